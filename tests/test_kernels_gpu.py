@@ -231,6 +231,25 @@ def test_gemm_tiled_rows_do_not_depend_on_the_batch():
         assert torch.equal(out, full[rows])
 
 
+@pytest.mark.parametrize("N,K,lda", [(7, 4, 4), (300, 132, 132), (300, 131, 131), (9001, 68, 72), (257, 1000, 1001)])
+def test_gemm_tiled_gives_the_same_bits_on_every_tile(N, K, lda):
+    """Row counts at the edges between tiles, narrow and wide N, rows that 16-byte copies can and cannot take: a row's
+    product is one chain of multiply-adds in ascending k whatever the tile, so all have the bits of the largest step."""
+    from infero_b200 import kernels as Kn
+    big = 1100
+    a, w = _rand((big, lda), torch.float32, 1)[:, :K], _rand((N, K), torch.float32, 2)
+    full = torch.empty((big, N), dtype=torch.float32, device=DEV)
+    Kn.gemm_tiled(a, w, None, full)
+    ref = a.double() @ w.double().T
+    # |error| <= K 2^-24 sum |a w| for a chain of K roundings; four times that of a random walk is far below it
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((full.double() - ref).abs() <= bound).all())
+    for M in (1, 2, 4, 5, 16, 17, 32, 33, 64, 129, 300):
+        out = torch.empty((M, N), dtype=torch.float32, device=DEV)
+        Kn.gemm_tiled(a[:M], w, None, out)
+        assert torch.equal(out, full[:M]), M
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
 def test_gemm_skinny(M):
     from infero_b200 import kernels as Kn
@@ -987,3 +1006,40 @@ def test_penalty_from_the_device_history_equals_the_host_statement():
                           torch.tensor([p.repetition_window for p in params], dtype=torch.int32, device=DEV), ring, ring_len)
     assert torch.equal(got, want)
     assert not torch.equal(got, z0)
+
+
+# ---- any-type attention ------------------------------------------------------------------------------
+@pytest.mark.parametrize("H,Hkv,D,V,window,page", [(4, 2, 64, 64, None, 16), (40, 1, 36, 36, 50, 32), (6, 2, 7, 10, 33, 16),
+                                                   (2, 2, 132, 256, None, 64), (3, 3, 16, 80, 1, 16)])
+def test_attention_generic_gives_the_same_bits_however_the_step_is_cut(H, Hkv, D, V, window, page):
+    """More tokens than a block per token is made for, blocks that several requests share, groups wider than a block, rows
+    that 16-byte copies can and cannot take: every token has the bits of the same token alone, and is right."""
+    from infero_b200 import kernels as Kn
+    lens, before = [270, 1, 1, 1, 5, 33], [0, 0, 31, 100, 60, 7]
+    blocks = max(-(-(n + p) // page) for n, p in zip(lens, before))
+    table = torch.randperm(len(lens) * blocks, generator=torch.Generator().manual_seed(3)).int().view(len(lens), blocks).to(DEV)
+    k, v = _rand((len(lens) * blocks, Hkv, page, D), torch.float32, 4), _rand((len(lens) * blocks, Hkv, page, V), torch.float32, 5)
+    q = _rand((sum(lens), H * D), torch.float32, 6)
+    entry = torch.tensor([e for e, n in enumerate(lens) for _ in range(n)], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p + i for n, p in zip(lens, before) for i in range(n)], dtype=torch.int32, device=DEV)
+
+    def run(rows):
+        out = torch.full((len(rows), H * V), float("nan"), dtype=torch.float32, device=DEV)
+        at = torch.tensor(rows, device=DEV)
+        Kn.attention_generic(q[at], out, k, v, table, entry[at].contiguous(), pos[at].contiguous(), H, Hkv, D, page, window, D ** -0.5,
+                             value_dim=V)
+        return out
+
+    full = run(list(range(sum(lens))))
+    for rows in ([0], [269], [270], [31, 32], list(range(250, 280)), list(range(100, 300))):
+        assert torch.equal(run(rows), full[rows])
+    for t in (0, 31, 32, 150, 269, 270, 272, 273, 277, sum(lens) - 1):
+        p, e = int(pos[t]), int(entry[t])
+        lo = max(0, p - window + 1) if window else 0
+        at = torch.arange(lo, p + 1)
+        pages, inside = table[e].cpu()[at // page].long(), at % page
+        for h in range(H):
+            kk, vv = (x.cpu().double()[pages, h // (H // Hkv), inside] for x in (k, v))
+            ref = torch.softmax(kk @ q[t, h * D:(h + 1) * D].cpu().double() * D ** -0.5, 0) @ vv
+            # scores and weights in 32-bit: D + keys roundings of 2^-24 in front of an exponential of scores of a few units
+            assert float((full[t, h * V:(h + 1) * V].cpu().double() - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max()))
