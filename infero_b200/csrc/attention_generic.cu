@@ -1,4 +1,4 @@
-// Attention over the paged cache for any batch of tokens: one warp per (token, query head).
+// Attention over the paged cache for any batch of tokens: a row per (token, query head).
 //
 // For token t of request entry e at position p, head h (kv head h / group):
 //   s_j = (q . K[j]) * scale - slope_h * (p - j)   for lo <= j <= p,  lo = window ? max(0, p - window + 1) : 0
@@ -15,95 +15,281 @@
 // depends only on its own position and window, never on how the step was cut or on what
 // else is in the batch.  It takes every head size up to 256 and every group size; it is the
 // whole of attention on the 32-bit path and the fallback of the bf16 path.
+//
+// A block has a few neighbouring tokens and the query heads of one kv head: their rows (token, head), R a warp, share the
+// chunks, which are fetched into shared memory ahead of the arithmetic (three with one row a warp, whose chain over the
+// chunks has nothing else to wait for; one with four, where more shared memory would cost blocks: 2.43 against 2.76 ms for
+// 2,048 tokens); a lane looks up its own key's page a chunk before that.  In the scores a lane has a key (rows of keys lie an
+// odd multiple of 16 bytes apart, so lanes read 16 bytes each without bank conflicts), in the sum over values it has every
+// 32nd column.  Tokens of different requests in one block take turns, so steps of few tokens get a block per token.
+// What bounds it: long prompts the multiply-adds and what feeds them from shared memory, single tokens the chain over the
+// chunks.  32-bit, before (a warp per row reading keys where they lie) and now: 301 tokens with 14 heads of 64 264 -> 68 us,
+// one token at 300 keys 125 -> 33, 64 tokens at 1,000 keys 516 -> 97, 2,048 tokens with 28 heads of 128 30.5 -> 2.4 ms.
 #include "common.cuh"
 #include <math_constants.h>
 
 namespace {
 
-constexpr int WARPS = 4;
+constexpr int WARPS = 8;
 constexpr int MAX_D = 256;
+constexpr int CHUNK = 32;
+constexpr int FEW_TOKENS = 256;         // up to here a block per token, one row a warp; beyond, 32 rows a block
 
-template <typename T, typename TO>
+struct GenericArgs {
+    const void* q;
+    void* out;
+    const void* k_cache;
+    const void* v_cache;
+    const int* block_table;
+    const int* tok_entry;
+    const int* positions;
+    const float* slopes;
+    const float* rel;
+    const float* sinks;
+    int q_stride, out_stride, max_blocks, n_tokens, n_heads, n_kv, head_dim, value_dim, page_size, window, sink, rel_len, cross;
+    int tokens_per_block, head_chunks;
+    float scale, softcap;
+};
+
+__host__ __device__ inline int key_stride(int head_dim) { return (((head_dim + 3) / 4) | 1) * 4; }
+__host__ __device__ inline int value_stride(int value_dim) { return (value_dim + 3) / 4 * 4; }
+
+inline size_t generic_smem(int head_dim, int value_dim, int rows, int stages) {
+    return ((size_t)stages * (CHUNK * (key_stride(head_dim) + value_stride(value_dim)) + 1) +
+            (size_t)rows * ((head_dim + 3) / 4 * 4 + CHUNK)) * sizeof(float);
+}
+
+// A chunk's rows of one array into shared memory, zeros where there is none; lane r brings the place of row r (or -1), a warp
+// fetches every n_warps-th row.  VEC: 32-bit rows of whole 16 bytes.
+template <typename T, bool VEC>
+__device__ __forceinline__ void fetch(float* dst, int stride, const T* cache, int width, long long row, int warp, int n_warps, int lane) {
+    const int per = VEC ? width / 4 : (width + 3) / 4 * 4;
+    for (int r = warp; r < CHUNK; r += n_warps) {
+        const long long at = __shfl_sync(0xffffffffu, row, r);
+        const T* src = cache + (at < 0 ? 0 : at * width);
+        for (int c = lane; c < per; c += 32) {
+            if constexpr (VEC) {
+                const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst + r * stride + c * 4);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(at < 0 ? cache : src + c * 4), "r"(at < 0 ? 0 : 16)
+                             : "memory");
+            } else {
+                dst[r * stride + c] = at >= 0 && c < width ? to_f32(src[c]) : 0.f;
+            }
+        }
+    }
+}
+
+template <typename T, typename TO, int R, int COLS, bool VEC, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_generic_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ out, int out_stride,
-                         const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                         const int* __restrict__ block_table, int max_blocks,
-                         const int* __restrict__ tok_entry, const int* __restrict__ positions,
-                         int n_tokens, int n_heads, int n_kv, int head_dim, int value_dim, int page_size,
-                         int window, float scale, int sink, const float* __restrict__ slopes,
-                         const float* __restrict__ rel, int rel_len, int cross, const float* __restrict__ sinks, float softcap) {
-    __shared__ float q_s[WARPS][MAX_D];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * WARPS + warp;
-    const int rows = cross ? n_heads * n_kv : n_heads;                // results per token
-    if (item >= (long long)n_tokens * rows) return;
-    const int t = (int)(item / rows), orow_i = (int)(item % rows), h = orow_i % n_heads;
-    const int group = n_heads / n_kv;
-    const int kvh = h / group, vh = cross ? orow_i / n_heads : kvh;
-    const int pos = positions[t];
-    const int* table = block_table + (size_t)tok_entry[t] * max_blocks;
-    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
-    const float slope = slopes ? slopes[h] : 0.f;
-    const float* rel_h = rel ? rel + (size_t)h * rel_len : nullptr;
+attention_generic_kernel(const GenericArgs a) {
+    extern __shared__ float4 smem4[];
+    float* smem = reinterpret_cast<float*>(smem4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    const int D = a.head_dim, V = a.value_dim, D4 = (D + 3) / 4 * 4, ks = key_stride(D), vs = value_stride(V);
+    float* k_s = smem;                                   // [STAGES][CHUNK][ks]
+    float* v_s = k_s + STAGES * CHUNK * ks;              // [STAGES][CHUNK][vs]
+    float* q_s = v_s + STAGES * CHUNK * vs + warp * R * D4;                                // this warp's [R][D4]
+    float* p_s = v_s + STAGES * CHUNK * vs + n_warps * R * D4 + warp * R * CHUNK;
+    unsigned int* here = reinterpret_cast<unsigned int*>(v_s + STAGES * CHUNK * vs + n_warps * R * (D4 + CHUNK));   // a bit per key
+    const int group = a.n_heads / a.n_kv;
+    const int kvh = a.cross ? blockIdx.y / a.n_kv : blockIdx.y, vh = a.cross ? blockIdx.y % a.n_kv : kvh;
+    const int t0 = blockIdx.x / a.head_chunks * a.tokens_per_block, g0 = blockIdx.x % a.head_chunks * (n_warps * R);
+    const int t1 = min(a.n_tokens, t0 + a.tokens_per_block);
+    const int heads = a.head_chunks > 1 ? min(group - g0, n_warps * R) : group;
 
-    const T* qrow = q + (size_t)t * q_stride + (size_t)h * head_dim;
-    for (int i = lane; i < head_dim; i += 32) q_s[warp][i] = to_f32(qrow[i]);
+    int tok[R], head[R], pos[R], lo[R];
+    float m[R], l[R], slope[R], acc[R][COLS];
+    const T* q = (const T*)a.q;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = warp * R + r;
+        tok[r] = t0 + i / heads;
+        head[r] = kvh * group + g0 + i % heads;
+        const bool mine = tok[r] < t1;
+        pos[r] = mine ? a.positions[tok[r]] : -1;
+        lo[r] = a.window > 0 ? max(0, pos[r] - a.window + 1) : 0;
+        if (!mine) tok[r] = -1;
+        slope[r] = mine && a.slopes ? a.slopes[head[r]] : 0.f;
+        // a sink is one more term of the softmax's sum, with score 0 and no value: the running maximum and sum start
+        // as if that key had been seen (with learned sinks its score is the head's own number)
+        m[r] = a.sink ? 0.f : mine && a.sinks ? a.sinks[head[r]] : -CUDART_INF_F;
+        l[r] = a.sink || a.sinks ? 1.f : 0.f;
+#pragma unroll
+        for (int i2 = 0; i2 < COLS; ++i2) acc[r][i2] = 0.f;
+        for (int d = lane; d < D4; d += 32)
+            q_s[r * D4 + d] = mine && d < D ? to_f32(q[(size_t)tok[r] * a.q_stride + (size_t)head[r] * D + d]) : 0.f;
+    }
     __syncwarp();
 
-    // a sink is one more term of the softmax's sum, with score 0 and no value: the running maximum and sum start
-    // as if that key had been seen
-    // (with learned sinks its score is the head's own number)
-    float m = sink ? 0.f : sinks ? sinks[h] : -CUDART_INF_F, l = sink || sinks ? 1.f : 0.f;
-    float acc[MAX_D / 32];
+    for (int first = t0; first < t1;) {                  // the tokens of one request after the other
+        const int entry = a.tok_entry[first];
+        const int* table = a.block_table + (size_t)entry * a.max_blocks;
+        int end = first, start = 0x7fffffff, last = -1;
+        for (; end < t1 && a.tok_entry[end] == entry; ++end) {
+            const int p = a.positions[end];
+            last = max(last, p);
+            start = min(start, a.window > 0 ? max(0, p - a.window + 1) : 0);
+        }
+        auto page_of = [&](int j0) {                     // of this lane's key in a chunk, -1 if there is none
+            const int j = j0 + lane;
+            return j <= last ? table[j / a.page_size] : -1;
+        };
+        auto load = [&](int j0, int page, int stage) {
+            if (j0 <= last) {
+                const long long row = page < 0 ? -1 : ((long long)page * a.n_kv + kvh) * a.page_size + (j0 + lane) % a.page_size;
+                const unsigned int there = __ballot_sync(0xffffffffu, page >= 0);
+                if (threadIdx.x == 0) here[stage] = there;
+                fetch<T, VEC>(k_s + stage * CHUNK * ks, ks, (const T*)a.k_cache, D, row, warp, n_warps, lane);
+                fetch<T, VEC>(v_s + stage * CHUNK * vs, vs, (const T*)a.v_cache, V, page < 0 ? -1 : row + (long long)(vh - kvh) * a.page_size, warp,
+                              n_warps, lane);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        start = start / CHUNK * CHUNK;
 #pragma unroll
-    for (int i = 0; i < MAX_D / 32; ++i) acc[i] = 0.f;
+        for (int s = 0; s < STAGES - 1; ++s) load(start + s * CHUNK, page_of(start + s * CHUNK), s);
+        int page = page_of(start + (STAGES - 1) * CHUNK), stage = 0;
+        for (int j0 = start; j0 <= last; j0 += CHUNK, stage = stage + 1 == STAGES ? 0 : stage + 1) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();                             // this chunk is here, and everyone is done with the one before,
+            load(j0 + (STAGES - 1) * CHUNK, page, stage == 0 ? STAGES - 1 : stage - 1);                 // whose place this takes
+            page = page_of(j0 + STAGES * CHUNK);
+            const int j = j0 + lane;
+            const bool there = here[stage] >> lane & 1;
+            bool sees[R];                                // does the row have keys in this chunk?
+            bool any = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                sees[r] = tok[r] >= first && tok[r] < end && j0 <= pos[r] && j0 + CHUNK > lo[r];
+                any |= sees[r];
+            }
+            if (any) {
+                float d[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) d[r] = 0.f;
+                const float* kr = k_s + (stage * CHUNK + lane) * ks;
+#pragma unroll 8
+                for (int i = 0; i < D4; i += 4) {        // (columns beyond D are zeros on both sides)
+                    const float4 k = *reinterpret_cast<const float4*>(kr + i);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float4 x = *reinterpret_cast<const float4*>(q_s + r * D4 + i);
+                        d[r] = fmaf(x.x, k.x, d[r]);
+                        d[r] = fmaf(x.y, k.y, d[r]);
+                        d[r] = fmaf(x.z, k.z, d[r]);
+                        d[r] = fmaf(x.w, k.w, d[r]);
+                    }
+                }
+                int from = CHUNK, to = -1;               // the values some row of this warp takes
+                bool whole = true;                       // every row takes all of them
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool valid = sees[r] && there && j >= lo[r] && j <= pos[r];
+                    float s = -CUDART_INF_F;
+                    if (valid) {
+                        s = d[r] * a.scale;
+                        if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+                        s -= slope[r] * (float)(pos[r] - j);
+                        if (a.rel) s += a.rel[(size_t)head[r] * a.rel_len + min(pos[r] - j, a.rel_len - 1)];
+                    }
+                    const float m_new = fmaxf(m[r], warp_max(s));
+                    if (m_new == -CUDART_INF_F) sees[r] = false;      // no readable key in this chunk
+                    float p = 0.f;
+                    if (sees[r]) {
+                        p = valid ? expf(s - m_new) : 0.f;
+                        const float corr = expf(m[r] - m_new);        // first chunk: exp(-inf) = 0
+                        l[r] = l[r] * corr + warp_sum(p);
+#pragma unroll
+                        for (int i = 0; i < COLS; ++i) acc[r][i] *= corr;
+                        m[r] = m_new;
+                        from = min(from, max(lo[r] - j0, 0)), to = max(to, min(pos[r] - j0, CHUNK - 1));
+                    }
+                    whole &= sees[r] && j0 >= lo[r] && j0 + CHUNK - 1 <= pos[r];
+                    p_s[r * CHUNK + lane] = p;
+                }
+                __syncwarp();
+                const float* vr = v_s + stage * CHUNK * vs + lane;
+                if (whole) {
+#pragma unroll
+                    for (int jj = 0; jj < CHUNK; jj += 4) {
+                        float4 p4[R];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) p4[r] = *reinterpret_cast<const float4*>(p_s + r * CHUNK + jj);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+#pragma unroll
+                            for (int i = 0; i < COLS; ++i) {
+                                const float v = i * 32 + lane < V ? vr[(jj + u) * vs + i * 32] : 0.f;
+#pragma unroll
+                                for (int r = 0; r < R; ++r) acc[r][i] = fmaf(reinterpret_cast<const float*>(&p4[r])[u], v, acc[r][i]);
+                            }
+                        }
+                    }
+                } else {
+                    for (int jj = from; jj <= to; ++jj) {
+                        float v[COLS];
+#pragma unroll
+                        for (int i = 0; i < COLS; ++i) v[i] = i * 32 + lane < V ? vr[jj * vs + i * 32] : 0.f;
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {    // (a key that a row must not see is not even multiplied by zero)
+                            if (!sees[r] || j0 + jj < lo[r] || j0 + jj > pos[r]) continue;
+                            const float p = p_s[r * CHUNK + jj];
+#pragma unroll
+                            for (int i = 0; i < COLS; ++i) acc[r][i] = fmaf(p, v[i], acc[r][i]);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                 // the next request's chunks take the same places
+        first = end;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (tok[r] < 0) continue;
+        const int at = a.cross ? vh * a.n_heads + head[r] : head[r];
+        TO* orow = (TO*)a.out + (size_t)tok[r] * a.out_stride + (size_t)at * V;
+        const float inv = 1.0f / l[r];
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) {
+            const int dd = i * 32 + lane;
+            if (dd < V) orow[dd] = from_f32<TO>(acc[r][i] * inv);
+        }
+    }
+}
 
-    for (int j0 = (lo / 32) * 32; j0 <= pos; j0 += 32) {
-        const int j = j0 + lane;
-        const bool valid = j >= lo && j <= pos;
-        long long row = -1;
-        float s = -CUDART_INF_F;
-        if (valid) {
-            const int page = table[j / page_size];
-            if (page >= 0) {
-                row = ((long long)page * n_kv + kvh) * page_size + (j % page_size);
-                const T* kr = k_cache + row * head_dim;
-                float d = 0.f;
-                for (int i = 0; i < head_dim; ++i) d = fmaf(q_s[warp][i], to_f32(kr[i]), d);
-                s = d * scale;
-                if (softcap > 0.f) s = softcap * tanhf(s / softcap);
-                s -= slope * (float)(pos - j);
-                if (rel_h) s += rel_h[min(pos - j, rel_len - 1)];
-                row += (long long)(vh - kvh) * page_size;      // from here on: the row of the values
-            }
-        }
-        const float m_new = fmaxf(m, warp_max(s));
-        if (m_new == -CUDART_INF_F) continue;         // no readable key in this chunk
-        const float p = (row >= 0) ? expf(s - m_new) : 0.f;
-        const float corr = expf(m - m_new);          // first chunk: exp(-inf) = 0
-        l = l * corr + warp_sum(p);
-#pragma unroll
-        for (int i = 0; i < MAX_D / 32; ++i) acc[i] *= corr;
-        for (int jj = 0; jj < 32; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const long long rj = __shfl_sync(0xffffffffu, row, jj);
-            if (rj < 0) continue;                      // uniform across the warp
-            const T* vr = v_cache + rj * value_dim;
-#pragma unroll
-            for (int i = 0; i < MAX_D / 32; ++i) {
-                const int dd = i * 32 + lane;
-                if (dd < value_dim) acc[i] = fmaf(pj, to_f32(vr[dd]), acc[i]);
-            }
-        }
-        m = m_new;
+template <typename T, typename TO, int R, int COLS, bool VEC, int STAGES>
+int launch(const GenericArgs& a, int warps, cudaStream_t stream) {
+    auto* kernel = attention_generic_kernel<T, TO, R, COLS, VEC, STAGES>;
+    const size_t smem = generic_smem(a.head_dim, a.value_dim, warps * R, STAGES);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        INFERO_REQUIRE(e == cudaSuccess, "attention: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
-    TO* orow = out + (size_t)t * out_stride + (size_t)orow_i * value_dim;
-    const float inv = 1.0f / l;
-#pragma unroll
-    for (int i = 0; i < MAX_D / 32; ++i) {
-        const int dd = i * 32 + lane;
-        if (dd < value_dim) orow[dd] = from_f32<TO>(acc[i] * inv);
-    }
+    const long long tiles = (long long)((a.n_tokens + a.tokens_per_block - 1) / a.tokens_per_block) * a.head_chunks;
+    kernel<<<dim3((unsigned)tiles, a.cross ? a.n_kv * a.n_kv : a.n_kv), warps * 32, smem, stream>>>(a);
+    return infero_check_launch("attention_generic");
+}
+
+template <typename T, typename TO, bool VEC>
+int launch_rows(GenericArgs& a, cudaStream_t stream) {
+    const int group = a.n_heads / a.n_kv;
+    const bool few = a.n_tokens <= FEW_TOKENS;
+    const int warps = few && group < WARPS ? group : WARPS, rows = few ? warps : WARPS * 4;
+    a.tokens_per_block = few || group > rows ? 1 : rows / group;
+    a.head_chunks = (group + rows - 1) / rows;
+#define COLUMNS(R)                                                                                         \
+    do {                                                                                                   \
+        constexpr int S = R == 1 ? 4 : 2;                                                                  \
+        if (a.head_dim > 128 || a.value_dim > 128) return launch<T, TO, R, 8, VEC, 2>(a, warps, stream);   \
+        if (a.value_dim > 64) return launch<T, TO, R, 4, VEC, S>(a, warps, stream);                        \
+        return launch<T, TO, R, 2, VEC, S>(a, warps, stream);                                              \
+    } while (0)
+    if (few) COLUMNS(1);
+    COLUMNS(4);
+#undef COLUMNS
 }
 
 }  // namespace
@@ -127,17 +313,16 @@ int infero_attention_generic_rel(const void* q, int q_stride, void* out, int out
     INFERO_REQUIRE(value_dim >= 1 && value_dim <= MAX_D, "attention: value width %d outside 1..%d", value_dim, MAX_D);
     INFERO_REQUIRE(n_kv > 0 && n_heads % n_kv == 0, "attention: %d heads not a multiple of %d kv heads", n_heads, n_kv);
     INFERO_REQUIRE(!rel || rel_len >= 1, "attention: an empty table of distances");
-    const long long items = (long long)n_tokens * n_heads * (cross ? n_kv : 1);
-    const unsigned blocks = (unsigned)((items + WARPS - 1) / WARPS);
-#define LAUNCH(T, TO)                                                                                                   \
-    attention_generic_kernel<T, TO><<<blocks, WARPS * 32, 0, stream>>>((const T*)q, q_stride, (TO*)out, out_stride,     \
-        (const T*)k_cache, (const T*)v_cache, block_table, max_blocks, tok_entry, positions, n_tokens, n_heads, n_kv,   \
-        head_dim, value_dim, page_size, window, scale, sink, slopes, rel, rel_len, cross, sinks, softcap)
-    if (dtype == INFERO_F32) LAUNCH(float, float);
-    else if (cross) LAUNCH(bf16, float);
-    else LAUNCH(bf16, bf16);
-#undef LAUNCH
-    return infero_check_launch("attention_generic");
+    INFERO_REQUIRE((long long)n_kv * (cross ? n_kv : 1) <= 65535, "attention: %d kv heads are too many", n_kv);
+    GenericArgs a;
+    a.q = q, a.out = out, a.k_cache = k_cache, a.v_cache = v_cache, a.block_table = block_table, a.tok_entry = tok_entry;
+    a.positions = positions, a.slopes = slopes, a.rel = rel, a.sinks = sinks, a.q_stride = q_stride, a.out_stride = out_stride;
+    a.max_blocks = max_blocks, a.n_tokens = n_tokens, a.n_heads = n_heads, a.n_kv = n_kv, a.head_dim = head_dim;
+    a.value_dim = value_dim, a.page_size = page_size, a.window = window, a.sink = sink, a.rel_len = rel_len, a.cross = cross;
+    a.scale = scale, a.softcap = softcap;
+    const bool vec = head_dim % 4 == 0 && value_dim % 4 == 0 && (uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0;
+    if (dtype == INFERO_F32) return vec ? launch_rows<float, float, true>(a, stream) : launch_rows<float, float, false>(a, stream);
+    return cross ? launch_rows<bf16, float, false>(a, stream) : launch_rows<bf16, bf16, false>(a, stream);
 }
 
 int infero_attention_generic_bias(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
