@@ -442,86 +442,114 @@ __device__ __forceinline__ void add_bias16(float* v, const void* __restrict__ bi
         if (at + e < end) v[e] += load_any(bias, bias_dtype, at + e);
 }
 
-// One epilogue warp's share of a finished accumulator: its 32 rows (TMEM lanes at lane_addr, result
-// row ra for this thread) by BN columns starting at feature b0, written as the epilogue EPI says.
+// Writes a warp's 32 rows of SEGS * 16 bytes (lane r holds row r) so that neighbouring lanes write neighbouring bytes: through
+// 32 * SEGS * 16 bytes of shared memory, 16-byte pieces placed so that neither side has bank conflicts.  dst: row 0's place.
+template <int SEGS>
+__device__ __forceinline__ void store_rows(uint8_t* stage, const uint4* mine, uint8_t* dst, size_t pitch, int rows, int lane) {
+    auto at = [&](int r, int s) { return reinterpret_cast<uint4*>(stage + r * (SEGS * 16) + ((s ^ ((r * SEGS >> 3) & (SEGS - 1))) << 4)); };
+    __syncwarp();                                        // the rows written before have been read
+#pragma unroll
+    for (int s = 0; s < SEGS; ++s) *at(lane, s) = mine[s];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < SEGS; ++i) {
+        const int r = i * (32 / SEGS) + lane / SEGS, s = lane % SEGS;
+        const uint4 v = *at(r, s);
+        if (r < rows) *reinterpret_cast<uint4*>(dst + r * pitch + s * 16) = v;
+    }
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
+
+// The epilogue of the many-token kernels.  Sixteen warps drain an accumulator, four per quarter of its rows: they take turns
+// at blocks of 32 columns.  What a warp does with a block is one chain of instructions (the TMEM load, divisions with a
+// branch each, packing), so a warp alone is bound by their latency, not by any unit: with one warp a quarter, each lane
+// writing its own row, a tile's SwiGLU took 15 us beside 5 us of MMAs at K = 896.  1032 x 9728 x 896 with SwiGLU: 44 us with
+// four warps, 36 with eight, 25 with sixteen; 1738 x 12800 x 2048 to 32-bit: 107 us before, 82 now (cuBLAS to bf16: 78).
+constexpr int DRAIN_WARPS = 16, MANY_THREADS = 64 + 32 * DRAIN_WARPS, DRAIN_STAGE = 32 * 64;
+
+// One warp's share of a finished accumulator: its 32 rows (TMEM lanes at lane_addr, result rows from row0) in every second
+// block of 32 of the BN columns that start at feature b0, written as the epilogue EPI says.
 template <int EPI, typename OutT>
-__device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int ra, int b0, int BN, int RA, int RB,
-                                                  OutT* __restrict__ out, const void* __restrict__ bias,
+__device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, int row0, int lane, uint8_t* stage, int b0, int BN,
+                                                  int RA, int RB, OutT* __restrict__ out, const void* __restrict__ bias,
                                                   int bias_dtype, long long ldc, int act_kind = GLU_SILU,
                                                   float act_limit = 0.f, float act_alpha = 1.f) {
+    constexpr bool GLU = EPI == EPI_ROW_SWIGLU;
     const int col_end = min(RB, b0 + BN);                // what this tile owns
+    const int ra = row0 + lane, rows = RA - row0;
+    const size_t pitch = (size_t)ldc * sizeof(OutT);
+    const bool wide = ((reinterpret_cast<uintptr_t>(out) | pitch) & 15u) == 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-        if (b0 + c0 >= col_end) break;               // uniform over the block
-        uint32_t u[32];
-        tmem_ld32_nowait(lane_addr + (uint32_t)c0, u);
-        tmem_wait_ld();
-        if (ra < RA) {
+    for (int c0 = turn * 32; c0 < BN; c0 += 8 * DRAIN_WARPS) {
+        const int rb = b0 + c0;
+        if (rb >= col_end) break;                        // uniform over the warp
+        float v[32];
+        {
+            uint32_t u[32];
+            tmem_ld32_nowait(lane_addr + (uint32_t)c0, u);
+            tmem_wait_ld();
 #pragma unroll
-            for (int hseg = 0; hseg < 2; ++hseg) {
-                const int rb = b0 + c0 + hseg * 16;
-                if (rb >= col_end) break;
-                float v[16];
+            for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(u[e]);
+        }
+        if (bias) {
+            add_bias16(v, bias, bias_dtype, rb, col_end);
+            add_bias16(v + 16, bias, bias_dtype, rb + 16, col_end);
+        }
+        if (GLU) {
 #pragma unroll
-                for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(u[hseg * 16 + e]);
-                if (EPI == EPI_ROW_SWIGLU) {
-                    OutT* dst = out + (size_t)ra * ldc + (rb >> 1);
-                    float h[8];
-                    if (bias) add_bias16(v, bias, bias_dtype, rb, RB);
+            for (int e = 0; e < 16; ++e) v[e] = glu_act(v[2 * e], v[2 * e + 1], act_kind, act_limit, act_alpha);
+        } else if (act_kind == ACT_RELU2) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        h[e] = act_kind == GLU_SILU ? silu_mul(v[2 * e], v[2 * e + 1])
-                                                    : glu_act(v[2 * e], v[2 * e + 1], act_kind, act_limit, act_alpha);
-                    if (rb + 16 <= RB && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0 && sizeof(OutT) == 2) {
-                        uint32_t pk[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            __nv_bfloat162 t2 = __floats2bfloat162_rn(h[2 * e], h[2 * e + 1]);
-                            pk[e] = *reinterpret_cast<uint32_t*>(&t2);
-                        }
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (rb + 2 * e + 1 < RB) dst[e] = from_f32<OutT>(h[e]);
-                    }
-                } else {
-                    OutT* dst = out + (size_t)ra * ldc + rb;
-                    if (bias) add_bias16(v, bias, bias_dtype, rb, RB);
-                    if (act_kind == ACT_RELU2) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const float r = fmaxf(v[e], 0.f);
-                            v[e] = r * r;
-                        }
-                    }
-                    if (rb + 16 <= RB) {
-                        store16<OutT>(dst, v, (reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            if (rb + e < RB) dst[e] = from_f32<OutT>(v[e]);
-                    }
-                }
+            for (int e = 0; e < 32; ++e) {
+                const float r = fmaxf(v[e], 0.f);
+                v[e] = r * r;
             }
         }
-        __syncwarp();
+        const int cols = min(32, col_end - rb), first = GLU ? rb >> 1 : rb, n = GLU ? cols >> 1 : cols;
+        uint8_t* dst = reinterpret_cast<uint8_t*>(out + first) + (size_t)row0 * pitch;
+        // (first is a multiple of 16 elements, or of 8 of bf16 behind a gated unit: pieces of 16 bytes start aligned)
+        if (wide && sizeof(OutT) == 4 && (cols == 32 || cols == 16)) {
+            const uint4* f = reinterpret_cast<const uint4*>(v);
+            store_rows<4>(stage, f, dst, pitch, rows, lane);
+            if (cols == 32) store_rows<4>(stage, f + 4, dst + 64, pitch, rows, lane);
+        } else if (wide && sizeof(OutT) == 2 && (cols == 32 || (cols == 16 && !GLU))) {
+            uint4 pk[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                pk[e] = make_uint4(pack_bf16(v[8 * e], v[8 * e + 1]), pack_bf16(v[8 * e + 2], v[8 * e + 3]),
+                                   pack_bf16(v[8 * e + 4], v[8 * e + 5]), pack_bf16(v[8 * e + 6], v[8 * e + 7]));
+            if (!GLU && cols == 32) store_rows<4>(stage, pk, dst, pitch, rows, lane);
+            else store_rows<2>(stage, pk, dst, pitch, rows, lane);
+        } else if (ra < RA) {
+            OutT* row = out + (size_t)ra * ldc + first;
+#pragma unroll
+            for (int e = 0; e < (GLU ? 16 : 32); ++e)
+                if (e < n) row[e] = from_f32<OutT>(v[e]);
+        }
     }
+    __syncwarp();
 }
 
 // ---- many tokens: persistent, two accumulators --------------------------------------------------
 // One CTA per SM walks over 128 x 256 tiles of the result (tile t = blockIdx.x, + gridDim.x, ...).
 // Tile numbers run over the token blocks of one block of 256 features first, so that at any
 // moment the CTAs together work on a few feature blocks and all token blocks, which L2 holds.  The shared-memory ring runs on across tiles; tensor memory
-// holds two accumulators of 256 columns, so the four epilogue warps drain tile i while the MMAs
+// holds two accumulators of 256 columns, so the epilogue warps drain tile i while the MMAs
 // of tile i + 1 run.  A = activations [RA, K], B = weights [RB, K].
 // The tile width bn (a multiple of 16 up to 256) is chosen per problem so that the tiles fill
 // whole rounds of the CTAs (3584 features in tiles of 256 are 224 tiles with 16 token blocks:
 // two rounds on 148 SMs, the second half empty; in tiles of 208 they are 288 and nearly fill two).
-constexpr int PERS_MAX_BN = 256, PERS_STAGES = 4;
+// Narrower tiles have smaller stages and more of them in the same RING_BYTES.
+constexpr int PERS_MAX_BN = 256, MAX_STAGES = 8, RING_BYTES = 192 * 1024;
+constexpr int MANY_BARRIERS = RING_BYTES, MANY_DRAIN = MANY_BARRIERS + 256, MANY_SMEM = MANY_DRAIN + DRAIN_WARPS * DRAIN_STAGE + 1024;
+static_assert((2 * MAX_STAGES + 4) * 8 + 12 <= 256 && MANY_SMEM <= 227 * 1024, "ring, barriers, staging rows, slack for the alignment");
 
 template <int EPI, typename OutT>
-__global__ void __launch_bounds__(GEMM_THREADS)
+__global__ void __launch_bounds__(MANY_THREADS)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           OutT* __restrict__ out, const void* __restrict__ bias, int bias_dtype,
                           int RA_bound, int RB, int K, long long ldc, int BN, int* __restrict__ err_flag,
@@ -537,16 +565,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         const int used = tile_group[(RA_bound + TILE_A - 1) / TILE_A];
         RA = used < RA_bound ? used : RA_bound;
     }
-    constexpr int STAGES = PERS_STAGES;
-    using Plan = SmemPlan<PERS_MAX_BN, STAGES>;             // where the barriers sit; stages are packed by BN
-    const int stage_bytes = A_STAGE_BYTES + BN * TILE_K * 2;
+    const int stage_bytes = A_STAGE_BYTES + BN * TILE_K * 2, STAGES = min(MAX_STAGES, RING_BYTES / stage_bytes);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Plan::BAR_OFFSET);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + MANY_BARRIERS);
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_full = empty_bar + STAGES;             // 2
-    uint64_t* acc_empty = acc_full + 2;                  // 2 (four arrivals: one per epilogue warp)
+    uint64_t* acc_empty = acc_full + 2;                  // 2 (an arrival per epilogue warp)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* never_flag = abort_flag + 1;
@@ -568,7 +594,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], 4);
+            mbar_init(&acc_empty[a], DRAIN_WARPS);
         }
         *abort_flag = 0;
         *never_flag = 0;
@@ -603,7 +629,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             };
             // weights of the first stages before the kernel in front has finished, activations after
             const int pre = (int)(total < STAGES ? total : STAGES);
-            int pa0[STAGES], pkx[STAGES];
+            int pa0[MAX_STAGES], pkx[MAX_STAGES];
             if (tile_group) pdl_wait();
             auto b_row = [&]() {                       // first row of this tile's weights in map_b
                 if (!tile_group) return b0;
@@ -677,17 +703,18 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         }
     } else {
         // ---- epilogue: tile i while the MMAs of tile i + 1 run ------------------------------------
-        const int q = warp & 3;
+        const int q = warp & 3, turn = (warp - 2) >> 2;
+        uint8_t* stage = smem + MANY_DRAIN + (warp - 2) * DRAIN_STAGE;
         bool ok = true;
         for (int i = 0; i < my_tiles; ++i) {
             const int a = i & 1;
             const int t = (int)blockIdx.x + i * (int)gridDim.x;
             const int a0 = (t % tiles_a) * TILE_A, b0 = (t / tiles_a) * BN;
-            const int ra = a0 + q * 32 + lane;
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[a], (uint32_t)(i >> 1) & 1u, abort_flag))) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t lane_addr = tmem_base + (uint32_t)a * PERS_MAX_BN + ((uint32_t)(q * 32) << 16);
-            drain_accumulator<EPI, OutT>(lane_addr, ra, b0, BN, RA, RB, out, bias, bias_dtype, ldc, act_kind, act_limit, act_alpha);
+            drain_accumulator<EPI, OutT>(lane_addr, turn, a0 + q * 32, lane, stage, b0, BN, RA, RB, out, bias, bias_dtype, ldc,
+                                         act_kind, act_limit, act_alpha);
             // this warp has read its quarter of the accumulator: hand it back
             tc_fence_before_sync();
             __syncwarp();
@@ -712,28 +739,26 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // rows of the activations and its own half of the tile's weight rows, so every byte enters the
 // pair's shared memory once and an SM's shared memory takes 128 + BN/2 rows per step of K instead
 // of 128 + BN; the CTA of rank 0 issues the MMAs for both, each CTA's tensor memory holds the
-// accumulator rows of its own tokens, and each CTA's four epilogue warps write those rows.  All
+// accumulator rows of its own tokens, and each CTA's epilogue warps write those rows.  All
 // loads of a stage report to rank 0's barrier; the commits that free a stage or publish an
 // accumulator reach both CTAs; the epilogue warps of both hand an accumulator back on rank 0's
 // barrier.  The pairs walk the tiles as the single CTAs above do.
-constexpr int PAIR_STAGES = 6, PAIR_ROWS = 2 * TILE_A;
+constexpr int PAIR_ROWS = 2 * TILE_A;
 
 template <int EPI, typename OutT>
-__global__ void __launch_bounds__(GEMM_THREADS)
+__global__ void __launch_bounds__(MANY_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     OutT* __restrict__ out, const void* __restrict__ bias, int bias_dtype,
                     int RA, int RB, int K, long long ldc, int BN, int* __restrict__ err_flag) {
-    constexpr int STAGES = PAIR_STAGES;
-    constexpr int BAR_OFFSET = STAGES * (A_STAGE_BYTES + (PERS_MAX_BN / 2) * TILE_K * 2);
     const int half_bn = BN >> 1;
-    const int stage_bytes = A_STAGE_BYTES + half_bn * TILE_K * 2;
+    const int stage_bytes = A_STAGE_BYTES + half_bn * TILE_K * 2, STAGES = min(MAX_STAGES, RING_BYTES / stage_bytes);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + BAR_OFFSET);    // used in rank 0
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + MANY_BARRIERS);    // used in rank 0
     uint64_t* empty_bar = full_bar + STAGES;                                 // in both
     uint64_t* acc_full = empty_bar + STAGES;                                 // 2, in both
-    uint64_t* acc_empty = acc_full + 2;                                      // 2, used in rank 0 (eight arrivals)
+    uint64_t* acc_empty = acc_full + 2;                                      // 2, used in rank 0 (an arrival per epilogue warp of both)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* never_flag = abort_flag + 1;
@@ -757,7 +782,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], 8);
+            mbar_init(&acc_empty[a], 2 * DRAIN_WARPS);
         }
         *abort_flag = 0;
         *never_flag = 0;
@@ -790,11 +815,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     b0 = (tile / tiles_a) * BN + (int)rank * half_bn;
                 }
             };
-            uint32_t lead_full[STAGES];
+            uint32_t lead_full[MAX_STAGES];
             for (int s = 0; s < STAGES; ++s) lead_full[s] = cluster_addr_of(&full_bar[s], 0);
             // weights of the first stages before the kernel in front has finished, activations after
             const int pre = (int)(total < STAGES ? total : STAGES);
-            int pa0[STAGES], pkx[STAGES];
+            int pa0[MAX_STAGES], pkx[MAX_STAGES];
             for (int it = 0; it < pre; ++it) {
                 if (rank == 0) mbar_expect_tx(&full_bar[it], 2 * stage_bytes);
                 tma_load_2d_pair(smem + it * stage_bytes + A_STAGE_BYTES, &map_b, kt * TILE_K, b0, lead_full[it]);
@@ -862,7 +887,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else {
         // ---- epilogue: each CTA its own 128 rows ------------------------------------------------------
-        const int q = warp & 3;
+        const int q = warp & 3, turn = (warp - 2) >> 2;
+        uint8_t* stage = smem + MANY_DRAIN + (warp - 2) * DRAIN_STAGE;
         bool ok = true;
         uint32_t lead_empty[2];
         for (int a = 0; a < 2; ++a) lead_empty[a] = cluster_addr_of(&acc_empty[a], 0);
@@ -870,11 +896,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int a = i & 1;
             const int t = pair + i * n_pairs;
             const int a0 = (t % tiles_a) * PAIR_ROWS + (int)rank * TILE_A, b0 = (t / tiles_a) * BN;
-            const int ra = a0 + q * 32 + lane;
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[a], (uint32_t)(i >> 1) & 1u, abort_flag))) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t lane_addr = tmem_base + (uint32_t)a * PERS_MAX_BN + ((uint32_t)(q * 32) << 16);
-            drain_accumulator<EPI, OutT>(lane_addr, ra, b0, BN, RA, RB, out, bias, bias_dtype, ldc);
+            drain_accumulator<EPI, OutT>(lane_addr, turn, a0 + q * 32, lane, stage, b0, BN, RA, RB, out, bias, bias_dtype, ldc);
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(lead_empty[a]);
@@ -1015,13 +1040,12 @@ int launch_persistent(const void* x, const void* w, void* out, const void* bias,
                       int RA, int RB, int K, int ldx, long long ldc, int sm_count, int* err, cudaStream_t stream,
                       const int* tile_group = nullptr, int n_groups = 1, int act_kind = GLU_SILU, float act_limit = 0.f,
                       float act_alpha = 1.f) {
-    using Plan = SmemPlan<PERS_MAX_BN, PERS_STAGES>;
     auto kern = gemm_tc_persistent_kernel<EPI, OutT>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);
         if (e != cudaSuccess) {
-            infero_set_error("gemm_tc: cannot get %d bytes of shared memory: %s", Plan::TOTAL, cudaGetErrorString(e));
+            infero_set_error("gemm_tc: cannot get %d bytes of shared memory: %s", MANY_SMEM, cudaGetErrorString(e));
             return 1;
         }
         configured = true;
@@ -1033,7 +1057,7 @@ int launch_persistent(const void* x, const void* w, void* out, const void* bias,
     if (get_map(w, RB * n_groups, K, K, bn, &mb)) return 1;
     const int n_tiles = ((RA + TILE_A - 1) / TILE_A) * ((RB + bn - 1) / bn);
     const int ctas = n_tiles < sms ? n_tiles : sms;
-    launch_pdl(kern, dim3(ctas), dim3(GEMM_THREADS), Plan::TOTAL, stream, ma, mb, (OutT*)out, bias, bias_dtype, RA, RB,
+    launch_pdl(kern, dim3(ctas), dim3(MANY_THREADS), MANY_SMEM, stream, ma, mb, (OutT*)out, bias, bias_dtype, RA, RB,
                K, ldc, bn, err, tile_group, act_kind, act_limit, act_alpha);
     return infero_check_launch("gemm_tc_persistent");
 }
@@ -1061,16 +1085,15 @@ int pick_pair_tile_n(int M, int N, int pairs, int multiple) {
 template <int EPI, typename OutT>
 int launch_pair(const void* x, const void* w, void* out, const void* bias, int bias_dtype,
                 int RA, int RB, int K, int ldx, long long ldc, int* err, cudaStream_t stream) {
-    constexpr int SMEM = PAIR_STAGES * (A_STAGE_BYTES + (PERS_MAX_BN / 2) * TILE_K * 2) + 256 + 1024;
     auto kern = gemm_tc_pair_kernel<EPI, OutT>;
     static int max_pairs = 0;
     if (max_pairs == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);
         if (e == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(2);
-            cfg.blockDim = dim3(GEMM_THREADS);
-            cfg.dynamicSmemBytes = SMEM;
+            cfg.blockDim = dim3(MANY_THREADS);
+            cfg.dynamicSmemBytes = MANY_SMEM;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = 2;
@@ -1095,8 +1118,8 @@ int launch_pair(const void* x, const void* w, void* out, const void* bias, int b
     const int pairs = n_tiles < max_pairs ? n_tiles : max_pairs;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.blockDim = dim3(MANY_THREADS);
+    cfg.dynamicSmemBytes = MANY_SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

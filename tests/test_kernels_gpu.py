@@ -151,6 +151,34 @@ def test_gemm_tensor_core_with_swiglu_epilogue(M, N, K, cta_pairs):
     assert tc_gemm.error_flag() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 224, 72), (300, 1008, 136), (300, 1000, 136), (641, 40, 64), (1032, 2064, 136)])
+@pytest.mark.parametrize("kind", ["f32", "bf16", "swiglu", "relu2"])
+def test_many_token_rows_stored_wide_and_narrow(M, N, K, kind, cta_pairs):
+    """A result whose rows start on 16 bytes (stored through shared memory) and one whose rows do not (element by element): the
+    same bits, nothing outside the rows and columns; blocks of 32 columns that end in 16, in 8 and past the matrix."""
+    from infero_b200.kernels import tc_gemm
+    a, w = _rand((M, K), torch.bfloat16, 1), _rand((N, K), torch.bfloat16, 2, 0.1)
+    n = N // 2 if kind == "swiglu" else N
+    dt = torch.float32 if kind == "f32" else torch.bfloat16
+    got = []
+    for pad, at in ((8, 0), (3, 1)):
+        big = torch.full((M + 2, n + pad), 7.0, dtype=dt, device=DEV)
+        out = big[1:M + 1, at:at + n]
+        if kind in ("swiglu", "relu2"):
+            assert tc_gemm.gemm_act(a, w, out, kind)
+        else:
+            tc_gemm.gemm(a, w, None, out)
+        got.append(out.clone())
+        out.fill_(7.0)
+        assert bool((big == 7.0).all()), "wrote outside its rows or columns"
+    assert tc_gemm.error_flag() == 0
+    assert torch.equal(*got)
+    y = a.double() @ w.double().T
+    ref = y if kind in ("f32", "bf16") else y.clamp(min=0) ** 2 if kind == "relu2" else y[:, 0::2] * torch.sigmoid(y[:, 0::2]) * y[:, 1::2]
+    tol = 1e-5 if kind == "f32" else 6e-3                   # (bf16 rounds to 2^-9)
+    assert float((got[0].double() - ref).abs().max() / ref.abs().max()) <= tol
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 3584, 18944), (1, 3584, 3584), (64, 896, 4864), (200, 1000, 2048), (5, 128, 320),
                                    (16, 256, 616), (33, 130, 1024)])
 @pytest.mark.parametrize("with_bias", [False, True])
