@@ -28,6 +28,7 @@
 // that runs out raises the error flag and the CTA leaves in order (TMEM freed).
 #include "attn_common.cuh"
 #include "tc_common.cuh"
+#include "tc_softmax.cuh"
 #include <math_constants.h>
 
 namespace {
@@ -58,28 +59,6 @@ struct PfPlan {
     static_assert(2 * KTILE + D <= 256, "S, S and O must fit 256 TMEM columns");
     static_assert(TOTAL > 116 * 1024, "one CTA per SM: it takes all of the SM's tensor memory");
 };
-
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-// max of three in one instruction, and a multiply-add on a pair of 32-bit floats in one instruction
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ void fma2(float& x0, float& x1, float a0, float a1, float b, float c) {
-    asm("{\n .reg .b64 ra, rb, rc, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %4};\n mov.b64 rc, {%5, %5};\n"
-        " fma.rn.f32x2 rd, ra, rb, rc;\n mov.b64 {%0, %1}, rd;\n}"
-        : "=f"(x0), "=f"(x1)
-        : "f"(a0), "f"(a1), "f"(b), "f"(c));
-}
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
 
 template <int D>
 __global__ void __launch_bounds__(PFT_THREADS)

@@ -29,29 +29,30 @@ constexpr int PREP_THREADS = 128;
 
 // The angle is position times frequency in 64-bit, brought into [-pi, pi] there and only then rounded: a 32-bit product
 // is off by its own size times 2^-24, which at position 1,000 is already 6e-5 of a turn's worth of radians.
-__device__ __forceinline__ void turn(float a, float b, double ang, float amp, float& ra, float& rb) {
+__device__ __forceinline__ float2 turn(double ang, float amp) {
     const double two_pi = 6.283185307179586476925286766559;
     ang -= two_pi * rint(ang / two_pi);
     float s, c;
     sincosf((float)ang, &s, &c);
-    s *= amp, c *= amp;
-    ra = a * c - b * s;
-    rb = b * c + a * s;
+    return make_float2(c * amp, s * amp);
 }
 
-// element i of a rotated part of width R: what it becomes at position p
-__device__ __forceinline__ float rotated(const float* __restrict__ part, int i, int rot, int pairing, int pos,
-                                         const double* __restrict__ freq, float amp) {
+// element i of a rotated part: what it becomes with the token's cosines and sines
+__device__ __forceinline__ float rotated(const float* __restrict__ part, int i, int rot, int pairing, const float2* cs) {
     if (i >= rot) return part[i];
     int ia, ib;
     if (pairing) ia = i & ~1, ib = ia + 1;
     else ia = i < rot / 2 ? i : i - rot / 2, ib = ia + rot / 2;
-    const int pair = pairing ? i >> 1 : ia;
-    float ra, rb;
-    turn(part[ia], part[ib], (double)pos * freq[pair], amp, ra, rb);
-    return i == ia ? ra : rb;
+    const float2 t = cs[pairing ? i >> 1 : ia];
+    const float a = part[ia], b = part[ib];
+    return i == ia ? a * t.x - b * t.y : b * t.x + a * t.y;
 }
 
+// The rotated part's width where the kernel that reads it takes blocks of 64 columns (zeros behind the R-th).
+constexpr int ROT_BLOCK = 64;
+
+// A token's cosines and sines are the same for all its heads and for the key part, and their 64-bit angles are most of the
+// work, so a block makes them once, into shared memory (2,048 tokens of 16 heads of 128 + 64: 30 us an element at a time, 24 from the table).
 template <typename T>
 __global__ void __launch_bounds__(PREP_THREADS)
 latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ q_src, int q_stride,
@@ -59,24 +60,26 @@ latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const flo
                       const float* __restrict__ norm_w, float eps, const double* __restrict__ freq, int rot, int pairing,
                       float amp, const int* __restrict__ positions, const int* __restrict__ tok_entry,
                       const int* __restrict__ block_table, int max_blocks, int page_size, T* __restrict__ cache,
-                      int write_cache, T* __restrict__ q_plain, float* __restrict__ q_rot, long long head_rows,
-                      int H, int D, int R, int C, int heads_per_block) {
+                      int write_cache, T* __restrict__ q_plain, float* __restrict__ q_rot, T* __restrict__ q_rot_block,
+                      long long head_rows, int H, int D, int R, int C, int heads_per_block) {
+    extern __shared__ float2 cs[];                       // [rot / 2]: amp * (cos, sin)
     __shared__ float red[32];
     const int t = blockIdx.x;
     const float* row = proj + (size_t)t * proj_stride;
     const int pos = positions[t];
+    if (blockIdx.y == 0 && !write_cache) return;
+    for (int i = threadIdx.x; i < rot / 2; i += blockDim.x) cs[i] = turn((double)pos * freq[i], amp);
+    __syncthreads();
     if (blockIdx.y == 0) {
         // the latent row
-        if (!write_cache) return;
         const float* kv = row + kv_off;
         float sq = 0.f;
         for (int i = threadIdx.x; i < C; i += blockDim.x) sq = fmaf(kv[i], kv[i], sq);
         const float rstd = 1.0f / sqrtf(block_sum(sq, red) / (float)C + eps);
-        const int p = positions[t];
-        const int page = block_table[(size_t)tok_entry[t] * max_blocks + p / page_size];
-        T* dst = cache + ((size_t)page * page_size + (p % page_size)) * (C + R);
+        const int page = block_table[(size_t)tok_entry[t] * max_blocks + pos / page_size];
+        T* dst = cache + ((size_t)page * page_size + (pos % page_size)) * (C + R);
         for (int i = threadIdx.x; i < C; i += blockDim.x) dst[i] = from_f32<T>(kv[i] * rstd * norm_w[i]);
-        for (int i = threadIdx.x; i < R; i += blockDim.x) dst[C + i] = from_f32<T>(rotated(kv + C, i, rot, pairing, pos, freq, amp));
+        for (int i = threadIdx.x; i < R; i += blockDim.x) dst[C + i] = from_f32<T>(rotated(kv + C, i, rot, pairing, cs));
         return;
     }
     // the queries of heads [n0, n1)
@@ -86,9 +89,17 @@ latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const flo
         const int n = i / D, c = i % D;
         q_plain[((size_t)n * head_rows + t) * D + c] = from_f32<T>(q[(size_t)n * (D + R) + c]);
     }
+    if (q_rot_block) {
+        for (int i = n0 * ROT_BLOCK + threadIdx.x; i < n1 * ROT_BLOCK; i += blockDim.x) {
+            const int n = i / ROT_BLOCK, c = i % ROT_BLOCK;
+            const float v = c < R ? rotated(q + (size_t)n * (D + R) + D, c, rot, pairing, cs) : 0.f;
+            q_rot_block[((size_t)n * head_rows + t) * ROT_BLOCK + c] = from_f32<T>(v);
+        }
+        return;
+    }
     for (int i = n0 * R + threadIdx.x; i < n1 * R; i += blockDim.x) {
         const int n = i / R, c = i % R;
-        q_rot[((size_t)n * head_rows + t) * R + c] = rotated(q + (size_t)n * (D + R) + D, c, rot, pairing, pos, freq, amp);
+        q_rot[((size_t)n * head_rows + t) * R + c] = rotated(q + (size_t)n * (D + R) + D, c, rot, pairing, cs);
     }
 }
 
@@ -183,14 +194,16 @@ extern "C" {
 // proj float32 [T, proj_stride]: the C + R columns of the latent row from kv_off.  q_src float32 [T, q_stride]: the
 // query's H * (D + R) columns from q_off (the same array as proj where one product gives both, another where the queries
 // come from a product of their own).  cache [pages, 1, page, C + R]; q_plain [H, head_rows, D] of the cache's type; q_rot
-// float32 [H, head_rows, R] (R may be 0: no rotated part).
+// float32 [H, head_rows, R] (R may be 0: no rotated part), or, where q_rot_block is given, [H, head_rows, 64] of the cache's
+// type there instead, zeros behind the R-th column.
 int infero_latent_prepare_from(const float* proj, int proj_stride, const float* q_src, int q_stride, int q_off, int kv_off,
                                const float* norm_w, float eps,
                           const double* freq, int rot, int pairing, float amp, const int* positions, const int* tok_entry,
                           const int* block_table, int max_blocks, int page_size, void* cache, int dtype, int write_cache,
-                          void* q_plain, float* q_rot, long long head_rows, int n_tokens, int H, int D, int R, int C,
-                          cudaStream_t stream) {
+                          void* q_plain, float* q_rot, void* q_rot_block, long long head_rows, int n_tokens, int H, int D,
+                          int R, int C, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
+    INFERO_REQUIRE(rot <= 8192 && (!q_rot_block || R <= ROT_BLOCK), "latent attention: a rotated part of %d (%d turned)", R, rot);
     INFERO_REQUIRE(rot >= 0 && rot <= R && rot % 2 == 0, "latent attention: %d rotated coordinates of %d", rot, R);
     INFERO_REQUIRE(head_rows >= n_tokens, "latent attention: %lld rows per head for %d tokens", head_rows, n_tokens);
     // one block for a token's latent row, and one per group of heads (all heads in one block where tokens alone fill
@@ -198,13 +211,13 @@ int infero_latent_prepare_from(const float* proj, int proj_stride, const float* 
     const int heads_per_block = n_tokens >= 512 ? H : max(1, H / 8);
     const dim3 grid(n_tokens, 1 + (H + heads_per_block - 1) / heads_per_block);
     if (dtype == INFERO_F32)
-        latent_prepare_kernel<float><<<grid, PREP_THREADS, 0, stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
+        latent_prepare_kernel<float><<<grid, PREP_THREADS, rot / 2 * sizeof(float2), stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
             rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (float*)cache, write_cache,
-            (float*)q_plain, q_rot, head_rows, H, D, R, C, heads_per_block);
+            (float*)q_plain, q_rot, (float*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
     else
-        latent_prepare_kernel<bf16><<<grid, PREP_THREADS, 0, stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
+        latent_prepare_kernel<bf16><<<grid, PREP_THREADS, rot / 2 * sizeof(float2), stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
             rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (bf16*)cache, write_cache,
-            (bf16*)q_plain, q_rot, head_rows, H, D, R, C, heads_per_block);
+            (bf16*)q_plain, q_rot, (bf16*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
     return infero_check_launch("latent_prepare");
 }
 
@@ -215,7 +228,7 @@ int infero_latent_prepare(const float* proj, int proj_stride, int q_off, int kv_
                           cudaStream_t stream) {
     return infero_latent_prepare_from(proj, proj_stride, proj, proj_stride, q_off, kv_off, norm_w, eps, freq, rot, pairing, amp,
                                       positions, tok_entry, block_table, max_blocks, page_size, cache, dtype, write_cache,
-                                      q_plain, q_rot, head_rows, n_tokens, H, D, R, C, stream);
+                                      q_plain, q_rot, nullptr, head_rows, n_tokens, H, D, R, C, stream);
 }
 
 // q_lat float32 [H, head_rows, C] (the plain query parts carried through Wuk^T), q_rot float32 [H, head_rows, R];

@@ -19,18 +19,20 @@ TILE = 128
 def prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, eps: float, freq: Optional[torch.Tensor],
             pairing: str, amp: float, positions, tok_entry, block_table, cache: torch.Tensor, page_size: int,
             q_plain: torch.Tensor, q_rot: torch.Tensor, n_tokens: int, H: int, D: int, R: int, C: int,
-            write_cache: bool = True, q_src: Optional[torch.Tensor] = None) -> None:
+            write_cache: bool = True, q_src: Optional[torch.Tensor] = None, rot_block: bool = False) -> None:
     """From the input product (float32 [T, >= ...]): the normed latent and the rotated key part go to the token's
     page, the plain query parts to q_plain [H, rows, D], the rotated ones to q_rot float32 [H, rows, R].  ``freq``: the
     rotary table in float64 (the angle is formed in 64-bit).  ``q_src`` (float32 [T, >= q_off + H (D + R)]): the
-    queries come from this array instead of ``proj`` (a product of their own)."""
+    queries come from this array instead of ``proj`` (a product of their own).  ``rot_block``: q_rot is [H, rows, 64] of the
+    cache's type instead, zeros behind the R-th column."""
     if q_src is None:
         q_src = proj
     assert q_src.dtype == torch.float32 and q_src.stride(1) == 1 and q_src.shape[0] == proj.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and cache.is_contiguous() and cache.shape[-1] == C + R
-    assert cache.shape[1] == 1 and q_plain.dtype == cache.dtype and q_plain.is_contiguous() and q_rot.dtype == torch.float32
+    assert cache.shape[1] == 1 and q_plain.dtype == cache.dtype and q_plain.is_contiguous()
+    assert q_rot.dtype == (cache.dtype if rot_block else torch.float32)
     rows = q_plain.shape[1]
-    assert tuple(q_plain.shape) == (H, rows, D) and tuple(q_rot.shape) == (H, rows, R) and q_rot.is_contiguous()
+    assert tuple(q_plain.shape) == (H, rows, D) and tuple(q_rot.shape) == (H, rows, 64 if rot_block else R) and q_rot.is_contiguous()
     assert freq is None or (freq.dtype == torch.float64 and freq.is_contiguous())
     rot = 0 if freq is None else 2 * freq.numel()
     _check(lib().infero_latent_prepare_from(
@@ -38,7 +40,7 @@ def prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, e
         _ptr(freq), c_int(rot), c_int(1 if pairing == "adjacent" else 0), c_float(amp),
         _ptr(_i32(positions, "positions")), _ptr(_i32(tok_entry, "tok_entry")), _ptr(_i32(block_table, "block_table")),
         c_int(block_table.shape[1]), c_int(page_size), _ptr(cache), c_int(_dt(cache)), c_int(1 if write_cache else 0),
-        _ptr(q_plain), _ptr(q_rot), c_longlong(rows), c_int(n_tokens), c_int(H), c_int(D), c_int(R), c_int(C), _stream()))
+        _ptr(q_plain), _ptr(None if rot_block else q_rot), _ptr(q_rot if rot_block else None), c_longlong(rows), c_int(n_tokens), c_int(H), c_int(D), c_int(R), c_int(C), _stream()))
 
 
 def grouped_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
@@ -83,18 +85,19 @@ def per_head_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n_rows
 
 def attention(ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor, kv, table, n_tokens: int, H: int, C: int,
               R: int, scale: float, window: Optional[int] = None, sinks: Optional[torch.Tensor] = None,
-              sinks_log2: Optional[torch.Tensor] = None) -> None:
+              sinks_log2: Optional[torch.Tensor] = None, singles_only: bool = False) -> None:
     """Causal softmax attention of every token over its request's cached latent rows: q_lat float32 [H, rows, C],
     q_rot float32 [H, rows, R], out [H, rows, C] of the cache's type.  ``window``: a token sees that many keys up to its own.
     ``sinks`` float32 [H] (``sinks_log2``: times log2 e, made here when absent): one more term exp(sinks[h]) in head h's sum,
-    without a value."""
+    without a value.  ``singles_only``: only the requests in front that bring one token each (``n_tokens`` of them)."""
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == H)
     cache = kv.k
     rows = q_lat.shape[1]
     assert q_lat.dtype == torch.float32 and q_rot.dtype == torch.float32 and q_lat.is_contiguous() and q_rot.is_contiguous()
     assert out.dtype == cache.dtype and out.is_contiguous() and tuple(out.shape) == (H, rows, C) and cache.is_contiguous()
     from . import latent_mma
-    if latent_mma.run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window, sinks, sinks_log2):
+    if latent_mma.run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window, sinks, sinks_log2,
+                      singles_only):
         return
     _check(lib().infero_latent_attention_generic(
         _ptr(q_lat), _ptr(q_rot), c_longlong(rows), _ptr(out), _ptr(cache), c_int(_dt(cache)),

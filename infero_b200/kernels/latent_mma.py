@@ -31,7 +31,8 @@ def plan_splits(n_tok: int, head_blocks: int, visible: int, sms: int):
     return chunk, -(-visible // chunk)
 
 
-def run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window=None, sinks=None, sinks_log2=None) -> bool:
+def run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window=None, sinks=None, sinks_log2=None,
+        singles_only=False) -> bool:
     cache = kv.k
     if not ENABLED or cache.dtype != torch.bfloat16 or not supported(C, R) or getattr(ctx, "h_q_len", None) is None:
         return False
@@ -61,7 +62,7 @@ def run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window=None
                                                  *common, c_int(0), c_int(n_dec), c_int(n_dec), c_int(1), c_int(H), c_int(C),
                                                  c_int(R), c_int(kv.page_size), c_float(scale), c_int(chunk), c_int(splits),
                                                  *more, _stream()))
-    if n_dec < E:
+    if n_dec < E and not singles_only:
         TQ = 64 // HC
         launches["tiled"] += 1
         tiles = sum(-(-int(n) // TQ) for n in ctx.h_q_len[n_dec:])

@@ -25,6 +25,9 @@ class LatentAttention(Mixer):
         ->  per-head product with Wuk^T  ->  attention over latent rows  ->  per-head product with Wuv
         ->  finish (gate, heads side by side)  ->  output product.
 
+    In bf16 steps, prompt portions of many tokens have the keys and values they see written out per head instead
+    (``kernels/latent_prefill.py``); the requests in front that bring one token each keep to the latent rows.
+
     Rotation: the position part's table (with any stretching of the frequencies and its amplitude) and pairing; R may
     be 0 (no rotated part: positions enter through the causal mask alone).
 
@@ -77,6 +80,7 @@ class LatentAttention(Mixer):
         return out
 
     def bind(self, tensors: Dict[str, torch.Tensor]) -> None:
+        from ..kernels.latent_prefill import supported as written_out
         H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
         rows = [tensors[self._n("q_down" if self.Q else "q")], tensors[self._n("down")]]
         if self.spec.out_gate:
@@ -97,37 +101,68 @@ class LatentAttention(Mixer):
             self.sinks_log2 = (self.sinks * 1.4426950408889634).contiguous()
         # [H, C, D]: head n's rows of Wuk, transposed, so that the product with the plain query parts is a @ w^T
         self.up_k_t = tensors[self._n("up_k")].view(H, D, C).transpose(1, 2).contiguous()
-        self.up_v = tensors[self._n("up_v")].view(H, V, C).contiguous()
+        # where prompts are written out: both up-projections as one matrix
+        up_k, up_v = tensors[self._n("up_k")], tensors[self._n("up_v")]
+        self.kv_up = torch.cat([up_k, up_v]) if up_k.dtype == up_v.dtype == torch.bfloat16 and written_out(D, V, R, C) else None
+        self.up_v = (up_v if self.kv_up is None else self.kv_up[H * D:]).view(H, V, C).contiguous()
         self.out = Linear(tensors[self._n("o")], None, self._n("o"))
 
     def forward(self, ctx, h, slot):
         from ..kernels import latent_attention as A
+        from ..kernels import latent_prefill as P
         H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
         T, dev = h.shape[0], h.device
         proj = self.qkv.forward(h, out_dtype=torch.float32)             # [T, H (D + R) + C + R (+ H)], never rounded
         kv = ctx.kv_cache(slot.cache)
         table = ctx.block_table(kv.group)
-        # whole 128-row tiles per head where the grouped tensor-core product runs
-        rows = -(-T // A.TILE) * A.TILE if (h.dtype == torch.bfloat16 and D % 8 == 0 and C % 8 == 0) else T
-        q_plain = torch.empty((H, rows, D), dtype=h.dtype, device=dev)
-        q_rot = torch.empty((H, rows, R), dtype=torch.float32, device=dev)
-        freq = self.rope.inv_freq64(dev) if self.rope is not None else None
         q_src = None
         if self.Q:
             from ..kernels import layer_ops as L
             cq = torch.empty((T, self.Q), dtype=h.dtype, device=dev)
             L.gated_group_norm(proj[:, :self.Q], None, self.q_norm, self.spec.norm_eps, 1, cq)
             q_src = self.q_up.forward(cq, out_dtype=torch.float32)
-        A.prepare(proj, self.q_off, self.kv_off, self.latent_norm, self.spec.norm_eps, freq, self.pairing, self.amp,
-                  ctx.positions, ctx.tok_entry, table, kv.k, kv.page_size, q_plain, q_rot, T, H, D, R, C,
-                  write_cache=slot.write_cache, q_src=q_src)
-        q_lat = torch.empty((H, rows, C), dtype=torch.float32, device=dev)
-        A.per_head_product(q_plain, self.up_k_t, q_lat, T)
-        o_lat = torch.empty((H, rows, C), dtype=h.dtype, device=dev)
-        A.attention(ctx, q_lat, q_rot, o_lat, kv, table, T, H, C, R, self.spec.scale, self.spec.window, self.sinks, self.sinks_log2)
-        val = torch.empty((H, rows, V), dtype=torch.float32, device=dev)
-        A.per_head_product(o_lat, self.up_v, val, T)
         attn = torch.empty((T, H * V), dtype=h.dtype, device=dev)
-        gate = proj[:, self.gate_off:self.gate_off + H] if self.spec.out_gate else None
-        A.finish(val, gate, attn, T, H, V)
+        plan = P.plan(ctx, h.dtype, H, D, V, R, C, self.spec.window) if self.kv_up is not None else None
+        singles = T if plan is None else plan.first_entry
+        if singles:
+            self._through_latents(ctx, A, proj, q_src, kv, table, slot, attn, singles, plan is not None)
+        if plan is not None:
+            self._written_out(ctx, A, P, plan, proj, q_src, kv, table, slot, attn)
         return self.out.forward(attn, defer=True, residual=True)
+
+    def _prepare(self, ctx, A, proj, q_src, kv, table, slot, t0, t1, rows, rot_block):
+        """Norm, rotation and cache append of tokens t0 .. t1 - 1; their queries, head-major."""
+        H, D, R, C = self.H, self.D, self.R, self.C
+        q_plain = torch.empty((H, rows, D), dtype=kv.k.dtype, device=proj.device)
+        q_rot = torch.empty((H, rows, 64 if rot_block else R), dtype=kv.k.dtype if rot_block else torch.float32, device=proj.device)
+        freq = self.rope.inv_freq64(proj.device) if self.rope is not None else None
+        A.prepare(proj[t0:t1], self.q_off, self.kv_off, self.latent_norm, self.spec.norm_eps, freq, self.pairing, self.amp,
+                  ctx.positions[t0:t1], ctx.tok_entry[t0:t1], table, kv.k, kv.page_size, q_plain, q_rot, t1 - t0, H, D, R, C,
+                  write_cache=slot.write_cache, q_src=None if q_src is None else q_src[t0:t1], rot_block=rot_block)
+        return q_plain, q_rot
+
+    def _gate(self, proj, t0, t1):
+        return proj[t0:t1, self.gate_off:self.gate_off + self.H] if self.spec.out_gate else None
+
+    def _through_latents(self, ctx, A, proj, q_src, kv, table, slot, attn, n, singles_only):
+        """Tokens 0 .. n - 1 against the latent rows where they lie, the up-projections carried to the query side."""
+        H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
+        dt, dev = kv.k.dtype, proj.device
+        # whole 128-row tiles per head where the grouped tensor-core product runs
+        rows = -(-n // A.TILE) * A.TILE if (dt == torch.bfloat16 and D % 8 == 0 and C % 8 == 0) else n
+        q_plain, q_rot = self._prepare(ctx, A, proj, q_src, kv, table, slot, 0, n, rows, False)
+        q_lat = torch.empty((H, rows, C), dtype=torch.float32, device=dev)
+        A.per_head_product(q_plain, self.up_k_t, q_lat, n)
+        o_lat = torch.empty((H, rows, C), dtype=dt, device=dev)
+        A.attention(ctx, q_lat, q_rot, o_lat, kv, table, n, H, C, R, self.spec.scale, self.spec.window, self.sinks, self.sinks_log2,
+                    singles_only=singles_only)
+        val = torch.empty((H, rows, V), dtype=torch.float32, device=dev)
+        A.per_head_product(o_lat, self.up_v, val, n)
+        A.finish(val, self._gate(proj, 0, n), attn[:n], n, H, V)
+
+    def _written_out(self, ctx, A, P, plan, proj, q_src, kv, table, slot, attn):
+        """The portions behind the single tokens, their visible keys and values written out per head."""
+        t0, T = plan.first_entry, proj.shape[0]
+        q_plain, q_rot = self._prepare(ctx, A, proj, q_src, kv, table, slot, t0, T, T - t0, True)
+        P.run(ctx, plan, q_plain, q_rot, kv, table, self.kv_up, self._gate(proj, t0, T), attn[t0:], self.H, self.D, self.R, self.C,
+              self.spec.scale, self.spec.window, self.sinks_log2)

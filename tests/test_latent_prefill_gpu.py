@@ -1,0 +1,87 @@
+"""Latent attention of prompt portions with their keys and values written out (``csrc/latent_prefill_tc.cu``), against the plain
+implementation in 64 bits; the rule that picks it."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from infero_b200.kernels import latent_prefill as P
+
+TOL = 2.5e-2          # bf16 operands, as the kernels that attend over the latent rows are held to
+
+
+def _ctx(lens, pos0):
+    return types.SimpleNamespace(h_q_len=np.array(lens, dtype=np.int32), h_pos0=np.array(pos0, dtype=np.int32), n_entries=len(lens))
+
+
+@pytest.mark.parametrize("lens,pos0,window,want", [
+    ([16], [0], None, (0, 1, 1)), ([15], [0], None, None), ([1, 1, 300], [9, 900, 0], None, (2, 5, 3)),
+    ([1, 1], [9, 900], None, None),                                  # single tokens only
+    ([100], [400], None, None), ([100], [300], None, (0, 7, 1)),     # behind too long a prefix; within the bound
+    ([100], [4000], 128, (0, 5, 1)),                                 # the window leaves 100 + 127 keys, from 3,840 on
+    ([40, 1, 129], [0, 5, 64], None, (0, 1 + 1 + 4, 1 + 1 + 2)),     # a single token behind a portion goes with it
+])
+def test_the_rule(lens, pos0, window, want):
+    got = P.plan(_ctx(lens, pos0), torch.bfloat16, 4, 64, 64, 32, 128, window)
+    assert got == (None if want is None else P.Plan(*want))
+    assert P.plan(_ctx(lens, pos0), torch.float32, 4, 64, 64, 32, 128, window) is None
+    for D, V, R, C in ((32, 32, 16, 128), (64, 128, 32, 256), (64, 64, 72, 256), (64, 64, 12, 256), (128, 128, 64, 128), (64, 64, 32, 132)):
+        assert P.plan(_ctx(lens, pos0), torch.bfloat16, 4, D, V, R, C, window) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,D,R,C,page", [(16, 128, 64, 512, 16), (3, 64, 32, 256, 64), (2, 128, 8, 256, 16), (5, 64, 64, 136, 16)])
+def test_portions_at_the_edges_of_tiles(H, D, R, C, page, monkeypatch):
+    """Portions of 1 to 300 tokens beside each other and behind prefixes, single tokens in front of them; shuffled pages."""
+    from test_gositar_gpu import _Latent, _rel
+    from infero_b200.kernels import tc_gemm
+    g = torch.Generator().manual_seed(D + R)
+    cuts = {"s": [2, 1, 1], "a": [64, 65, 128], "b": [129, 300], "c": [127, 1, 63], "d": [193, 192]}
+    hs = None
+    for least in (1, 1 << 30):                          # written out, and through the latent rows
+        # (queries and keys grow with the input's width here: the scale leaves scores a spread of a few units)
+        a = _Latent("bfloat16", H, D, R, D, C, gated=H != 3, pairing="half" if H == 3 else "adjacent", seed=H, page=page, pages=120,
+                    scale=3.0 / (max(64, H * D) * C * (D + R)) ** 0.5)
+        if hs is None:
+            hs = {r: torch.randn(sum(n), a.d, generator=g).to(torch.bfloat16).float() for r, n in cuts.items()}
+            want = {r: a.plain(h) for r, h in hs.items()}
+        monkeypatch.setattr(P, "MIN_TOKENS", least)
+        got, before = {r: [] for r in cuts}, P.launches["steps"]
+        for i in range(3):
+            entries = [(r, hs[r][sum(n[:i]):sum(n[:i]) + n[i]]) for r, n in cuts.items() if i < len(n)]
+            for r, rows in a.step(entries).items():
+                got[r].append(rows)
+        assert P.launches["steps"] == before + (3 if least == 1 else 0) and tc_gemm.error_flag() == 0
+        for r in hs:
+            assert _rel(torch.cat(got[r]), want[r]) < TOL, (r, least)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window", [1, 64, 100, 129])
+def test_windows_and_sinks(window, monkeypatch):
+    import plain_dukolorn as PD
+    from test_dukolorn_gpu import EPS, _inputs, _latent_alone, _rel, latent
+    from infero_b200.kernels import tc_gemm
+    monkeypatch.setattr(P, "MIN_TOKENS", 1)
+    H, D, R, C, scale = 3, 64, 32, 128, 0.08
+    a = _latent_alone(H, D, R, D, C, scale, window, "bfloat16", pages=128)
+    m, w, d = latent(H, D, R, D, C, scale, 500.0, window), a.weights(), a.spec.hidden
+    hs = {r: _inputs(n, d, "bfloat16", n, 0.4) for r, n in (("a", 500), ("b", 90))}
+    before = P.launches["steps"]
+    first = a.step([("a", hs["a"][:201]), ("b", hs["b"])])
+    then = a.step([("a", hs["a"][201:])])
+    assert P.launches["steps"] == before + 2 and tc_gemm.error_flag() == 0
+    for r, rows in (("a", torch.cat([first["a"], then["a"]])), ("b", first["b"])):
+        assert _rel(rows[:, :H * D], PD.latent_inner(hs[r].double(), w, "mix", m, EPS)) < TOL, r
+
+
+@pytest.mark.gpu
+def test_one_requests_infinities_stay_its_own():
+    """Tiles of a request end in rows of zeros, not in the next request's keys."""
+    from test_gositar_gpu import _Latent, _rel
+    a = _Latent("bfloat16", 2, 64, 32, 64, 128, seed=3, scale=0.06, pages=40)
+    g = torch.Generator().manual_seed(1)
+    h = torch.randn(70, a.d, generator=g).to(torch.bfloat16).float()
+    got = a.step([("x", h), ("y", torch.full((64, a.d), float("inf")))])
+    assert _rel(got["x"], a.plain(h)) < TOL and not bool(torch.isfinite(got["y"]).all())
