@@ -19,6 +19,8 @@ __device__ __forceinline__ float summed(const TI* __restrict__ v, int splits, lo
 template <typename TI, typename TO>
 __global__ void glu_act_kernel(const TI* __restrict__ v, int splits, long long split_stride, TO* __restrict__ out, int ff,
                                size_t total, int kind, float limit, float alpha, const float* __restrict__ bias) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / ff, j = i % ff;
@@ -30,6 +32,8 @@ __global__ void glu_act_kernel(const TI* __restrict__ v, int splits, long long s
 
 template <typename TI, typename TO>
 __global__ void relu2_kernel(const TI* __restrict__ v, int splits, long long split_stride, TO* __restrict__ out, size_t total) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const float x = fmaxf(summed(v, splits, split_stride, i), 0.f);
@@ -42,10 +46,10 @@ extern "C" {
 
 #define DISPATCH(KERNEL, ...)                                                                                      \
     do {                                                                                                           \
-        if (in_dtype == INFERO_F32 && out_dtype == INFERO_F32) KERNEL<float, float><<<blocks, 256, 0, stream>>>((const float*)v, splits, split_stride, (float*)out, __VA_ARGS__); \
-        else if (in_dtype == INFERO_F32) KERNEL<float, bf16><<<blocks, 256, 0, stream>>>((const float*)v, splits, split_stride, (bf16*)out, __VA_ARGS__); \
-        else if (out_dtype == INFERO_F32) KERNEL<bf16, float><<<blocks, 256, 0, stream>>>((const bf16*)v, splits, split_stride, (float*)out, __VA_ARGS__); \
-        else KERNEL<bf16, bf16><<<blocks, 256, 0, stream>>>((const bf16*)v, splits, split_stride, (bf16*)out, __VA_ARGS__); \
+        if (in_dtype == INFERO_F32 && out_dtype == INFERO_F32) launch_pdl(KERNEL<float, float>, dim3(blocks), dim3(256), 0, stream, (const float*)v, splits, split_stride, (float*)out, __VA_ARGS__); \
+        else if (in_dtype == INFERO_F32) launch_pdl(KERNEL<float, bf16>, dim3(blocks), dim3(256), 0, stream, (const float*)v, splits, split_stride, (bf16*)out, __VA_ARGS__); \
+        else if (out_dtype == INFERO_F32) launch_pdl(KERNEL<bf16, float>, dim3(blocks), dim3(256), 0, stream, (const bf16*)v, splits, split_stride, (float*)out, __VA_ARGS__); \
+        else launch_pdl(KERNEL<bf16, bf16>, dim3(blocks), dim3(256), 0, stream, (const bf16*)v, splits, split_stride, (bf16*)out, __VA_ARGS__); \
     } while (0)
 
 // v: splits arrays of [n_tokens, 2 * ff], split_stride elements apart; out [n_tokens, ff]; bias (may be null) float32 [2 * ff],

@@ -62,6 +62,8 @@ latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const flo
                       const int* __restrict__ block_table, int max_blocks, int page_size, T* __restrict__ cache,
                       int write_cache, T* __restrict__ q_plain, float* __restrict__ q_rot, T* __restrict__ q_rot_block,
                       long long head_rows, int H, int D, int R, int C, int heads_per_block) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ float2 cs[];                       // [rot / 2]: amp * (cos, sin)
     __shared__ float red[32];
     const int t = blockIdx.x;
@@ -178,6 +180,8 @@ latent_attention_generic_kernel(const float* __restrict__ q_lat, const float* __
 template <typename T>
 __global__ void latent_finish_kernel(const float* __restrict__ val, long long head_rows, const float* __restrict__ gate,
                                      int gate_stride, T* __restrict__ out, int out_stride, int H, int V) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t t = blockIdx.x;
     for (int i = threadIdx.x; i < H * V; i += blockDim.x) {
         const int n = i / V, v = i % V;
@@ -211,11 +215,11 @@ int infero_latent_prepare_from(const float* proj, int proj_stride, const float* 
     const int heads_per_block = n_tokens >= 512 ? H : max(1, H / 8);
     const dim3 grid(n_tokens, 1 + (H + heads_per_block - 1) / heads_per_block);
     if (dtype == INFERO_F32)
-        latent_prepare_kernel<float><<<grid, PREP_THREADS, rot / 2 * sizeof(float2), stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
+        launch_pdl(latent_prepare_kernel<float>, grid, dim3(PREP_THREADS), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
             rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (float*)cache, write_cache,
             (float*)q_plain, q_rot, (float*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
     else
-        latent_prepare_kernel<bf16><<<grid, PREP_THREADS, rot / 2 * sizeof(float2), stream>>>(proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
+        launch_pdl(latent_prepare_kernel<bf16>, grid, dim3(PREP_THREADS), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
             rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (bf16*)cache, write_cache,
             (bf16*)q_plain, q_rot, (bf16*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
     return infero_check_launch("latent_prepare");
@@ -258,9 +262,9 @@ int infero_latent_finish(const float* val, long long head_rows, const float* gat
                          int out_stride, int dtype, int n_tokens, int H, int V, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
     if (dtype == INFERO_F32)
-        latent_finish_kernel<float><<<n_tokens, 256, 0, stream>>>(val, head_rows, gate, gate_stride, (float*)out, out_stride, H, V);
+        launch_pdl(latent_finish_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, val, head_rows, gate, gate_stride, (float*)out, out_stride, H, V);
     else
-        latent_finish_kernel<bf16><<<n_tokens, 256, 0, stream>>>(val, head_rows, gate, gate_stride, (bf16*)out, out_stride, H, V);
+        launch_pdl(latent_finish_kernel<bf16>, dim3(n_tokens), dim3(256), 0, stream, val, head_rows, gate, gate_stride, (bf16*)out, out_stride, H, V);
     return infero_check_launch("latent_finish");
 }
 

@@ -38,6 +38,8 @@ latent_mma_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_r
                   const int* __restrict__ entry_q_start, const int* __restrict__ entry_q_len,
                   const int* __restrict__ entry_pos0, int entry_first, int n_entries, int TQ, int HC, int H, int R,
                   int page_size, float scale_log2, int chunk, int splits, int window, const float* __restrict__ sinks) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int ROWS = ROWG * 16, NT = ROWG * NW * 32, CW = C / NW, NO = CW / 8;
     constexpr int KW = KT / NW, NTW = KW / 8;              // keys, and n-tiles of 8 keys, whose scores a warp forms
     const int W = C + R, LD = W + 8;                       // padded row of a tile, in elements
@@ -314,6 +316,8 @@ constexpr int MAX_SPLITS = 64;
 __global__ void __launch_bounds__(256)
 latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, bf16* __restrict__ out,
                     long long head_rows, int H, int C, int splits, const float* __restrict__ sinks) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float w_s[MAX_SPLITS];
     __shared__ float inv_s;
     const int t = blockIdx.x / H, n = blockIdx.x % H;
@@ -366,7 +370,7 @@ int launch_one(const float* q_lat, const float* q_rot, long long head_rows, bf16
         }
     }
     const dim3 grid(n_tiles, (H + HC - 1) / HC, splits);
-    kern<<<grid, ROWG * NW * 32, sh, stream>>>(q_lat, q_rot, head_rows, out, part_o, part_ml, cache, block_table, max_blocks,
+    launch_pdl(kern, grid, dim3(ROWG * NW * 32), sh, stream, q_lat, q_rot, head_rows, out, part_o, part_ml, cache, block_table, max_blocks,
                                           entry_q_start, entry_q_len, entry_pos0, entry_first, n_entries, TQ, HC, H, R,
                                           page_size, scale * 1.4426950408889634f, chunk, splits, window, sinks);
     return 0;
@@ -424,7 +428,7 @@ int infero_latent_attention_mma(const float* q_lat, const float* q_rot, long lon
     if (rc) return rc;
     if (splits > 1) {
         // the tokens of the leading single-token entries are the first rows of the step
-        latent_merge_kernel<<<n_tiles * H, C >= 256 ? 256 : 128, 0, stream>>>(part_o, part_ml, (bf16*)out, head_rows, H, C, splits, sinks);
+        launch_pdl(latent_merge_kernel, dim3(n_tiles * H), dim3(C >= 256 ? 256 : 128), 0, stream, part_o, part_ml, (bf16*)out, head_rows, H, C, splits, sinks);
     }
     return infero_check_launch("latent_attention_mma");
 }

@@ -54,6 +54,8 @@ __device__ __forceinline__ float warp_dot(const bf16* __restrict__ a, const bf16
 __global__ void __launch_bounds__(RWARPS * 32)
 moe_select_kernel(const float* __restrict__ logits, int stride, int gate_col, int* __restrict__ top_idx,
                   float* __restrict__ top_w, float* __restrict__ gate_out, int n_tokens, int E, int top) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float z[RWARPS][MAX_E];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RWARPS + warp;
@@ -96,6 +98,8 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int gate_col, in
 __global__ void __launch_bounds__(RWARPS * 32)
 moe_select_scored_kernel(const float* __restrict__ logits, int stride, int splits, long long split_stride,
                          int* __restrict__ top_idx, float* __restrict__ top_w, int n_tokens, int E, int top, int renorm) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float sc[RWARPS][MAX_E];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RWARPS + warp;
@@ -144,6 +148,8 @@ __global__ void __launch_bounds__(RWARPS * 32)
 moe_select_grouped_kernel(const float* __restrict__ logits, int stride, const float* __restrict__ correction,
                           int* __restrict__ top_idx, float* __restrict__ top_w, int n_tokens, int E, int top, int n_groups,
                           int keep) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float sc[RWARPS][MAX_E];          // softmax scores
     __shared__ float pk[RWARPS][MAX_E];          // pick scores (minus infinity once taken or shut out)
     __shared__ float gs[RWARPS][MAX_E];          // group scores
@@ -224,6 +230,8 @@ template <typename T>
 __global__ void __launch_bounds__(EWARPS * 32)
 moe_up_kernel(const T* __restrict__ h, int h_stride, const T* __restrict__ gate_up, const int* __restrict__ top_idx,
               T* __restrict__ act, int d, int ff, int top, int act_kind, float act_limit, float act_alpha) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.y;                              // token * top + choice
     const int t = item / top;
@@ -242,6 +250,8 @@ template <typename T>
 __global__ void __launch_bounds__(EWARPS * 32)
 moe_up_plain_kernel(const T* __restrict__ h, int h_stride, const T* __restrict__ up, const int* __restrict__ top_idx,
                     const float* __restrict__ in_w, T* __restrict__ act, int d, int ff, int top) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.y;                              // token * top + choice
     const int t = item / top;
@@ -259,6 +269,8 @@ __global__ void __launch_bounds__(EWARPS * 32)
 moe_down_kernel(const T* __restrict__ act, const T* __restrict__ down, const int* __restrict__ top_idx,
                 const float* __restrict__ top_w, const float* __restrict__ shared, const float* __restrict__ shared_gate,
                 float* __restrict__ y, int d, int ff, int top, int shared_splits = 1, long long shared_stride = 0) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.y;
     const int i = blockIdx.x * EWARPS + warp;
@@ -288,7 +300,7 @@ int infero_moe_select(const float* logits, int stride, int gate_col, int* top_id
     if (n_tokens == 0) return 0;
     INFERO_REQUIRE(E >= 1 && E <= MAX_E && top >= 1 && top <= E && top <= MAX_TOP,
                    "moe select: %d experts (at most %d), top %d (at most %d)", E, MAX_E, top, MAX_TOP);
-    moe_select_kernel<<<(n_tokens + RWARPS - 1) / RWARPS, RWARPS * 32, 0, stream>>>(logits, stride, gate_col, top_idx, top_w,
+    launch_pdl(moe_select_kernel, dim3((n_tokens + RWARPS - 1) / RWARPS), dim3(RWARPS * 32), 0, stream, logits, stride, gate_col, top_idx, top_w,
                                                                                   gate_out, n_tokens, E, top);
     return infero_check_launch("moe_select");
 }
@@ -300,7 +312,7 @@ int infero_moe_select_grouped(const float* logits, int stride, const float* corr
                    "moe select: %d experts (at most %d), top %d (at most %d)", E, MAX_E, top, MAX_TOP);
     INFERO_REQUIRE(n_groups >= 1 && E % n_groups == 0 && keep >= 1 && keep <= n_groups && (E / n_groups) * keep >= top,
                    "moe select: %d groups of %d experts, %d kept, cannot give %d choices", n_groups, E, keep, top);
-    moe_select_grouped_kernel<<<(n_tokens + RWARPS - 1) / RWARPS, RWARPS * 32, 0, stream>>>(
+    launch_pdl(moe_select_grouped_kernel, dim3((n_tokens + RWARPS - 1) / RWARPS), dim3(RWARPS * 32), 0, stream, 
         logits, stride, correction, top_idx, top_w, n_tokens, E, top, n_groups, keep);
     return infero_check_launch("moe_select_grouped");
 }
@@ -312,7 +324,7 @@ int infero_moe_select_scored(const float* logits, int stride, int splits, long l
     INFERO_REQUIRE(E >= 1 && E <= MAX_E && top >= 1 && top <= E && top <= MAX_TOP,
                    "moe select: %d experts (at most %d), top %d (at most %d)", E, MAX_E, top, MAX_TOP);
     INFERO_REQUIRE(splits >= 1, "moe select: %d splits", splits);
-    moe_select_scored_kernel<<<(n_tokens + RWARPS - 1) / RWARPS, RWARPS * 32, 0, stream>>>(logits, stride, splits, split_stride,
+    launch_pdl(moe_select_scored_kernel, dim3((n_tokens + RWARPS - 1) / RWARPS), dim3(RWARPS * 32), 0, stream, logits, stride, splits, split_stride,
                                                                                          top_idx, top_w, n_tokens, E, top, renorm);
     return infero_check_launch("moe_select_scored");
 }
@@ -330,14 +342,14 @@ int infero_moe_experts_plain_streamed(const void* h, int h_stride, const void* u
     const float* in_w = weight_input ? top_w : nullptr;
     const float* out_w = weight_input ? nullptr : top_w;
     if (dtype == INFERO_F32) {
-        moe_up_plain_kernel<float><<<gu, EWARPS * 32, 0, stream>>>((const float*)h, h_stride, (const float*)up, top_idx, in_w,
+        launch_pdl(moe_up_plain_kernel<float>, gu, dim3(EWARPS * 32), 0, stream, (const float*)h, h_stride, (const float*)up, top_idx, in_w,
                                                                   (float*)act, d, ff, top);
-        moe_down_kernel<float><<<gd, EWARPS * 32, 0, stream>>>((const float*)act, (const float*)down, top_idx, out_w, shared,
+        launch_pdl(moe_down_kernel<float>, gd, dim3(EWARPS * 32), 0, stream, (const float*)act, (const float*)down, top_idx, out_w, shared,
                                                               nullptr, y, d, ff, top, shared_splits, shared_stride);
     } else {
-        moe_up_plain_kernel<bf16><<<gu, EWARPS * 32, 0, stream>>>((const bf16*)h, h_stride, (const bf16*)up, top_idx, in_w,
+        launch_pdl(moe_up_plain_kernel<bf16>, gu, dim3(EWARPS * 32), 0, stream, (const bf16*)h, h_stride, (const bf16*)up, top_idx, in_w,
                                                                  (bf16*)act, d, ff, top);
-        moe_down_kernel<bf16><<<gd, EWARPS * 32, 0, stream>>>((const bf16*)act, (const bf16*)down, top_idx, out_w, shared,
+        launch_pdl(moe_down_kernel<bf16>, gd, dim3(EWARPS * 32), 0, stream, (const bf16*)act, (const bf16*)down, top_idx, out_w, shared,
                                                              nullptr, y, d, ff, top, shared_splits, shared_stride);
     }
     return infero_check_launch("moe_experts_plain_streamed");
@@ -352,15 +364,15 @@ int infero_moe_experts_streamed(const void* h, int h_stride, const void* gate_up
     INFERO_REQUIRE(n_tokens * (long long)top <= 65535 && n_tokens <= 65535, "moe: %d tokens are too many for the streaming path", n_tokens);
     const dim3 gu((ff + EWARPS - 1) / EWARPS, n_tokens * top), gd((d + EWARPS - 1) / EWARPS, n_tokens);
     if (dtype == INFERO_F32) {
-        moe_up_kernel<float><<<gu, EWARPS * 32, 0, stream>>>((const float*)h, h_stride, (const float*)gate_up, top_idx,
+        launch_pdl(moe_up_kernel<float>, gu, dim3(EWARPS * 32), 0, stream, (const float*)h, h_stride, (const float*)gate_up, top_idx,
                                                             (float*)act, d, ff, top, act_kind, act_limit, act_alpha);
-        moe_down_kernel<float><<<gd, EWARPS * 32, 0, stream>>>((const float*)act, (const float*)down, top_idx, top_w,
-                                                              shared, shared_gate, y, d, ff, top);
+        launch_pdl(moe_down_kernel<float>, gd, dim3(EWARPS * 32), 0, stream, (const float*)act, (const float*)down, top_idx, top_w,
+                                                              shared, shared_gate, y, d, ff, top, 1, 0LL);
     } else {
-        moe_up_kernel<bf16><<<gu, EWARPS * 32, 0, stream>>>((const bf16*)h, h_stride, (const bf16*)gate_up, top_idx,
+        launch_pdl(moe_up_kernel<bf16>, gu, dim3(EWARPS * 32), 0, stream, (const bf16*)h, h_stride, (const bf16*)gate_up, top_idx,
                                                            (bf16*)act, d, ff, top, act_kind, act_limit, act_alpha);
-        moe_down_kernel<bf16><<<gd, EWARPS * 32, 0, stream>>>((const bf16*)act, (const bf16*)down, top_idx, top_w,
-                                                             shared, shared_gate, y, d, ff, top);
+        launch_pdl(moe_down_kernel<bf16>, gd, dim3(EWARPS * 32), 0, stream, (const bf16*)act, (const bf16*)down, top_idx, top_w,
+                                                             shared, shared_gate, y, d, ff, top, 1, 0LL);
     }
     return infero_check_launch("moe_experts_streamed");
 }

@@ -27,6 +27,8 @@ __global__ void moe_align_kernel(const int* __restrict__ top_idx, int n_pairs, i
                                  int* __restrict__ sorted_pair, int* __restrict__ tile_expert, int max_tiles,
                                  int* __restrict__ a_rows /* token of each row, -1 in padding */, int BM,
                                  int* __restrict__ pair_row /* row of each pair, or null */) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int sh[];
     int* count = sh;                        // [E]
     int* start = sh + E;                    // [E + 1], in rows, padded
@@ -70,6 +72,8 @@ __global__ void moe_align_kernel(const int* __restrict__ top_idx, int n_pairs, i
 __global__ void moe_gather_rows_kernel(const bf16* __restrict__ h, int h_stride, const int* __restrict__ a_rows,
                                        bf16* __restrict__ xs, int d, const int* __restrict__ sorted_pair,
                                        const float* __restrict__ pair_w) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int src = a_rows[r];
     const float f = (pair_w && src >= 0) ? pair_w[sorted_pair[r]] : 1.0f;
@@ -94,6 +98,8 @@ __global__ void moe_gather_rows_kernel(const bf16* __restrict__ h, int h_stride,
 __global__ void moe_combine_rows_kernel(const float* __restrict__ rows, const int* __restrict__ pair_row,
                                         const float* __restrict__ top_w, const float* __restrict__ shared,
                                         const float* __restrict__ shared_gate, float* __restrict__ y, int d, int top) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t t = blockIdx.x;
     for (int i = threadIdx.x; i < d; i += blockDim.x) {
         float acc = 0.f;
@@ -226,6 +232,8 @@ void launch_grouped(const bf16* A, int lda, const int* a_rows, const bf16* B, co
 __global__ void moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ top_w,
                                    const float* __restrict__ shared, const float* __restrict__ shared_gate,
                                    float* __restrict__ y, int d, int top) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t t = blockIdx.x;
     for (int i = threadIdx.x; i < d; i += blockDim.x) {
         float acc = 0.f;
@@ -258,7 +266,7 @@ int infero_moe_experts_grouped(const void* h, int h_stride, const void* gate_up,
     const int BM = infero_moe_grouped_tile_rows(n_pairs, E);
     const size_t sh = (size_t)(3 * E + 1) * sizeof(int);
     INFERO_REQUIRE(sh <= 48 * 1024, "moe grouped: %d experts are too many", E);
-    moe_align_kernel<<<1, 1024, sh, stream>>>(top_idx, n_pairs, E, top, sorted_pair, tile_expert, tiles, a_rows, BM, nullptr);
+    launch_pdl(moe_align_kernel, dim3(1), dim3(1024), sh, stream, top_idx, n_pairs, E, top, sorted_pair, tile_expert, tiles, a_rows, BM, nullptr);
     if (BM == 128) {
         launch_grouped<EPI_SWIGLU, 128, 128, 4, 2, 3>((const bf16*)h, h_stride, a_rows, (const bf16*)gate_up, tile_expert, tiles,
                                                       2 * ff, d, act, ff, nullptr, stream, act_kind, act_limit, act_alpha);
@@ -270,7 +278,7 @@ int infero_moe_experts_grouped(const void* h, int h_stride, const void* gate_up,
         launch_grouped<EPI_SCATTER, 64, 64, 4, 1, 2>((const bf16*)act, ff, nullptr, (const bf16*)down, tile_expert, tiles,
                                                      d, ff, part, d, sorted_pair, stream);
     }
-    moe_combine_kernel<<<n_tokens, 256, 0, stream>>>(part, top_w, shared, shared_gate, y, d, top);
+    launch_pdl(moe_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, part, top_w, shared, shared_gate, y, d, top);
     return infero_check_launch("moe_experts_grouped");
 }
 
@@ -287,8 +295,8 @@ int infero_moe_tc_prepare_scaled(const void* h, int h_stride, const int* top_idx
     const int n_pairs = n_tokens * top, tiles = infero_moe_tc_tiles(n_pairs, E);
     const size_t sh = (size_t)(3 * E + 1) * sizeof(int);
     INFERO_REQUIRE(sh <= 48 * 1024, "moe grouped: %d experts are too many", E);
-    moe_align_kernel<<<1, 1024, sh, stream>>>(top_idx, n_pairs, E, top, sorted_pair, tile_expert, tiles, a_rows, 128, pair_row);
-    moe_gather_rows_kernel<<<tiles * 128, 128, 0, stream>>>((const bf16*)h, h_stride, a_rows, (bf16*)xs, d, sorted_pair, pair_w);
+    launch_pdl(moe_align_kernel, dim3(1), dim3(1024), sh, stream, top_idx, n_pairs, E, top, sorted_pair, tile_expert, tiles, a_rows, 128, pair_row);
+    launch_pdl(moe_gather_rows_kernel, dim3(tiles * 128), dim3(128), 0, stream, (const bf16*)h, h_stride, a_rows, (bf16*)xs, d, sorted_pair, pair_w);
     return infero_check_launch("moe_tc_prepare");
 }
 
@@ -301,7 +309,7 @@ int infero_moe_tc_prepare(const void* h, int h_stride, const int* top_idx, int* 
 int infero_moe_tc_combine(const float* rows, const int* pair_row, const float* top_w, const float* shared,
                           const float* shared_gate, float* y, int n_tokens, int d, int top, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
-    moe_combine_rows_kernel<<<n_tokens, 256, 0, stream>>>(rows, pair_row, top_w, shared, shared_gate, y, d, top);
+    launch_pdl(moe_combine_rows_kernel, dim3(n_tokens), dim3(256), 0, stream, rows, pair_row, top_w, shared, shared_gate, y, d, top);
     return infero_check_launch("moe_tc_combine");
 }
 
