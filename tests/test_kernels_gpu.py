@@ -724,6 +724,36 @@ def _paged_requests(totals, Hkv, D, P, dt, seed, dead_before):
     return table, kc, vc, Ks, Vs
 
 
+@pytest.mark.parametrize("n", [15, 16, 33, 64, 256, 257])
+@pytest.mark.parametrize("window", [None, 700])
+def test_decode_splits_shared_out_by_length(n, window):
+    """Plans of several splits of 400 to 1,024 keys on batches of very uneven requests (1 to 2,047 keys, one far longer than the
+    rest), at the edges of what the sharing out takes: every key found, whoever has it, and nothing left in the counters."""
+    from infero_b200.kernels import attention as A, tc_gemm
+    H, Hkv, D, P, dt = 6, 2, 64, 16, torch.bfloat16
+    rng = np.random.default_rng(n)
+    for case in ("spread", "one long", "equal"):
+        lengths = {"spread": [int(round(16 * 128 ** (i / (n - 1)))) - (i == n - 1) for i in range(n)],
+                   "one long": [1] * (n - 1) + [2047], "equal": [1500] * min(n, 40) + [1500 if n <= 40 else 1] * max(0, n - 40)}[case]
+        rng.shuffle(lengths)
+        table, kc, vc, Ks, Vs = _paged_requests(lengths, Hkv, D, P, dt, 3, [0] * n)
+        q = _rand((n, H * D), dt, 7)
+        positions = torch.tensor([L - 1 for L in lengths], dtype=torch.int32, device=DEV)
+        entry = torch.arange(n, dtype=torch.int32, device=DEV)
+        scale = 2.0 / math.sqrt(D)
+        vis = min(max(lengths), window + 15) if window else max(lengths)
+        for chunk in (400, 1024):
+            out = torch.zeros((n, H * D), dtype=dt, device=DEV)
+            for _ in range(2):                          # (the second launch finds the counters as the first left them)
+                A.decode(q, out, kc, vc, table.to(DEV), entry, positions, 0, n, H, Hkv, D, P, window, scale, chunk, -(-vis // chunk))
+            worst = 0.0
+            for e in range(0, n, max(1, n // 20)):
+                ref = _attention_ref(q.view(n, H, D)[e].double().cpu(), Ks[e].double().cpu(), Vs[e].double().cpu(), scale, window)
+                worst = max(worst, float((out[e].double().cpu().view(H, D) - ref).abs().max() / ref.abs().max()))
+            assert worst <= 1.5e-2, f"{case}, splits of {chunk}: {worst:.3e}"
+    assert tc_gemm.error_flag() == 0
+
+
 @pytest.mark.parametrize("H,Hkv,D", [(4, 2, 64), (7, 1, 128)])
 @pytest.mark.parametrize("window", [48, 100])
 @pytest.mark.parametrize("P", [16, 64])
