@@ -42,8 +42,9 @@ struct ChannelScanArgs {
     float* y;                // [T, H V]
     int* err;
     long long v_stride, state_stride, s_off;
-    int slots, H, K, V, wide_state, wide_v;
+    int slots, H, K, V, wide_state, wide_v, n_entries;
     float q_scale;
+    Segments seg;
 };
 
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -63,8 +64,10 @@ template <bool DELTA, int Kp, int C> struct ChannelPlan {
 
 template <int N> struct Int { static constexpr int value = N; };
 
-template <bool DELTA, int NR, int LG, int C, int CPT>
+// ENDS (gated linear attention): every segment but a request's last from an empty state, without read-outs.
+template <bool DELTA, int NR, int LG, int C, int CPT, bool ENDS = false>
 __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs a) {
+    static_assert(!(DELTA && ENDS), "the delta rule's state does not come apart into segments");
     constexpr int Kp = NR * LG, NP = NR / 2, N4 = NR / 4, SHARE = LG / CPT, V4 = 3 * Kp / 4;
     using Plan = ChannelPlan<DELTA, Kp, C>;
     constexpr int TPS = Plan::TPS, REC = Plan::REC;
@@ -76,12 +79,15 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
     float* vs = sm + Plan::RING * Plan::STAGE;           // [Plan::RING][TPS][COLS]
     f2* us = reinterpret_cast<f2*>(vs + Plan::RING * TPS * COLS);         // [2][COLS][C] the u's, twice each
     pdl_launch_dependents();
-    const int e = blockIdx.x, h = blockIdx.y, pb = blockIdx.z;
-    const int n_new = a.entry_q_len[e];
-    if (n_new <= 0) return;
+    const Segment part = segment_at(a.seg, blockIdx.x, a.entry_q_len, a.n_entries);
+    const int e = part.e, h = blockIdx.y, pb = blockIdx.z;
+    const int n_new = part.n;
+    if (n_new <= 0 || (ENDS && part.last)) return;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int first = a.entry_q_start[e], n_stages = (n_new + TPS - 1) / TPS;
+    const int first = a.entry_q_start[e] + part.t0, n_stages = (n_new + TPS - 1) / TPS;
     float* S_head = a.state + (long long)a.entry_slot[e] * a.state_stride + a.s_off + (size_t)h * a.V * a.K;
+    float* S_part = a.seg.starts + ((size_t)part.slot * a.H + h) * a.V * a.K;
+    const float* S_from = part.count > 1 ? S_part : S_head;
     if (tid == 0) {
         never = 0;
         for (int i = 0; i < Plan::RING; ++i) tc::mbar_init(&full[i], 1);
@@ -159,9 +165,10 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
 #pragma unroll
         for (int n = 0; n < N4; ++n) {
             const int row = (n * LG + l) * 4, cc = c + (p ^ mine);
-            const float* s = S_head + (size_t)cc * a.K + row;
+            const float* s = S_from + (size_t)cc * a.K + row;
             float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (cc < a.V && a.wide_state) {
+            if (ENDS) {
+            } else if (cc < a.V && a.wide_state) {
                 if (row < a.K) f = *reinterpret_cast<const float4*>(s);
             } else if (cc < a.V) {
                 if (row < a.K) f.x = s[0];
@@ -186,6 +193,9 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
         scatter_sum<N, SHARE>(dots, lane);
     };
     int turn = 0;
+    f2 total[NP];                                    // ENDS: the product of the decays
+#pragma unroll
+    for (int n = 0; n < NP; ++n) total[n] = f2_of(1.f, 1.f);
     for (int s = 0; s < n_stages; ++s) {
         __syncthreads();
         const int buf = s % Plan::RING, nt = min(TPS, n_new - s * TPS);
@@ -285,6 +295,27 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
                             S[p][2 * n + 1] = f2_fma(fw.y, uu[p][j], S[p][2 * n + 1]);
                         }
                     }
+            } else if constexpr (ENDS) {
+#pragma unroll
+                for (int j = 0; j < C; ++j) {
+                    f2 pp[CPT];
+#pragma unroll
+                    for (int p = 0; p < CPT; ++p) {
+                        const float pv = vb[(t0 + j) * COLS + (p ^ mine)];
+                        pp[p] = f2_of(pv, pv);
+                    }
+#pragma unroll
+                    for (int n = 0; n < N4; ++n) {
+                        const ulonglong2 fd = tok[j * V4 + n * LG], fk = tok[j * V4 + Kp / 4 + n * LG];
+                        total[2 * n] = f2_mul(fd.x, total[2 * n]);
+                        total[2 * n + 1] = f2_mul(fd.y, total[2 * n + 1]);
+#pragma unroll
+                        for (int p = 0; p < CPT; ++p) {
+                            S[p][2 * n] = f2_fma(fk.x, pp[p], f2_mul(fd.x, S[p][2 * n]));
+                            S[p][2 * n + 1] = f2_fma(fk.y, pp[p], f2_mul(fd.y, S[p][2 * n + 1]));
+                        }
+                    }
+                }
             } else {
                 float dots[C * CPT];
 #pragma unroll
@@ -321,6 +352,19 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
             }
         }
     }
+    if (!ENDS && !part.last) return;
+    float* S_to = ENDS ? S_part : S_head;
+    if (ENDS && pb == 0 && tid < LG) {
+        float* d = a.seg.totals + ((size_t)part.slot * a.H + h) * a.K;
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            float x, y;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(total[n]));
+            const int row = (n / 2 * LG + l) * 4 + n % 2 * 2;
+            if (row < a.K) d[row] = x;
+            if (row + 1 < a.K) d[row + 1] = y;
+        }
+    }
 #pragma unroll
     for (int p = 0; p < CPT; ++p) {
         const int cc = c + (p ^ mine);
@@ -328,7 +372,7 @@ __global__ void __launch_bounds__(288) channel_scan_kernel(const ChannelScanArgs
 #pragma unroll
         for (int n = 0; n < N4; ++n) {
             const int row = (n * LG + l) * 4;
-            float* s = S_head + (size_t)cc * a.K + row;
+            float* s = S_to + (size_t)cc * a.K + row;
             float4 f;
             asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(S[p][2 * n]));
             asm("mov.b64 {%0, %1}, %2;" : "=f"(f.z), "=f"(f.w) : "l"(S[p][2 * n + 1]));
@@ -352,10 +396,12 @@ inline int forced_columns() {
 }
 
 template <bool DELTA>
-int launch_channel_scan(ChannelScanArgs a, int n_entries, bool single, int sm_count, cudaStream_t stream) {
+int launch_channel_scan(ChannelScanArgs a, int n_entries, int n_segments, bool single, int sm_count, cudaStream_t stream) {
     const int NR = a.K <= 128 ? 4 : a.K <= 256 ? 8 : 16, LG = a.K <= 32 ? 8 : a.K <= 64 ? 16 : 32;
     const int sms = sm_count > 0 ? sm_count : 148;
-    auto blocks = [&](int cols) { return (long long)n_entries * a.H * ((a.V + cols - 1) / cols); };
+    a.n_entries = n_entries;
+    const int parts = a.seg.len > 0 ? n_segments : n_entries;
+    auto blocks = [&](int cols) { return (long long)parts * a.H * ((a.V + cols - 1) / cols); };
     int CPT = 4;
     while (CPT > 1 && blocks(32 / LG * CPT) < 2 * sms) CPT /= 2;         // (blocks of one warp: warps)
     if (single) CPT = CPT == 4 ? 4 : 1;
@@ -363,7 +409,7 @@ int launch_channel_scan(ChannelScanArgs a, int n_entries, bool single, int sm_co
     int threads = single ? 256 : 128;
     while (threads > 32 && blocks(threads / LG * CPT) * 5 < 4 * sms) threads /= 2;
     const int COLS = threads / LG * CPT;
-    const dim3 grid(n_entries, a.H, (a.V + COLS - 1) / COLS);
+    const dim3 grid(parts, a.H, (a.V + COLS - 1) / COLS);
     INFERO_REQUIRE(grid.z <= 65535, "channel_scan: %d columns are too many for one launch", a.V);
     a.wide_v = a.wide_v && COLS % 4 == 0;
     if (infero_tc_err_flag(&a.err)) return 1;
@@ -376,7 +422,16 @@ int launch_channel_scan(ChannelScanArgs a, int n_entries, bool single, int sm_co
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
         /* a portion's blocks run long: started under the kernel in front, they would crowd on the first free SMs */         \
         if (single) launch_pdl(k, grid, dim3(threads + 32), smem, stream, a);                                           \
-        else k<<<grid, threads + 32, smem, stream>>>(a);                                                                \
+        else {                                                                                                          \
+            if (!DELTA && a.seg.len > 0) {                                                                              \
+                auto ends = CPT == 4 ? channel_scan_kernel<false, R, L, GROUP, 4, true>                                 \
+                          : CPT == 2 ? channel_scan_kernel<false, R, L, GROUP, 2, true> : channel_scan_kernel<false, R, L, GROUP, 1, true>; \
+                if (smem > 48 * 1024) cudaFuncSetAttribute(ends, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+                ends<<<grid, threads + 32, smem, stream>>>(a);                                                          \
+                if (chain_segments(a.seg, a.state, a.state_stride, a.s_off, a.entry_q_len, a.entry_slot, n_entries, a.H, a.V, a.K, stream)) return 1; \
+            }                                                                                                           \
+            k<<<grid, threads + 32, smem, stream>>>(a);                                                                 \
+        }                                                                                                               \
     } while (0)
     if (LG == 8) GO(4, 8);
     else if (LG == 16) GO(4, 16);
@@ -390,16 +445,17 @@ int launch_channel_scan(ChannelScanArgs a, int n_entries, bool single, int sm_co
 template <bool DELTA>
 int channel_scan(const float* rec, int slots, const float* v, long long v_stride, float* state, long long state_stride, long long s_off,
                  const int* entry_q_start, const int* entry_q_len, const int* entry_slot, float* y, float q_scale, int n_entries, int single,
-                 int H, int K, int V, int sm_count, cudaStream_t stream) {
+                 int H, int K, int V, int sm_count, cudaStream_t stream, Segments seg = {}, int n_segments = 0) {
     if (n_entries == 0) return 0;
     INFERO_REQUIRE(K >= 1 && K <= MAX_K && V >= 1 && H >= 1 && H <= 65535, "channel_scan: %d heads of %d x %d", H, K, V);
     INFERO_REQUIRE(al16(rec), "channel_scan: unaligned records");
     ChannelScanArgs a = {};
     a.rec = rec, a.v = v, a.state = state, a.entry_q_start = entry_q_start, a.entry_q_len = entry_q_len, a.entry_slot = entry_slot, a.y = y;
     a.v_stride = v_stride, a.state_stride = state_stride, a.s_off = s_off, a.slots = slots, a.H = H, a.K = K, a.V = V, a.q_scale = q_scale;
+    if (!single) a.seg = seg;
     a.wide_state = K % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 && al16(state);
     a.wide_v = V % 4 == 0 && v_stride % 4 == 0 && al16(v);
-    return launch_channel_scan<DELTA>(a, n_entries, single != 0, sm_count, stream);
+    return launch_channel_scan<DELTA>(a, n_entries, n_segments, single != 0, sm_count, stream);
 }
 
 }  // namespace memory

@@ -48,6 +48,35 @@ template <int N, int L> struct Scattered {
     static constexpr int per_lane = N / L > 1 ? N / L : 1, stride = L / N > 1 ? L / N : 1;
 };
 
+// ---- long portions in segments -------------------------------------------------------------------------------------------
+// A rule whose state only decays and takes in k v^T (no delta) is linear in its state, so a long portion can be cut into segments
+// that run side by side: one scan without read-outs gives every segment's end from an empty state and the product of its decays,
+// a small kernel chains them into every segment's start, and the ordinary scan runs over all segments at once.  One long
+// portion alone leaves a scan one or two warps a scheduler and the latency of its chain of tokens: two layers of 16 heads of
+// 128 x 128 over 2,047 tokens 482 us whole, 360 in segments of 256; a model's pass over them 2.26 and 2.14 ms, over 1,201 + 37 + 500
+// tokens 2.09 and 1.96.  Portions beside one another fill the schedulers by themselves (four of 512: 1.79 ms whole, 1.91 cut).
+struct Segments {
+    int len;                 // tokens of a segment (a multiple of the stages' tokens); 0: portions run whole
+    float* starts;           // [segments of the requests that have more than one][heads, columns, K]
+    float* totals;           // [the same][heads, K] the products of their decays
+};
+// From the segments' ends and decays to their starts, in place (channel_memory_decayed.cu).
+int chain_segments(const Segments& seg, const float* state, long long state_stride, long long s_off, const int* entry_q_len,
+                   const int* entry_slot, int n_entries, int H, int W, int K, cudaStream_t stream);
+struct Segment { int e, t0, n, count, slot; bool last; };      // request, first token and tokens of the segment; segments of the request
+__device__ __forceinline__ int segments_of(int n, int len) { return len > 0 && n > len ? (n + len - 1) / len : 1; }
+__device__ __forceinline__ Segment segment_at(const Segments& g, int index, const int* __restrict__ entry_q_len, int n_entries) {
+    if (g.len == 0) return {index, 0, entry_q_len[index], 1, 0, true};
+    int slot = 0;
+    for (int e = 0; e < n_entries; ++e) {
+        const int n = entry_q_len[e], count = segments_of(n, g.len);
+        if (index < count) return {e, index * g.len, min(g.len, n - index * g.len), count, slot + index, index == count - 1};
+        index -= count;
+        if (count > 1) slot += count;
+    }
+    return {0, 0, 0, 1, 0, true};
+}
+
 // ---- prepare -----------------------------------------------------------------------------------------------------------
 struct PrepareArgs {
     const float* proj;       // [T, >= x_off + CH]; CH = 2 G K + H V channels [q | k | v]

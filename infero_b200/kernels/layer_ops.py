@@ -760,14 +760,29 @@ def channel_prepare(proj: torch.Tensor, x_off: int, step_off: int, conv_w: torch
     return v, rec
 
 
-def _channel_scan(f, rec, n, v, extra, state, s_off, entry_q_start, entry_q_len, entry_slot, n_entries, H, K, V, single):
+SEGMENT = 256             # tokens of a segment
+
+
+def _segments(lens, H: int, V: int, K: int, device):
+    """(tokens of a segment or 0, segments in all, scratch for their starts and their decays) of a step whose requests bring
+    ``lens`` tokens (host numbers; None: not known, portions run whole).  Portions are cut where one of four segments and more
+    brings at least half of the step's tokens (csrc/outer_memory.cuh has both sides' times)."""
+    if lens is None or max(lens) < 4 * SEGMENT or 2 * int(max(lens)) < sum(int(n) for n in lens):
+        return 0, 0, None, None
+    counts = [-(-int(n) // SEGMENT) if n > SEGMENT else 1 for n in lens]
+    slots = sum(c for c in counts if c > 1)
+    return (SEGMENT, sum(counts), torch.empty((slots, H, V, K), dtype=torch.float32, device=device),
+            torch.empty((slots, H, K), dtype=torch.float32, device=device))
+
+
+def _channel_scan(f, rec, n, v, extra, state, s_off, entry_q_start, entry_q_len, entry_slot, n_entries, H, K, V, single, more=()):
     from .tc_gemm import sm_count
     assert rec.is_contiguous() and rec.dtype == v.dtype == torch.float32 and v.stride(1) == 1 and v.shape[1] == H * V
     assert state.dtype == torch.float32 and state.is_contiguous() and s_off + H * V * K <= state.shape[1]
     y = torch.empty((v.shape[0], H * V), dtype=torch.float32, device=v.device)
     _check(f(_ptr(rec), c_int(n), _ptr(v), c_longlong(v.stride(0)), *extra, _ptr(state), c_longlong(state.stride(0)), c_longlong(s_off),
              _ptr(_i32(entry_q_start, "entry_q_start")), _ptr(_i32(entry_q_len, "entry_q_len")), _ptr(_i32(entry_slot, "entry_slot")), _ptr(y),
-             c_int(n_entries), c_int(1 if single else 0), c_int(H), c_int(K), c_int(V), c_int(sm_count(v.device)), _stream()))
+             c_int(n_entries), c_int(1 if single else 0), c_int(H), c_int(K), c_int(V), *more, c_int(sm_count(v.device)), _stream()))
     return y
 
 
@@ -780,12 +795,14 @@ def channel_scan(v: torch.Tensor, rec: torch.Tensor, state: torch.Tensor, s_off:
 
 
 def decayed_scan(v: torch.Tensor, rec: torch.Tensor, state: torch.Tensor, s_off: int, entry_q_start, entry_q_len, entry_slot,
-                 n_entries: int, H: int, K: int, V: int, single: bool = False) -> torch.Tensor:
+                 n_entries: int, H: int, K: int, V: int, single: bool = False, lens=None) -> torch.Tensor:
     """Gated linear attention of every request over its new tokens, from the values (columns of the product's rows) and
-    ``decayed_records``; float32 [T, H V], q times K^-1/2.  S [H, V, K] at ``s_off``."""
+    ``decayed_records``; float32 [T, H V], q times K^-1/2.  S [H, V, K] at ``s_off``.  ``lens``: the requests' new tokens on the
+    host, for long portions to run in segments."""
     assert tuple(rec.shape[:2]) == (H, v.shape[0])
+    seg, n_seg, starts, totals = _segments(None if single else lens, H, V, K, v.device)
     return _channel_scan(lib().infero_decayed_scan, rec, rec.shape[1], v, (c_float(K ** -0.5),), state, s_off, entry_q_start, entry_q_len,
-                         entry_slot, n_entries, H, K, V, single)
+                         entry_slot, n_entries, H, K, V, single, (c_int(seg), c_int(n_seg), _ptr(starts), _ptr(totals)))
 
 
 def memory_finish(y: torch.Tensor, den: Optional[torch.Tensor], gate: torch.Tensor, act: str, norm_w: torch.Tensor, eps: float,
