@@ -20,7 +20,8 @@
 //   With a window W a query at position p sees the keys p - W + 1 .. p; with sinks (one number per head) the softmax's
 //   denominator has one more term exp(sink) without a value.
 // finish: out[t, n * V + v] = val[n, t, v] * sigmoid(gate[t, n]).
-#include "common.cuh"
+#include "attn_common.cuh"
+#include "outer_memory.cuh"
 #include <math_constants.h>
 
 namespace {
@@ -191,6 +192,185 @@ __global__ void latent_finish_kernel(const float* __restrict__ val, long long he
     }
 }
 
+// ---- steps of few single tokens (bf16) ---------------------------------------------------------------------------------
+// What is around the attention of up to FEW_TOKENS tokens in two launches instead of five: every launch costs more than its
+// work here, and the tiles of 128 rows of the grouped products were mostly padding.  Both kernels ask for their weights before they
+// wait for the kernel in front.  A layer of 16 heads of 128 + 64, latent 512, eight tokens: the launches around the attention
+// 27 us (in five, one after the other), 15 in two; a step of four such layers with experts 462 us before, 404 now.
+constexpr int FEW_TOKENS = 16, FEW_COLS = 64, FEW_MAX_D = 128;
+
+// Blocks 0 .. T - 1: a token's latent row.  Then for every head the blocks of FEW_COLS latent columns, a warp 16 of them, and
+// one block that turns the rotated parts.  q_lat = bf16(q plain) Wuk^T on mma.sync with the columns as rows of the tile and the
+// tokens as its eight columns; a lane's 16 bytes of a row serve two steps of k (the order of k is the same on both sides).
+template <int OCT>
+__global__ void __launch_bounds__(128)
+latent_query_few_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ q_src, int q_stride, int q_off,
+                        int kv_off, const float* __restrict__ norm_w, float eps, const double* __restrict__ freq, int rot, int pairing,
+                        float amp, const int* __restrict__ positions, const int* __restrict__ tok_entry,
+                        const int* __restrict__ block_table, int max_blocks, int page_size, bf16* __restrict__ cache, int write_cache,
+                        const bf16* __restrict__ w_k, float* __restrict__ q_lat, float* __restrict__ q_rot, long long head_rows,
+                        int T, int H, int D, int R, int C) {
+    extern __shared__ float2 cs[];                       // a latent row: [rot / 2]
+    __shared__ __align__(16) bf16 qs[8 * OCT][FEW_MAX_D + 8];
+    __shared__ float red[32];
+    pdl_launch_dependents();
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x < T) {
+        pdl_wait();
+        if (!write_cache) return;
+        const int t = blockIdx.x, pos = positions[t];
+        for (int i = tid; i < rot / 2; i += blockDim.x) cs[i] = turn((double)pos * freq[i], amp);
+        __syncthreads();
+        const float* kv = proj + (size_t)t * proj_stride + kv_off;
+        float sq = 0.f;
+        for (int i = tid; i < C; i += blockDim.x) sq = fmaf(kv[i], kv[i], sq);
+        const float rstd = 1.0f / sqrtf(block_sum(sq, red) / (float)C + eps);
+        const int page = block_table[(size_t)tok_entry[t] * max_blocks + pos / page_size];
+        bf16* dst = cache + ((size_t)page * page_size + (pos % page_size)) * (C + R);
+        for (int i = tid; i < C; i += blockDim.x) dst[i] = from_f32<bf16>(kv[i] * rstd * norm_w[i]);
+        for (int i = tid; i < R; i += blockDim.x) dst[C + i] = from_f32<bf16>(rotated(kv + C, i, rot, pairing, cs));
+        return;
+    }
+    const int chunks = C / FEW_COLS, n = ((int)blockIdx.x - T) / (chunks + 1), ch = ((int)blockIdx.x - T) % (chunks + 1);
+    const float* q0 = q_src + q_off + (size_t)n * (D + R);
+    if (ch == chunks) {
+        pdl_wait();
+        for (int i = tid; i < T * R; i += blockDim.x) {
+            const int t = i / R, c = i % R;
+            const float* part = q0 + (size_t)t * q_stride + D;
+            float v = part[c];
+            if (c < rot) {
+                const int ia = pairing ? c & ~1 : c < rot / 2 ? c : c - rot / 2, ib = pairing ? ia + 1 : ia + rot / 2;
+                const float2 f = turn((double)positions[t] * freq[pairing ? c >> 1 : ia], amp);
+                v = c == ia ? part[ia] * f.x - part[ib] * f.y : part[ib] * f.x + part[ia] * f.y;
+            }
+            q_rot[((size_t)n * head_rows + t) * R + c] = v;
+        }
+        return;
+    }
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, c4 = lane & 3, col0 = ch * FEW_COLS + warp * 16;
+    const bf16* wr = w_k + ((size_t)n * C + col0 + g) * D + c4 * 8;
+    uint4 wa[FEW_MAX_D / 32], wb[FEW_MAX_D / 32];
+#pragma unroll
+    for (int k = 0; k < FEW_MAX_D / 32; ++k)
+        if (k * 32 < D) {
+            wa[k] = __ldg(reinterpret_cast<const uint4*>(wr + k * 32));
+            wb[k] = __ldg(reinterpret_cast<const uint4*>(wr + (size_t)8 * D + k * 32));
+        }
+    pdl_wait();
+    for (int i = tid; i < 8 * OCT * D; i += blockDim.x) {
+        const int t = i / D, c = i % D;
+        qs[t][c] = from_f32<bf16>(t < T ? q0[(size_t)t * q_stride + c] : 0.f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < OCT; ++o) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < FEW_MAX_D / 32; ++k)
+            if (k * 32 < D) {
+                const uint4 qb = *reinterpret_cast<const uint4*>(&qs[o * 8 + g][k * 32 + c4 * 8]);
+                const uint32_t a0[4] = {wa[k].x, wb[k].x, wa[k].y, wb[k].y}, a1[4] = {wa[k].z, wb[k].z, wa[k].w, wb[k].w};
+                attn::mma16816(acc, a0, qb.x, qb.y);
+                attn::mma16816(acc, a1, qb.z, qb.w);
+            }
+        const int t = o * 8 + c4 * 2;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (t + x < T) {
+                float* dst = q_lat + ((size_t)n * head_rows + t + x) * C + col0 + g;
+                dst[0] = acc[x];
+                dst[8] = acc[2 + x];
+            }
+    }
+}
+
+// A block per (head, token): the ranges' results merged (or the finished one read), rounded to bf16 as the product's operand, then
+// out[t, n V + v] = (Wuv row v . that) * sigmoid(gate): a warp eight rows at a time, a lane eight neighbouring columns of each 256.
+constexpr int FEW_ROWS = 8, FEW_MAX_C = 512, FEW_MAX_SPLITS = 64;
+__global__ void __launch_bounds__(256)
+latent_result_few_kernel(const bf16* __restrict__ o_lat, long long head_rows, const float* __restrict__ part_o,
+                         const float* __restrict__ part_ml, int splits, const float* __restrict__ sinks_log2, const bf16* __restrict__ w_v,
+                         const float* __restrict__ gate, int gate_stride, bf16* __restrict__ out, int out_stride, int H, int C, int V) {
+    __shared__ float w_s[FEW_MAX_SPLITS];
+    __shared__ float inv_s;
+    __shared__ __align__(16) bf16 o_s[FEW_MAX_C];
+    pdl_launch_dependents();
+    const int n = blockIdx.x, t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NJ = FEW_MAX_C / 256;
+    uint4 w[FEW_ROWS][NJ];
+    auto fetch = [&](int v0) {
+#pragma unroll
+        for (int r = 0; r < FEW_ROWS; ++r)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const int k = j * 256 + lane * 8;
+                w[r][j] = make_uint4(0, 0, 0, 0);
+                if (v0 + r < V && k < C) w[r][j] = __ldg(reinterpret_cast<const uint4*>(w_v + ((size_t)n * V + v0 + r) * C + k));
+            }
+    };
+    fetch(warp * FEW_ROWS);
+    pdl_wait();
+    if (splits > 1) {
+        const size_t item0 = ((size_t)t * H + n) * splits;
+        if (warp == 0) {
+            const float2* ml = reinterpret_cast<const float2*>(part_ml) + item0;
+            const float2 none = make_float2(-CUDART_INF_F, 0.f);
+            const float2 a = lane < splits ? ml[lane] : none, b = lane + 32 < splits ? ml[lane + 32] : none;
+            const float M = warp_max(fmaxf(a.x, b.x));
+            const float w0 = a.x == -CUDART_INF_F ? 0.f : exp2f(a.x - M), w1 = b.x == -CUDART_INF_F ? 0.f : exp2f(b.x - M);
+            w_s[lane] = w0, w_s[lane + 32] = w1;
+            float L = warp_sum(w0 * a.y + w1 * b.y);
+            if (sinks_log2) L += exp2f(sinks_log2[n] - M);
+            if (lane == 0) inv_s = 1.0f / L;
+        }
+        __syncthreads();
+        for (int c = threadIdx.x; c < C; c += blockDim.x) {
+            const float* src = part_o + item0 * C + c;
+            float acc = 0.f;
+            for (int s0 = 0; s0 < splits; s0 += 8) {
+                float v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = s0 + k < splits ? src[(size_t)(s0 + k) * C] : 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (s0 + k < splits) acc = fmaf(w_s[s0 + k], v[k], acc);
+            }
+            o_s[c] = from_f32<bf16>(acc * inv_s);
+        }
+    } else {
+        for (int c = threadIdx.x; c < C; c += blockDim.x) o_s[c] = o_lat[((size_t)n * head_rows + t) * C + c];
+    }
+    __syncthreads();
+    float o[NJ][8];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[j][i] = j * 256 + lane * 8 + i < C ? to_f32(o_s[j * 256 + lane * 8 + i]) : 0.f;
+    const float sg = gate ? 1.0f / (1.0f + expf(-gate[(size_t)t * gate_stride + n])) : 1.0f;
+    for (int v0 = warp * FEW_ROWS; v0 < V; v0 += 8 * FEW_ROWS) {
+        float dot[FEW_ROWS];
+#pragma unroll
+        for (int r = 0; r < FEW_ROWS; ++r) {
+            dot[r] = 0.f;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&w[r][j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __bfloat1622float2(p[i]);
+                    dot[r] = fmaf(f.x, o[j][2 * i], dot[r]);
+                    dot[r] = fmaf(f.y, o[j][2 * i + 1], dot[r]);
+                }
+            }
+        }
+        if (v0 + 8 * FEW_ROWS < V) fetch(v0 + 8 * FEW_ROWS);
+        memory::scatter_sum<FEW_ROWS, 32>(dot, lane);        // row r's in lane 4 r
+        const int v = v0 + (lane >> 2);
+        if (!(lane & 3) && v < V) out[(size_t)t * out_stride + (size_t)n * V + v] = from_f32<bf16>(dot[0] * sg);
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -266,6 +446,45 @@ int infero_latent_finish(const float* val, long long head_rows, const float* gat
     else
         launch_pdl(latent_finish_kernel<bf16>, dim3(n_tokens), dim3(256), 0, stream, val, head_rows, gate, gate_stride, (bf16*)out, out_stride, H, V);
     return infero_check_launch("latent_finish");
+}
+
+// Steps of up to 16 single tokens in bf16 (every token's request brings it alone).
+int infero_latent_few_supported(int n_tokens, int D, int C) {
+    return n_tokens >= 1 && n_tokens <= FEW_TOKENS && D >= 32 && D <= FEW_MAX_D && D % 32 == 0 && C >= FEW_COLS && C % FEW_COLS == 0 && C <= FEW_MAX_C;
+}
+
+// infero_latent_prepare_from and the product with Wuk^T [H, C, D] in one: q_lat float32 [H, head_rows, C], q_rot float32
+// [H, head_rows, R]; the tokens' latent rows go to the cache.
+int infero_latent_query_few(const float* proj, int proj_stride, const float* q_src, int q_stride, int q_off, int kv_off,
+                            const float* norm_w, float eps, const double* freq, int rot, int pairing, float amp, const int* positions,
+                            const int* tok_entry, const int* block_table, int max_blocks, int page_size, void* cache, int write_cache,
+                            const void* w_k, float* q_lat, float* q_rot, long long head_rows, int n_tokens, int H, int D, int R, int C,
+                            cudaStream_t stream) {
+    INFERO_REQUIRE(infero_latent_few_supported(n_tokens, D, C) && (reinterpret_cast<uintptr_t>(w_k) & 15u) == 0,
+                   "latent_query_few: %d tokens, %d x %d, not supported", n_tokens, D, C);
+    INFERO_REQUIRE(rot >= 0 && rot <= R && rot % 2 == 0 && rot <= 8192 && head_rows >= n_tokens, "latent attention: %d rotated coordinates of %d", rot, R);
+    const dim3 grid(n_tokens + H * (C / FEW_COLS + 1));
+#define GO(O_)                                                                                                                      \
+    launch_pdl(latent_query_few_kernel<O_>, grid, dim3(128), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, \
+               kv_off, norm_w, eps, freq, rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (bf16*)cache, \
+               write_cache, (const bf16*)w_k, q_lat, q_rot, head_rows, n_tokens, H, D, R, C)
+    if (n_tokens <= 8) GO(1);
+    else GO(2);
+#undef GO
+    return infero_check_launch("latent_query_few");
+}
+
+// From the attention's ranges (splits > 1: part_o, part_ml as infero_latent_attention_mma leaves them) or its finished result o_lat
+// (splits = 1) to out [tokens, H V]: merge, product with Wuv [H, V, C], gate.
+int infero_latent_result_few(const void* o_lat, long long head_rows, const float* part_o, const float* part_ml, int splits,
+                             const float* sinks_log2, const void* w_v, const float* gate, int gate_stride, void* out, int out_stride,
+                             int n_tokens, int H, int D, int C, int V, cudaStream_t stream) {
+    INFERO_REQUIRE(infero_latent_few_supported(n_tokens, D, C) && V >= 1 && splits >= 1 && splits <= FEW_MAX_SPLITS &&
+                       (reinterpret_cast<uintptr_t>(w_v) & 15u) == 0 && (splits == 1 ? o_lat != nullptr : part_o && part_ml),
+                   "latent_result_few: %d tokens, latent %d, %d ranges, not supported", n_tokens, C, splits);
+    launch_pdl(latent_result_few_kernel, dim3(H, n_tokens), dim3(256), 0, stream, (const bf16*)o_lat, head_rows, part_o, part_ml, splits,
+               sinks_log2, (const bf16*)w_v, gate, gate_stride, (bf16*)out, out_stride, H, C, V);
+    return infero_check_launch("latent_result_few");
 }
 
 }  // extern "C"

@@ -392,14 +392,14 @@ int infero_latent_mma_heads(int H) { return H <= 16 ? 16 : H <= 32 ? 32 : 64; }
 // Entries [entry_first, n_entries) of the step; n_tiles = sum over them of ceil(q_len / TQ) (the host knows the lengths).
 // single != 0: every entry brings one token (TQ = 1) and the keys are cut into `splits` ranges of `chunk` (a multiple of
 // 32); with splits > 1 part_o float32 [tokens * H * splits * C] and part_ml [tokens * H * splits * 2] are scratch, indexed
-// by the token's row in the step, and the merge runs behind.  Otherwise TQ = 64 / heads per CTA and splits = 1.
+// by the token's row in the step, and the merge runs behind (merge 0: the caller does it).  Otherwise TQ = 64 / heads per CTA and splits = 1.
 // window > 0: a token sees that many keys up to its own (the ranges then start at the tile of its lowest key); sinks float32
 // [H] (times log2 e) or null: one more term 2^sink of a head's sum.
 int infero_latent_attention_mma(const float* q_lat, const float* q_rot, long long head_rows, void* out, float* part_o,
                                 float* part_ml, const void* cache, const int* block_table, int max_blocks,
                                 const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int entry_first,
                                 int n_entries, int n_tiles, int single, int H, int C, int R, int page_size, float scale,
-                                int chunk, int splits, int window, const float* sinks, cudaStream_t stream) {
+                                int chunk, int splits, int window, const float* sinks, int merge, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
     INFERO_REQUIRE(infero_latent_mma_supported(C, R), "latent attention: no tensor-core instance for a latent of %d + %d", C, R);
     INFERO_REQUIRE(splits <= MAX_SPLITS, "latent attention: %d ranges of keys, at most %d", splits, MAX_SPLITS);
@@ -426,7 +426,7 @@ int infero_latent_attention_mma(const float* q_lat, const float* q_rot, long lon
 #undef BY_ROWS
 #undef GO
     if (rc) return rc;
-    if (splits > 1) {
+    if (splits > 1 && merge) {
         // the tokens of the leading single-token entries are the first rows of the step
         launch_pdl(latent_merge_kernel, dim3(n_tiles * H), dim3(C >= 256 ? 256 : 128), 0, stream, part_o, part_ml, (bf16*)out, head_rows, H, C, splits, sinks);
     }

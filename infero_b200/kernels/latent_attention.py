@@ -43,6 +43,44 @@ def prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, e
         _ptr(q_plain), _ptr(None if rot_block else q_rot), _ptr(q_rot if rot_block else None), c_longlong(rows), c_int(n_tokens), c_int(H), c_int(D), c_int(R), c_int(C), _stream()))
 
 
+def few_ok(ctx, cache: torch.Tensor, n_tokens: int, D: int, R: int, C: int) -> bool:
+    """Do the first ``n_tokens`` tokens go through ``query_few`` and ``result_few``?  Up to 16 of them, each its request's only one,
+    in bf16, in sizes those and the tensor-core attention take."""
+    from . import latent_mma
+    return (cache.dtype == torch.bfloat16 and n_tokens <= 16 and D % 32 == 0 and D <= 128 and latent_mma.ENABLED
+            and getattr(ctx, "h_q_len", None) is not None and len(ctx.h_q_len) >= n_tokens and bool((ctx.h_q_len[:n_tokens] == 1).all())
+            and latent_mma.supported(C, R))
+
+
+def query_few(proj, q_off, kv_off, norm_w, eps, freq, pairing, amp, positions, tok_entry, block_table, cache, page_size, w_k, q_lat, q_rot,
+              n_tokens, H, D, R, C, write_cache=True, q_src=None) -> None:
+    """``prepare`` and the product of the plain query parts with Wuk^T (``w_k`` [H, C, D]) in one launch: q_lat float32 [H, rows, C],
+    q_rot float32 [H, rows, R]."""
+    if q_src is None:
+        q_src = proj
+    assert proj.dtype == q_src.dtype == torch.float32 and proj.stride(1) == q_src.stride(1) == 1 and cache.is_contiguous()
+    assert cache.dtype == w_k.dtype == torch.bfloat16 and tuple(w_k.shape) == (H, C, D) and w_k.is_contiguous() and cache.shape[-1] == C + R
+    rows = q_lat.shape[1]
+    assert tuple(q_lat.shape) == (H, rows, C) and tuple(q_rot.shape) == (H, rows, R) and q_lat.is_contiguous() and q_rot.is_contiguous()
+    assert q_lat.dtype == q_rot.dtype == torch.float32 and (freq is None or (freq.dtype == torch.float64 and freq.is_contiguous()))
+    _check(lib().infero_latent_query_few(
+        _ptr(proj), c_int(proj.stride(0)), _ptr(q_src), c_int(q_src.stride(0)), c_int(q_off), c_int(kv_off), _ptr(_f32(norm_w, "norm_w")),
+        c_float(eps), _ptr(freq), c_int(0 if freq is None else 2 * freq.numel()), c_int(1 if pairing == "adjacent" else 0), c_float(amp),
+        _ptr(_i32(positions, "positions")), _ptr(_i32(tok_entry, "tok_entry")), _ptr(_i32(block_table, "block_table")),
+        c_int(block_table.shape[1]), c_int(page_size), _ptr(cache), c_int(1 if write_cache else 0), _ptr(w_k), _ptr(q_lat), _ptr(q_rot),
+        c_longlong(rows), c_int(n_tokens), c_int(H), c_int(D), c_int(R), c_int(C), _stream()))
+
+
+def result_few(o_lat, splits: int, part_o, part_ml, sinks_log2, w_v, gate, out, n_tokens: int, H: int, D: int, C: int, V: int) -> None:
+    """The attention's ranges merged (``splits`` > 1; else o_lat [H, rows, C] as it is), the product with Wuv (``w_v`` [H, V, C]) and the
+    gate (float32 [tokens, H] or None) in one launch; out [tokens, H V] bf16."""
+    assert w_v.dtype == out.dtype == torch.bfloat16 and tuple(w_v.shape) == (H, V, C) and w_v.is_contiguous()
+    assert out.shape[1] == H * V and out.stride(1) == 1 and (gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1))
+    _check(lib().infero_latent_result_few(_ptr(o_lat), c_longlong(o_lat.shape[1]), _ptr(part_o), _ptr(part_ml), c_int(splits), _ptr(sinks_log2),
+                                          _ptr(w_v), _ptr(gate), c_int(gate.stride(0) if gate is not None else 0), _ptr(out),
+                                          c_int(out.stride(0)), c_int(n_tokens), c_int(H), c_int(D), c_int(C), c_int(V), _stream()))
+
+
 def grouped_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Can the tcgen05 grouped product take a [H, rows, K] x w [H, N, K]?"""
     from .tc_gemm import supported

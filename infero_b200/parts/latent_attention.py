@@ -148,6 +148,19 @@ class LatentAttention(Mixer):
         """Tokens 0 .. n - 1 against the latent rows where they lie, the up-projections carried to the query side."""
         H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
         dt, dev = kv.k.dtype, proj.device
+        if self.up_k_t.dtype == self.up_v.dtype == torch.bfloat16 and A.few_ok(ctx, kv.k, n, D, R, C):
+            from ..kernels import latent_mma
+            q_lat = torch.empty((H, n, C), dtype=torch.float32, device=dev)
+            q_rot = torch.empty((H, n, R), dtype=torch.float32, device=dev)
+            freq = self.rope.inv_freq64(dev) if self.rope is not None else None
+            A.query_few(proj[:n], self.q_off, self.kv_off, self.latent_norm, self.spec.norm_eps, freq, self.pairing, self.amp,
+                        ctx.positions[:n], ctx.tok_entry[:n], table, kv.k, kv.page_size, self.up_k_t, q_lat, q_rot, n, H, D, R, C,
+                        write_cache=slot.write_cache, q_src=None if q_src is None else q_src[:n])
+            o_lat = torch.empty((H, n, C), dtype=dt, device=dev)
+            parts = latent_mma.single(ctx, q_lat, q_rot, o_lat, kv, table, n, H, C, R, self.spec.scale, self.spec.window, self.sinks_log2,
+                                      merge=False)
+            A.result_few(o_lat, *parts, self.sinks_log2, self.up_v, self._gate(proj, 0, n), attn[:n], n, H, D, C, V)
+            return
         # whole 128-row tiles per head where the grouped tensor-core product runs
         rows = -(-n // A.TILE) * A.TILE if (dt == torch.bfloat16 and D % 8 == 0 and C % 8 == 0) else n
         q_plain, q_rot = self._prepare(ctx, A, proj, q_src, kv, table, slot, 0, n, rows, False)

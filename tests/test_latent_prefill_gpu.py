@@ -85,3 +85,33 @@ def test_one_requests_infinities_stay_its_own():
     h = torch.randn(70, a.d, generator=g).to(torch.bfloat16).float()
     got = a.step([("x", h), ("y", torch.full((64, a.d), float("inf")))])
     assert _rel(got["x"], a.plain(h)) < TOL and not bool(torch.isfinite(got["y"]).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,D,R,V,C", [(16, 128, 64, 128, 512), (3, 96, 16, 20, 64), (5, 32, 0, 72, 256)])
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17])
+def test_few_single_tokens_in_two_launches(H, D, R, V, C, n, monkeypatch):
+    """Steps of 1 to 17 single tokens behind prefixes of 3 to 200 tokens: 16 and fewer without the grouped products, 17 with them; against
+    64 bits and, where both can run, no further from it."""
+    from test_gositar_gpu import _Latent, _rel
+    from infero_b200.kernels import latent_attention as A, tc_gemm
+    g = torch.Generator().manual_seed(n + D)
+    lens = [3 + (197 * i) // max(1, n - 1) for i in range(n)]
+    a = None
+    calls = []
+    real = A.query_few
+    monkeypatch.setattr(A, "query_few", lambda *x, **k: (calls.append(1), real(*x, **k))[1])
+    for few in (True, False):
+        a = _Latent("bfloat16", H, D, R, V, C, gated=H != 3, pairing="half", seed=H, pages=16 * n + 16, scale=3.0 / (max(64, H * V) * C * (D + R)) ** 0.5)
+        if few:
+            hs = [torch.randn(m + 2, a.d, generator=g).to(torch.bfloat16).float() for m in lens]
+            want = torch.cat([a.plain(h)[-2:] for h in hs])
+        else:
+            monkeypatch.setattr(A, "few_ok", lambda *x: False)
+        for i, h in enumerate(hs):
+            a.step([(i, h[:-2])])
+        calls.clear()
+        got = [a.step([(i, h[h.shape[0] - 2 + k:h.shape[0] - 1 + k]) for i, h in enumerate(hs)]) for k in range(2)]
+        assert len(calls) == (2 if few and n <= 16 else 0) and tc_gemm.error_flag() == 0
+        out = torch.cat([torch.cat([got[0][i], got[1][i]]) for i in range(n)])
+        assert _rel(out, want) < TOL, few
