@@ -212,6 +212,7 @@ struct Share { int token, split, splits, keys, first; };          // which token
 __device__ __forceinline__ Share share_out(const int* __restrict__ positions, int n_tok, int chunk, int window, int id, int budget, int lane) {
     constexpr int PER = BALANCED_TOKENS / 32;
     const int per = (n_tok + 31) / 32;                   // a lane has `per` neighbouring tokens
+    const int cover = budget / n_tok * chunk;            // (what the plan covers, in a token's keys)
     int vis[PER], longest = 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -219,7 +220,7 @@ __device__ __forceinline__ Share share_out(const int* __restrict__ positions, in
         vis[i] = 0;
         if (i < per && t < n_tok) {
             const int pos = positions[t], lo = window > 0 ? max(0, pos - window + 1) : 0;
-            vis[i] = pos + 1 - lo / KEYS16 * KEYS16;
+            vis[i] = min(cover, pos + 1 - lo / KEYS16 * KEYS16);
             longest = max(longest, vis[i]);
         }
     }
