@@ -370,7 +370,11 @@ int launch_one(const float* q_lat, const float* q_rot, long long head_rows, bf16
         }
     }
     const dim3 grid(n_tiles, (H + HC - 1) / HC, splits);
-    launch_pdl(kern, grid, dim3(ROWG * NW * 32), sh, stream, q_lat, q_rot, head_rows, out, part_o, part_ml, cache, block_table, max_blocks,
+    // (a portion's blocks run long: started under the kernel in front, they would crowd on the first free SMs)
+    if (TQ == 1) launch_pdl(kern, grid, dim3(ROWG * NW * 32), sh, stream, q_lat, q_rot, head_rows, out, part_o, part_ml, cache, block_table, max_blocks,
+                                          entry_q_start, entry_q_len, entry_pos0, entry_first, n_entries, TQ, HC, H, R,
+                                          page_size, scale * 1.4426950408889634f, chunk, splits, window, sinks);
+    else kern<<<grid, ROWG * NW * 32, sh, stream>>>(q_lat, q_rot, head_rows, out, part_o, part_ml, cache, block_table, max_blocks,
                                           entry_q_start, entry_q_len, entry_pos0, entry_first, n_entries, TQ, HC, H, R,
                                           page_size, scale * 1.4426950408889634f, chunk, splits, window, sinks);
     return 0;

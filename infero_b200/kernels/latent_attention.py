@@ -48,7 +48,7 @@ def few_ok(ctx, cache: torch.Tensor, n_tokens: int, D: int, R: int, C: int) -> b
     in bf16, in sizes those and the tensor-core attention take."""
     from . import latent_mma
     return (cache.dtype == torch.bfloat16 and n_tokens <= 16 and D % 32 == 0 and D <= 128 and latent_mma.ENABLED
-            and getattr(ctx, "h_q_len", None) is not None and len(ctx.h_q_len) >= n_tokens and bool((ctx.h_q_len[:n_tokens] == 1).all())
+            and getattr(ctx, "h_q_len", None) is not None and len(ctx.h_q_len) >= n_tokens and all(int(n) == 1 for n in ctx.h_q_len[:n_tokens])
             and latent_mma.supported(C, R))
 
 
