@@ -7,12 +7,13 @@
 //   * one elected thread issues tcgen05.mma (M=128, N=BN, K=16) four times per stage; the
 //     accumulator lives in tensor memory (128 lanes x BN 32-bit columns);
 //   * tcgen05.commit hands finished stages back to the loader and the finished accumulator
-//     to four epilogue warps, which read it with tcgen05.ld and write the result.
-// Warp roles: 0 loads, 1 owns TMEM and issues MMAs, 2..5 run the epilogue.
+//     to the epilogue warps, which read it with tcgen05.ld and write the result.
+// Warp roles: 0 loads, 1 owns TMEM and issues MMAs, the others run the epilogue (four; sixteen in
+// the persistent kernels for many tokens).
 //
 // Which matrix is "A" is the launcher's choice:
 //   many tokens (M > 256): A = activations, B = weights; an epilogue thread owns one token
-//     row and writes BN consecutive features (ROW mode).
+//     row, and a warp's rows are written side by side (ROW mode).
 //   few tokens (decode, small chunks): A = weights, B = activations, so that the 128-wide
 //     side of the MMA is always full and the token side is as narrow as 16.  The CTAs then
 //     number N/128 x splits of K, enough to keep every SM streaming weights; with more than
