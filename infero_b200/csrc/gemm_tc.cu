@@ -489,6 +489,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, 
         const int rb = b0 + c0;
         if (rb >= col_end) break;                        // uniform over the warp
         float v[32];
+        __syncwarp();                                    // (lanes part where they store the block before; tcgen05.ld wants them together)
         {
             uint32_t u[32];
             tmem_ld32_nowait(lane_addr + (uint32_t)c0, u);

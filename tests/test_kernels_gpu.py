@@ -179,6 +179,29 @@ def test_many_token_rows_stored_wide_and_narrow(M, N, K, kind, cta_pairs):
     assert float((got[0].double() - ref).abs().max() / ref.abs().max()) <= tol
 
 
+@pytest.mark.parametrize("kind", ["f32", "bf16", "swiglu"])
+@pytest.mark.parametrize("M", [257, 271, 287, 511])
+def test_ragged_rows_of_the_widest_tiles(M, kind, cta_pairs, monkeypatch):
+    """Tiles of 256 columns, of which a warp drains two blocks: its lanes part at the first block's stores (rows past the last one
+    have none, stored element by element above all) and have to be together again for the second one's load."""
+    from infero_b200.kernels import tc_gemm
+    monkeypatch.setenv("INFERO_GEMM_TILE_N", "256")
+    N, K = 536, 72
+    a, w = _rand((M, K), torch.bfloat16, 1), _rand((N, K), torch.bfloat16, 2, 0.1)
+    n = N // 2 if kind == "swiglu" else N
+    y = a.double() @ w.double().T
+    ref = y[:, 0::2] * torch.sigmoid(y[:, 0::2]) * y[:, 1::2] if kind == "swiglu" else y
+    for pad, at in ((8, 0), (3, 1)):
+        out = torch.full((M, n + pad), 7.0, dtype=torch.float32 if kind == "f32" else torch.bfloat16, device=DEV)[:, at:at + n]
+        if kind == "swiglu":
+            assert tc_gemm.gemm_act(a, w, out, kind)
+        else:
+            tc_gemm.gemm(a, w, None, out)
+        # (32-bit sums of 72 products; bf16 rounds to 2^-9)
+        assert float((out.double() - ref).abs().max() / ref.abs().max()) <= (1e-5 if kind == "f32" else 6e-3)
+    assert tc_gemm.error_flag() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 3584, 18944), (1, 3584, 3584), (64, 896, 4864), (200, 1000, 2048), (5, 128, 320),
                                    (16, 256, 616), (33, 130, 1024)])
 @pytest.mark.parametrize("with_bias", [False, True])
