@@ -47,7 +47,7 @@ struct GenericArgs {
     const float* rel;
     const float* sinks;
     int q_stride, out_stride, max_blocks, n_tokens, n_heads, n_kv, head_dim, value_dim, page_size, window, sink, rel_len, cross;
-    int tokens_per_block, head_chunks;
+    int tokens_per_block, head_chunks, tiles;            // tiles: blocks of one kv head
     float scale, softcap;
 };
 
@@ -92,8 +92,9 @@ attention_generic_kernel(const GenericArgs a) {
     float* p_s = v_s + STAGES * CHUNK * vs + n_warps * R * D4 + warp * R * CHUNK;
     unsigned int* here = reinterpret_cast<unsigned int*>(v_s + STAGES * CHUNK * vs + n_warps * R * (D4 + CHUNK));   // a bit per key
     const int group = a.n_heads / a.n_kv;
-    const int kvh = a.cross ? blockIdx.y / a.n_kv : blockIdx.y, vh = a.cross ? blockIdx.y % a.n_kv : kvh;
-    const int t0 = blockIdx.x / a.head_chunks * a.tokens_per_block, g0 = blockIdx.x % a.head_chunks * (n_warps * R);
+    const int side = blockIdx.x / a.tiles, tile = blockIdx.x % a.tiles;
+    const int kvh = a.cross ? side / a.n_kv : side, vh = a.cross ? side % a.n_kv : kvh;
+    const int t0 = tile / a.head_chunks * a.tokens_per_block, g0 = tile % a.head_chunks * (n_warps * R);
     const int t1 = min(a.n_tokens, t0 + a.tokens_per_block);
     const int heads = a.head_chunks > 1 ? min(group - g0, n_warps * R) : group;
 
@@ -261,7 +262,7 @@ attention_generic_kernel(const GenericArgs a) {
 }
 
 template <typename T, typename TO, int R, int COLS, bool VEC, int STAGES>
-int launch(const GenericArgs& a, int warps, cudaStream_t stream) {
+int launch(GenericArgs& a, int warps, cudaStream_t stream) {
     auto* kernel = attention_generic_kernel<T, TO, R, COLS, VEC, STAGES>;
     const size_t smem = generic_smem(a.head_dim, a.value_dim, warps * R, STAGES);
     if (smem > 48 * 1024) {
@@ -269,7 +270,10 @@ int launch(const GenericArgs& a, int warps, cudaStream_t stream) {
         INFERO_REQUIRE(e == cudaSuccess, "attention: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
     const long long tiles = (long long)((a.n_tokens + a.tokens_per_block - 1) / a.tokens_per_block) * a.head_chunks;
-    kernel<<<dim3((unsigned)tiles, a.cross ? a.n_kv * a.n_kv : a.n_kv), warps * 32, smem, stream>>>(a);
+    const long long blocks = tiles * a.n_kv * (a.cross ? a.n_kv : 1);
+    INFERO_REQUIRE(blocks < (1ll << 31), "attention: %d tokens of %d kv heads are too many for one launch", a.n_tokens, a.n_kv);
+    a.tiles = (int)tiles;
+    kernel<<<(unsigned)blocks, warps * 32, smem, stream>>>(a);
     return infero_check_launch("attention_generic");
 }
 
@@ -313,7 +317,6 @@ int infero_attention_generic_rel(const void* q, int q_stride, void* out, int out
     INFERO_REQUIRE(value_dim >= 1 && value_dim <= MAX_D, "attention: value width %d outside 1..%d", value_dim, MAX_D);
     INFERO_REQUIRE(n_kv > 0 && n_heads % n_kv == 0, "attention: %d heads not a multiple of %d kv heads", n_heads, n_kv);
     INFERO_REQUIRE(!rel || rel_len >= 1, "attention: an empty table of distances");
-    INFERO_REQUIRE((long long)n_kv * (cross ? n_kv : 1) <= 65535, "attention: %d kv heads are too many", n_kv);
     GenericArgs a;
     a.q = q, a.out = out, a.k_cache = k_cache, a.v_cache = v_cache, a.block_table = block_table, a.tok_entry = tok_entry;
     a.positions = positions, a.slopes = slopes, a.rel = rel, a.sinks = sinks, a.q_stride = q_stride, a.out_stride = out_stride;

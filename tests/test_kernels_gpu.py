@@ -1124,3 +1124,19 @@ def test_attention_generic_gives_the_same_bits_however_the_step_is_cut(H, Hkv, D
             ref = torch.softmax(kk @ q[t, h * D:(h + 1) * D].cpu().double() * D ** -0.5, 0) @ vv
             # scores and weights in 32-bit: D + keys roundings of 2^-24 in front of an exponential of scores of a few units
             assert float((full[t, h * V:(h + 1) * V].cpu().double() - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max()))
+
+
+def test_attention_generic_of_very_many_kv_heads():
+    """256 kv heads whose every head's weights meet every kv head's values: 65,536 pairs of them."""
+    from infero_b200 import kernels as Kn
+    G, D, page, n = 256, 4, 16, 2
+    k, v = _rand((1, G, page, D), torch.float32, 1), _rand((1, G, page, D), torch.float32, 2)
+    q = _rand((n, G * D), torch.float32, 3)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)               # noqa: E731
+    out = torch.full((n, G * G * D), float("nan"), dtype=torch.float32, device=DEV)
+    Kn.attention_generic(q, out, k, v, i32([[0]]), i32([0, 0]), i32([5, 6]), G, G, D, page, None, 0.5, cross=True)
+    for t, last in ((0, 5), (1, 6)):
+        kk, vv = k[0, :, :last + 1].double(), v[0, :, :last + 1].double()
+        w = torch.softmax(torch.einsum("hd,hjd->hj", q[t].double().view(G, D), kk) * 0.5, -1)
+        ref = torch.einsum("hj,cjd->chd", w, vv)
+        assert float((out[t].double().view(G, G, D) - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
