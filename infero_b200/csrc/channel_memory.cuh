@@ -20,7 +20,8 @@
 // follow by forward substitution from the products in the table, the lanes shared out among the columns (a lane keeps its columns
 // in an order of its own, the one that it ends up with first, so that the exchanges need no selection).  A helper warp brings
 // the stages in, two ahead.  Groups are counted from a request's own first new token: a token's arithmetic does not depend on the
-// batch, nor beyond rounding on how its prompt was cut.  Steps of single tokens run the same code in groups of one.
+// batch (beyond rounding in bf16 steps, where the step decides which portions run in segments: outer_memory.cuh), nor beyond
+// rounding on how its prompt was cut.  Steps of single tokens run the same code in groups of one.
 #pragma once
 #include "outer_memory.cuh"
 #include "tc_common.cuh"

@@ -55,6 +55,7 @@ template <int N, int L> struct Scattered {
 // portion alone leaves a scan one or two warps a scheduler and the latency of its chain of tokens: two layers of 16 heads of
 // 128 x 128 over 2,047 tokens 482 us whole, 360 in segments of 256; a model's pass over them 2.26 and 2.14 ms, over 1,201 + 37 + 500
 // tokens 2.09 and 1.96.  Portions beside one another fill the schedulers by themselves (four of 512: 1.79 ms whole, 1.91 cut).
+// Which portions are cut is therefore decided by the whole step, and only in bf16: a cut changes the rounding.
 struct Segments {
     int len;                 // tokens of a segment (a multiple of the stages' tokens); 0: portions run whole
     float* starts;           // [segments of the requests that have more than one][heads, columns, K]

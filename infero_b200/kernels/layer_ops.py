@@ -767,7 +767,7 @@ def _segments(lens, H: int, V: int, K: int, device):
     """(tokens of a segment or 0, segments in all, scratch for their starts and their decays) of a step whose requests bring
     ``lens`` tokens (host numbers; None: not known, portions run whole).  Portions are cut where one of four segments and more
     brings at least half of the step's tokens (csrc/outer_memory.cuh has both sides' times)."""
-    if lens is None or max(lens) < 4 * SEGMENT or 2 * int(max(lens)) < sum(int(n) for n in lens) or V * K > 65535 * 256:
+    if lens is None or not len(lens) or max(lens) < 4 * SEGMENT or 2 * int(max(lens)) < sum(int(n) for n in lens) or V * K > 65535 * 256:
         return 0, 0, None, None
     counts = [-(-int(n) // SEGMENT) if n > SEGMENT else 1 for n in lens]
     slots = sum(c for c in counts if c > 1)

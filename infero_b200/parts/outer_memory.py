@@ -303,7 +303,10 @@ class DecayedMemory(_ChannelDecayed):
         H, K, V, o = self.H, self.K, self.V, self.off
         rec = L.decayed_records(self._narrow(proj, off, "decay_down"), self.decay_up, self.decay_bias, float(self.spec.decay_tau), proj,
                                 off + o["q"], off + o["k"], H, K)
+        # which portions run in segments depends on the whole step, and a cut changes the rounding: never on the 32-bit path, where a
+        # request's numbers are the same whoever shares its steps
+        lens = getattr(ctx, "h_q_len", None) if out.dtype == torch.bfloat16 else None
         y = L.decayed_scan(proj[:, off + o["v"]:off + o["v"] + H * V], rec, ctx.state(slot.cache), 0, ctx.entry_q_start, ctx.entry_q_len,
-                           ctx.entry_slot, ctx.n_entries, H, K, V, single_tokens(ctx), getattr(ctx, "h_q_len", None))
+                           ctx.entry_slot, ctx.n_entries, H, K, V, single_tokens(ctx), lens)
         L.memory_finish(y, None, proj[:, off + o["gate"]:off + o["gate"] + H * V], "silu", self.norm_w, float(self.spec.norm_eps), out,
                         H, V, scale)

@@ -9,7 +9,7 @@ DEV = "cuda:0"
 
 def test_which_portions_are_cut():
     cut = lambda lens: L._segments(lens, 2, 4, 8, "cpu")[:2]                      # noqa: E731
-    assert cut(None) == cut([1023]) == (0, 0) and cut([1024]) == (256, 4) and cut([3, 1201, 257, 256]) == (256, 1 + 5 + 2 + 1)
+    assert cut(None) == cut([]) == cut([1023]) == (0, 0) and cut([1024]) == (256, 4) and cut([3, 1201, 257, 256]) == (256, 1 + 5 + 2 + 1)
     assert cut([1200, 1300]) == (256, 5 + 6) and cut([1100, 600, 600]) == (0, 0)
     starts, totals = L._segments([3, 1201, 257, 256], 2, 4, 8, "cpu")[2:]
     assert tuple(starts.shape) == (7, 2, 4, 8) and tuple(totals.shape) == (7, 2, 8)
@@ -19,7 +19,6 @@ def test_which_portions_are_cut():
 @pytest.mark.parametrize("K,V", [(128, 128), (64, 36), (32, 5), (20, 16), (200, 8)])
 def test_segments_against_whole_portions_and_64_bits(K, V, monkeypatch):
     """Portions around multiples of a segment, beside short ones, from states of their own: read-outs and the states left."""
-    monkeypatch.setattr(L, "_segments", L._segments)
     H, lens = 2, [1, 49, 32, 0, 127, 33]
     T, E = sum(lens), len(lens)
     g = torch.Generator().manual_seed(K)

@@ -545,12 +545,13 @@ def test_mixed_batches_with_slots_and_pages_used_again(name, dtype):
     assert runner.manager.pages_reused > 0
 
 
-def test_a_batch_equals_each_request_alone_bitwise_in_32_bit():
+@pytest.mark.parametrize("lens", [[50, 21, 37], [1100, 600, 600], [1100, 300]])       # (alone, 1,100 tokens are most of their step)
+def test_a_batch_equals_each_request_alone_bitwise_in_32_bit(lens):
     mdir = model_dir("A")
-    reqs = make_requests("A", [50, 21, 37], seed=9)
-    together = R.replay_inprocess(make_runner(mdir, "float32", 256, max_seqs=3), [
+    reqs = make_requests("A", lens, seed=9)
+    together = R.replay_inprocess(make_runner(mdir, "float32", max(256, sum(lens) + 48), max_seqs=3), [
         {"step": 0, "entries": [{"id": r, "tokens": t, "want": list(range(len(t)))} for r, t in reqs.items()], "end": list(reqs)}])
-    alone = R.replay_inprocess(make_runner(mdir, "float32", 256, max_seqs=3), R.steps_whole(reqs))
+    alone = R.replay_inprocess(make_runner(mdir, "float32", max(256, sum(lens) + 48), max_seqs=3), R.steps_whole(reqs))
     assert together.keys() == alone.keys()
     for k in alone:
         assert np.array_equal(together[k], alone[k]), k
