@@ -38,13 +38,14 @@ __device__ __forceinline__ float2 turn(double ang, float amp) {
     return make_float2(c * amp, s * amp);
 }
 
-// element i of a rotated part: what it becomes with the token's cosines and sines
-__device__ __forceinline__ float rotated(const float* __restrict__ part, int i, int rot, int pairing, const float2* cs) {
+// element i of a rotated part: what it becomes with the token's cosines and sines, cs(pair)
+template <typename CS>
+__device__ __forceinline__ float rotated(const float* __restrict__ part, int i, int rot, int pairing, CS cs) {
     if (i >= rot) return part[i];
     int ia, ib;
     if (pairing) ia = i & ~1, ib = ia + 1;
     else ia = i < rot / 2 ? i : i - rot / 2, ib = ia + rot / 2;
-    const float2 t = cs[pairing ? i >> 1 : ia];
+    const float2 t = cs(pairing ? i >> 1 : ia);
     const float a = part[ia], b = part[ib];
     return i == ia ? a * t.x - b * t.y : b * t.x + a * t.y;
 }
@@ -53,8 +54,10 @@ __device__ __forceinline__ float rotated(const float* __restrict__ part, int i, 
 constexpr int ROT_BLOCK = 64;
 
 // A token's cosines and sines are the same for all its heads and for the key part, and their 64-bit angles are most of the
-// work, so a block makes them once, into shared memory (2,048 tokens of 16 heads of 128 + 64: 30 us an element at a time, 24 from the table).
-template <typename T>
+// work, so a block makes them once, into shared memory (2,048 tokens of 16 heads of 128 + 64: 30 us an element at a time, 24 from the
+// table).  TABLE off: more of them than fit there, made where they are used.
+constexpr int MAX_TABLE = 4096;
+template <typename T, bool TABLE>
 __global__ void __launch_bounds__(PREP_THREADS)
 latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ q_src, int q_stride,
                       int q_off, int kv_off,
@@ -65,14 +68,17 @@ latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, const flo
                       long long head_rows, int H, int D, int R, int C, int heads_per_block) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float2 cs[];                       // [rot / 2]: amp * (cos, sin)
+    extern __shared__ float2 table[];                    // [rot / 2]: amp * (cos, sin)
     __shared__ float red[32];
     const int t = blockIdx.x;
     const float* row = proj + (size_t)t * proj_stride;
     const int pos = positions[t];
     if (blockIdx.y == 0 && !write_cache) return;
-    for (int i = threadIdx.x; i < rot / 2; i += blockDim.x) cs[i] = turn((double)pos * freq[i], amp);
-    __syncthreads();
+    if (TABLE) {
+        for (int i = threadIdx.x; i < rot / 2; i += blockDim.x) table[i] = turn((double)pos * freq[i], amp);
+        __syncthreads();
+    }
+    auto cs = [&](int pair) { return TABLE ? table[pair] : turn((double)pos * freq[pair], amp); };
     if (blockIdx.y == 0) {
         // the latent row
         const float* kv = row + kv_off;
@@ -210,7 +216,7 @@ latent_query_few_kernel(const float* __restrict__ proj, int proj_stride, const f
                         const int* __restrict__ block_table, int max_blocks, int page_size, bf16* __restrict__ cache, int write_cache,
                         const bf16* __restrict__ w_k, float* __restrict__ q_lat, float* __restrict__ q_rot, long long head_rows,
                         int T, int H, int D, int R, int C) {
-    extern __shared__ float2 cs[];                       // a latent row: [rot / 2]
+    extern __shared__ float2 table[];                    // a latent row: [rot / 2]
     __shared__ __align__(16) bf16 qs[8 * OCT][FEW_MAX_D + 8];
     __shared__ float red[32];
     pdl_launch_dependents();
@@ -219,8 +225,9 @@ latent_query_few_kernel(const float* __restrict__ proj, int proj_stride, const f
         pdl_wait();
         if (!write_cache) return;
         const int t = blockIdx.x, pos = positions[t];
-        for (int i = tid; i < rot / 2; i += blockDim.x) cs[i] = turn((double)pos * freq[i], amp);
+        for (int i = tid; i < rot / 2; i += blockDim.x) table[i] = turn((double)pos * freq[i], amp);
         __syncthreads();
+        auto cs = [&](int pair) { return table[pair]; };
         const float* kv = proj + (size_t)t * proj_stride + kv_off;
         float sq = 0.f;
         for (int i = tid; i < C; i += blockDim.x) sq = fmaf(kv[i], kv[i], sq);
@@ -387,21 +394,26 @@ int infero_latent_prepare_from(const float* proj, int proj_stride, const float* 
                           void* q_plain, float* q_rot, void* q_rot_block, long long head_rows, int n_tokens, int H, int D,
                           int R, int C, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
-    INFERO_REQUIRE(rot <= 8192 && (!q_rot_block || R <= ROT_BLOCK), "latent attention: a rotated part of %d (%d turned)", R, rot);
+    INFERO_REQUIRE(!q_rot_block || R <= ROT_BLOCK, "latent attention: a rotated part of %d in one block of %d", R, ROT_BLOCK);
     INFERO_REQUIRE(rot >= 0 && rot <= R && rot % 2 == 0, "latent attention: %d rotated coordinates of %d", rot, R);
     INFERO_REQUIRE(head_rows >= n_tokens, "latent attention: %lld rows per head for %d tokens", head_rows, n_tokens);
     // one block for a token's latent row, and one per group of heads (all heads in one block where tokens alone fill
     // the multiprocessors)
     const int heads_per_block = n_tokens >= 512 ? H : max(1, H / 8);
     const dim3 grid(n_tokens, 1 + (H + heads_per_block - 1) / heads_per_block);
-    if (dtype == INFERO_F32)
-        launch_pdl(latent_prepare_kernel<float>, grid, dim3(PREP_THREADS), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
-            rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (float*)cache, write_cache,
-            (float*)q_plain, q_rot, (float*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
-    else
-        launch_pdl(latent_prepare_kernel<bf16>, grid, dim3(PREP_THREADS), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, kv_off, norm_w, eps, freq,
-            rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size, (bf16*)cache, write_cache,
-            (bf16*)q_plain, q_rot, (bf16*)q_rot_block, head_rows, H, D, R, C, heads_per_block);
+    const bool table = rot / 2 <= MAX_TABLE;
+#define PREPARE(T_, TABLE_)                                                                                                              \
+    launch_pdl(latent_prepare_kernel<T_, TABLE_>, grid, dim3(PREP_THREADS), TABLE_ ? rot / 2 * sizeof(float2) : 0, stream, proj, proj_stride, \
+               q_src, q_stride, q_off, kv_off, norm_w, eps, freq, rot, pairing, amp, positions, tok_entry, block_table, max_blocks, page_size,  \
+               (T_*)cache, write_cache, (T_*)q_plain, q_rot, (T_*)q_rot_block, head_rows, H, D, R, C, heads_per_block)
+    if (dtype == INFERO_F32) {
+        if (table) PREPARE(float, true);
+        else PREPARE(float, false);
+    } else {
+        if (table) PREPARE(bf16, true);
+        else PREPARE(bf16, false);
+    }
+#undef PREPARE
     return infero_check_launch("latent_prepare");
 }
 
@@ -462,7 +474,7 @@ int infero_latent_query_few(const float* proj, int proj_stride, const float* q_s
                             cudaStream_t stream) {
     INFERO_REQUIRE(infero_latent_few_supported(n_tokens, D, C) && (reinterpret_cast<uintptr_t>(w_k) & 15u) == 0,
                    "latent_query_few: %d tokens, %d x %d, not supported", n_tokens, D, C);
-    INFERO_REQUIRE(rot >= 0 && rot <= R && rot % 2 == 0 && rot <= 8192 && head_rows >= n_tokens, "latent attention: %d rotated coordinates of %d", rot, R);
+    INFERO_REQUIRE(rot >= 0 && rot <= R && rot % 2 == 0 && rot / 2 <= MAX_TABLE && head_rows >= n_tokens, "latent attention: %d rotated coordinates of %d", rot, R);
     const dim3 grid(n_tokens + H * (C / FEW_COLS + 1));
 #define GO(O_)                                                                                                                      \
     launch_pdl(latent_query_few_kernel<O_>, grid, dim3(128), rot / 2 * sizeof(float2), stream, proj, proj_stride, q_src, q_stride, q_off, \

@@ -156,6 +156,30 @@ def test_rotary_tables_on_the_device_and_both_pairings():
             assert _rel(got[C:], PG.rotate(row[t:t + 1, C:].unsqueeze(1), torch.tensor([p]), freqs, amp, pairing)[0, 0]) < 2e-6
 
 
+@pytest.mark.parametrize("dims", [8190, 8192, 8194, 8260])
+def test_rotated_parts_around_what_a_table_of_sines_holds(dims):
+    """The prepare kernel keeps up to 4,096 pairs' sines of a token in shared memory and works out wider ones where they are used."""
+    from infero_b200.config.spec import PositionSpec
+    from infero_b200.kernels import latent_attention as A
+    from infero_b200.parts.rope import RopeNeox
+    g = torch.Generator().manual_seed(dims)
+    H, D, R, C, page, pos = 2, 3, dims + 6, 5, 16, [3, 1000]
+    rope = RopeNeox(PositionSpec("x", 500.0, dims))
+    freqs, amp = PG.rotary_table(dims, 500.0, None)
+    T = len(pos)
+    proj = torch.randn(T, H * (D + R) + C + R, generator=g)
+    cache, table = torch.zeros(T, 1, page, C + R, device=DEV), torch.zeros(T, 1000 // page + 1, dtype=torch.int32)
+    table[1] = 1
+    q_plain, q_rot = torch.empty(H, T, D, device=DEV), torch.empty(H, T, R, device=DEV)
+    A.prepare(proj.to(DEV), 0, H * (D + R), torch.ones(C, device=DEV), 1e-5, rope.inv_freq64(DEV), "half", rope.amplitude, _i32(pos), _i32(range(T)),
+              table.to(DEV), cache, page, q_plain, q_rot, T, H, D, R, C)
+    q = proj[:, :H * (D + R)].double().view(T, H, D + R)
+    assert _rel(q_rot.permute(1, 0, 2), PG.rotate(q[..., D:], torch.tensor(pos), freqs, amp, "half")) < 2e-6
+    for t, p in enumerate(pos):
+        want = PG.rotate(proj[t:t + 1, H * (D + R) + C:].double().unsqueeze(1), torch.tensor([p]), freqs, amp, "half")[0, 0]
+        assert _rel(cache[t, 0, p % page, C:].cpu(), want) < 2e-6
+
+
 @pytest.mark.parametrize("E,top,groups,keep", [(8, 3, 4, 2), (6, 3, 3, 2), (16, 5, 4, 3), (5, 5, 1, 1), (12, 1, 6, 1), (9, 2, 3, 3), (64, 8, 8, 4), (8, 2, 4, 2)])
 def test_routing_with_groups_and_a_correction(E, top, groups, keep):
     """Choice and weights against the plain statement.  The corrections are large and mostly negative, so pick scores
