@@ -472,7 +472,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // four warps, 36 with eight, 25 with sixteen; 1738 x 12800 x 2048 to 32-bit: 107 us before, 82 now (cuBLAS to bf16: 78).
 constexpr int DRAIN_WARPS = 16, MANY_THREADS = 64 + 32 * DRAIN_WARPS, DRAIN_STAGE = 32 * 64;
 
-// One warp's share of a finished accumulator: its 32 rows (TMEM lanes at lane_addr, result rows from row0) in every second
+// One warp's share of a finished accumulator: its 32 rows (TMEM lanes at lane_addr, result rows from row0) in every fourth
 // block of 32 of the BN columns that start at feature b0, written as the epilogue EPI says.
 template <int EPI, typename OutT>
 __device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, int row0, int lane, uint8_t* stage, int b0, int BN,
@@ -514,10 +514,10 @@ __device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, 
         const int cols = min(32, col_end - rb), first = GLU ? rb >> 1 : rb, n = GLU ? cols >> 1 : cols;
         uint8_t* dst = reinterpret_cast<uint8_t*>(out + first) + (size_t)row0 * pitch;
         // (first is a multiple of 16 elements, or of 8 of bf16 behind a gated unit: pieces of 16 bytes start aligned)
-        if (wide && sizeof(OutT) == 4 && (cols == 32 || cols == 16)) {
+        if (wide && sizeof(OutT) == 4 && (n == 32 || n == 16)) {
             const uint4* f = reinterpret_cast<const uint4*>(v);
             store_rows<4>(stage, f, dst, pitch, rows, lane);
-            if (cols == 32) store_rows<4>(stage, f + 4, dst + 64, pitch, rows, lane);
+            if (n == 32) store_rows<4>(stage, f + 4, dst + 64, pitch, rows, lane);
         } else if (wide && sizeof(OutT) == 2 && (cols == 32 || (cols == 16 && !GLU))) {
             uint4 pk[4];
 #pragma unroll
