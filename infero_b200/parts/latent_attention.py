@@ -148,7 +148,7 @@ class LatentAttention(Mixer):
         """Tokens 0 .. n - 1 against the latent rows where they lie, the up-projections carried to the query side."""
         H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
         dt, dev = kv.k.dtype, proj.device
-        if self.up_k_t.dtype == self.up_v.dtype == torch.bfloat16 and A.few_ok(ctx, kv.k, n, D, R, C):
+        if A.few_ok(ctx, kv.k, n, D, R, C, self.up_k_t, self.up_v):
             from ..kernels import latent_mma
             q_lat = torch.empty((H, n, C), dtype=torch.float32, device=dev)
             q_rot = torch.empty((H, n, R), dtype=torch.float32, device=dev)

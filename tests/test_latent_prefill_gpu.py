@@ -115,3 +115,23 @@ def test_few_single_tokens_in_two_launches(H, D, R, V, C, n, monkeypatch):
         assert len(calls) == (2 if few and n <= 16 else 0) and tc_gemm.error_flag() == 0
         out = torch.cat([torch.cat([got[0][i], got[1][i]]) for i in range(n)])
         assert _rel(out, want) < TOL, few
+
+
+@pytest.mark.gpu
+def test_up_projections_that_start_anywhere():
+    """Values of another width than the keys keep the caller's own projection, here two bytes behind a multiple of 16."""
+    from test_gositar_gpu import DEV, _Latent, _rel
+    a = _Latent("bfloat16", 3, 64, 16, 20, 64, seed=2, scale=0.05, pages=40)
+    bound = {k: v.to(DEV) for k, v in a.w.items()}
+    name = a.part._n("up_v")
+    up_v = bound[name]
+    moved = torch.empty(up_v.numel() + 8, dtype=up_v.dtype, device=DEV)[1:1 + up_v.numel()].view(up_v.shape)
+    assert moved.data_ptr() % 16
+    bound[name] = moved.copy_(up_v)
+    a.part.bind(bound)
+    g = torch.Generator().manual_seed(1)
+    hs = [torch.randn(n + 1, a.d, generator=g).to(torch.bfloat16).float() for n in (5, 30)]
+    first = a.step([(i, h[:-1]) for i, h in enumerate(hs)])
+    last = a.step([(i, h[-1:]) for i, h in enumerate(hs)])
+    for i, h in enumerate(hs):
+        assert _rel(torch.cat([first[i], last[i]]), a.plain(h)) < TOL
