@@ -23,6 +23,7 @@
 #include "tc_common.cuh"
 
 extern "C" int infero_attn_decode_tma_supported(int head_dim, int page_size);
+extern "C" int infero_attn_decode_min_chunk();     // runtime.cu
 
 namespace {
 
@@ -203,13 +204,14 @@ __device__ __forceinline__ void merge_if_last(int* counter, float* wbuf, const f
 }
 
 // Requests of a step seldom have equally many keys, and a plan that cuts every one into as many splits as the longest wants
-// leaves that one's CTAs working long after the others.  SHARED: the grid's n_tok x n_splits CTAs per kv head are shared out by length instead: every token gets ceil(keys / c) of them, c the
-// fewest keys (in sixteens, at least MIN_KEYS and no more than the plan's) for which they suffice; the CTAs left over leave at
-// once.  Every warp works it out for itself from the positions, ahead of the wait for the kernel in front.  64 tokens
-// behind 16 to 2,047 keys, 14 heads of 64 over 2: a step of 24 layers 1.34 ms in equal splits, 1.15 shared out.
-constexpr int BALANCED_TOKENS = 256, BALANCED_SPLITS = 256, MIN_KEYS = 256;       // (the merge keeps a weight per split in shared memory)
+// leaves that one's CTAs working long after the others.  SHARED: the grid's n_tok x n_splits CTAs per kv head are shared out by
+// length instead: every token gets ceil(keys / c) of them, c the fewest keys (in sixteens, at least the plan's least and no more
+// than its chunk) for which they suffice; the CTAs left over leave at once.  Every warp works it out for itself from the
+// positions, ahead of the wait for the kernel in front.  64 tokens behind 16 to 2,047 keys, 14 heads of 64 over 2: a step of 24
+// layers 1.34 ms in equal splits, 1.15 shared out.
+constexpr int BALANCED_TOKENS = 256, BALANCED_SPLITS = 256;       // (the merge keeps a weight per split in shared memory)
 struct Share { int token, split, splits, keys, first; };          // which token and split; splits of the token, keys of a split; CTAs of the tokens before
-__device__ __forceinline__ Share share_out(const int* __restrict__ positions, int n_tok, int chunk, int window, int id, int budget, int lane) {
+__device__ __forceinline__ Share share_out(const int* __restrict__ positions, int n_tok, int chunk, int window, int least, int id, int budget, int lane) {
     constexpr int PER = BALANCED_TOKENS / 32;
     const int per = (n_tok + 31) / 32;                   // a lane has `per` neighbouring tokens
     const int cover = budget / n_tok * chunk;            // (what the plan covers, in a token's keys)
@@ -232,7 +234,7 @@ __device__ __forceinline__ Share share_out(const int* __restrict__ positions, in
             if (i < per) n += (vis[i] + c - 1) / c;
         return n;
     };
-    int hi = chunk, lo = min(chunk, max(MIN_KEYS, (longest / BALANCED_SPLITS + 16) / 16 * 16));
+    int hi = chunk, lo = min(chunk, max((least + 15) / 16 * 16, (longest / BALANCED_SPLITS + 16) / 16 * 16));
     while (lo < hi) {                                    // (hi always suffices; both are multiples of 16)
         const int mid = (lo + hi) / 32 * 16;
         if ((int)__reduce_add_sync(0xffffffffu, (unsigned)wanted(mid)) <= budget) hi = mid;
@@ -284,7 +286,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        int tok_first, int n_heads, int n_kv, int page_size, int window, float scale_log2,
                        int chunk, int n_splits, float* __restrict__ partial_o, float* __restrict__ partial_ml,
                        bf16* __restrict__ out, int out_stride, int* __restrict__ counters,
-                       int* __restrict__ err_flag, const FusedQkv fq, int sink) {
+                       int* __restrict__ err_flag, const FusedQkv fq, int sink, int least) {
     using Plan = TdPlan<D>;
     using Layout = Swizzled128<D, 16>;
     constexpr int STAGES = Plan::STAGES;
@@ -310,7 +312,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     // kernel in front (which writes q and the token's own key and value) has finished
     int split = blockIdx.x, ti = blockIdx.z, splits_before = ti * n_splits;
     if (SHARED) {                                                     // the splits are shared out by length
-        const Share s = share_out(positions + tok_first, (int)gridDim.z, chunk, window, (int)(blockIdx.z * gridDim.x + blockIdx.x),
+        const Share s = share_out(positions + tok_first, (int)gridDim.z, chunk, window, least, (int)(blockIdx.z * gridDim.x + blockIdx.x),
                                   (int)(gridDim.z * gridDim.x), lane);
         if (s.token < 0) return;                                      // (uniform over the block)
         split = s.split, ti = s.token, chunk = s.keys, n_splits = s.splits, splits_before = s.first;
@@ -707,7 +709,7 @@ int launch_tma(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, int 
     dim3 grid(n_splits, n_kv * ((group + 15) / 16) * (fq.ex.cross ? n_kv : 1), n_tok);
     launch_pdl(kern, grid, dim3(TD_THREADS), SMEM, stream, mk, mv, (const bf16*)q, q_stride, block_table,
                max_blocks, tok_entry, positions, tok_first, n_heads, n_kv, page_size, window, scale_log2, chunk,
-               n_splits, po, pml, (bf16*)out, out_stride, counters, err, fq, sink);
+               n_splits, po, pml, (bf16*)out, out_stride, counters, err, fq, sink, infero_attn_decode_min_chunk());
     return infero_check_launch(FUSED ? "attn_decode_tma_fused" : "attn_decode_tma");
 }
 

@@ -65,6 +65,16 @@ int infero_sm_count() {
     return cached[dev];
 }
 
+// Fewest keys per split of decode attention (INFERO_DECODE_MIN_CHUNK).
+int infero_attn_decode_min_chunk() {
+    static int min_chunk = -1;
+    if (min_chunk < 0) {
+        const char* e = getenv("INFERO_DECODE_MIN_CHUNK");
+        min_chunk = e && atoi(e) > 0 ? atoi(e) : 256;
+    }
+    return min_chunk;
+}
+
 // How decode attention cuts the keys of a step into splits: (keys per split, number of splits) such
 // that the splits cover max_visible keys and the grid of n_tok x n_kv x ceil(group / 16) x splits CTAs
 // has about two CTAs per multiprocessor; a split has at least INFERO_DECODE_MIN_CHUNK keys (256) and
@@ -72,11 +82,7 @@ int infero_sm_count() {
 // statement of the plan: the Python parts, the native launcher of a block and the scratch sizing all
 // call this.
 void infero_attn_plan_decode(int n_tok, int n_kv, int group, int max_visible, int sm_count, int* chunk, int* splits) {
-    static int min_chunk = -1;
-    if (min_chunk < 0) {
-        const char* e = getenv("INFERO_DECODE_MIN_CHUNK");
-        min_chunk = e && atoi(e) > 0 ? atoi(e) : 256;
-    }
+    const int min_chunk = infero_attn_decode_min_chunk();
     const int target = 2 * (sm_count > 0 ? sm_count : infero_sm_count()), max_splits = 256;
     const int per_split = n_tok * n_kv * ((group + 15) / 16) > 0 ? n_tok * n_kv * ((group + 15) / 16) : 1;
     const int want = target / per_split > 0 ? target / per_split : 1;

@@ -777,6 +777,34 @@ def test_decode_splits_shared_out_by_length(n, window):
     assert tc_gemm.error_flag() == 0
 
 
+def _decode_with_the_fewest_keys_a_split_has():
+    """Run with INFERO_DECODE_MIN_CHUNK = 1024: splits of 1,024 keys may not be cut further, so tokens that share a call's splits out
+    by length have the bits of the same tokens in calls too small for that."""
+    from infero_b200.kernels import attention as A
+    H, Hkv, D, P, n = 6, 2, 64, 16, 40
+    lengths = [16 + 50 * i for i in range(n)]
+    table, kc, vc, _, _ = _paged_requests(lengths, Hkv, D, P, torch.bfloat16, 3, [0] * n)
+    q = _rand((n, H * D), torch.bfloat16, 7)
+    positions = torch.tensor([L - 1 for L in lengths], dtype=torch.int32, device=DEV)
+    entry, table = torch.arange(n, dtype=torch.int32, device=DEV), table.to(DEV)
+    whole, parts = (torch.zeros((n, H * D), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    A.decode(q, whole, kc, vc, table, entry, positions, 0, n, H, Hkv, D, P, None, 0.2, 1024, 2)
+    for t in range(0, n, 10):
+        A.decode(q, parts, kc, vc, table, entry, positions, t, 10, H, Hkv, D, P, None, 0.2, 1024, 2)
+    assert torch.equal(whole, parts)
+
+
+def test_decode_splits_shared_out_keep_to_the_fewest_keys():
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    run = subprocess.run([sys.executable, "-c", "import test_kernels_gpu as t; t._decode_with_the_fewest_keys_a_split_has()"], text=True,
+                         capture_output=True, timeout=300, cwd=here,
+                         env=dict(os.environ, INFERO_DECODE_MIN_CHUNK="1024", PYTHONPATH=os.path.dirname(here) + os.pathsep + here))
+    assert run.returncode == 0, run.stderr[-2000:]
+
+
 @pytest.mark.parametrize("H,Hkv,D", [(4, 2, 64), (7, 1, 128)])
 @pytest.mark.parametrize("window", [48, 100])
 @pytest.mark.parametrize("P", [16, 64])
