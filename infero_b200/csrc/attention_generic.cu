@@ -17,14 +17,15 @@
 // whole of attention on the 32-bit path and the fallback of the bf16 path.
 //
 // A block has a few neighbouring tokens and the query heads of one kv head: their rows (token, head), R a warp, share the
-// chunks, which are fetched into shared memory ahead of the arithmetic (three with one row a warp, whose chain over the
-// chunks has nothing else to wait for; one with four, where more shared memory would cost blocks: 2.43 against 2.76 ms for
-// 2,048 tokens); a lane looks up its own key's page a chunk before that.  In the scores a lane has a key (rows of keys lie an
-// odd multiple of 16 bytes apart, so lanes read 16 bytes each without bank conflicts), in the sum over values it has every
-// 32nd column.  Tokens of different requests in one block take turns, so steps of few tokens get a block per token.
+// chunks, which are fetched into shared memory a chunk ahead of the arithmetic; a lane looks up its own key's page a chunk before
+// that.  In the scores a lane has a key, in the sum over values it has every 32nd column.  Tokens of different requests in one
+// block take turns, so single tokens and short portions get a block per token, with warps that only fetch where a kv head has
+// fewer query heads than a block wants warps.
 // What bounds it: long prompts the multiply-adds and what feeds them from shared memory, single tokens the chain over the
-// chunks.  32-bit, before (a warp per row reading keys where they lie) and now: 301 tokens with 14 heads of 64 264 -> 68 us,
-// one token at 300 keys 125 -> 33, 64 tokens at 1,000 keys 516 -> 97, 2,048 tokens with 28 heads of 128 30.5 -> 2.4 ms.
+// chunks.  A warp per row reading keys where they lie, and now, in us.  32-bit, 14 heads of 64 over 2: 301 tokens 265 and 64, one token
+// at 300 keys 127 and 24, 64 at 1,000 518 and 68; 16 heads of 64 over 16: 250 single tokens at 1,000 keys 1,248 and 426, 10 of them at
+// 2,000 beside 250 prompt tokens 1,412 and 208; 16 of 128 over 16: 1,500 tokens 9,560 and 742.  bf16, 16 of 36 over 16: 250 single
+// tokens 523 and 308.  (A chunk ahead is enough: two or three ahead made blocks too large, 707 instead of 428 for the 250 of 64.)
 #include "common.cuh"
 #include <math_constants.h>
 
@@ -32,8 +33,9 @@ namespace {
 
 constexpr int WARPS = 8;
 constexpr int MAX_D = 256;
-constexpr int CHUNK = 32;
-constexpr int FEW_TOKENS = 256;         // up to here a block per token, one row a warp; beyond, 32 rows a block
+constexpr int CHUNK = 32, STAGES = 2;
+constexpr int FEW_TOKENS = 256;         // portions of up to so many tokens: a block per token, one row a warp; beyond, 32 rows a block
+constexpr int WIDE_ROWS = WARPS * 4;
 
 struct GenericArgs {
     const void* q;
@@ -47,55 +49,82 @@ struct GenericArgs {
     const float* rel;
     const float* sinks;
     int q_stride, out_stride, max_blocks, n_tokens, n_heads, n_kv, head_dim, value_dim, page_size, window, sink, rel_len, cross;
-    int tokens_per_block, head_chunks, tiles;            // tiles: blocks of one kv head
+    int tokens_per_block, head_chunks, tiles, singles;   // tiles: blocks of one kv head; singles: tokens in front with a block each
     float scale, softcap;
 };
 
+// Elements between rows of keys (an odd multiple of four: lanes read four elements of neighbouring rows each without bank conflicts)
+// and of values.
 __host__ __device__ inline int key_stride(int head_dim) { return (((head_dim + 3) / 4) | 1) * 4; }
 __host__ __device__ inline int value_stride(int value_dim) { return (value_dim + 3) / 4 * 4; }
 
-inline size_t generic_smem(int head_dim, int value_dim, int rows, int stages) {
-    return ((size_t)stages * (CHUNK * (key_stride(head_dim) + value_stride(value_dim)) + 1) +
-            (size_t)rows * ((head_dim + 3) / 4 * 4 + CHUNK)) * sizeof(float);
+// VEC: rows of whole pieces of four elements, 16 bytes of 32-bit or 8 of bf16, stay in their type in shared memory; other rows are
+// widened to 32-bit element by element.
+template <typename T, bool VEC> struct Stored { using type = float; };
+template <> struct Stored<bf16, true> { using type = bf16; };
+
+template <typename S>
+inline size_t generic_smem(int head_dim, int value_dim, int rows) {
+    return (size_t)STAGES * CHUNK * (key_stride(head_dim) + value_stride(value_dim)) * sizeof(S) +
+           (STAGES + (size_t)rows * ((head_dim + 3) / 4 * 4 + CHUNK)) * sizeof(float);
 }
 
-// A chunk's rows of one array into shared memory, zeros where there is none; lane r brings the place of row r (or -1), a warp
-// fetches every n_warps-th row.  VEC: 32-bit rows of whole 16 bytes.
-template <typename T, bool VEC>
-__device__ __forceinline__ void fetch(float* dst, int stride, const T* cache, int width, long long row, int warp, int n_warps, int lane) {
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four(const bf16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// The pieces (VEC: four elements; else one) of a row, and what divides by their number.
+struct Pieces { int per; unsigned int inverse; };
+template <bool VEC> __device__ __forceinline__ Pieces pieces_of(int width) {
     const int per = VEC ? width / 4 : (width + 3) / 4 * 4;
-    for (int r = warp; r < CHUNK; r += n_warps) {
+    return {per, 0xffffffffu / per + 1};                 // (exact for numbers below 2^32 / per; 0 for one piece a row)
+}
+
+// A chunk's rows of one array into shared memory, zeros where there is none; lane r brings the place of row r (or -1).  Neighbouring
+// lanes take neighbouring pieces, whichever row they are of, and a warp every n_warps-th 32 of them.  (A row at a time left half of the
+// lanes of a 256-byte row idle and took 240 cycles a row in one chain: all of the time of a block with one warp.)
+template <typename T, bool VEC, typename S>
+__device__ __forceinline__ void fetch(S* dst, int stride, const T* cache, int width, const Pieces p, long long row, int warp, int n_warps, int lane) {
+#pragma unroll 4
+    for (int i = warp; i < p.per; i += n_warps) {
+        const int e = i * 32 + lane, r = p.per == 1 ? e : (int)__umulhi((unsigned)e, p.inverse), c = (e - r * p.per) * (VEC ? 4 : 1);
         const long long at = __shfl_sync(0xffffffffu, row, r);
-        const T* src = cache + (at < 0 ? 0 : at * width);
-        for (int c = lane; c < per; c += 32) {
-            if constexpr (VEC) {
-                const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst + r * stride + c * 4);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(at < 0 ? cache : src + c * 4), "r"(at < 0 ? 0 : 16)
-                             : "memory");
-            } else {
-                dst[r * stride + c] = at >= 0 && c < width ? to_f32(src[c]) : 0.f;
-            }
+        if constexpr (VEC) {
+            const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst + r * stride + c);
+            const T* src = at < 0 ? cache : cache + at * width + c;
+            if constexpr (sizeof(T) == 4)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(at < 0 ? 0 : 16) : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(at < 0 ? 0 : 8) : "memory");
+        } else {
+            dst[r * stride + c] = at >= 0 && c < width ? to_f32(__ldg(cache + at * width + c)) : 0.f;
         }
     }
 }
 
-template <typename T, typename TO, int R, int COLS, bool VEC, int STAGES>
+template <typename T, typename TO, int R, int COLS, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_generic_kernel(const GenericArgs a) {
+    using S = typename Stored<T, VEC>::type;
     extern __shared__ float4 smem4[];
-    float* smem = reinterpret_cast<float*>(smem4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     const int D = a.head_dim, V = a.value_dim, D4 = (D + 3) / 4 * 4, ks = key_stride(D), vs = value_stride(V);
-    float* k_s = smem;                                   // [STAGES][CHUNK][ks]
-    float* v_s = k_s + STAGES * CHUNK * ks;              // [STAGES][CHUNK][vs]
-    float* q_s = v_s + STAGES * CHUNK * vs + warp * R * D4;                                // this warp's [R][D4]
-    float* p_s = v_s + STAGES * CHUNK * vs + n_warps * R * D4 + warp * R * CHUNK;
-    unsigned int* here = reinterpret_cast<unsigned int*>(v_s + STAGES * CHUNK * vs + n_warps * R * (D4 + CHUNK));   // a bit per key
+    S* k_s = reinterpret_cast<S*>(smem4);                // [STAGES][CHUNK][ks]
+    S* v_s = k_s + STAGES * CHUNK * ks;                  // [STAGES][CHUNK][vs]
+    float* rows_s = reinterpret_cast<float*>(v_s + STAGES * CHUNK * vs);
+    float* q_s = rows_s + warp * R * D4;                 // this warp's [R][D4]
+    float* p_s = rows_s + n_warps * R * D4 + warp * R * CHUNK;
+    unsigned int* here = reinterpret_cast<unsigned int*>(rows_s + n_warps * R * (D4 + CHUNK));   // a bit per key
+    const Pieces k_pieces = pieces_of<VEC>(D), v_pieces = pieces_of<VEC>(V);
     const int group = a.n_heads / a.n_kv;
     const int side = blockIdx.x / a.tiles, tile = blockIdx.x % a.tiles;
     const int kvh = a.cross ? side / a.n_kv : side, vh = a.cross ? side % a.n_kv : kvh;
-    const int t0 = tile / a.head_chunks * a.tokens_per_block, g0 = tile % a.head_chunks * (n_warps * R);
-    const int t1 = min(a.n_tokens, t0 + a.tokens_per_block);
+    const int at = tile / a.head_chunks, g0 = tile % a.head_chunks * (n_warps * R);
+    const int t0 = at < a.singles ? at : a.singles + (at - a.singles) * a.tokens_per_block;
+    const int t1 = at < a.singles ? t0 + 1 : min(a.n_tokens, t0 + a.tokens_per_block);
     const int heads = a.head_chunks > 1 ? min(group - g0, n_warps * R) : group;
 
     int tok[R], head[R], pos[R], lo[R];
@@ -140,21 +169,20 @@ attention_generic_kernel(const GenericArgs a) {
                 const long long row = page < 0 ? -1 : ((long long)page * a.n_kv + kvh) * a.page_size + (j0 + lane) % a.page_size;
                 const unsigned int there = __ballot_sync(0xffffffffu, page >= 0);
                 if (threadIdx.x == 0) here[stage] = there;
-                fetch<T, VEC>(k_s + stage * CHUNK * ks, ks, (const T*)a.k_cache, D, row, warp, n_warps, lane);
-                fetch<T, VEC>(v_s + stage * CHUNK * vs, vs, (const T*)a.v_cache, V, page < 0 ? -1 : row + (long long)(vh - kvh) * a.page_size, warp,
-                              n_warps, lane);
+                fetch<T, VEC>(k_s + stage * CHUNK * ks, ks, (const T*)a.k_cache, D, k_pieces, row, warp, n_warps, lane);
+                fetch<T, VEC>(v_s + stage * CHUNK * vs, vs, (const T*)a.v_cache, V, v_pieces,
+                              page < 0 ? -1 : row + (long long)(vh - kvh) * a.page_size, warp, n_warps, lane);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         start = start / CHUNK * CHUNK;
-#pragma unroll
-        for (int s = 0; s < STAGES - 1; ++s) load(start + s * CHUNK, page_of(start + s * CHUNK), s);
-        int page = page_of(start + (STAGES - 1) * CHUNK), stage = 0;
-        for (int j0 = start; j0 <= last; j0 += CHUNK, stage = stage + 1 == STAGES ? 0 : stage + 1) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        load(start, page_of(start), 0);
+        int page = page_of(start + CHUNK), stage = 0;
+        for (int j0 = start; j0 <= last; j0 += CHUNK, stage ^= 1) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();                             // this chunk is here, and everyone is done with the one before,
-            load(j0 + (STAGES - 1) * CHUNK, page, stage == 0 ? STAGES - 1 : stage - 1);                 // whose place this takes
-            page = page_of(j0 + STAGES * CHUNK);
+            load(j0 + CHUNK, page, stage ^ 1);           // whose place this takes
+            page = page_of(j0 + 2 * CHUNK);
             const int j = j0 + lane;
             const bool there = here[stage] >> lane & 1;
             bool sees[R];                                // does the row have keys in this chunk?
@@ -168,10 +196,10 @@ attention_generic_kernel(const GenericArgs a) {
                 float d[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) d[r] = 0.f;
-                const float* kr = k_s + (stage * CHUNK + lane) * ks;
+                const S* kr = k_s + (stage * CHUNK + lane) * ks;
 #pragma unroll 8
                 for (int i = 0; i < D4; i += 4) {        // (columns beyond D are zeros on both sides)
-                    const float4 k = *reinterpret_cast<const float4*>(kr + i);
+                    const float4 k = four(kr + i);
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const float4 x = *reinterpret_cast<const float4*>(q_s + r * D4 + i);
@@ -209,7 +237,7 @@ attention_generic_kernel(const GenericArgs a) {
                     p_s[r * CHUNK + lane] = p;
                 }
                 __syncwarp();
-                const float* vr = v_s + stage * CHUNK * vs + lane;
+                const S* vr = v_s + stage * CHUNK * vs + lane;
                 if (whole) {
 #pragma unroll
                     for (int jj = 0; jj < CHUNK; jj += 4) {
@@ -220,7 +248,7 @@ attention_generic_kernel(const GenericArgs a) {
                         for (int u = 0; u < 4; ++u) {
 #pragma unroll
                             for (int i = 0; i < COLS; ++i) {
-                                const float v = i * 32 + lane < V ? vr[(jj + u) * vs + i * 32] : 0.f;
+                                const float v = i * 32 + lane < V ? to_f32(vr[(jj + u) * vs + i * 32]) : 0.f;
 #pragma unroll
                                 for (int r = 0; r < R; ++r) acc[r][i] = fmaf(reinterpret_cast<const float*>(&p4[r])[u], v, acc[r][i]);
                             }
@@ -230,7 +258,7 @@ attention_generic_kernel(const GenericArgs a) {
                     for (int jj = from; jj <= to; ++jj) {
                         float v[COLS];
 #pragma unroll
-                        for (int i = 0; i < COLS; ++i) v[i] = i * 32 + lane < V ? vr[jj * vs + i * 32] : 0.f;
+                        for (int i = 0; i < COLS; ++i) v[i] = i * 32 + lane < V ? to_f32(vr[jj * vs + i * 32]) : 0.f;
 #pragma unroll
                         for (int r = 0; r < R; ++r) {    // (a key that a row must not see is not even multiplied by zero)
                             if (!sees[r] || j0 + jj < lo[r] || j0 + jj > pos[r]) continue;
@@ -261,15 +289,15 @@ attention_generic_kernel(const GenericArgs a) {
     }
 }
 
-template <typename T, typename TO, int R, int COLS, bool VEC, int STAGES>
+template <typename T, typename TO, int R, int COLS, bool VEC>
 int launch(GenericArgs& a, int warps, cudaStream_t stream) {
-    auto* kernel = attention_generic_kernel<T, TO, R, COLS, VEC, STAGES>;
-    const size_t smem = generic_smem(a.head_dim, a.value_dim, warps * R, STAGES);
+    auto* kernel = attention_generic_kernel<T, TO, R, COLS, VEC>;
+    const size_t smem = generic_smem<typename Stored<T, VEC>::type>(a.head_dim, a.value_dim, warps * R);
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         INFERO_REQUIRE(e == cudaSuccess, "attention: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
-    const long long tiles = (long long)((a.n_tokens + a.tokens_per_block - 1) / a.tokens_per_block) * a.head_chunks;
+    const long long tiles = (a.singles + (long long)(a.n_tokens - a.singles + a.tokens_per_block - 1) / a.tokens_per_block) * a.head_chunks;
     const long long blocks = tiles * a.n_kv * (a.cross ? a.n_kv : 1);
     INFERO_REQUIRE(blocks < (1ll << 31), "attention: %d tokens of %d kv heads are too many for one launch", a.n_tokens, a.n_kv);
     a.tiles = (int)tiles;
@@ -277,19 +305,28 @@ int launch(GenericArgs& a, int warps, cudaStream_t stream) {
     return infero_check_launch("attention_generic");
 }
 
+// Tokens a block of 32 rows takes at a time, 0 for a block per token.  A block's tokens of different requests take turns and all but
+// one request's rows idle meanwhile, so what counts is the portions' tokens (the single ones in front have blocks of their own
+// either way) and that a portion has about a block's tokens and more.
+int block_tokens(int n_tokens, int singles, int portions, int group) {
+    const int rest = n_tokens - singles, tokens = group > WIDE_ROWS ? 1 : WIDE_ROWS / group;
+    return rest <= FEW_TOKENS || 2 * rest < (long long)portions * tokens ? 0 : tokens;
+}
+
 template <typename T, typename TO, bool VEC>
-int launch_rows(GenericArgs& a, cudaStream_t stream) {
-    const int group = a.n_heads / a.n_kv;
-    const bool few = a.n_tokens <= FEW_TOKENS;
-    const int warps = few && group < WARPS ? group : WARPS, rows = few ? warps : WARPS * 4;
-    a.tokens_per_block = few || group > rows ? 1 : rows / group;
+int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
+    const int group = a.n_heads / a.n_kv, tokens = block_tokens(a.n_tokens, a.singles, portions, group);
+    const bool few = tokens == 0;
+    // (warps without a row help to fetch: four suffice for narrow rows)
+    const int least = a.head_dim > 64 || a.value_dim > 64 ? WARPS : WARPS / 2;
+    const int warps = few ? (group < least ? least : group < WARPS ? group : WARPS) : WARPS, rows = few ? warps : WIDE_ROWS;
+    a.tokens_per_block = few ? 1 : tokens;
     a.head_chunks = (group + rows - 1) / rows;
-#define COLUMNS(R)                                                                                         \
-    do {                                                                                                   \
-        constexpr int S = R == 1 ? 4 : 2;                                                                  \
-        if (a.head_dim > 128 || a.value_dim > 128) return launch<T, TO, R, 8, VEC, 2>(a, warps, stream);   \
-        if (a.value_dim > 64) return launch<T, TO, R, 4, VEC, S>(a, warps, stream);                        \
-        return launch<T, TO, R, 2, VEC, S>(a, warps, stream);                                              \
+#define COLUMNS(R)                                                                                      \
+    do {                                                                                                \
+        if (a.head_dim > 128 || a.value_dim > 128) return launch<T, TO, R, 8, VEC>(a, warps, stream);   \
+        if (a.value_dim > 64) return launch<T, TO, R, 4, VEC>(a, warps, stream);                        \
+        return launch<T, TO, R, 2, VEC>(a, warps, stream);                                              \
     } while (0)
     if (few) COLUMNS(1);
     COLUMNS(4);
@@ -300,19 +337,26 @@ int launch_rows(GenericArgs& a, cudaStream_t stream) {
 
 extern "C" {
 
+int infero_attention_generic_block_tokens(int n_tokens, int singles, int portions, int group) {
+    return block_tokens(n_tokens, singles, portions, group);
+}
+
 // Keys of width head_dim, values of width value_dim (the cache's two arrays have their own row widths); ``sink``:
 // the softmax's denominator has one more term exp(0), which carries no value; ``slopes``: float32 [n_heads] or null,
 // head h's score loses slopes[h] times the distance between the query and the key; ``rel``: float32 [n_heads, rel_len] or
 // null, what a score gains at every distance (the last entry also beyond it); ``cross``: every head meets the values of
 // every kv head, out float32 [n_tokens, n_heads * n_kv * value_dim]; ``sinks``: float32 [n_heads] or null, one more term
-// exp(sinks[h]) of the denominator; ``softcap`` > 0: scaled scores are soft-capped.
+// exp(sinks[h]) of the denominator; ``softcap`` > 0: scaled scores are soft-capped; ``singles`` tokens in front are their requests'
+// only ones and ``portions`` requests bring the others (they choose the blocks and change no result).
 int infero_attention_generic_rel(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
                                  const void* v_cache, int dtype, const int* block_table, int max_blocks,
                                  const int* tok_entry, const int* positions, int n_tokens, int n_heads,
                                  int n_kv, int head_dim, int value_dim, int page_size, int window, float scale,
                                  int sink, const float* slopes, const float* rel, int rel_len, int cross,
-                                 const float* sinks, float softcap, cudaStream_t stream) {
+                                 const float* sinks, float softcap, int singles, int portions, cudaStream_t stream) {
     if (n_tokens == 0) return 0;
+    INFERO_REQUIRE(singles >= 0 && singles <= n_tokens && portions >= 0, "attention: %d single tokens and %d portions of %d tokens", singles,
+                   portions, n_tokens);
     INFERO_REQUIRE(head_dim >= 1 && head_dim <= MAX_D, "attention: head_dim %d outside 1..%d", head_dim, MAX_D);
     INFERO_REQUIRE(value_dim >= 1 && value_dim <= MAX_D, "attention: value width %d outside 1..%d", value_dim, MAX_D);
     INFERO_REQUIRE(n_kv > 0 && n_heads % n_kv == 0, "attention: %d heads not a multiple of %d kv heads", n_heads, n_kv);
@@ -322,10 +366,12 @@ int infero_attention_generic_rel(const void* q, int q_stride, void* out, int out
     a.positions = positions, a.slopes = slopes, a.rel = rel, a.sinks = sinks, a.q_stride = q_stride, a.out_stride = out_stride;
     a.max_blocks = max_blocks, a.n_tokens = n_tokens, a.n_heads = n_heads, a.n_kv = n_kv, a.head_dim = head_dim;
     a.value_dim = value_dim, a.page_size = page_size, a.window = window, a.sink = sink, a.rel_len = rel_len, a.cross = cross;
-    a.scale = scale, a.softcap = softcap;
-    const bool vec = head_dim % 4 == 0 && value_dim % 4 == 0 && (uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0;
-    if (dtype == INFERO_F32) return vec ? launch_rows<float, float, true>(a, stream) : launch_rows<float, float, false>(a, stream);
-    return cross ? launch_rows<bf16, float, false>(a, stream) : launch_rows<bf16, bf16, false>(a, stream);
+    a.scale = scale, a.softcap = softcap, a.singles = singles;
+    const size_t piece = dtype == INFERO_F32 ? 16 : 8;
+    const bool vec = head_dim % 4 == 0 && value_dim % 4 == 0 && (uintptr_t)k_cache % piece == 0 && (uintptr_t)v_cache % piece == 0;
+    if (dtype == INFERO_F32) return vec ? launch_rows<float, float, true>(a, portions, stream) : launch_rows<float, float, false>(a, portions, stream);
+    if (cross) return vec ? launch_rows<bf16, float, true>(a, portions, stream) : launch_rows<bf16, float, false>(a, portions, stream);
+    return vec ? launch_rows<bf16, bf16, true>(a, portions, stream) : launch_rows<bf16, bf16, false>(a, portions, stream);
 }
 
 int infero_attention_generic_bias(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
@@ -335,7 +381,7 @@ int infero_attention_generic_bias(const void* q, int q_stride, void* out, int ou
                                   int sink, const float* slopes, cudaStream_t stream) {
     return infero_attention_generic_rel(q, q_stride, out, out_stride, k_cache, v_cache, dtype, block_table, max_blocks,
                                         tok_entry, positions, n_tokens, n_heads, n_kv, head_dim, value_dim, page_size,
-                                        window, scale, sink, slopes, nullptr, 0, 0, nullptr, 0.f, stream);
+                                        window, scale, sink, slopes, nullptr, 0, 0, nullptr, 0.f, 0, 1, stream);
 }
 
 int infero_attention_generic_ex(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,

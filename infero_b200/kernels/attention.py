@@ -169,15 +169,16 @@ def attention_any(q, out, k_cache, v_cache, table, tok_entry, positions, n_heads
     ``rel`` (float32 [H, L]; ``rel_log2``: the same times log2 e, for the bf16 kernels) and ``cross``: see
     ``paged_attention_cross``; out [T, G*H*D] then, float32 where the any-type kernel runs.  ``sinks`` (float32 [H];
     ``sinks_log2``: the same times log2 e) and ``softcap``: see ``paged_attention_ex``."""
+    if batch_shape is None:
+        batch_shape = shape_of_batch(q_lens, pos0)
     if q.dtype != torch.bfloat16 or not mma_supported(head_dim, page_size):
         attention_generic(q, out, k_cache, v_cache, table, tok_entry, positions, n_heads, n_kv, head_dim,
-                          page_size, window, scale, sink=sink, slopes=slopes, rel=rel, cross=cross, sinks=sinks, softcap=softcap)
+                          page_size, window, scale, sink=sink, slopes=slopes, rel=rel, cross=cross, sinks=sinks, softcap=softcap,
+                          batch=(batch_shape[0], len(q_lens) - batch_shape[0]))
         return
     more = dict(sink=sink, slopes=slopes, rel=rel_log2, cross=cross, sinks=sinks_log2, softcap=softcap)
     sides = n_kv if cross else 1
     E = len(q_lens)
-    if batch_shape is None:
-        batch_shape = shape_of_batch(q_lens, pos0)
     n_dec, vis_now, tiles_128, tiles_mma = batch_shape
     if n_dec:
         vis = vis_now if kv_bound is None else int(kv_bound)
@@ -224,6 +225,14 @@ def _batch_shape(ctx):
     return memo
 
 
+def _singles_and_portions(ctx):
+    """``batch`` of ``attention_generic``."""
+    if getattr(ctx, "h_q_len", None) is None:
+        return 0, 1
+    n_dec = _batch_shape(ctx)[0]
+    return n_dec, ctx.n_entries - n_dec
+
+
 LOG2E = 1.4426950408889634
 
 
@@ -249,7 +258,7 @@ def paged_attention_ex(ctx, q, out, kv, table, n_heads, n_kv, head_dim, value_di
                       rel_log2=rel_log2, sinks=sinks, sinks_log2=sinks_log2, softcap=softcap)
         return
     attention_generic(q, out, kv.k, kv.v, table, ctx.tok_entry, ctx.positions, n_heads, n_kv, head_dim, kv.page_size,
-                      window, scale, value_dim=value_dim, sink=sink, slopes=slopes, rel=rel, sinks=sinks, softcap=softcap)
+                      window, scale, value_dim=value_dim, sink=sink, slopes=slopes, rel=rel, sinks=sinks, softcap=softcap, batch=_singles_and_portions(ctx))
 
 
 def paged_attention_cross(ctx, q, kv, table, n_heads, n_kv, head_dim, value_dim, window, scale, rel=None,
@@ -268,5 +277,5 @@ def paged_attention_cross(ctx, q, kv, table, n_heads, n_kv, head_dim, value_dim,
                       kv_bound=getattr(ctx, "kv_bound", None), batch_shape=_batch_shape(ctx), rel=rel, rel_log2=rel_log2, cross=True)
     else:
         attention_generic(q, out, kv.k, kv.v, table, ctx.tok_entry, ctx.positions, n_heads, n_kv, head_dim, kv.page_size,
-                          window, scale, value_dim=value_dim, rel=rel, cross=True)
+                          window, scale, value_dim=value_dim, rel=rel, cross=True, batch=_singles_and_portions(ctx))
     return out

@@ -1168,3 +1168,33 @@ def test_attention_generic_of_very_many_kv_heads():
         w = torch.softmax(torch.einsum("hd,hjd->hj", q[t].double().view(G, D), kk) * 0.5, -1)
         ref = torch.einsum("hj,cjd->chd", w, vv)
         assert float((out[t].double().view(G, G, D) - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("H,G,D,dt", [(3, 3, 24, "f32"), (14, 2, 24, "f32"), (3, 3, 7, "f32"), (3, 3, 36, "bf16"), (4, 2, 200, "bf16"),
+                                      (6, 2, 10, "bf16")])
+def test_attention_generic_blocks_of_single_tokens_and_portions(H, G, D, dt):
+    """What the caller says of the step (single tokens in front, how many requests bring the others) chooses the blocks, not the bits;
+    rows in pieces of four elements and rows that come one by one."""
+    from infero_b200 import kernels as Kn
+    dt = torch.float32 if dt == "f32" else torch.bfloat16
+    lens, before, page = [1] * 40 + [300, 9], [(53 * i) % 301 for i in range(40)] + [0, 60], 16
+    blocks = max(-(-(n + p) // page) for n, p in zip(lens, before))
+    table = torch.randperm(len(lens) * blocks, generator=torch.Generator().manual_seed(3)).int().view(len(lens), blocks).to(DEV)
+    k, v = (_rand((len(lens) * blocks, G, page, D), dt, i) for i in (4, 5))
+    q = _rand((sum(lens), H * D), dt, 6)
+    entry = torch.tensor([e for e, n in enumerate(lens) for _ in range(n)], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p + i for n, p in zip(lens, before) for i in range(n)], dtype=torch.int32, device=DEV)
+    outs = []
+    for batch in ((0, 1), (40, 2), (39, 1), (0, 1000), (40, 1000)):
+        outs.append(torch.full((sum(lens), H * D), float("nan"), dtype=dt, device=DEV))
+        Kn.attention_generic(q, outs[-1], k, v, table, entry, pos, H, G, D, page, None, D ** -0.5, batch=batch)
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+    for t in (0, 17, 39, 40, 339, 340, 348):
+        at = torch.arange(int(pos[t]) + 1)
+        pages, inside = table[int(entry[t])].cpu()[at // page].long(), at % page
+        for h in range(H):
+            kk, vv = (x.cpu().double()[pages, h // (H // G), inside] for x in (k, v))
+            ref = torch.softmax(kk @ q[t, h * D:(h + 1) * D].cpu().double() * D ** -0.5, 0) @ vv
+            tol = 1e-5 if dt == torch.float32 else 2.0 ** -8        # (32-bit sums; the result rounded to bf16)
+            assert float((outs[0][t, h * D:(h + 1) * D].cpu().double() - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))

@@ -61,3 +61,12 @@ def test_decode_attention_splits_cover_the_keys(n_tok, n_kv, group, visible):
     assert 1 <= splits.value <= 256
     assert chunk.value * splits.value >= visible, "the splits cover every visible key"
     assert chunk.value * (splits.value - 1) < max(visible, 16), "and none of them is empty by plan"
+
+
+@pytest.mark.parametrize("n,singles,portions,group,want", [
+    (256, 0, 1, 1, 0), (257, 0, 1, 1, 32), (257, 0, 1, 7, 4), (257, 0, 1, 40, 1),
+    (300, 300, 0, 1, 0), (266, 10, 1, 1, 0), (267, 10, 1, 1, 32),      # single tokens do not make a step one of many tokens
+    (300, 0, 100, 1, 0), (300, 0, 100, 16, 2), (320, 0, 20, 1, 32), (320, 0, 21, 1, 0),      # portions of half a block's tokens and more
+])
+def test_any_type_attention_shares_blocks_among_a_portions_tokens(n, singles, portions, group, want):
+    assert K.lib().infero_attention_generic_block_tokens(c_int(n), c_int(singles), c_int(portions), c_int(group)) == want
