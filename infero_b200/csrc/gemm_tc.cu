@@ -48,7 +48,7 @@ constexpr int A_STAGE_BYTES = TILE_A * TILE_K * 2;
 // EPI_CLUSTER: the CTAs that share a tile and differ in their split of K form a cluster; each leaves its
 // 32-bit tile in its own shared memory and the cluster adds the tiles up through distributed shared
 // memory, in ascending order of the splits, each CTA a share of the token columns: out[token, feature].
-enum : int { EPI_ROW = 0, EPI_COL = 1, EPI_PARTIAL = 2, EPI_ROW_SWIGLU = 3, EPI_COL_SWIGLU = 4, EPI_CLUSTER = 5 };
+enum : int { EPI_ROW = 0, EPI_COL = 1, EPI_PARTIAL = 2, EPI_ROW_SWIGLU = 3, EPI_COL_SWIGLU = 4, EPI_CLUSTER = 5, EPI_ROW_HALVES = 6 };
 
 __device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + expf(-g)) * u; }
 
@@ -464,6 +464,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&t);
 }
+__device__ __forceinline__ uint32_t pack_half(float a, float b) {
+    const __half2 t = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
 
 // The epilogue of the many-token kernels.  Sixteen warps drain an accumulator, four per quarter of its rows: they take turns
 // at blocks of 32 columns.  What a warp does with a block is one chain of instructions (the TMEM load, divisions with a
@@ -511,6 +515,9 @@ __device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, 
                 v[e] = r * r;
             }
         }
+        // (EPI_ROW_HALVES: the second half of the columns are IEEE halves; blocks of 32 lie on one side of the line)
+        const bool half = EPI == EPI_ROW_HALVES && rb >= RB / 2;
+        auto pack = [&](float a, float b) { return half ? pack_half(a, b) : pack_bf16(a, b); };
         const int cols = min(32, col_end - rb), first = GLU ? rb >> 1 : rb, n = GLU ? cols >> 1 : cols;
         uint8_t* dst = reinterpret_cast<uint8_t*>(out + first) + (size_t)row0 * pitch;
         // (first is a multiple of 16 elements, or of 8 of bf16 behind a gated unit: pieces of 16 bytes start aligned)
@@ -522,15 +529,18 @@ __device__ __forceinline__ void drain_accumulator(uint32_t lane_addr, int turn, 
             uint4 pk[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                pk[e] = make_uint4(pack_bf16(v[8 * e], v[8 * e + 1]), pack_bf16(v[8 * e + 2], v[8 * e + 3]),
-                                   pack_bf16(v[8 * e + 4], v[8 * e + 5]), pack_bf16(v[8 * e + 6], v[8 * e + 7]));
+                pk[e] = make_uint4(pack(v[8 * e], v[8 * e + 1]), pack(v[8 * e + 2], v[8 * e + 3]), pack(v[8 * e + 4], v[8 * e + 5]),
+                                   pack(v[8 * e + 6], v[8 * e + 7]));
             if (!GLU && cols == 32) store_rows<4>(stage, pk, dst, pitch, rows, lane);
             else store_rows<2>(stage, pk, dst, pitch, rows, lane);
         } else if (ra < RA) {
             OutT* row = out + (size_t)ra * ldc + first;
 #pragma unroll
             for (int e = 0; e < (GLU ? 16 : 32); ++e)
-                if (e < n) row[e] = from_f32<OutT>(v[e]);
+                if (e < n) {
+                    if (half) reinterpret_cast<__half*>(row)[e] = __float2half_rn(v[e]);
+                    else row[e] = from_f32<OutT>(v[e]);
+                }
         }
     }
     __syncwarp();
@@ -1053,7 +1063,7 @@ int launch_persistent(const void* x, const void* w, void* out, const void* bias,
         configured = true;
     }
     const int sms = sm_count > 0 ? sm_count : 148;
-    const int bn = pick_tile_n(RA, RB, sms, EPI == EPI_ROW_SWIGLU ? 32 : 16);
+    const int bn = pick_tile_n(RA, RB, sms, EPI == EPI_ROW_SWIGLU || EPI == EPI_ROW_HALVES ? 32 : 16);
     CUtensorMap ma, mb;
     if (get_map(x, RA, K, ldx, TILE_A, &ma)) return 1;
     if (get_map(w, RB * n_groups, K, K, bn, &mb)) return 1;
@@ -1428,6 +1438,20 @@ int infero_gemm_tc_swiglu_bias(const void* x, const void* w, const void* bias, i
 int infero_gemm_tc_swiglu(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldc,
                           int sm_count, cudaStream_t stream) {
     return infero_gemm_tc_swiglu_bias(x, w, nullptr, 0, out, M, N, K, ldx, ldc, sm_count, stream);
+}
+
+// out[M, N] = x[M, K] w[N, K]^T, the first N / 2 columns bf16, the others IEEE half (N a multiple of 64); rows of out on 16 bytes.
+int infero_gemm_tc_halves(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldc, int sm_count, cudaStream_t stream) {
+    if (M == 0 || N == 0) return 0;
+    INFERO_REQUIRE(infero_gemm_tc_supported(x, w, M, N, K, ldx), "gemm_tc_halves: shape M=%d N=%d K=%d ldx=%d not supported", M, N, K, ldx);
+    INFERO_REQUIRE(N % 64 == 0 && ldc >= N, "gemm_tc_halves: N=%d must be a multiple of 64 and ldc=%d at least N", N, ldc);
+    int* err;
+    if (err_flag_ptr(&err)) return 1;
+    if (M > 256 && pairs_wanted(M)) {
+        const int r = launch_pair<EPI_ROW_HALVES, bf16>(x, w, out, nullptr, 0, M, N, K, ldx, ldc, err, stream);
+        if (r >= 0) return r;
+    }
+    return launch_persistent<EPI_ROW_HALVES, bf16>(x, w, out, nullptr, 0, M, N, K, ldx, ldc, sm_count, err, stream);
 }
 
 // A product of many rows with an activation in the epilogue of the persistent kernel (bf16 out):

@@ -5,11 +5,14 @@
 // 2 D + R.  A step runs
 //     gather: the visible latent rows of every portion, from their pages, side by side: c [keys, C] and the rotated part
 //             [keys, 64]; a request's rows start at a multiple of 64 keys of its positions and end in zeros
-//     one product (gemm_tc.cu): [Wuk; Wuv] c -> [keys, H D + H D], bf16
+//     one product (gemm_tc.cu): [Wuk; Wuv] c -> [keys, H D + H D], the keys bf16, the values IEEE halves
 //     this file's attention over it, the output gate in its epilogue.
 // At 2,048 tokens, 16 heads of 128 + 64 and a latent of 512 a layer's attention with its up-projections took 600 us
 // through the latent rows (73 GFLOP of scores and sums, on mma.sync) and takes 71 written out (21.5 GFLOP, of it 38 us in the
-// attention kernel).  Against 64 bits whole passes come out alike: 0.0055 to 0.0072 either way over prompts of 8 to 2,048 tokens.
+// attention kernel).  Weights and values are IEEE halves: bf16 for both left a layer 1 to 6 % further from 64 bits than the latent
+// rows do, halves leave it 17 to 23 % nearer (16 to 600 tokens, 8 heads of 64 + 32 and 16 of 128 + 64), in the same time.  A weight is
+// 256 at most, and layers whose values could leave the range of halves (their weights bound them: the latent row is normed) keep to
+// the latent rows.
 //
 // One CTA = 128 query rows of one request and one head; it walks the visible keys in tiles of 64.  The tensor memory holds
 // two results: tiles of even number (of the absolute position) belong to warps 0..3, odd ones to warps 4..7, each with its
@@ -17,12 +20,13 @@
 // added up, every thread for its row and half of the columns.  (A head's keys are its own here, so there is no second head
 // that could share them, as attention_prefill_tc.cu has it; 256 rows a CTA would leave too few CTAs: 128 at the size above.)
 // Per tile: S = [q | q_rot] [k | k_rot]^T over D / 64 + 1 blocks of 64 columns (tcgen05.mma from shared memory, TMA with
-// 128-byte swizzle), P = 2^(S c - m) by one thread a row, back over S as bf16, O += P V.  Two S buffers a parity, so the
+// 128-byte swizzle), P = 2^(S c - m) by one thread a row, back over S as halves, O += P V.  Two S buffers a parity, so the
 // products of the next two tiles are issued ahead.  Scores, maxima, sums and O are 32-bit.
 //
 // Same formula as latent_attention.cu: key j is visible from position p iff lo <= j <= p, lo = max(0, p - window + 1); a learned
-// sink is one more term of the sum.  What is computed for a token depends on its position only, not on how its prompt was cut:
-// tiles sit at multiples of 64 of the absolute position.  Every wait is bounded, as in attention_prefill_tc.cu.
+// sink is one more term of the sum.  What is computed for a token here depends on its position only: tiles sit at multiples of 64
+// of the absolute position.  (Which of the two routes it takes depends on the step: kernels/latent_prefill.py.)  Every wait is
+// bounded, as in attention_prefill_tc.cu.
 #include "tc_common.cuh"
 #include "tc_softmax.cuh"
 #include <math_constants.h>
@@ -208,7 +212,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // ---- MMA issue: tile j belongs to parity (kt_begin + j) & 1 and is its (j >> 1)-th ----------------------
         if (n_kt > 0 && elect_one()) {
             constexpr uint32_t idesc_qk = idesc_bf16_f32(QROWS, KTILE);
-            constexpr uint32_t idesc_pv = idesc_bf16_f32_b_mn(QROWS, D);
+            constexpr uint32_t idesc_pv = idesc_f16_f32_b_mn(QROWS, D);
             const uint32_t q_addr = smem_u32(smem);
             const int k_steps = (DB + rot_blocks) * (BLOCK / 16);
             bool ok = true;
@@ -242,7 +246,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const uint32_t p_tmem = tmem_base + side * Plan::SIDE_COLS + buf * KTILE;
 #pragma unroll
                 for (int ks = 0; ks < KTILE / 16; ++ks)
-                    // 16 keys: 8 columns of P (two bf16 each), 16 rows of V (2048 bytes)
+                    // 16 keys: 8 columns of P (two halves each), 16 rows of V (2048 bytes)
                     umma_bf16_ts(o_tmem, p_tmem + (uint32_t)ks * 8u, smem_desc_mn_sw128(v_addr + (uint32_t)ks * 2048u, Plan::KBLOCK_BYTES, 1024u),
                                  idesc_pv, (j > 1 || ks > 0) ? 1u : 0u);
                 umma_commit(&o_done[side]);
@@ -304,7 +308,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 fma2(x0, x1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), scale_log2, -sub);
                 const float p0 = ex2(x0), p1 = ex2(x1);
                 sum4[(i >> 1) & 3] += p0 + p1;
-                pk[i >> 1] = pack2(p0, p1);
+                pk[i >> 1] = pack2_half(p0, p1);
             }
 #pragma unroll
             for (int c = 0; c < KTILE / 32; ++c) tmem_st16(s_addr + (uint32_t)c * 16u, pk + c * 16);
@@ -434,7 +438,7 @@ int infero_latent_gather(const void* cache, const int* block_table, int max_bloc
 }
 
 // q [H, head_rows, D] and q_rot [H, head_rows, 64] (bf16; row t is token first_token + t), kv [64 * n_key_tiles, 2 H D] = head
-// by head the plain keys, then the values, of the gathered rows, k_rot their rotated parts; out [tokens, >= H D] bf16;
+// by head the plain keys (bf16), then the values (IEEE halves), of the gathered rows, k_rot their rotated parts; out [tokens, >= H D] bf16;
 // gate float32 [tokens, H] (row stride gate_stride) or null; n_tiles = the sum of ceil(q_len / 128) over the portions.
 int infero_latent_prefill_tc(const void* q, const void* q_rot, int head_rows, const void* kv, const void* k_rot, int n_key_tiles,
                              void* out, int out_stride, const float* gate, int gate_stride, const int* entry_q_start,

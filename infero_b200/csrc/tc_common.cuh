@@ -286,6 +286,8 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
 }
 // The same with an MN-major B operand.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32_b_mn(int m, int n) { return idesc_bf16_f32(m, n) | (1u << 16); }
+// And with both operands IEEE halves (format 0).
+__host__ __device__ constexpr uint32_t idesc_f16_f32_b_mn(int m, int n) { return idesc_bf16_f32_b_mn(m, n) & ~((1u << 7) | (1u << 10)); }
 
 }  // namespace tc
 

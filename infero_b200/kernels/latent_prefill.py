@@ -26,6 +26,13 @@ def supported(D: int, V: int, R: int, C: int) -> bool:
     return (D in (64, 128) and V == D and 0 <= R <= BLOCK and R % 8 == 0 and C >= 2 * D and C % 8 == 0)
 
 
+def values_fit(up_v: torch.Tensor, norm_w: torch.Tensor, C: int) -> bool:
+    """Can no value of these weights leave the range of IEEE halves?  A latent row is norm_w times a row of 2-norm sqrt(C) at most
+    (rounded to bf16: 1 + 2^-8), a value its product with a row of Wuv."""
+    rows = (up_v.float() * norm_w.float()).norm(dim=1)
+    return bool(float(rows.max()) * C ** 0.5 * (1 + 2.0 ** -8) < 65504.0)
+
+
 def plan(ctx, dtype, H: int, D: int, V: int, R: int, C: int, window: Optional[int]) -> Optional[Plan]:
     """None, or how the portions behind the leading single tokens are cut.  Writing keys and values out costs 2 C (D + V)
     a key and head and saves about 2 (2 C - D - V) a (query, key) pair, so not a short portion behind a long cached prefix.
@@ -70,7 +77,7 @@ def run(ctx, p: Plan, q: torch.Tensor, q_rot: torch.Tensor, kv, table: torch.Ten
     _check(lib().infero_latent_gather(_ptr(cache), _ptr(_i32(table, "block_table")), c_int(table.shape[1]), c_int(kv.page_size), entry[1], entry[2],
                                       *where, c_int(p.key_tiles), c_int(window or 0), c_int(C), c_int(R), _ptr(lat), _ptr(k_rot), _stream()))
     wide = torch.empty((keys, 2 * H * D), dtype=torch.bfloat16, device=dev)
-    tc_gemm.gemm(lat, w_kv, None, wide)
+    tc_gemm.gemm_halves(lat, w_kv, wide)                 # keys bf16, values halves
     _check(lib().infero_latent_prefill_tc(_ptr(q), _ptr(q_rot), c_int(rows), _ptr(wide), _ptr(k_rot), c_int(p.key_tiles), _ptr(out),
                                           c_int(out.stride(0)), _ptr(gate), c_int(gate.stride(0) if gate is not None else 0), *entry, *where,
                                           c_int(p.first_entry), c_int(p.query_tiles), c_int(H), c_int(D), c_int(D), c_int(R), c_int(C),

@@ -67,6 +67,15 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: to
                                 c_int(tile_n), _stream()))
 
 
+def gemm_halves(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """a @ w^T with the first half of the columns bf16 and the others IEEE halves, side by side in ``out`` [M, N] (bf16 by name)."""
+    M, K = a.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and out.shape == (M, N) and out.stride(1) == 1 and out.dtype == torch.bfloat16
+    _check(lib().infero_gemm_tc_halves(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)), c_int(out.stride(0)),
+                                       c_int(sm_count(a.device)), _stream()))
+
+
 def set_cluster(on: bool) -> None:
     """Few-row products whose K is cut into splits: add the splits up inside the kernel (a cluster
     per tile, through distributed shared memory) or return them as partial sums (the default;

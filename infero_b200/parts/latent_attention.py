@@ -80,7 +80,7 @@ class LatentAttention(Mixer):
         return out
 
     def bind(self, tensors: Dict[str, torch.Tensor]) -> None:
-        from ..kernels.latent_prefill import supported as written_out
+        from ..kernels import latent_prefill as P
         H, D, R, V, C = self.H, self.D, self.R, self.V, self.C
         rows = [tensors[self._n("q_down" if self.Q else "q")], tensors[self._n("down")]]
         if self.spec.out_gate:
@@ -103,7 +103,8 @@ class LatentAttention(Mixer):
         self.up_k_t = tensors[self._n("up_k")].view(H, D, C).transpose(1, 2).contiguous()
         # where prompts are written out: both up-projections as one matrix
         up_k, up_v = tensors[self._n("up_k")], tensors[self._n("up_v")]
-        self.kv_up = torch.cat([up_k, up_v]) if up_k.dtype == up_v.dtype == torch.bfloat16 and written_out(D, V, R, C) else None
+        out = up_k.dtype == up_v.dtype == torch.bfloat16 and P.supported(D, V, R, C) and P.values_fit(up_v, self.latent_norm, C)
+        self.kv_up = torch.cat([up_k, up_v]) if out else None
         self.up_v = (up_v if self.kv_up is None else self.kv_up[H * D:]).view(H, V, C).contiguous()
         self.out = Linear(tensors[self._n("o")], None, self._n("o"))
 

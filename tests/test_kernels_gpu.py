@@ -179,6 +179,25 @@ def test_many_token_rows_stored_wide_and_narrow(M, N, K, kind, cta_pairs):
     assert float((got[0].double() - ref).abs().max() / ref.abs().max()) <= tol
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 128, 136), (192, 640, 64), (257, 2048, 72), (1032, 4096, 136)])
+def test_product_with_keys_in_bf16_and_values_in_halves(M, N, K, cta_pairs):
+    """Left half of the columns bf16, right half IEEE halves; rows beside one another untouched, narrow rows included."""
+    from infero_b200.kernels import tc_gemm
+    a, w = _rand((M, K), torch.bfloat16, 1), _rand((N, K), torch.bfloat16, 2, 0.1)
+    ref = a.double() @ w.double().T
+    for pad, at in ((8, 0), (3, 1)):
+        big = torch.full((M + 2, N + pad), 7.0, dtype=torch.bfloat16, device=DEV)
+        out = big[1:M + 1, at:at + N]
+        tc_gemm.gemm_halves(a, w, out)
+        left, right = out[:, :N // 2].double(), out[:, N // 2:].contiguous().view(torch.float16).double()
+        # (half a unit in the last place, and the 32-bit sums' own error)
+        assert bool(((left - ref[:, :N // 2]).abs() <= ref[:, :N // 2].abs() * 2.0 ** -8 + 1e-4).all())
+        assert bool(((right - ref[:, N // 2:]).abs() <= ref[:, N // 2:].abs() * 2.0 ** -11 + 1e-4).all())
+        out.fill_(7.0)
+        assert bool((big == 7.0).all()), "wrote outside its rows or columns"
+    assert tc_gemm.error_flag() == 0
+
+
 @pytest.mark.parametrize("kind", ["f32", "bf16", "swiglu"])
 @pytest.mark.parametrize("M", [257, 271, 287, 511])
 def test_ragged_rows_of_the_widest_tiles(M, kind, cta_pairs, monkeypatch):

@@ -58,6 +58,46 @@ def test_portions_at_the_edges_of_tiles(H, D, R, C, page, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("H,D,R,C", [(16, 128, 64, 512), (8, 64, 32, 256)])
+@pytest.mark.parametrize("n", [16, 130])
+def test_written_out_is_no_further_from_64_bits(H, D, R, C, n, monkeypatch):
+    from test_gositar_gpu import _Latent
+    g = torch.Generator().manual_seed(n)
+    errors = []
+    for least in (1, 1 << 30):                          # written out, and through the latent rows
+        monkeypatch.setattr(P, "MIN_TOKENS", least)
+        a = _Latent("bfloat16", H, D, R, D, C, pairing="half", pages=n // 16 + 8, scale=2.0 / (H * D * C * (D + R)) ** 0.5)
+        if not errors:
+            h = torch.randn(n, a.d, generator=g).to(torch.bfloat16).float()
+            want = a.plain(h).cpu()
+        got = a.step([("x", h)])["x"].double().cpu()
+        errors.append(float((got - want).norm() / want.norm()))
+    assert errors[0] <= errors[1]
+
+
+def test_values_that_halves_hold():
+    w, norm = torch.full((3, 64), 10.0), torch.ones(64)              # 2-norm of a row: 80; of a latent row: 8
+    assert P.values_fit(w, norm, 64) and P.values_fit(w * 100, norm, 64)
+    w[1] *= 102                                                      # 65,280 in exact numbers, more with the latents rounded up
+    assert not P.values_fit(w, norm, 64) and P.values_fit(w, norm * 0.9, 64) and not P.values_fit(w * 0.9, norm * 2, 64)
+    assert not P.values_fit(w * float("nan"), norm, 64)
+
+
+@pytest.mark.gpu
+def test_values_that_halves_do_not_hold_keep_to_the_latent_rows():
+    from test_gositar_gpu import DEV, _Latent, _rel
+    for times in (1.0, 3.0e4):
+        a = _Latent("bfloat16", 2, 64, 32, 64, 128, seed=3, scale=0.06, pages=40)
+        name = a.part._n("up_v")
+        a.w[name] = a.w[name] * times
+        a.part.bind({k: v.to(DEV) for k, v in a.w.items()})
+        before = P.launches["steps"]
+        h = torch.randn(70, a.d, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).float()
+        assert _rel(a.step([("x", h)])["x"], a.plain(h)) < TOL
+        assert P.launches["steps"] == before + (times == 1.0)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("window", [1, 64, 100, 129])
 def test_windows_and_sinks(window, monkeypatch):
     import plain_dukolorn as PD
