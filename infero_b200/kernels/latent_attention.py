@@ -47,7 +47,8 @@ def few_ok(ctx, cache: torch.Tensor, n_tokens: int, D: int, R: int, C: int, w_k:
     """Do the first ``n_tokens`` tokens go through ``query_few`` and ``result_few``?  Up to 16 of them, each its request's only one,
     in bf16, in sizes those and the tensor-core attention take, with up-projections that start on 16 bytes."""
     from . import latent_mma
-    return (cache.dtype == w_k.dtype == w_v.dtype == torch.bfloat16 and w_k.data_ptr() % 16 == 0 and w_v.data_ptr() % 16 == 0 and n_tokens <= 16 and D % 32 == 0 and D <= 128 and latent_mma.ENABLED
+    return (n_tokens <= 16 and cache.dtype == w_k.dtype == w_v.dtype == torch.bfloat16 and D % 32 == 0 and D <= 128 and latent_mma.ENABLED
+            and w_k.data_ptr() % 16 == 0 and w_v.data_ptr() % 16 == 0
             and getattr(ctx, "h_q_len", None) is not None and len(ctx.h_q_len) >= n_tokens and all(int(n) == 1 for n in ctx.h_q_len[:n_tokens])
             and latent_mma.supported(C, R))
 

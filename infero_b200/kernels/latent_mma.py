@@ -6,6 +6,7 @@ single tokens behind one) to its tiled form, 64 / heads-per-CTA tokens a tile.  
 launched, where the kernel has no instance (sizes, element type) or the step gives no host copy of its lengths."""
 from __future__ import annotations
 
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong
 
@@ -18,8 +19,14 @@ MIN_CHUNK = int(os.environ.get("INFERO_LATENT_MIN_CHUNK", "64"))     # fewest ke
 launches = {"single": 0, "tiled": 0, "cut": 0}      # how often each form ran (tests look at it)
 
 
+@functools.lru_cache(maxsize=64)
 def supported(C: int, R: int) -> bool:
     return bool(lib().infero_latent_mma_supported(c_int(C), c_int(R)))
+
+
+@functools.lru_cache(maxsize=64)
+def heads_per_cta(H: int) -> int:
+    return int(lib().infero_latent_mma_heads(c_int(H)))
 
 
 def plan_splits(n_tok: int, head_blocks: int, visible: int, sms: int):
@@ -31,12 +38,12 @@ def plan_splits(n_tok: int, head_blocks: int, visible: int, sms: int):
     return chunk, -(-visible // chunk)
 
 
-def single(ctx, q_lat, q_rot, out, kv, table, n_dec, H, C, R, scale, window, sinks_log2, merge: bool = True):
+def single(ctx, q_lat, q_rot, out, kv, table, n_dec, H, C, R, scale, window, sinks_log2, merge: bool = True, common=None):
     """The leading ``n_dec`` single-token requests; (ranges, their results, their maxima and sums), merged into ``out`` unless
     ``merge`` is off and there is more than one range."""
     from .attention import _batch_shape
     from .tc_gemm import sm_count
-    cache, HC = kv.k, int(lib().infero_latent_mma_heads(c_int(H)))
+    HC = heads_per_cta(H)
     vis = _batch_shape(ctx)[1] if getattr(ctx, "kv_bound", None) is None else int(ctx.kv_bound)
     if window:
         vis = min(vis, int(window) + 31)                 # (ranges start at the tile of the lowest key seen)
@@ -48,7 +55,7 @@ def single(ctx, q_lat, q_rot, out, kv, table, n_dec, H, C, R, scale, window, sin
         part_o = torch.empty(n_dec * H * splits * C, dtype=torch.float32, device=q_lat.device)
         part_ml = torch.empty(n_dec * H * splits * 2, dtype=torch.float32, device=q_lat.device)
     _check(lib().infero_latent_attention_mma(_ptr(q_lat), _ptr(q_rot), c_longlong(q_lat.shape[1]), _ptr(out), _ptr(part_o), _ptr(part_ml),
-                                             *_common(ctx, cache, table), c_int(0), c_int(n_dec), c_int(n_dec), c_int(1), c_int(H), c_int(C),
+                                             *(common or _common(ctx, kv.k, table)), c_int(0), c_int(n_dec), c_int(n_dec), c_int(1), c_int(H), c_int(C),
                                              c_int(R), c_int(kv.page_size), c_float(scale), c_int(chunk), c_int(splits),
                                              c_int(window or 0), _ptr(sinks_log2), c_int(1 if merge else 0), _stream()))
     return splits, part_o, part_ml
@@ -69,16 +76,15 @@ def run(ctx, q_lat, q_rot, out, kv, table, n_tokens, H, C, R, scale, window=None
     if sinks is not None and sinks_log2 is None:
         sinks_log2 = sinks * 1.4426950408889634
     E = ctx.n_entries
-    HC = int(lib().infero_latent_mma_heads(c_int(H)))
-    rows = q_lat.shape[1]
+    rows, common = q_lat.shape[1], _common(ctx, cache, table)
     if n_dec:
-        single(ctx, q_lat, q_rot, out, kv, table, n_dec, H, C, R, scale, window, sinks_log2)
+        single(ctx, q_lat, q_rot, out, kv, table, n_dec, H, C, R, scale, window, sinks_log2, common=common)
     if n_dec < E and not singles_only:
-        TQ = 64 // HC
+        TQ = 64 // heads_per_cta(H)
         launches["tiled"] += 1
         tiles = sum(-(-int(n) // TQ) for n in ctx.h_q_len[n_dec:])
         _check(lib().infero_latent_attention_mma(_ptr(q_lat), _ptr(q_rot), c_longlong(rows), _ptr(out), _ptr(None), _ptr(None),
-                                                 *_common(ctx, cache, table), c_int(n_dec), c_int(E), c_int(tiles), c_int(0), c_int(H), c_int(C),
+                                                 *common, c_int(n_dec), c_int(E), c_int(tiles), c_int(0), c_int(H), c_int(C),
                                                  c_int(R), c_int(kv.page_size), c_float(scale), c_int(0), c_int(1),
                                                  c_int(window or 0), _ptr(sinks_log2), c_int(1), _stream()))
     return True

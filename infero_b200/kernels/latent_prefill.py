@@ -13,6 +13,7 @@ from . import _check, _i32, _ptr, _stream, lib
 KTILE, QROWS, BLOCK = 64, 128, 64
 MIN_TOKENS = 16            # of all portions together
 MAX_KEYS_PER_TOKEN = 4
+MIN_BESIDE = 1 << 31       # multiply-adds that writing out has to save where single tokens stand in front
 launches = {"steps": 0}    # (tests look at it)
 
 
@@ -42,19 +43,52 @@ def plan(ctx, dtype, H: int, D: int, V: int, R: int, C: int, window: Optional[in
     the memory: at most 16 D bytes a token and head, where the latent queries and results take 6 C + 4 V (C >= 2 D)."""
     if dtype != torch.bfloat16 or getattr(ctx, "h_q_len", None) is None or not supported(D, V, R, C):
         return None
-    E, n = ctx.n_entries, 0
-    while n < E and ctx.h_q_len[n] == 1:
+    lens, starts = [int(n) for n in ctx.h_q_len], [int(p) for p in ctx.h_pos0]
+    n = 0
+    while n < len(lens) and lens[n] == 1:
         n += 1
-    tokens = keys = tiles = 0
-    for e in range(n, E):
-        q, p0 = int(ctx.h_q_len[e]), int(ctx.h_pos0[e])
+    tokens = sum(lens[n:])
+    if tokens < MIN_TOKENS:
+        return None
+    keys = tiles = 0
+    for q, p0 in zip(lens[n:], starts[n:]):
         start = max(0, p0 - window + 1) // KTILE * KTILE if window else 0
-        tokens += q
         keys += -(-(p0 + q - start) // KTILE)
         tiles += -(-q // QROWS)
-    if tokens < MIN_TOKENS or keys * KTILE > MAX_KEYS_PER_TOKEN * tokens + KTILE * (E - n):
+    if keys * KTILE > MAX_KEYS_PER_TOKEN * tokens + KTILE * (len(lens) - n):
         return None
     return Plan(n, keys, tiles)
+
+
+def worth_it(ctx, p: Plan, H: int, D: int, V: int, C: int, window: Optional[int]) -> bool:
+    """Beside single tokens the portions' four launches come on top of the single tokens' own three to six, where everything
+    through the latent rows is seven together; such steps are never captured, so the host's launches bound them, and writing out has to
+    save more than these cost.  Four layers, through the latent rows and written out: 16 heads of 128, latent 512 (the line lies at 591
+    prompt tokens): 17 single tokens and 100 prompt tokens 1.61 and 1.92 ms, 17 + 400 1.64 and 1.85, 17 + 700 2.06 and 1.92, 2 + 400 1.55 and
+    1.58, 64 + 1,500 3.38 and 2.25; 8 of 64, latent 256 (1,182): 64 + 24 1.72 and 2.01, 17 + 700 1.45 and 1.73, 17 + 1,500 1.92 and 1.78."""
+    if p.first_entry == 0:
+        return True
+    pairs = 0
+    for q, p0 in zip(ctx.h_q_len[p.first_entry:], ctx.h_pos0[p.first_entry:]):
+        q, p0 = int(q), int(p0)
+        pairs += q * min(p0 + (q + 1) // 2, window or p0 + q)
+    return H * (2 * C - D - V) * pairs >= MIN_BESIDE
+
+
+def step_plan(ctx, dtype, H: int, D: int, V: int, R: int, C: int, window: Optional[int]) -> Optional[Plan]:
+    """The plan that the step's layers of these sizes go by, worked out by the first of them."""
+    memo = getattr(ctx, "_latent_plans", None)
+    if memo is None:
+        memo = {}
+        try:
+            ctx._latent_plans = memo
+        except AttributeError:          # a context that takes no new attributes
+            pass
+    key = (dtype, H, D, V, R, C, window)
+    if key not in memo:
+        p = plan(ctx, *key)
+        memo[key] = p if p is not None and worth_it(ctx, p, H, D, V, C, window) else None
+    return memo[key]
 
 
 def run(ctx, p: Plan, q: torch.Tensor, q_rot: torch.Tensor, kv, table: torch.Tensor, w_kv: torch.Tensor, gate: Optional[torch.Tensor],

@@ -123,7 +123,7 @@ class LatentAttention(Mixer):
             L.gated_group_norm(proj[:, :self.Q], None, self.q_norm, self.spec.norm_eps, 1, cq)
             q_src = self.q_up.forward(cq, out_dtype=torch.float32)
         attn = torch.empty((T, H * V), dtype=h.dtype, device=dev)
-        plan = P.plan(ctx, h.dtype, H, D, V, R, C, self.spec.window) if self.kv_up is not None else None
+        plan = P.step_plan(ctx, h.dtype, H, D, V, R, C, self.spec.window) if self.kv_up is not None else None
         singles = T if plan is None else plan.first_entry
         if singles:
             self._through_latents(ctx, A, proj, q_src, kv, table, slot, attn, singles, plan is not None)
@@ -134,16 +134,23 @@ class LatentAttention(Mixer):
     def _prepare(self, ctx, A, proj, q_src, kv, table, slot, t0, t1, rows, rot_block):
         """Norm, rotation and cache append of tokens t0 .. t1 - 1; their queries, head-major."""
         H, D, R, C = self.H, self.D, self.R, self.C
+        n, positions, tok_entry = t1 - t0, ctx.positions, ctx.tok_entry
+        if n < proj.shape[0]:                           # (steps that the host's work bounds come whole: no views of everything)
+            proj, positions, tok_entry = proj[t0:t1], positions[t0:t1], tok_entry[t0:t1]
+            q_src = None if q_src is None else q_src[t0:t1]
         q_plain = torch.empty((H, rows, D), dtype=kv.k.dtype, device=proj.device)
         q_rot = torch.empty((H, rows, 64 if rot_block else R), dtype=kv.k.dtype if rot_block else torch.float32, device=proj.device)
         freq = self.rope.inv_freq64(proj.device) if self.rope is not None else None
-        A.prepare(proj[t0:t1], self.q_off, self.kv_off, self.latent_norm, self.spec.norm_eps, freq, self.pairing, self.amp,
-                  ctx.positions[t0:t1], ctx.tok_entry[t0:t1], table, kv.k, kv.page_size, q_plain, q_rot, t1 - t0, H, D, R, C,
-                  write_cache=slot.write_cache, q_src=None if q_src is None else q_src[t0:t1], rot_block=rot_block)
+        A.prepare(proj, self.q_off, self.kv_off, self.latent_norm, self.spec.norm_eps, freq, self.pairing, self.amp,
+                  positions, tok_entry, table, kv.k, kv.page_size, q_plain, q_rot, n, H, D, R, C,
+                  write_cache=slot.write_cache, q_src=q_src, rot_block=rot_block)
         return q_plain, q_rot
 
     def _gate(self, proj, t0, t1):
-        return proj[t0:t1, self.gate_off:self.gate_off + self.H] if self.spec.out_gate else None
+        if not self.spec.out_gate:
+            return None
+        gate = proj[:, self.gate_off:self.gate_off + self.H]
+        return gate if t1 - t0 == proj.shape[0] else gate[t0:t1]
 
     def _through_latents(self, ctx, A, proj, q_src, kv, table, slot, attn, n, singles_only):
         """Tokens 0 .. n - 1 against the latent rows where they lie, the up-projections carried to the query side."""
@@ -172,7 +179,7 @@ class LatentAttention(Mixer):
                     singles_only=singles_only)
         val = torch.empty((H, rows, V), dtype=torch.float32, device=dev)
         A.per_head_product(o_lat, self.up_v, val, n)
-        A.finish(val, self._gate(proj, 0, n), attn[:n], n, H, V)
+        A.finish(val, self._gate(proj, 0, n), attn if n == attn.shape[0] else attn[:n], n, H, V)
 
     def _written_out(self, ctx, A, P, plan, proj, q_src, kv, table, slot, attn):
         """The portions behind the single tokens, their visible keys and values written out per head."""

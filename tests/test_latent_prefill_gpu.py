@@ -30,6 +30,21 @@ def test_the_rule(lens, pos0, window, want):
         assert P.plan(_ctx(lens, pos0), torch.bfloat16, 4, D, V, R, C, window) is None
 
 
+@pytest.mark.parametrize("lens,pos0,window,want", [
+    ([600], [0], None, True), ([1, 600], [40, 0], None, True), ([1, 500], [40, 0], None, False), ([1] * 64 + [24], [99] * 64 + [0], None, False),
+    ([1, 200, 300, 220], [7, 0, 0, 0], None, False), ([1, 200], [7, 500], None, False), ([1, 300], [7, 900], None, True),       # (pairs count)
+    ([1, 600], [40, 0], 256, False), ([1, 1500], [40, 0], 256, True),                  # a window bounds them
+])
+def test_beside_single_tokens_only_portions_that_are_worth_it(lens, pos0, window, want):
+    """16 heads of 128 with a latent of 512 save 12,288 multiply-adds a pair: from about 174,763 pairs on."""
+    args = (torch.bfloat16, 16, 128, 128, 64, 512, window)
+    ctx = _ctx(lens, pos0)
+    p = P.step_plan(ctx, *args)
+    assert (p is not None) == want and P.plan(ctx, *args) is not None
+    ctx.h_q_len = None                                               # (the layers behind the first one ask no more)
+    assert P.step_plan(ctx, *args) is p
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("H,D,R,C,page", [(16, 128, 64, 512, 16), (3, 64, 32, 256, 64), (2, 128, 8, 256, 16), (5, 64, 64, 136, 16)])
 def test_portions_at_the_edges_of_tiles(H, D, R, C, page, monkeypatch):
@@ -47,6 +62,7 @@ def test_portions_at_the_edges_of_tiles(H, D, R, C, page, monkeypatch):
             hs = {r: torch.randn(sum(n), a.d, generator=g).to(torch.bfloat16).float() for r, n in cuts.items()}
             want = {r: a.plain(h) for r, h in hs.items()}
         monkeypatch.setattr(P, "MIN_TOKENS", least)
+        monkeypatch.setattr(P, "MIN_BESIDE", 0)         # (single tokens in front or not)
         got, before = {r: [] for r in cuts}, P.launches["steps"]
         for i in range(3):
             entries = [(r, hs[r][sum(n[:i]):sum(n[:i]) + n[i]]) for r, n in cuts.items() if i < len(n)]
