@@ -208,39 +208,63 @@ __device__ __forceinline__ void merge_if_last(int* counter, float* wbuf, const f
 // length instead: every token gets ceil(keys / c) of them, c the fewest keys (in sixteens, at least the plan's least and no more
 // than its chunk) for which they suffice; the CTAs left over leave at once.  Every warp works it out for itself from the
 // positions, ahead of the wait for the kernel in front.  64 tokens behind 16 to 2,047 keys, 14 heads of 64 over 2: a step of 24
-// layers 1.34 ms in equal splits, 1.15 shared out.
+// layers 1.34 ms in equal splits, 1.15 shared out.  Where the plan's splits are full to seven eighths and more there is no more to
+// gain than the search costs, and they stay as they are.
 constexpr int BALANCED_TOKENS = 256, BALANCED_SPLITS = 256;       // (the merge keeps a weight per split in shared memory)
-struct Share { int token, split, splits, keys, first; };          // which token and split; splits of the token, keys of a split; CTAs of the tokens before
-__device__ __forceinline__ Share share_out(const int* __restrict__ positions, int n_tok, int chunk, int window, int least, int id, int budget, int lane) {
-    constexpr int PER = BALANCED_TOKENS / 32;
-    const int per = (n_tok + 31) / 32;                   // a lane has `per` neighbouring tokens
-    const int cover = budget / n_tok * chunk;            // (what the plan covers, in a token's keys)
-    int vis[PER], longest = 0;
+// A read at this place in the program, not where its result is first wanted.
+__device__ __forceinline__ int read_now(const int* p) {
+    int v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+// Which token and split; splits of the token, keys of a split, CTAs of the tokens before; the token's position.
+struct Share { int token, split, splits, keys, first, pos; };
+// Positions of a lane's tokens (`per` neighbouring ones), asked for ahead of everything else a block does.
+struct Lengths {
+    static constexpr int PER = BALANCED_TOKENS / 32;
+    int per, pos[PER];
+    __device__ __forceinline__ void ask(const int* positions, int n_tok, int lane) {
+        per = (n_tok + 31) / 32;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int t = lane * per + i;
-        vis[i] = 0;
-        if (i < per && t < n_tok) {
-            const int pos = positions[t], lo = window > 0 ? max(0, pos - window + 1) : 0;
-            vis[i] = min(cover, pos + 1 - lo / KEYS16 * KEYS16);
-            longest = max(longest, vis[i]);
+        for (int i = 0; i < PER; ++i) {
+            pos[i] = 0;
+            if (i < per) pos[i] = read_now(positions + min(lane * per + i, n_tok - 1));
         }
     }
+};
+struct Ceil {
+    unsigned int by, inverse;
+    __device__ __forceinline__ explicit Ceil(int c) : by(c), inverse(0xffffffffu / (unsigned)c + 1) {}
+    __device__ __forceinline__ int operator()(int v) const {
+        const unsigned int n = (unsigned)v + by - 1, q = __umulhi(n, inverse);         // right or one too many
+        return (int)(q - (q * by > n ? 1u : 0u));
+    }
+};
+struct Visible { int keys[Lengths::PER]; };               // of a lane's tokens
+// The sharing out itself, a call: its instructions would stand between a block's start and its body and be fetched there in every
+// layer, whether they are wanted or not (16 requests of 4,095 keys, 24 layers: 0.916 ms a step in place, 0.884 as a call, as without any).
+__device__ __noinline__ Share shared_out(const Visible vis, const Lengths of, int chunk, int budget, int id, int least, int lane) {
+    constexpr int PER = Lengths::PER;
+    const int per = of.per;
+    int longest = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) longest = max(longest, vis.keys[i]);
     longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)longest);
-    auto wanted = [&](int c) {                           // CTAs of this lane's tokens with c keys a split
+    auto wanted = [&](const Ceil splits) {               // CTAs of this lane's tokens
         int n = 0;
 #pragma unroll
         for (int i = 0; i < PER; ++i)
-            if (i < per) n += (vis[i] + c - 1) / c;
+            if (i < per) n += splits(vis.keys[i]);
         return n;
     };
     int hi = chunk, lo = min(chunk, max((least + 15) / 16 * 16, (longest / BALANCED_SPLITS + 16) / 16 * 16));
     while (lo < hi) {                                    // (hi always suffices; both are multiples of 16)
         const int mid = (lo + hi) / 32 * 16;
-        if ((int)__reduce_add_sync(0xffffffffu, (unsigned)wanted(mid)) <= budget) hi = mid;
+        if ((int)__reduce_add_sync(0xffffffffu, (unsigned)wanted(Ceil(mid))) <= budget) hi = mid;
         else lo = mid + 16;
     }
-    const int mine = wanted(hi);
+    const Ceil splits(hi);
+    const int mine = wanted(splits);
     int before = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -249,23 +273,38 @@ __device__ __forceinline__ Share share_out(const int* __restrict__ positions, in
     }
     before -= mine;
     const unsigned owner = __ballot_sync(0xffffffffu, id >= before && id < before + mine);
-    Share s = {-1, 0, 0, hi, 0};
+    Share s = {-1, 0, 0, hi, 0, 0};
     if (owner) {
-        int at = before, token = 0, first = 0, splits = 1;
+        int at = before, token = 0, first = 0, n_splits = 1, pos = 0;
 #pragma unroll
         for (int i = 0; i < PER; ++i)
             if (i < per) {
-                const int n = (vis[i] + hi - 1) / hi;
-                if (id >= at && id < at + n) token = lane * per + i, first = at, splits = n;
+                const int n = splits(vis.keys[i]);
+                if (id >= at && id < at + n) token = lane * per + i, first = at, n_splits = n, pos = of.pos[i];
                 at += n;
             }
         const int src = __ffs(owner) - 1;
         s.token = __shfl_sync(0xffffffffu, token, src);
         s.first = __shfl_sync(0xffffffffu, first, src);
-        s.splits = __shfl_sync(0xffffffffu, splits, src);
+        s.splits = __shfl_sync(0xffffffffu, n_splits, src);
+        s.pos = __shfl_sync(0xffffffffu, pos, src);
         s.split = id - s.first;
     }
     return s;
+}
+__device__ __forceinline__ Share share_out(const Share plan, const Lengths& of, int n_tok, int window, int least, int lane) {
+    const int budget = n_tok * plan.splits, cover = plan.splits * plan.keys;          // cover: what the plan does of a token's keys
+    Visible vis;
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < Lengths::PER; ++i) {
+        const int lo = window > 0 ? max(0, of.pos[i] - window + 1) : 0;
+        vis.keys[i] = i < of.per && lane * of.per + i < n_tok ? max(0, min(cover, of.pos[i] + 1 - lo / KEYS16 * KEYS16)) : 0;
+        total += vis.keys[i];
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (8ll * total >= 7ll * budget * plan.keys) return plan;
+    return shared_out(vis, of, plan.keys, budget, plan.first + plan.split, least, lane);
 }
 
 // partial_o [n_tok, n_heads, n_splits, D] float (unnormalised), partial_ml [n_tok, n_heads, n_splits, 2]; shared out by length, a
@@ -298,6 +337,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     TL_BEGIN();
+    // positions and block tables are set before the step's first kernel, and every cached key
+    // but the token's own was written by earlier steps: all of that may be read before the
+    // kernel in front (which writes q and the token's own key and value) has finished
+    int pos = read_now(positions + tok_first + blockIdx.z), entry = read_now(tok_entry + tok_first + blockIdx.z);
+    Lengths lengths;
+    if (SHARED) lengths.ask(positions + tok_first, (int)gridDim.z, lane);
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         tc::prefetch_tensormap(&map_k);
@@ -307,15 +352,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         tc::fence_barrier_init();
         tc::fence_proxy_async();
     }
-    // positions and block tables are set before the step's first kernel, and every cached key
-    // but the token's own was written by earlier steps: all of that may be read before the
-    // kernel in front (which writes q and the token's own key and value) has finished
     int split = blockIdx.x, ti = blockIdx.z, splits_before = ti * n_splits;
     if (SHARED) {                                                     // the splits are shared out by length
-        const Share s = share_out(positions + tok_first, (int)gridDim.z, chunk, window, least, (int)(blockIdx.z * gridDim.x + blockIdx.x),
-                                  (int)(gridDim.z * gridDim.x), lane);
+        const Share s = share_out(Share{ti, split, n_splits, chunk, splits_before, pos}, lengths, (int)gridDim.z, window, least, lane);
         if (s.token < 0) return;                                      // (uniform over the block)
-        split = s.split, ti = s.token, chunk = s.keys, n_splits = s.splits, splits_before = s.first;
+        if (s.token != ti) entry = tok_entry[tok_first + s.token];
+        split = s.split, ti = s.token, chunk = s.keys, n_splits = s.splits, splits_before = s.first, pos = s.pos;
     }
     const int group = n_heads / n_kv;
     const int gtiles = (group + 15) / 16;
@@ -323,8 +365,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const int vh = fq.ex.cross ? blockIdx.y / (gtiles * n_kv) : kvh;  // the kv head whose values are summed
     const int rows = fq.ex.cross ? n_heads * n_kv : n_heads;          // result rows per token
     const int t = tok_first + ti;
-    const int pos = positions[t];
-    const int* table = block_table + (size_t)tok_entry[t] * max_blocks;
+    const int* table = block_table + (size_t)entry * max_blocks;
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int base = (lo / KEYS16) * KEYS16;
     const int k_begin = base + split * chunk;
