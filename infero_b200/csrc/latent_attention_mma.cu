@@ -10,7 +10,7 @@
 // forms the rows' scores with its share of a tile's 32 keys, they exchange the rows' maxima and their softmax weights
 // (as tensor-core fragments, whose layout is the same lane by lane) through shared memory, and each owns its share of the
 // C result columns, so the result tile of 16 x C/2 (or C/4) stays in registers.  Key tiles start at multiples of 32 of the absolute position, so what is
-// computed for a token does not depend on how its prompt was cut.
+// computed for a token here does not depend on how its prompt was cut (which route a portion takes does: kernels/latent_prefill.py).
 //
 // With a window every row has a lowest key too, and the ranges start at the tile of the first row's lowest key; a learned sink
 // per head is one more term of the rows' sums, added where a row's result is divided by its sum.
