@@ -37,6 +37,7 @@ gated matrix memory) of the same width, depth, head counts, memory sizes and fee
 from __future__ import annotations
 
 import argparse
+import gc
 import json
 import os
 import random
@@ -232,6 +233,8 @@ class _Timer:
             # a kernel alone: replayed from a captured graph, so that the host's share of a launch is not timed
             fn()
             torch.cuda.synchronize()
+            was_enabled = gc.isenabled()
+            gc.disable()                               # (an old graph that the collector frees meanwhile invalidates a capture)
             try:
                 graph = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(graph):
@@ -241,6 +244,9 @@ class _Timer:
                 fn = graph.replay
             except Exception:                          # noqa: BLE001  (something in fn cannot be captured: time it as it is)
                 torch.cuda.synchronize()
+            finally:
+                if was_enabled:
+                    gc.enable()
         times = []
         for i in range(warmup + reps):
             if setup:
@@ -444,7 +450,7 @@ def time_gositar_kernels(z, T, context, batch, timer, peaks):
     import numpy as np
     import torch
     from infero_b200 import kernels as K
-    from infero_b200.kernels import attention as A, latent_attention as LA, layer_ops as L, moe as M, tc_gemm
+    from infero_b200.kernels import attention as A, latent_attention as LA, latent_prefill as LP, layer_ops as L, moe as M, tc_gemm
     from infero_b200.parts.linear import Linear
     dev, bf = "cuda:0", torch.bfloat16
     d, H, D, R, V, C, S = z["width"], z["heads"], z["dim"], z["rot"], z["vdim"], z["rank"], z["streams"]
@@ -494,6 +500,13 @@ def time_gositar_kernels(z, T, context, batch, timer, peaks):
         ms = timer(lambda: LA.attention(ctx, q_lat, q_rot, o_lat, kv, table, n, H, C, R, (D + R) ** -0.5))
         note(f"latent_attention_{label}", ms, 2.0 * (C + R) * keys + n * H * (4.0 * (C + R) + 2.0 * C), 2.0 * H * (2 * C + R) * pairs)
         rows[f"latent_attention_{label}"]["unabsorbed_tflops"] = round(2.0 * H * (D + R + V) * pairs / ms / 1e9, 1)
+        # ---- keys and values written out (what a prompt step takes): gather, product, attention ---------------------
+        written = LP.plan(ctx, bf, H, D, V, R, C, None)
+        if written is not None:
+            q_out, qr_out, w_kv, res = rnd(H, n, D), rnd(H, n, 64), rnd(2 * H * D, C, k=0.05), torch.empty(n, H * V, dtype=bf, device=dev)
+            ms = timer(lambda: LP.run(ctx, written, q_out, qr_out, kv, table, w_kv, None, res, H, D, R, C, (D + R) ** -0.5, None, None))
+            note(f"latent_written_out_{label}", ms, 2.0 * (C + R) * keys + n * H * (2.0 * (D + R) + 2.0 * V) + 2.0 * 2 * H * D * C,
+                 2.0 * keys * C * 2 * H * D + 2.0 * H * (D + R + V) * pairs)
         # ---- the per-head products around it -----------------------------------------------------------------------
         q_plain, up_k = rnd(H, rows_h, D), rnd(H, C, D, k=0.05)
         ms = timer(lambda: LA.per_head_product(q_plain, up_k, q_lat, n))

@@ -45,6 +45,37 @@ def test_one_kernel_alone():
     assert "attn_decode_fused:" in out and "us per launch" in out and "error flag" not in out
 
 
+def test_old_graphs_are_not_collected_while_the_design_bench_captures():
+    """Runners sit in reference cycles with their captured graphs; one that the collector frees during another capture ends it."""
+    import gc
+
+    import torch
+    from infero_b200.tools.design_bench import _Timer
+    x = torch.zeros(8, device="cuda:0")
+
+    class Runner:
+        pass
+
+    def garbage():
+        old = Runner()
+        old.me, old.graph = old, torch.cuda.CUDAGraph()
+        with torch.cuda.graph(old.graph):
+            x.add_(1.0)
+
+    calls = []
+
+    def work():
+        calls.append(torch.cuda.is_current_stream_capturing())
+        if calls[-1]:
+            assert not gc.isenabled()
+        x.add_(1.0)
+
+    garbage()
+    assert _Timer()(work, reps=1, warmup=1) > 0
+    assert calls == [False, True] and gc.isenabled()                 # (captured once, replayed from then on)
+    assert torch.rand(4, device="cuda:0").shape == (4,)
+
+
 def test_design_bench_prints_both_designs_and_the_kernels(capsys):
     """``bench.py --designs`` at a size made for tests: both models step, every kernel row has a time."""
     import json
