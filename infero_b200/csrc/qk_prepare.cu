@@ -25,6 +25,9 @@
 // may put on its result.
 #include "common.cuh"
 
+// (These launch the ordinary way, behind the whole of the kernel in front: launched early they let attention's blocks in while the
+// product still ran, and a step of eight tokens took 0.354 ms instead of 0.337 on Banelix's smallest layers, 0.538 instead of 0.513 on
+// Pibavik's.)
 namespace {
 
 constexpr int THREADS = 256;
@@ -37,8 +40,6 @@ qk_prepare_kernel(const float* __restrict__ proj, int proj_stride, int q_off, in
                   const int* __restrict__ tok_entry, const int* __restrict__ block_table, int max_blocks, int page_size,
                   T* __restrict__ q_out, int q_stride, T* __restrict__ k_cache, T* __restrict__ v_cache, int write_cache,
                   int H, int G, int D, int V, float temp_coef, float temp_every, float v_scale) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float smem[];
     __shared__ float red[32];
     const int half = rot / 2;
@@ -140,8 +141,6 @@ qk_prepare_kernel(const float* __restrict__ proj, int proj_stride, int q_off, in
 template <typename T>
 __global__ void head_gate_kernel(const T* __restrict__ a, int a_stride, const float* __restrict__ gate, int gate_stride,
                                  T* __restrict__ out, int out_stride, int n_tokens, int H, int V, float scale) {
-    pdl_launch_dependents();
-    pdl_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)n_tokens * H * V) return;
     const int t = (int)(i / (H * V)), c = (int)(i % (H * V)), h = c / V;
@@ -153,8 +152,6 @@ __global__ void head_gate_kernel(const T* __restrict__ a, int a_stride, const fl
 // Eight neighbouring columns a thread (they lie in one head when V is a multiple of 8): 16-byte loads and stores.
 __global__ void head_gate_vec_kernel(const bf16* __restrict__ a, int a_stride, const float* __restrict__ gate, int gate_stride,
                                      bf16* __restrict__ out, int out_stride, int n_tokens, int H, int V, float scale) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int per_row = H * V / 8;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)n_tokens * per_row) return;
@@ -194,7 +191,7 @@ int infero_qk_prepare(const float* proj, int proj_stride, int q_off, int k_off, 
     do {                                                                                                                 \
         auto k = qk_prepare_kernel<T>;                                                                                   \
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
-        launch_pdl(k, dim3(n_tokens), dim3(THREADS), smem, stream, proj, proj_stride, q_off, k_off, v_off, norm_mode, q_norm_w, k_norm_w,    \
+        k<<<n_tokens, THREADS, smem, stream>>>(proj, proj_stride, q_off, k_off, v_off, norm_mode, q_norm_w, k_norm_w,    \
                                                norm_w_dtype, eps, freq, rot, amp, positions, tok_entry, block_table,      \
                                                max_blocks, page_size, (T*)q_out, q_stride, (T*)k_cache, (T*)v_cache,      \
                                                write_cache, H, G, D, V, temp_coef, temp_every, v_scale);                                                  \
@@ -212,15 +209,15 @@ int infero_head_gate(const void* a, int a_stride, const float* gate, int gate_st
     const unsigned blocks = (unsigned)((total + 255) / 256);
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (dtype != INFERO_F32 && V % 8 == 0 && a_stride % 8 == 0 && out_stride % 8 == 0 && al16(a) && al16(out)) {
-        launch_pdl(head_gate_vec_kernel, dim3((unsigned)((total / 8 + 255) / 256)), dim3(256), 0, stream, (const bf16*)a, a_stride, gate, gate_stride,
+        head_gate_vec_kernel<<<(unsigned)((total / 8 + 255) / 256), 256, 0, stream>>>((const bf16*)a, a_stride, gate, gate_stride,
                                                                                      (bf16*)out, out_stride, n_tokens, H, V, scale);
         return infero_check_launch("head_gate");
     }
     if (dtype == INFERO_F32)
-        launch_pdl(head_gate_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)a, a_stride, gate, gate_stride, (float*)out,
+        head_gate_kernel<float><<<blocks, 256, 0, stream>>>((const float*)a, a_stride, gate, gate_stride, (float*)out,
                                                              out_stride, n_tokens, H, V, scale);
     else
-        launch_pdl(head_gate_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, (const bf16*)a, a_stride, gate, gate_stride, (bf16*)out,
+        head_gate_kernel<bf16><<<blocks, 256, 0, stream>>>((const bf16*)a, a_stride, gate, gate_stride, (bf16*)out,
                                                             out_stride, n_tokens, H, V, scale);
     return infero_check_launch("head_gate");
 }
