@@ -1,8 +1,8 @@
 // Matrix products on the ordinary cores: out[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
 //
 //  * gemm_tiled: any shape, any mix of float / bf16 operands, 32-bit accumulation with one
-//    fused multiply-add per k in ascending k.  The value of out[m,n] therefore does not
-//    depend on M, on the tile it falls in or on its batch-mates: this is the product of the
+//    fused multiply-add per k, in an order that depends on K alone.  The value of out[m,n] therefore
+//    does not depend on M, on the tile it falls in or on its batch-mates: this is the product of the
 //    true 32-bit path (no reduced-precision matrix mode anywhere).
 //  * gemm_skinny: up to 4 rows of A (decode at tiny batch): one warp per pair of output
 //    features streams the weight rows with 16-byte loads.  The reference switches to its
@@ -18,94 +18,171 @@ namespace {
 // One block works out BM x BN results, TM x TN a thread.  Both operands keep their rows in shared memory as they lie in
 // memory ([row][k], rows padded by 16 bytes): a stage of BK columns arrives by 16-byte asynchronous copies, STAGES - 1 stages
 // ahead, and a thread reads four k of a row at a time.  Thread (ty, tx) has rows ty + i * (BM / TM) and columns
-// tx + j * (BN / TN), so that eight neighbouring lanes read eight neighbouring rows, whose starts lie 4 banks apart
-// (BK + 4 is an odd multiple of 4): no bank conflict.  Operands that 16-byte copies cannot take (bf16, rows that
-// start anywhere) come by plain loads into the same ring.
-// Every result is one chain of fused multiply-adds in ascending k whatever the tile, so the choice of a tile never
-// shows in the numbers.
+// tx + j * (BN / TN); a warp is eight threads wide and four high where there are so many rows, so that eight neighbouring lanes
+// read eight neighbouring rows, whose starts lie 4 banks apart (BK + 4 is an odd multiple of 4): no bank conflict.  Operands that
+// 16-byte copies cannot take (bf16, rows that start anywhere) come by plain loads into the same ring.
+//
+// K is cut into parts of equal length that depend on K alone (parts_of).  A part's result is two chains of fused multiply-adds,
+// over its even and its odd k in ascending order (one instruction takes a step of both), and their sum; a result is the sum of its
+// parts in ascending order.  That holds whatever the tile and whether a block runs through all parts or (SPLIT) the blocks of a
+// cluster take one each and add them up through each other's shared memory, so the choice never shows in the numbers.  Against
+// 64-bit products of normal numbers: 2.7e-7 (2-norm) at K = 896 and 3.2e-7 at 4,864; one chain in ascending k had 5.4e-7 and 1.3e-6.
 template <int BM, int BN, int TM, int TN, int BK, int STAGES>
 struct Tile {
     static constexpr int TX = BN / TN, TY = BM / TM, WORK = TX * TY, THREADS = WORK < 32 ? 32 : WORK;
+    static constexpr int LY = TY < 4 ? TY : 4, LX = WORK < 32 ? TX : 32 / LY;              // a warp has LX x LY threads
     static constexpr int LD = BK + 4, A_FLOATS = BM * LD, STAGE = (BM + BN) * LD;
-    static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float);
+    static constexpr int Q = BK / 4, ROWS = THREADS / Q;                                   // rows that one round of copies covers
+    static constexpr int FLOATS = STAGES * STAGE > BM * BN ? STAGES * STAGE : BM * BN;     // (a part's results take the ring's place)
+    static constexpr size_t SMEM = (size_t)FLOATS * sizeof(float);
     static_assert(SMEM <= 48 * 1024, "more shared memory than a launch gets without asking");
-    static_assert(BK % 4 == 0 && (BK / 4) % 2 == 0, "");
+    static_assert(BK % 4 == 0 && (BK / 4) % 2 == 0 && THREADS % Q == 0, "");
+    static_assert(TX % LX == 0 && TY % LY == 0, "");
 };
 
-__device__ __forceinline__ void copy16(float* dst, const float* src, bool ok) {
-    const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
-    const int bytes = ok ? 16 : 0;                          // (nothing is read of a row that is not there: zeros)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+constexpr int PART = 640, MAX_SPLIT = 8;
+struct Parts { int n, len; };
+Parts parts_of(int K) {
+    const int n = (K + PART - 1) / PART, len = ((K + n - 1) / n + 31) / 32 * 32;
+    return {(K + len - 1) / len, len};
 }
 
-// ROWS rows of BK columns from column k0 on
-template <int ROWS, int BK, int LD, int THREADS, bool VEC, typename T>
-__device__ __forceinline__ void fill(float* dst, const T* src, int row0, int n_rows, int k0, int K, long long ld, int tid) {
-    if constexpr (VEC) {
-        constexpr int Q = BK / 4;
-        for (int e = tid; e < ROWS * Q; e += THREADS) {
-            const int r = e / Q, k = k0 + (e % Q) * 4;
-            const bool ok = row0 + r < n_rows && k < K;     // (K is a multiple of 4 here)
-            copy16(dst + r * LD + (e % Q) * 4, ok ? src + (long long)(row0 + r) * ld + k : src, ok);
-        }
-    } else {
-        for (int e = tid; e < ROWS * BK; e += THREADS) {
-            const int r = e / BK, k = k0 + e % BK;
-            dst[r * LD + e % BK] = row0 + r < n_rows && k < K ? to_f32(src[(long long)(row0 + r) * ld + k]) : 0.f;
-        }
+// a + b * c for two numbers at a time, each rounded once
+__device__ __forceinline__ void fma2(unsigned long long& a, unsigned long long b, unsigned long long c) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(b), "l"(c));
+}
+
+// The rows of an operand in a stage, zeros from column k_end on and where there is no row.  This thread copies 16 bytes of every
+// STEP-th row from row `row` on, src being its place in the first of them.
+template <int ROWS, int LD, int STEP>
+__device__ __forceinline__ void copy_rows(unsigned int dst, const float* src, const float* any, long long ld, int row, int n_rows, bool in) {
+#pragma unroll
+    for (int i = 0; i < (ROWS + STEP - 1) / STEP; ++i, src += ld * STEP) {
+        if (ROWS % STEP != 0 && row + i * STEP >= ROWS) break;
+        const bool ok = in && row + i * STEP < n_rows;          // (nothing is read of a row that is not there)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * STEP * LD * 4), "l"(ok ? src : any), "r"(ok ? 16 : 0) : "memory");
     }
 }
+template <int ROWS, int BK, int LD, int THREADS, typename T>
+__device__ __forceinline__ void widen_rows(float* dst, const T* src, int row0, int n_rows, int k0, int k_end, long long ld, int tid) {
+    for (int e = tid; e < ROWS * BK; e += THREADS) {
+        const int r = e / BK, k = k0 + e % BK;
+        dst[r * LD + e % BK] = row0 + r < n_rows && k < k_end ? to_f32(src[(long long)(row0 + r) * ld + k]) : 0.f;
+    }
+}
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
-template <typename TL, int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC, typename TA, typename TW, typename TC>
+template <typename TL, int BM, int BN, int TM, int TN, int BK, int STAGES, bool SPLIT, bool VEC, typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(TL::THREADS)
 gemm_tiled_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const void* __restrict__ bias,
-                  int bias_dtype, TC* __restrict__ C, int M, int N, int K, int lda, int ldc) {
+                  int bias_dtype, TC* __restrict__ C, int M, int N, int K, int lda, int ldc, int part_len) {
     extern __shared__ float4 ring4[];
     float* ring = reinterpret_cast<float*>(ring4);
     constexpr int LD = TL::LD;
-    const int tid = threadIdx.x;
-    const int ty = tid / TL::TX, tx = tid % TL::TX;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int ty = warp / (TL::TX / TL::LX) * TL::LY + lane / TL::LX, tx = warp % (TL::TX / TL::LX) * TL::LX + lane % TL::LX;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const bool works = TL::WORK == TL::THREADS || tid < TL::WORK;
-    const int n_stages = (K + BK - 1) / BK;
-    auto load = [&](int s) {
-        if (s < n_stages) {
-            float* at = ring + (s % STAGES) * TL::STAGE;
-            fill<BM, BK, LD, TL::THREADS, VEC>(at, A, m0, M, s * BK, K, lda, tid);
-            fill<BN, BK, LD, TL::THREADS, VEC>(at + TL::A_FLOATS, W, n0, N, s * BK, K, K, tid);
+    const int k_first = SPLIT ? blockIdx.z * part_len : 0, k_last = SPLIT ? min(K, k_first + part_len) : K;
+    const int row = tid / TL::Q, col = tid % TL::Q * 4;
+    const TA* a_src = A + (long long)(m0 + row) * lda + col;
+    const TW* w_src = W + (long long)(n0 + row) * K + col;
+    const unsigned int ring_at = (unsigned int)__cvta_generic_to_shared(ring);
+    int next_k = k_first, next_end = min(K, k_first + part_len), slot = 0;      // the next stage to load
+    auto load = [&]() {
+        if (next_k < k_last) {
+            if constexpr (VEC) {
+                const unsigned int dst = ring_at + (slot * TL::STAGE + row * LD + col) * 4;
+                const bool in = next_k + col < next_end;        // (K is a multiple of 4 here)
+                copy_rows<BM, LD, TL::ROWS>(dst, a_src + next_k, A, lda, row, M - m0, in);
+                copy_rows<BN, LD, TL::ROWS>(dst + TL::A_FLOATS * 4, w_src + next_k, W, K, row, N - n0, in);
+            } else {
+                float* at = ring + slot * TL::STAGE;
+                widen_rows<BM, BK, LD, TL::THREADS>(at, A, m0, M, next_k, next_end, lda, tid);
+                widen_rows<BN, BK, LD, TL::THREADS>(at + TL::A_FLOATS, W, n0, N, next_k, next_end, K, tid);
+            }
+            next_k += BK;
+            if (next_k >= next_end) next_k = next_end, next_end = min(K, next_end + part_len);
+            slot = slot + 1 == STAGES ? 0 : slot + 1;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[TM][TN];
+    float sum[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-    for (int s = 0; s < STAGES - 1; ++s) load(s);
-    for (int s = 0; s < n_stages; ++s) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncthreads();                                    // stage s is here, and everyone is done with stage s - 1,
-        load(s + STAGES - 1);                               // whose place this fills
-        if (!works) continue;
-        const float* a_s = ring + (s % STAGES) * TL::STAGE + ty * LD;
-        const float* w_s = ring + (s % STAGES) * TL::STAGE + TL::A_FLOATS + tx * LD;
+        for (int j = 0; j < TN; ++j) sum[i][j] = 0.f;
+    for (int s = 0; s < STAGES - 1; ++s) load();
+    int here = 0, first = k_first;
+    do {                                                        // a part
+        const int end = min(K, first + part_len);
+        unsigned long long acc[TM][TN];
 #pragma unroll
-        for (int k = 0; k < BK; k += 4) {
-            float4 w[TN];
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(w_s + j * TL::TX * LD + k);
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+        for (int k0 = first; k0 < end; k0 += BK) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();                                    // this stage is here, and everyone is done with the one before,
+            load();                                             // whose place this fills
+            const float* a_s = ring + here * TL::STAGE + ty * LD;
+            const float* w_s = ring + here * TL::STAGE + TL::A_FLOATS + tx * LD;
+            here = here + 1 == STAGES ? 0 : here + 1;
+            if (!works) continue;
 #pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(a_s + i * TL::TY * LD + k);
+            for (int k = 0; k < BK; k += 4) {
+                ulonglong2 w[TN], a[TM];
 #pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    acc[i][j] = fmaf(a.x, w[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(a.y, w[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(a.z, w[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(a.w, w[j].w, acc[i][j]);
-                }
+                for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + j * TL::TX * LD + k);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * TL::TY * LD + k);
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) fma2(acc[i][j], a[i].x, w[j].x);
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) fma2(acc[i][j], a[i].y, w[j].y);
             }
         }
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) sum[i][j] += __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+        first = end;
+    } while (!SPLIT && first < K);
+    if constexpr (SPLIT) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                        // the ring's place is free: this block's part of the results
+        if (works) {
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) ring[(ty + i * TL::TY) * BN + tx + j * TL::TX] = sum[i][j];
+        }
+        cluster_meet();
+        for (int e = blockIdx.z * TL::THREADS + tid; e < BM * BN; e += gridDim.z * TL::THREADS) {
+            const int gm = m0 + e / BN, gn = n0 + e % BN;
+            if (gm >= M || gn >= N) continue;
+            float part[MAX_SPLIT], v = 0.f;
+#pragma unroll
+            for (int p = 0; p < MAX_SPLIT; ++p)
+                if (p < gridDim.z) {
+                    unsigned int at;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(ring_at + e * 4), "r"(p));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[p]) : "r"(at) : "memory");
+                }
+#pragma unroll
+            for (int p = 0; p < MAX_SPLIT; ++p)
+                if (p < gridDim.z) v += part[p];
+            if (bias) v += load_any(bias, bias_dtype, gn);
+            C[(size_t)gm * ldc + gn] = from_f32<TC>(v);
+        }
+        cluster_meet();                                         // nobody's part goes before it has been read
+        return;
     }
     if (!works) return;
 #pragma unroll
@@ -116,7 +193,7 @@ gemm_tiled_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const void
         for (int j = 0; j < TN; ++j) {
             const int gn = n0 + tx + j * TL::TX;
             if (gn >= N) continue;
-            float v = acc[i][j];
+            float v = sum[i][j];
             if (bias) v += load_any(bias, bias_dtype, gn);
             C[(size_t)gm * ldc + gn] = from_f32<TC>(v);
         }
@@ -179,40 +256,66 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, const
         }
 }
 
-template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC, typename TA, typename TW, typename TC>
+template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool SPLIT, bool VEC, typename TA, typename TW, typename TC>
 int launch_tile(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N,
                 int K, int lda, int ldc, cudaStream_t stream) {
     using TL = Tile<BM, BN, TM, TN, BK, STAGES>;
-    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_tiled_kernel<TL, BM, BN, TM, TN, BK, STAGES, VEC, TA, TW, TC><<<grid, TL::THREADS, TL::SMEM, stream>>>(
-        (const TA*)A, (const TW*)W, bias, bias_dtype, (TC*)C, M, N, K, lda, ldc);
+    const Parts parts = parts_of(K);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, SPLIT ? parts.n : 1);
+    cfg.blockDim = TL::THREADS;
+    cfg.dynamicSmemBytes = TL::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = parts.n;
+    cfg.attrs = attr;
+    cfg.numAttrs = SPLIT ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, gemm_tiled_kernel<TL, BM, BN, TM, TN, BK, STAGES, SPLIT, VEC, TA, TW, TC>,
+                       (const TA*)A, (const TW*)W, bias, bias_dtype, (TC*)C, M, N, K, lda, ldc, parts.len);
     return infero_check_launch("gemm_tiled");
 }
 
-// The tile.  Few rows: a block streams rows of W past all rows of A; where N is small, few rows of W a block, so that every
-// SM streams some (1 x 896, K = 4,864: 25 us with 8 rows of W a block, 37 with 16, 47 with 32; the chain alone is 10).  Many
-// rows: the largest tile that still gives nearly every SM a block (301 x 9,728, K = 896: 157 us with 64 x 128, 178 with
-// 64 x 64; 301 x 896, K = 4,864: 144 with 32 x 32, 166 with twice the results a thread; 64 x 896: 60 with 32 x 16, 112 with
-// 32 x 32).  In large products the bound is the rate at which shared memory feeds the multiply-adds (42 TFLOP/s of the 74 that
-// the cores have; pairs of multiply-adds in one instruction need more moves than they save: 1,160 against 840 us at
-// 2,048 x 9,728).  Before, with one 64 x 64 tile and loads waited for in place: 1 x 896, K = 4,864 342 us, 301 x 9,728 285 us,
-// 2,048 x 9,728 1,512 us, 1 x 151,936 782 us (now 95: 5.7 TB/s).
+// The tile.  Few rows: a block streams rows of W past all rows of A; where N is small, few rows of W a block and a block per part
+// of K, so that every multiprocessor streams some and no chain is long (us, before one block ran one chain over all of K: 1 x 896,
+// K = 4,864 25 and 8.4; 8 rows 33 and 13; 1 x 1,152, K = 896 6.8 and 6.3); where N alone gives four blocks a multiprocessor, all
+// parts to a block (8 x 151,936, K = 896 132, split 146; before 228).  Many rows: the largest tile that gives three blocks a
+// multiprocessor, 64 rows only where they are not much more than 32 would be (301 x 896, K = 4,864: 148 before, 73 with 64 x 64,
+// 104 with 32 x 64; 301 x 9,728, K = 896: 156 before, 138 and 141; 150 x 9,728 121 before, 93 with 32 x 64; 301 x 1,152 35 before,
+// 29 with 32 x 32, 31 with 32 x 64; 64 x 896 14.5 before, 12.4 with four results a thread, 14.4 with eight).  In large products
+// (2,048 x 9,728, K = 896: 857 before, 795 now) the bound is the rate of the paired multiply-adds, two thirds of it reached.
 template <bool VEC, typename TA, typename TW, typename TC>
 int launch_tiled(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N,
                  int K, int lda, int ldc, cudaStream_t stream) {
-#define TILE(...) return launch_tile<__VA_ARGS__, VEC, TA, TW, TC>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, stream)
-    const int enough = infero_sm_count() * 7 / 8;
+    // (operands that are widened on the way come with all parts to a block)
+#define TILE(...)                                                                                                                      \
+    do {                                                                                                                               \
+        if constexpr (VEC)                                                                                                             \
+            if (split) return launch_tile<__VA_ARGS__, true, VEC, TA, TW, TC>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, stream);   \
+        return launch_tile<__VA_ARGS__, false, VEC, TA, TW, TC>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, stream);                 \
+    } while (0)
+    const int parts = parts_of(K).n, sms = infero_sm_count();
+    bool split = VEC && parts >= 2 && parts <= MAX_SPLIT;
+    const int by = split ? parts : 1;
     auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
     if (M <= 16) {
-        const bool narrow = blocks(16, 32) < 2 * enough;
+        const bool narrow = blocks(16, 32) < 2 * sms;
+        split = split && blocks(16, 32) < 4 * sms;
+        if (M == 1 && narrow && split) TILE(1, 16, 1, 1, 128, 4);
         if (M == 1 && narrow) TILE(1, 8, 1, 1, 128, 6);
-        if (narrow) TILE(16, 8, 1, 1, 64, 4);
         if (M == 1) TILE(1, 32, 1, 1, 64, 4);
+        if (M <= 4 && narrow) TILE(4, 8, 1, 1, 128, 4);
         if (M <= 4) TILE(4, 32, 4, 1, 64, 4);
+        if (M <= 8 && narrow) TILE(4, 16, 2, 1, 64, 5);
+        if (M <= 8) TILE(8, 32, 4, 1, 64, 3);
+        if (narrow) TILE(16, 16, 2, 1, 64, 4);
         TILE(16, 32, 4, 1, 64, 3);
     }
-    if (blocks(64, 128) >= enough) TILE(64, 128, 8, 8, 16, 3);
-    if (blocks(32, 32) >= enough) TILE(32, 32, 4, 2, 32, 3);
+    if (blocks(64, 64) * by >= 3 * sms && (M + 63) / 64 * 64 <= (M + 31) / 32 * 35) TILE(64, 64, 8, 4, 32, 2);
+    if (blocks(32, 64) * by >= 3 * sms) TILE(32, 64, 4, 4, 32, 3);
+    if (blocks(32, 32) * by >= sms) TILE(32, 32, 4, 2, 32, 3);
+    if (3 * blocks(32, 32) * by >= 2 * sms) TILE(32, 32, 2, 2, 32, 3);
     TILE(32, 16, 2, 1, 32, 4);
 #undef TILE
 }
@@ -230,7 +333,7 @@ int launch_f32(const void* A, const void* W, const void* bias, int bias_dtype, v
 
 extern "C" {
 
-// Any of A, W, C may be float or bf16; accumulation is 32-bit in ascending k.
+// Any of A, W, C may be float or bf16; accumulation is 32-bit in an order that depends on K alone.
 int infero_gemm_tiled(const void* A, int a_dtype, const void* W, int w_dtype, const void* bias,
                       int bias_dtype, void* C, int c_dtype, int M, int N, int K, int lda, int ldc,
                       cudaStream_t stream) {

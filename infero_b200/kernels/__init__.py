@@ -232,7 +232,7 @@ def swiglu(gate_up, out: torch.Tensor) -> None:
 
 # ---- matrix products ------------------------------------------------------------------------
 def gemm_tiled(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> None:
-    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias); 32-bit accumulation in ascending k."""
+    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias); 32-bit accumulation in an order that depends on K alone."""
     M, K = a.shape
     N = w.shape[0]
     assert w.shape[1] == K and out.shape == (M, N) and w.is_contiguous()
