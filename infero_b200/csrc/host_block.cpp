@@ -15,6 +15,8 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "decode_resident.h"
+
 extern "C" {
 // elementwise.cu, rope_cache.cu, gemm_tc.cu, attention_*.cu, runtime.cu
 int infero_embed_gather(const void* table, int table_dtype, const int* ids, const int* device_tokens, float* x,
@@ -189,7 +191,9 @@ long long infero_block_arena_bytes(const InferoBlock* b, int max_tokens, int sm_
     const int probes[] = {1, 16, 32, 64, 128, 256, 257, max_tokens};
     for (int t : probes)
         if (t <= max_tokens || t == 1) most = std::max(most, plan_arena(*b, std::min(t, std::max(1, max_tokens)), sm_count).total);
-    return most;
+    ResidentStep r = {};
+    r.hidden = b->hidden, r.n_heads = b->n_heads, r.n_kv = b->n_kv, r.ff = b->intermediate;
+    return std::max(most, infero_resident_scratch(&r, nullptr, b->head_dim, sm_count));
 }
 
 // Can this block run here at all?  (Shapes the tensor-core kernels take, head sizes the TMA-fed
@@ -268,6 +272,40 @@ static bool cluster_plan_ok(int T, int N, int K, int sm_count, int* splits, int*
 void infero_block_set_fusion(int fused_decode_on, int fused_norm_on) {
     g_fused_decode = fused_decode_on ? 1 : 0;
     g_fused_norm = fused_norm_on ? 1 : 0;
+}
+
+// A step of a few single tokens through blocks of equal sizes, each with a cache of its own, can run as one resident kernel
+// (decode_resident.cu), where INFERO_RESIDENT=1 asks for it and neither of the two switches above is off.
+static int g_resident = -1;
+void infero_block_set_resident(int on) { g_resident = on ? 1 : 0; }
+static bool resident_step(const InferoBlock* b, int n, const InferoStep& s, const int* const* tables, const int* entry_group, int max_blocks,
+                          ResidentStep* r, ResidentLayer* layers, int* num_pages) {
+    if (g_resident < 0) { const char* e = getenv("INFERO_RESIDENT"); g_resident = e && e[0] == '1' ? 1 : 0; }
+    if (g_fused_decode < 0) g_fused_decode = env_on("INFERO_FUSED_DECODE") ? 1 : 0;
+    if (!g_resident || !g_fused_decode || !fused_norm_wanted() || n < 1 || n > RESIDENT_LAYERS) return false;
+    if (s.n_decode != s.n_entries || s.n_decode != s.n_tokens) return false;
+    *r = ResidentStep{};
+    r->n_tok = s.n_tokens, r->n_layers = n, r->hidden = b->hidden, r->n_heads = b->n_heads, r->n_kv = b->n_kv, r->ff = b->intermediate;
+    r->rotary_dim = b->rotary_dim, r->page_size = b->page_size, r->max_blocks = max_blocks;
+    r->norm_dtype = b->norm_dtype, r->qkv_bias_dtype = b->qkv_bias_dtype, r->o_bias_dtype = b->o_bias_dtype;
+    r->inv_hidden = 1.0f / (float)b->hidden, r->positions = s.positions, r->tok_entry = s.tok_entry, r->x = s.x;
+    if (!infero_resident_supported(r, b->head_dim, s.sm_count)) return false;
+    for (int i = 0; i < n; ++i) {
+        const InferoBlock& o = b[i];
+        if (o.hidden != b->hidden || o.n_heads != b->n_heads || o.n_kv != b->n_kv || o.head_dim != b->head_dim || o.intermediate != b->intermediate ||
+            o.rotary_dim != b->rotary_dim || o.page_size != b->page_size || o.norm_dtype != b->norm_dtype || o.qkv_bias_dtype != b->qkv_bias_dtype ||
+            o.o_bias_dtype != b->o_bias_dtype || !o.write_cache)
+            return false;
+        for (const void* w : {o.w_qkv, o.w_o, o.w_gate_up, o.w_down, (const void*)o.k_cache, (const void*)o.v_cache})
+            if ((uintptr_t)w % 16 != 0) return false;
+        for (int j = 0; j < i; ++j)
+            if (b[j].k_cache == o.k_cache || b[j].v_cache == o.v_cache) return false;      // (keys of this step are not read ahead)
+        layers[i] = ResidentLayer{(const __nv_bfloat16*)o.w_qkv, (const __nv_bfloat16*)o.w_o, (const __nv_bfloat16*)o.w_gate_up, (const __nv_bfloat16*)o.w_down,
+                                  o.b_qkv, o.b_o, o.w_norm_mixer, o.w_norm_ffn, o.inv_freq, (__nv_bfloat16*)o.k_cache, (__nv_bfloat16*)o.v_cache,
+                                  tables[entry_group[i]], o.eps_mixer, o.eps_ffn, o.scale * 1.4426950408889634f, o.window};
+        num_pages[i] = o.num_pages;
+    }
+    return infero_resident_scratch(r, s.arena, b->head_dim, s.sm_count) <= s.arena_bytes;
 }
 
 // x += pending; the block; leaves its own feed-forward output pending in *delta.  layer_parity picks
@@ -437,14 +475,22 @@ int infero_decoder_forward(const InferoDecoder* m, const InferoStep* s, const in
                            float* logits, void* head_ws, long long head_ws_bytes) {
     const int T = s->n_tokens;
     if (T == 0) return 0;
-    if (int rc = infero_embed_gather(m->embed, m->embed_dtype, token_ids, device_tokens, s->x, T, m->hidden, m->vocab,
-                                     m->embed_scale, s->stream))
-        return rc;
     InferoDelta delta = {};
-    for (int i = 0; i < m->n_entries; ++i) {
+    ResidentStep r;
+    ResidentLayer layers[RESIDENT_LAYERS];
+    int num_pages[RESIDENT_LAYERS], rc = 2;
+    if (resident_step(m->blocks, m->n_entries, *s, tables, m->entry_group, max_blocks, &r, layers, num_pages)) {
+        rc = infero_decode_resident(&r, layers, m->blocks->head_dim, num_pages, m->embed, m->embed_dtype, token_ids, device_tokens, m->vocab,
+                                    m->embed_scale, s->sm_count, s->stream);
+        if (rc == 1) return rc;
+    }
+    if (rc == 2)
+        if (int rc2 = infero_embed_gather(m->embed, m->embed_dtype, token_ids, device_tokens, s->x, T, m->hidden, m->vocab, m->embed_scale, s->stream))
+            return rc2;
+    for (int i = 0; rc == 2 && i < m->n_entries; ++i) {
         const InferoBlock* next = i + 1 < m->n_entries ? &m->blocks[i + 1] : nullptr;
-        if (int rc = infero_block_forward(&m->blocks[i], s, tables[m->entry_group[i]], max_blocks, i & 1, &delta, next))
-            return rc;
+        if (int rc2 = infero_block_forward(&m->blocks[i], s, tables[m->entry_group[i]], max_blocks, i & 1, &delta, next))
+            return rc2;
     }
     if (n_rows == 0) return 0;
     const bool pending = delta.data && delta.dtype != PRENORMED;
