@@ -36,6 +36,7 @@ constexpr int MAX_D = 256;
 constexpr int CHUNK = 32, STAGES = 2;
 constexpr int FEW_TOKENS = 256;         // portions of up to so many tokens: a block per token, one row a warp; beyond, 32 rows a block
 constexpr int WIDE_ROWS = WARPS * 4;
+constexpr int AHEAD_BLOCKS = 296;       // so few blocks cannot cover one another's waits for memory: keys are sent for far ahead
 
 struct GenericArgs {
     const void* q;
@@ -176,6 +177,19 @@ attention_generic_kernel(const GenericArgs a) {
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         start = start / CHUNK * CHUNK;
+        // Few blocks of a row a warp (single tokens, short portions) would wait for every chunk to come from memory.  Every warp asks for a chunk of its own on the way to L2, then for the one n_warps chunks on.
+        auto send_for = [&](int j0, int page) {
+            if (page < 0) return;
+            const long long row = ((long long)page * a.n_kv + kvh) * a.page_size + (j0 + lane) % a.page_size, v_row = row + (long long)(vh - kvh) * a.page_size;
+            for (int b = 0; b < D * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)((const T*)a.k_cache + row * D) + b));
+            for (int b = 0; b < V * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)((const T*)a.v_cache + v_row * V) + b));
+        };
+        const bool ahead = R == 1 && gridDim.x <= AHEAD_BLOCKS;
+        int far = start + warp * CHUNK, far_page = -1;
+        if (ahead) {
+            send_for(far, page_of(far));
+            far += n_warps * CHUNK, far_page = page_of(far);
+        }
         load(start, page_of(start), 0);
         int page = page_of(start + CHUNK), stage = 0;
         for (int j0 = start; j0 <= last; j0 += CHUNK, stage ^= 1) {
@@ -183,6 +197,10 @@ attention_generic_kernel(const GenericArgs a) {
             __syncthreads();                             // this chunk is here, and everyone is done with the one before,
             load(j0 + CHUNK, page, stage ^ 1);           // whose place this takes
             page = page_of(j0 + 2 * CHUNK);
+            if (ahead && j0 + n_warps * CHUNK >= far) {         // (once for every n_warps chunks)
+                send_for(far, far_page);
+                far += n_warps * CHUNK, far_page = page_of(far);
+            }
             const int j = j0 + lane;
             const bool there = here[stage] >> lane & 1;
             bool sees[R];                                // does the row have keys in this chunk?
