@@ -67,6 +67,11 @@ struct FusedQkv {
     const float* sumsq_in;
     int in_tiles;
     float inv_d, eps;
+    // The kernel in front in the stream is prompt attention of the same step: it has let this one in after its own wait (so
+    // finished queries, keys and values are there), and touches nothing that this one reads or writes.  No block waits for it at the
+    // start; the grid's first block does before it leaves, so that whoever waits for this grid waits for both.  (40 single tokens of 16
+    // to 2,047 keys beside prompts of 700, 37 and 255 tokens, 14 heads of 64 over 2: 27 and 15 us a layer one after the other.)
+    int beside;
     // Biases by distance and the choice of values (attn_common.cuh).  They ride here because they are one more thing the
     // kernel needs about the queries.
     Extras ex;
@@ -352,10 +357,14 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         tc::fence_barrier_init();
         tc::fence_proxy_async();
     }
+    const bool last_to_leave = !FUSED && fq.beside && (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
     int split = blockIdx.x, ti = blockIdx.z, splits_before = ti * n_splits;
     if (SHARED) {                                                     // the splits are shared out by length
         const Share s = share_out(Share{ti, split, n_splits, chunk, splits_before, pos}, lengths, (int)gridDim.z, window, least, lane);
-        if (s.token < 0) return;                                      // (uniform over the block)
+        if (s.token < 0) {                                            // (uniform over the block)
+            if (last_to_leave) pdl_wait();
+            return;
+        }
         if (s.token != ti) entry = tok_entry[tok_first + s.token];
         split = s.split, ti = s.token, chunk = s.keys, n_splits = s.splits, splits_before = s.first, pos = s.pos;
     }
@@ -383,7 +392,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     float* pml = partial_ml + part * 2;
     if (k_begin >= k_end) {
         // nothing in this split: leave (m, l) = (-inf, 0) so the merge skips it
-        pdl_wait();
+        if (FUSED || !fq.beside) pdl_wait();
         for (int r = threadIdx.x; r < valid; r += TD_THREADS) {
             pml[(size_t)r * n_splits * 2] = -CUDART_INF_F;
             pml[(size_t)r * n_splits * 2 + 1] = 0.f;
@@ -392,6 +401,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             merge_if_last<D>(counters + (size_t)ti * gridDim.y + blockIdx.y, reinterpret_cast<float*>(smem),
                              po - (size_t)split * D, pml - (size_t)split * 2, n_splits, valid,
                              out + (size_t)t * out_stride + (size_t)row_first * D, sink, fq.ex.sinks ? fq.ex.sinks + h0 : nullptr);
+        if (last_to_leave) pdl_wait();
         return;
     }
     float2* sc = reinterpret_cast<float2*>(smem + Plan::FUSED_OFFSET);            // [rotary_dim / 2] (sine, cosine)
@@ -450,7 +460,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
         __syncthreads();
     }
-    pdl_wait();                                        // q and this step's key and value
+    if (FUSED || !fq.beside) pdl_wait();               // q and this step's key and value
     TL_MARK(51);
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i)
@@ -678,6 +688,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         merge_if_last<D>(counters + (size_t)ti * gridDim.y + blockIdx.y, reinterpret_cast<float*>(smem),
                          po - (size_t)split * D, pml - (size_t)split * 2, n_splits, valid,
                          out + (size_t)t * out_stride + (size_t)row_first * D, sink, fq.ex.sinks ? fq.ex.sinks + h0 : nullptr);
+    if (last_to_leave) pdl_wait();
     TL_END(TL_ATTN_DECODE);
 }
 
@@ -824,6 +835,19 @@ int infero_attn_decode_tma(const void* q, int q_stride, void* out, int out_strid
                            int n_kv, int head_dim, int page_size, int window, float scale, int chunk, int n_splits,
                            void* scratch, int* counters, int n_counters, cudaStream_t stream) {
     FusedQkv none = {};
+    return decode_tma(q, q_stride, none, out, out_stride, k_cache, v_cache, num_pages, block_table, max_blocks, tok_entry,
+                      positions, tok_first, n_tok, n_heads, n_kv, head_dim, page_size, window, scale, chunk, n_splits,
+                      scratch, counters, n_counters, 0, stream);
+}
+
+// The same right behind infero_attn_prefill_tc of the same step's prompt portions (see FusedQkv::beside).
+int infero_attn_decode_tma_beside(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
+                                  const void* v_cache, int num_pages, const int* block_table, int max_blocks,
+                                  const int* tok_entry, const int* positions, int tok_first, int n_tok, int n_heads,
+                                  int n_kv, int head_dim, int page_size, int window, float scale, int chunk, int n_splits,
+                                  void* scratch, int* counters, int n_counters, cudaStream_t stream) {
+    FusedQkv none = {};
+    none.beside = 1;
     return decode_tma(q, q_stride, none, out, out_stride, k_cache, v_cache, num_pages, block_table, max_blocks, tok_entry,
                       positions, tok_first, n_tok, n_heads, n_kv, head_dim, page_size, window, scale, chunk, n_splits,
                       scratch, counters, n_counters, 0, stream);

@@ -88,7 +88,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     volatile int* never_flag = abort_flag + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_q);
         prefetch_tensormap(&map_k);
@@ -120,6 +119,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                                        // q, the tables and this step's keys come from earlier kernels
+    // (behind the wait: decode attention of the same step may follow and take what is here for granted, see attention_decode.cu)
+    pdl_launch_dependents();
 
     // ---- which kv head and pair of heads, which request and which block of 128 query rows? ------
     const int group = n_heads / n_kv;

@@ -56,6 +56,11 @@ int infero_attn_decode_tma(const void* q, int q_stride, void* out, int out_strid
                            const int* tok_entry, const int* positions, int tok_first, int n_tok, int n_heads,
                            int n_kv, int head_dim, int page_size, int window, float scale, int chunk, int n_splits,
                            void* scratch, int* counters, int n_counters, cudaStream_t stream);
+int infero_attn_decode_tma_beside(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
+                                  const void* v_cache, int num_pages, const int* block_table, int max_blocks,
+                                  const int* tok_entry, const int* positions, int tok_first, int n_tok, int n_heads,
+                                  int n_kv, int head_dim, int page_size, int window, float scale, int chunk, int n_splits,
+                                  void* scratch, int* counters, int n_counters, cudaStream_t stream);
 int infero_attn_decode_fused_supported(const float* partial, long long split_stride, int n_heads, int n_kv,
                                        int head_dim, int page_size, int rotary_dim, const void* k_cache,
                                        const void* v_cache);
@@ -367,6 +372,15 @@ int infero_block_forward(const InferoBlock* b, const InferoStep* s, const int* b
             return rc;
     }
     void* attn = A + p.attn;
+    // the portions first: single tokens then run on the multiprocessors and in the shared memory that these leave
+    const bool beside = s->n_decode > 0 && s->n_decode < s->n_entries && s->prefill_tiles > 0;
+    if (s->n_decode < s->n_entries) {
+        if (int rc = infero_attn_prefill_tc(q, q_stride, T, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table,
+                                            max_blocks, s->entry_q_start, s->entry_q_len, s->entry_pos0, s->n_entries,
+                                            s->n_decode, s->prefill_tiles, H, Hkv, D, b->page_size, b->window, b->scale,
+                                            s->stream))
+            return rc;
+    }
     if (s->n_decode > 0) {
         int vis = s->decode_visible;
         if (b->window > 0) vis = std::min(vis, b->window + 15);
@@ -385,18 +399,11 @@ int infero_block_forward(const InferoBlock* b, const InferoStep* s, const int* b
                                               A + p.scratch, s->counters, s->n_counters, ss_mixer, tiles, inv_d,
                                               b->eps_mixer, s->stream);
         else
-            rc = infero_attn_decode_tma(q, q_stride, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table,
-                                        max_blocks, s->tok_entry, s->positions, 0, s->n_decode, H, Hkv, D,
-                                        b->page_size, b->window, b->scale, chunk, splits, A + p.scratch, s->counters,
-                                        s->n_counters, s->stream);
+            rc = (beside ? infero_attn_decode_tma_beside : infero_attn_decode_tma)(
+                q, q_stride, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table, max_blocks, s->tok_entry, s->positions, 0,
+                s->n_decode, H, Hkv, D, b->page_size, b->window, b->scale, chunk, splits, A + p.scratch, s->counters, s->n_counters,
+                s->stream);
         if (rc) return rc;
-    }
-    if (s->n_decode < s->n_entries) {
-        if (int rc = infero_attn_prefill_tc(q, q_stride, T, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table,
-                                            max_blocks, s->entry_q_start, s->entry_q_len, s->entry_pos0, s->n_entries,
-                                            s->n_decode, s->prefill_tiles, H, Hkv, D, b->page_size, b->window, b->scale,
-                                            s->stream))
-            return rc;
     }
     // ---- output projection, second norm, feed-forward ----------------------------------------------
     void* act = A + p.act;
