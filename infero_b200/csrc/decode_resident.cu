@@ -28,6 +28,7 @@
 #include "tc_common.cuh"
 #include "decode_resident.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace {
@@ -38,17 +39,19 @@ constexpr int CW = 7, CT = CW * 32, THREADS = CT + 32;          // consumer warp
 constexpr int TOKENS = 8;                                       // tokens a step may have
 constexpr int PIECE = 896;                                      // columns of a weight piece: four steps of 32 for each warp
 constexpr int ROW_BYTES = PIECE * 2 + 64;                       // rows in a slot start 64 bytes apart mod 128: no bank conflicts
-constexpr int SLOT = 15360, SLOTS = 13;                         // bytes and number of ring slots
+constexpr int SLOT = 15360, SLOTS = 10;                         // bytes and number of ring slots
 constexpr int STEPS = (PIECE / 32 + CW - 1) / CW;               // k-steps of 32 columns a warp has in a piece, at most
 constexpr int UNITS = 8;                                        // units a warp accumulates at a time
 constexpr int RED_BYTES = CW * 8 * 68 * 4;                      // the warps' sums, or 64 columns of their attention results
+constexpr int ACT_BYTES = 44 * 1024;                            // a product's activations in shared memory (DIRECT)
 constexpr int MAX_ROWS = 64;                                    // columns of the residual stream one block owns, at most
 constexpr int GROUP = 8;                                        // query heads of a kv head, at most
 static_assert(8 * ROW_BYTES <= SLOT && SLOT % 1024 == 0 && CW * UNITS * TOKENS * 8 * 4 <= RED_BYTES && GROUP == 8 && TOKENS == 8, "");
 
 struct Smem {                                                   // offsets behind the ring (from a 1,024-byte boundary)
     static constexpr int RED = SLOT * SLOTS;
-    static constexpr int X = RED + RED_BYTES;                   // [TOKENS][MAX_ROWS] float
+    static constexpr int ACT = RED + RED_BYTES;                 // [tokens][K] bf16 (DIRECT)
+    static constexpr int X = ACT + ACT_BYTES;                   // [TOKENS][MAX_ROWS] float
     static constexpr int ANGLES = X + TOKENS * MAX_ROWS * 4;    // [64] float2
     static constexpr int Q = ANGLES + 64 * 8;                   // [GROUP][D + 8] bf16
     static constexpr int KV = Q + GROUP * 136 * 2;              // the token's own key and value [2][D] bf16
@@ -110,13 +113,6 @@ __device__ __forceinline__ uint32_t tagged(float v, uint32_t tag) {
 __device__ __forceinline__ void tell(uint32_t* p, uint32_t word) { asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(p), "r"(word) : "memory"); }
 __device__ __forceinline__ void tell(uint2* p, float v, uint32_t tag) {
     asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
-}
-// Eight words to four pairs of bf16; false unless all have the tag.
-__device__ __forceinline__ bool untag(const uint4 a, const uint4 b, uint32_t tag, uint4& out) {
-    const uint32_t T = tag << 16;
-    const uint32_t off = (a.x ^ T) | (a.y ^ T) | (a.z ^ T) | (a.w ^ T) | (b.x ^ T) | (b.y ^ T) | (b.z ^ T) | (b.w ^ T);
-    out = make_uint4(__byte_perm(a.x, a.y, 0x5410), __byte_perm(a.z, a.w, 0x5410), __byte_perm(b.x, b.y, 0x5410), __byte_perm(b.z, b.w, 0x5410));
-    return off >> 16 == 0;
 }
 
 // ---- who takes which keys ------------------------------------------------------------------------------------------------
@@ -231,10 +227,23 @@ struct Block {
           warp(threadIdx.x >> 5), lane(threadIdx.x & 31), seq(passed) {}
     __device__ __forceinline__ const ResidentStep& s() const { return p.s; }
 
+    // A wait that looks at the clock late: reading it takes about as long as a slot's work.
+    __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) {
+        unsigned long long t0 = 0;
+        for (unsigned int i = 1;; ++i) {
+            if (tc::mbar_try_wait(bar, parity)) return true;
+            if ((i & 255u) == 0) {
+                if (*abort_flag) return false;
+                const unsigned long long now = tc::global_ns();
+                if (!t0) t0 = now;
+                if (now - t0 > tc::WAIT_LIMIT_NS) return false;
+            }
+        }
+    }
     // The bytes of the ring's q-th slot are here.  A wait that runs out is reported; the caller goes on (with whatever is there) to
     // the next meeting, where all of the block's consumers leave together.
     __device__ __forceinline__ void arrived(uint32_t q) {
-        if (!tc::mbar_wait(&full[q % SLOTS], (q / SLOTS) & 1u, abort_flag)) {
+        if (!wait(&full[q % SLOTS], (q / SLOTS) & 1u)) {
             *abort_flag = 1;
             if (lane == 0) atomicExch(p.err_flag, 6);
         }
@@ -242,7 +251,7 @@ struct Block {
 
     // ---- the loader ------------------------------------------------------------------------------------------------------
     __device__ __forceinline__ bool acquire() {                 // the slot `seq` is free
-        return seq < SLOTS || tc::mbar_wait(&empty[seq % SLOTS], (seq / SLOTS - 1) & 1u, abort_flag);
+        return seq < SLOTS || wait(&empty[seq % SLOTS], (seq / SLOTS - 1) & 1u);
     }
     __device__ __forceinline__ bool load_matrix(const bf16* w, int r0, int r1, int K, uint64_t policy) {
         const int units = (r1 - r0 + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
@@ -354,46 +363,47 @@ struct Block {
         }
     }
 
+    // DIRECT: n tagged words of all blocks to shared memory, as bf16 (n is a multiple of 64).
+    __device__ __forceinline__ void gather(const bf16* in, int n, uint32_t tag) {
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(in);
+        uint2* act = reinterpret_cast<uint2*>(smem + Smem::ACT);
+        const uint32_t T = tag << 16;
+        for (int v0 = threadIdx.x; v0 < n / 4; v0 += 8 * CT) {
+            uint4 w[8];
+            until([&] {
+                uint32_t off = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (v0 + k * CT < n / 4) w[k] = look16(words + (v0 + k * CT) * 4);
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (v0 + k * CT < n / 4) off |= (w[k].x ^ T) | (w[k].y ^ T) | (w[k].z ^ T) | (w[k].w ^ T);
+                return off >> 16 == 0;
+            });
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (v0 + k * CT < n / 4) act[v0 + k * CT] = make_uint2(__byte_perm(w[k].x, w[k].y, 0x5410), __byte_perm(w[k].z, w[k].w, 0x5410));
+        }
+        consumers_sync();
+    }
+
     // ---- a product -----------------------------------------------------------------------------------------------------------
     // in [tokens, K] times the next `rows` weight rows of the ring; each(first, n) when the sums of n rows from `first` on are
     // in shared memory (total)
     template <typename F>
-    __device__ __forceinline__ void product(const bf16* in, int K, int rows, uint32_t tag, F each) {
+    __device__ __forceinline__ void product(const bf16* in, int K, int rows, F each) {
         const int units = (rows + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
         const int g = lane >> 2, c = lane & 3, M = s().n_tok;
         const bf16* mine = in + (size_t)g * K + warp * 32 + c * 8;
-        const uint32_t* words = reinterpret_cast<const uint32_t*>(in) + (size_t)g * K + warp * 32 + c * 8;
-        // A lane's activations of a piece: `ask` sends for them, `take` has them (DIRECT: with the tag they are to have).
-        constexpr int RAW = DIRECT ? 2 * STEPS : STEPS;
+        const uint8_t* act = smem + Smem::ACT + ((size_t)g * K + warp * 32 + c * 8) * 2;
+        // A lane's activations of a piece: sent for a piece ahead (from L2), or from shared memory (DIRECT).
         auto there = [&](int k0, int i) { return g < M && k0 + i * (CW * 32) + warp * 32 < K && i * (CW * 32) + warp * 32 < PIECE; };
-        auto ask = [&](uint4* raw, int k0) {
+        auto fetch = [&](uint4* x, int k0) {
 #pragma unroll
             for (int i = 0; i < STEPS; ++i) {
-                if constexpr (DIRECT) {
-                    if (there(k0, i)) raw[2 * i] = look16(words + k0 + i * (CW * 32)), raw[2 * i + 1] = look16(words + k0 + i * (CW * 32) + 4);
-                } else {
-                    raw[i] = there(k0, i) ? ld_l2_16(mine + k0 + i * (CW * 32)) : make_uint4(0, 0, 0, 0);
-                }
-            }
-        };
-        auto take = [&](uint4* x, uint4* raw, int k0) {
-            if constexpr (DIRECT) {
-                bool first = true;
-                until([&] {
-                    if (!first) ask(raw, k0);
-                    first = false;
-                    bool all = true;
-#pragma unroll
-                    for (int i = 0; i < STEPS; ++i) {
-                        if (there(k0, i)) all &= untag(raw[2 * i], raw[2 * i + 1], tag, x[i]);
-                        else x[i] = make_uint4(0, 0, 0, 0);
-                    }
-                    return all;
-                });
-                __syncwarp();
-            } else {
-#pragma unroll
-                for (int i = 0; i < STEPS; ++i) x[i] = raw[i];
+                if (!there(k0, i)) x[i] = make_uint4(0, 0, 0, 0);
+                else if constexpr (DIRECT) x[i] = *reinterpret_cast<const uint4*>(act + (k0 + i * (CW * 32)) * 2);
+                else x[i] = ld_l2_16(mine + k0 + i * (CW * 32));
             }
         };
 #pragma unroll 1
@@ -404,12 +414,17 @@ struct Block {
             for (int u = 0; u < UNITS / 2; ++u)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[u][0][i] = acc[u][1][i] = 0.f;
-            uint4 x[STEPS], raw[RAW];
-            ask(raw, 0);
+            uint4 x[STEPS], next[STEPS];
+            if (!DIRECT) fetch(next, 0);
 #pragma unroll 1
             for (int k0 = 0; k0 < K; k0 += PIECE) {
-                take(x, raw, k0);
-                if (k0 + PIECE < K) ask(raw, k0 + PIECE);
+                if constexpr (DIRECT) {
+                    fetch(x, k0);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < STEPS; ++i) x[i] = next[i];
+                    if (k0 + PIECE < K) fetch(next, k0 + PIECE);
+                }
                 const int steps = min(PIECE, K - k0) / 32;
 #pragma unroll
                 for (int u = 0; u < UNITS / 2; ++u) {
@@ -679,12 +694,13 @@ struct Block {
         const bool last = which == 3 && l + 1 == s().n_layers, residual = which == 1 || which == 3;
         const int n = which == 0 ? nqkv : which == 2 ? s().ff : H, pairs = which == 2 ? 2 : 1;
         const int r0 = share(b, n, G) * pairs, rows = share(b + 1, n, G) * pairs - r0;
-        if (!residual) load_rms(s().sums[which / 2], l + which == 0 ? 1 : G, which == 0 ? L.eps_mixer : L.eps_ffn, tag);
         const bf16* in = which == 0 ? s().h[0] : which == 1 ? s().attn : which == 2 ? s().h[1] : s().act;
+        if (DIRECT) gather(in, M * (which == 1 ? da : which == 3 ? s().ff : H), tag);
+        if (!residual) load_rms(s().sums[which / 2], l + which == 0 ? 1 : G, which == 0 ? L.eps_mixer : L.eps_ffn, tag);
         const void* bias = which == 0 ? L.b_qkv : which == 1 ? L.b_o : nullptr;
         const void* norm_w = which == 1 ? L.norm_ffn : which == 3 && !last ? p.layer[l + 1].norm_mixer : nullptr;
         const int next = which == 1;                            // whose h and sums a residual product hands on
-        product(in, which == 1 ? da : which == 3 ? s().ff : H, rows, tag, [&](int first, int here) {
+        product(in, which == 1 ? da : which == 3 ? s().ff : H, rows, [&](int first, int here) {
             const int mine = here / pairs;                      // results of this block (a gate and its up row make one)
 #pragma unroll 1
             for (int e = threadIdx.x; e < mine * M; e += CT) {
@@ -867,7 +883,8 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
                            cudaStream_t stream) {
     static std::mutex mutex;
     static int fits[4] = {-1, -1, -1, -1};                      // blocks a multiprocessor holds, by kernel
-    const bool direct = s->n_tok <= DIRECT_TOKENS;
+    const int widest = std::max({s->ff, s->hidden, s->n_heads * head_dim});
+    const bool direct = s->n_tok <= DIRECT_TOKENS && s->n_tok * widest * 2 <= ACT_BYTES;
     void* kernel = head_dim == 64 ? (direct ? (void*)decode_resident_kernel<64, true> : (void*)decode_resident_kernel<64, false>)
                                   : (direct ? (void*)decode_resident_kernel<128, true> : (void*)decode_resident_kernel<128, false>);
     {
