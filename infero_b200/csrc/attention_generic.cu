@@ -29,6 +29,8 @@
 #include "common.cuh"
 #include <math_constants.h>
 
+extern "C" int infero_sm_count();
+
 namespace {
 
 constexpr int WARPS = 8;
@@ -36,7 +38,6 @@ constexpr int MAX_D = 256;
 constexpr int CHUNK = 32, STAGES = 2;
 constexpr int FEW_TOKENS = 256;         // portions of up to so many tokens: a block per token, one row a warp; beyond, 32 rows a block
 constexpr int WIDE_ROWS = WARPS * 4;
-constexpr int AHEAD_BLOCKS = 296;       // so few blocks cannot cover one another's waits for memory: keys are sent for far ahead
 
 struct GenericArgs {
     const void* q;
@@ -177,19 +178,6 @@ attention_generic_kernel(const GenericArgs a) {
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         start = start / CHUNK * CHUNK;
-        // Few blocks of a row a warp (single tokens, short portions) would wait for every chunk to come from memory.  Every warp asks for a chunk of its own on the way to L2, then for the one n_warps chunks on.
-        auto send_for = [&](int j0, int page) {
-            if (page < 0) return;
-            const long long row = ((long long)page * a.n_kv + kvh) * a.page_size + (j0 + lane) % a.page_size, v_row = row + (long long)(vh - kvh) * a.page_size;
-            for (int b = 0; b < D * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)((const T*)a.k_cache + row * D) + b));
-            for (int b = 0; b < V * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)((const T*)a.v_cache + v_row * V) + b));
-        };
-        const bool ahead = R == 1 && gridDim.x <= AHEAD_BLOCKS;
-        int far = start + warp * CHUNK, far_page = -1;
-        if (ahead) {
-            send_for(far, page_of(far));
-            far += n_warps * CHUNK, far_page = page_of(far);
-        }
         load(start, page_of(start), 0);
         int page = page_of(start + CHUNK), stage = 0;
         for (int j0 = start; j0 <= last; j0 += CHUNK, stage ^= 1) {
@@ -197,10 +185,6 @@ attention_generic_kernel(const GenericArgs a) {
             __syncthreads();                             // this chunk is here, and everyone is done with the one before,
             load(j0 + CHUNK, page, stage ^ 1);           // whose place this takes
             page = page_of(j0 + 2 * CHUNK);
-            if (ahead && j0 + n_warps * CHUNK >= far) {         // (once for every n_warps chunks)
-                send_for(far, far_page);
-                far += n_warps * CHUNK, far_page = page_of(far);
-            }
             const int j = j0 + lane;
             const bool there = here[stage] >> lane & 1;
             bool sees[R];                                // does the row have keys in this chunk?
@@ -337,8 +321,14 @@ int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
     const bool few = tokens == 0;
     // (warps without a row help to fetch: four suffice for narrow rows)
     const int least = a.head_dim > 64 || a.value_dim > 64 ? WARPS : WARPS / 2;
-    const int warps = few ? (group < least ? least : group < WARPS ? group : WARPS) : WARPS, rows = few ? warps : WIDE_ROWS;
-    a.tokens_per_block = few ? 1 : tokens;
+    const int warps = few ? (group < least ? least : group < WARPS ? group : WARPS) : WARPS;
+    // Where blocks of 32 rows are fewer than two a multiprocessor, half as many rows a warp: what a chunk costs a warp is latency, and
+    // twice the warps cover it.
+    const long long wide = few ? 0 : (a.singles + (long long)(a.n_tokens - a.singles + tokens - 1) / tokens) * ((group + WIDE_ROWS - 1) / WIDE_ROWS) *
+                                         a.n_kv * (a.cross ? a.n_kv : 1);
+    const bool half = !few && wide < 2 * infero_sm_count();
+    const int rows = few ? warps : half ? WIDE_ROWS / 2 : WIDE_ROWS;
+    a.tokens_per_block = few ? 1 : half ? (group > rows ? 1 : rows / group) : tokens;
     a.head_chunks = (group + rows - 1) / rows;
 #define COLUMNS(R)                                                                                      \
     do {                                                                                                \
@@ -347,6 +337,7 @@ int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
         return launch<T, TO, R, 2, VEC>(a, warps, stream);                                              \
     } while (0)
     if (few) COLUMNS(1);
+    if (half) COLUMNS(2);
     COLUMNS(4);
 #undef COLUMNS
 }

@@ -86,6 +86,12 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(tc::smem_u32(bar)), "l"(policy) : "memory");
 }
+// (a read where it stands, behind the wait for its slot; 32-bit addresses)
+__device__ __forceinline__ uint4 lds16(uint32_t at) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
 __device__ __forceinline__ void arrive_n(uint64_t* bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
 }
@@ -172,23 +178,23 @@ __device__ __forceinline__ void merge(const ResidentStep& s, const Segment g, ui
     for (int e = threadIdx.x; e < group * (D / 4); e += CT) {
         const int r = e / (D / 4), d = (e - r * (D / 4)) * 4;
         float M = -CUDART_INF_F, sum = 0.f, v[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k0 = 0; k0 < n; k0 += 16) {                    // sixteen blocks' loads in flight at a time
-            float2 x[16];
-            uint4 y[16];
+        for (int k0 = 0; k0 < n; k0 += 8) {                     // eight blocks' loads in flight at a time
+            float2 x[8];
+            uint4 y[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
+            for (int k = 0; k < 8; ++k)
                 if (k0 + k < n) {
                     x[k] = __ldcg(reinterpret_cast<const float2*>(ml0 + (size_t)(k0 + k) * (GROUP * 2)) + r);
                     y[k] = ld_l2_16(po0 + (size_t)(k0 + k) * (GROUP * D) + r * D + d);
                 }
             float Mn = M;
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
+            for (int k = 0; k < 8; ++k)
                 if (k0 + k < n) Mn = fmaxf(Mn, x[k].x);
             const float fix = M == -CUDART_INF_F ? 0.f : exp2f(M - Mn);
             M = Mn, sum *= fix, v[0] *= fix, v[1] *= fix, v[2] *= fix, v[3] *= fix;
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
+            for (int k = 0; k < 8; ++k)
                 if (k0 + k < n && x[k].x != -CUDART_INF_F) {
                     const float w = exp2f(x[k].x - M);
                     sum = fmaf(x[k].y, w, sum);
@@ -395,14 +401,15 @@ struct Block {
         const int units = (rows + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
         const int g = lane >> 2, c = lane & 3, M = s().n_tok;
         const bf16* mine = in + (size_t)g * K + warp * 32 + c * 8;
-        const uint8_t* act = smem + Smem::ACT + ((size_t)g * K + warp * 32 + c * 8) * 2;
+        const uint32_t act = tc::smem_u32(smem) + Smem::ACT + (g * K + warp * 32 + c * 8) * 2;
+        const uint32_t mine_at = tc::smem_u32(smem) + g * ROW_BYTES + warp * 64 + c * 16;
         // A lane's activations of a piece: sent for a piece ahead (from L2), or from shared memory (DIRECT).
         auto there = [&](int k0, int i) { return g < M && k0 + i * (CW * 32) + warp * 32 < K && i * (CW * 32) + warp * 32 < PIECE; };
         auto fetch = [&](uint4* x, int k0) {
 #pragma unroll
             for (int i = 0; i < STEPS; ++i) {
                 if (!there(k0, i)) x[i] = make_uint4(0, 0, 0, 0);
-                else if constexpr (DIRECT) x[i] = *reinterpret_cast<const uint4*>(act + (k0 + i * (CW * 32)) * 2);
+                else if constexpr (DIRECT) x[i] = lds16(act + (k0 + i * (CW * 32)) * 2);
                 else x[i] = ld_l2_16(mine + k0 + i * (CW * 32));
             }
         };
@@ -430,18 +437,17 @@ struct Block {
                 for (int u = 0; u < UNITS / 2; ++u) {
                     if (2 * u < n) {
                         const bool two = 2 * u + 1 < n;
-                        const uint8_t* w0 = smem + (seq % SLOTS) * SLOT + g * ROW_BYTES + warp * 64 + c * 16;
-                        const uint8_t* w1 = smem + ((seq + 1) % SLOTS) * SLOT + g * ROW_BYTES + warp * 64 + c * 16;
+                        const uint32_t w0 = mine_at + (seq % SLOTS) * SLOT, w1 = mine_at + ((seq + 1) % SLOTS) * SLOT;
                         uint4 a0[STEPS], a1[STEPS];
                         arrived(seq);
 #pragma unroll
                         for (int i = 0; i < STEPS; ++i)
-                            if (i * CW + warp < steps) a0[i] = *reinterpret_cast<const uint4*>(w0 + i * (CW * 64));
+                            if (i * CW + warp < steps) a0[i] = lds16(w0 + i * (CW * 64));
                         if (two) {
                             arrived(seq + 1);
 #pragma unroll
                             for (int i = 0; i < STEPS; ++i)
-                                if (i * CW + warp < steps) a1[i] = *reinterpret_cast<const uint4*>(w1 + i * (CW * 64));
+                                if (i * CW + warp < steps) a1[i] = lds16(w1 + i * (CW * 64));
                         } else {
 #pragma unroll
                             for (int i = 0; i < STEPS; ++i) a1[i] = make_uint4(0, 0, 0, 0);
@@ -753,12 +759,12 @@ struct Block {
 // return how far the ring has been passed, or GIVE_UP.
 constexpr uint32_t GIVE_UP = 0xffffffffu;
 template <int D, bool DIRECT>
-__device__ __noinline__ uint32_t attend(const Params& p, uint8_t* smem, int layer, uint32_t seq) {
+__device__ __forceinline__ uint32_t attend(const Params& p, uint8_t* smem, int layer, uint32_t seq) {
     Block<D, DIRECT> block(p, smem, seq);
     return block.attention(layer) ? block.seq : GIVE_UP;
 }
 template <int D, bool DIRECT>
-__device__ __noinline__ uint32_t multiply(const Params& p, uint8_t* smem, int layer, int which, uint32_t seq) {
+__device__ __forceinline__ uint32_t multiply(const Params& p, uint8_t* smem, int layer, int which, uint32_t seq) {
     Block<D, DIRECT> block(p, smem, seq);
     return block.multiply(layer, which) ? block.seq : GIVE_UP;
 }
