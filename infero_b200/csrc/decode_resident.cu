@@ -4,10 +4,9 @@
 // every kernel starts its stream of weights anew: about 3.5 us of a launch, a wait and an empty ring each, during which the
 // memory system idles.  Here one block per multiprocessor stays for the whole step.  One warp of it (the loader) knows the
 // order in which the block will want its bytes, for all products and all attention of all layers, and keeps a ring of shared
-// memory filled with them through the bulk-copy engine, ahead of everything that the other warps wait for.  Between the phases of a
-// layer (q/k/v, attention, output, gate/up, down) the blocks meet at a counter in global memory, or, in steps of one or two
-// tokens, look at tagged words (below); meanwhile the ring fills with the weights of the phases behind it, so that the stream
-// hardly stops.
+// memory filled with them through the bulk-copy engine, ahead of everything that the other warps wait for.  What the phases of a
+// layer (q/k/v, attention, output, gate/up, down) hand to one another goes through tagged words in global memory (below), without
+// a barrier; meanwhile the ring fills with the weights of the phases behind it.
 //
 //   products   Every block has an equal share of a matrix's rows, and all of K: no partial sums leave a block.  Rows come eight
 //              at a time (a unit), K in pieces of 896 columns; a unit's piece is one slot of the ring.  The seven consumer
@@ -36,27 +35,27 @@ namespace {
 using namespace attn;
 
 constexpr int CW = 7, CT = CW * 32, THREADS = CT + 32;          // consumer warps, their threads, all threads (eight warps: 255 registers)
-constexpr int TOKENS = 8;                                       // tokens a step may have
+constexpr int TOKENS = 2;                                       // tokens a step may have (a product has room for eight columns)
 constexpr int PIECE = 896;                                      // columns of a weight piece: four steps of 32 for each warp
 constexpr int ROW_BYTES = PIECE * 2 + 64;                       // rows in a slot start 64 bytes apart mod 128: no bank conflicts
 constexpr int SLOT = 15360, SLOTS = 10;                         // bytes and number of ring slots
 constexpr int STEPS = (PIECE / 32 + CW - 1) / CW;               // k-steps of 32 columns a warp has in a piece, at most
 constexpr int UNITS = 8;                                        // units a warp accumulates at a time
 constexpr int RED_BYTES = CW * 8 * 68 * 4;                      // the warps' sums, or 64 columns of their attention results
-constexpr int ACT_BYTES = 44 * 1024;                            // a product's activations in shared memory (DIRECT)
+constexpr int ACT_BYTES = 44 * 1024;                            // a product's activations in shared memory
 constexpr int MAX_ROWS = 64;                                    // columns of the residual stream one block owns, at most
 constexpr int GROUP = 8;                                        // query heads of a kv head, at most
-static_assert(8 * ROW_BYTES <= SLOT && SLOT % 1024 == 0 && CW * UNITS * TOKENS * 8 * 4 <= RED_BYTES && GROUP == 8 && TOKENS == 8, "");
+static_assert(8 * ROW_BYTES <= SLOT && SLOT % 1024 == 0 && CW * UNITS * 8 * 8 * 4 <= RED_BYTES && GROUP == 8, "");
 
 struct Smem {                                                   // offsets behind the ring (from a 1,024-byte boundary)
     static constexpr int RED = SLOT * SLOTS;
-    static constexpr int ACT = RED + RED_BYTES;                 // [tokens][K] bf16 (DIRECT)
+    static constexpr int ACT = RED + RED_BYTES;                 // [tokens][K] bf16
     static constexpr int X = ACT + ACT_BYTES;                   // [TOKENS][MAX_ROWS] float
     static constexpr int ANGLES = X + TOKENS * MAX_ROWS * 4;    // [64] float2
     static constexpr int Q = ANGLES + 64 * 8;                   // [GROUP][D + 8] bf16
     static constexpr int KV = Q + GROUP * 136 * 2;              // the token's own key and value [2][D] bf16
     static constexpr int ML = KV + 2 * 128 * 2;                 // [CW][GROUP] float2
-    static constexpr int MISC = ML + CW * GROUP * 8;            // rms, positions, entries [8] each; abort, leave; [28] last to arrive
+    static constexpr int MISC = ML + CW * GROUP * 8;            // rms, positions, entries [8] each; abort; [28] last to arrive
     static constexpr int BARS = MISC + 32 * 4;                  // full[SLOTS], empty[SLOTS]
     static constexpr int TOTAL = BARS + 2 * SLOTS * 8 + 1024;
 };
@@ -97,12 +96,11 @@ __device__ __forceinline__ void arrive_n(uint64_t* bar, uint32_t n) {
 }
 
 // ---- values that carry a tag --------------------------------------------------------------------------------------------------
-// DIRECT (steps of up to DIRECT_TOKENS tokens): what one block hands to the others needs no meeting.  Every value lies in a word of
-// its own beside a tag (bf16 with 16 bits of tag, 32-bit values with 32), the number of the layer that will read it, and a reader
-// looks at the word until the tag is there: a store and a load on the way instead of a fence, a counter, and then the load.
+// What one block hands to the others needs no meeting.  Every value lies in a word of its own beside a tag (bf16 with 16 bits of
+// tag, 32-bit values with 32), the number of the layer that will read it, and a reader looks at the word until the tag is there: a
+// store and a load on the way, instead of a fence, a counter (4 to 6 thousand cycles a phase, measured) and then the load.
 // The step's first kernel clears all tags.  No word is written again before all have read it: a block writes its
 // words of a phase after it has read everything of the phase before, and every block has words of gate/up in every layer.
-constexpr int DIRECT_TOKENS = 2;
 __device__ __forceinline__ uint4 look16(const uint32_t* p) {
     uint4 v;
     asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -170,7 +168,7 @@ __device__ __forceinline__ int slices_per_slot(int n) {
 }
 
 // The blocks' results of a pair, merged in their order.
-template <int D, bool DIRECT>
+template <int D>
 __device__ __forceinline__ void merge(const ResidentStep& s, const Segment g, uint32_t tag) {
     const int group = s.n_heads / s.n_kv, h0 = g.kvh * group, t = g.token, n = g.last - g.first + 1;
     const float* po0 = s.part_o + (size_t)(g.first + g.pair) * (GROUP * D);
@@ -204,22 +202,18 @@ __device__ __forceinline__ void merge(const ResidentStep& s, const Segment g, ui
         }
         const float inv = 1.0f / sum;
         const size_t to = ((size_t)t * s.n_heads + h0 + r) * D + d;
-        if (DIRECT) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) tell(reinterpret_cast<uint32_t*>(s.attn) + to + k, tagged(v[k] * inv, tag));
-        } else {
-            *reinterpret_cast<uint2*>(s.attn + to) = make_uint2(pack_bf16(v[0] * inv, v[1] * inv), pack_bf16(v[2] * inv, v[3] * inv));
-        }
+        for (int k = 0; k < 4; ++k) tell(s.attn + to + k, tagged(v[k] * inv, tag));
     }
 }
 
-template <int D, bool DIRECT>
+template <int D>
 struct Block {
     const Params& p;
     uint8_t* smem;
     uint64_t *full, *empty;
     int *pos, *entries;             // of the step's tokens
-    volatile int *abort_flag, *leave;   // a wait ran out; the consumers leave
+    volatile int* abort_flag;       // a wait ran out
     float* red;
     float* x_s;
     float* rms;
@@ -228,7 +222,7 @@ struct Block {
 
     __device__ __forceinline__ Block(const Params& params, uint8_t* at, uint32_t passed = 0)
         : p(params), smem(at), full(reinterpret_cast<uint64_t*>(at + Smem::BARS)), empty(full + SLOTS),
-          pos(reinterpret_cast<int*>(at + Smem::MISC) + 8), entries(pos + 8), abort_flag(pos + 16), leave(pos + 17),
+          pos(reinterpret_cast<int*>(at + Smem::MISC) + 8), entries(pos + 8), abort_flag(pos + 16),
           red(reinterpret_cast<float*>(at + Smem::RED)), x_s(reinterpret_cast<float*>(at + Smem::X)), rms(reinterpret_cast<float*>(at + Smem::MISC)),
           warp(threadIdx.x >> 5), lane(threadIdx.x & 31), seq(passed) {}
     __device__ __forceinline__ const ResidentStep& s() const { return p.s; }
@@ -246,12 +240,26 @@ struct Block {
             }
         }
     }
-    // The bytes of the ring's q-th slot are here.  A wait that runs out is reported; the caller goes on (with whatever is there) to
-    // the next meeting, where all of the block's consumers leave together.
+    // Nobody waits any more: the block runs through the rest of the step with whatever is there, as the other blocks do.
+    __device__ __forceinline__ void give_up() {
+        *abort_flag = 1;
+        *(volatile unsigned int*)s().stop = 1;
+        atomicExch(p.err_flag, 6);
+    }
+    // The bytes of the ring's q-th slot are here.
     __device__ __forceinline__ void arrived(uint32_t q) {
-        if (!wait(&full[q % SLOTS], (q / SLOTS) & 1u)) {
-            *abort_flag = 1;
-            if (lane == 0) atomicExch(p.err_flag, 6);
+        if (!wait(&full[q % SLOTS], (q / SLOTS) & 1u)) give_up();
+    }
+    // look() until it is true or the time is up
+    template <typename F>
+    __device__ __forceinline__ void until(F look) {
+        unsigned long long t0 = 0;
+        for (unsigned int i = 1; !look(); ++i) {
+            if (*abort_flag) return;
+            if ((i & 63u) == 0) {
+                if (!t0) t0 = tc::global_ns();
+                if (tc::global_ns() - t0 > tc::WAIT_LIMIT_NS || *(volatile unsigned int*)s().stop) give_up();
+            }
         }
     }
 
@@ -325,53 +333,9 @@ struct Block {
         for (uint32_t q = seq > SLOTS ? seq - SLOTS : 0; q < seq; ++q) tc::mbar_wait(&full[q % SLOTS], (q / SLOTS) & 1u, &never);
     }
 
-    // ---- the blocks meet ---------------------------------------------------------------------------------------------------
-    // Everything that this block's consumers wrote before `arrive` can be read by any block's consumers after their `meet`.
-    __device__ __forceinline__ void arrive() {
-        consumers_sync();
-        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s().sync) : "memory");
-    }
-    __device__ __forceinline__ void give_up() {
-        *abort_flag = 1;
-        *(volatile unsigned int*)(s().sync + 1) = 1;
-        atomicExch(p.err_flag, 6);
-    }
-    // The step's number-th meeting; false (for all consumers alike): give up.
-    __device__ __forceinline__ bool meet(unsigned int number) {
-        if (threadIdx.x == 0) {
-            const unsigned int want = number * gridDim.x;
-            unsigned long long t0 = 0;
-            for (unsigned int i = 1;; ++i) {
-                unsigned int have;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(s().sync) : "memory");
-                if (have >= want || *abort_flag) break;
-                if ((i & 63u) == 0) {
-                    if (!t0) t0 = tc::global_ns();
-                    if (tc::global_ns() - t0 > tc::WAIT_LIMIT_NS || *(volatile unsigned int*)(s().sync + 1)) *abort_flag = 1;
-                }
-            }
-            leave[0] = *abort_flag;                             // (one thread decides, so that all consumers leave or stay alike)
-            if (leave[0]) give_up();
-        }
-        consumers_sync();
-        return leave[0] == 0;
-    }
-    // look() until it is true or the time is up (then the block runs through the rest of the step without waiting)
-    template <typename F>
-    __device__ __forceinline__ void until(F look) {
-        unsigned long long t0 = 0;
-        for (unsigned int i = 1; !look(); ++i) {
-            if (*abort_flag) return;
-            if ((i & 63u) == 0) {
-                if (!t0) t0 = tc::global_ns();
-                if (tc::global_ns() - t0 > tc::WAIT_LIMIT_NS || *(volatile unsigned int*)(s().sync + 1)) give_up();
-            }
-        }
-    }
-
-    // DIRECT: n tagged words of all blocks to shared memory, as bf16 (n is a multiple of 64).
-    __device__ __forceinline__ void gather(const bf16* in, int n, uint32_t tag) {
-        const uint32_t* words = reinterpret_cast<const uint32_t*>(in);
+    // ---- a product -----------------------------------------------------------------------------------------------------------
+    // n tagged words of all blocks to shared memory, as bf16 (n is a multiple of 64)
+    __device__ __forceinline__ void gather(const uint32_t* words, int n, uint32_t tag) {
         uint2* act = reinterpret_cast<uint2*>(smem + Smem::ACT);
         const uint32_t T = tag << 16;
         for (int v0 = threadIdx.x; v0 < n / 4; v0 += 8 * CT) {
@@ -393,26 +357,14 @@ struct Block {
         consumers_sync();
     }
 
-    // ---- a product -----------------------------------------------------------------------------------------------------------
-    // in [tokens, K] times the next `rows` weight rows of the ring; each(first, n) when the sums of n rows from `first` on are
-    // in shared memory (total)
+    // The gathered [tokens, K] times the next `rows` weight rows of the ring; each(first, n) when the sums of n rows from `first` on
+    // are in shared memory (total).
     template <typename F>
-    __device__ __forceinline__ void product(const bf16* in, int K, int rows, F each) {
+    __device__ __forceinline__ void product(int K, int rows, F each) {
         const int units = (rows + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
         const int g = lane >> 2, c = lane & 3, M = s().n_tok;
-        const bf16* mine = in + (size_t)g * K + warp * 32 + c * 8;
         const uint32_t act = tc::smem_u32(smem) + Smem::ACT + (g * K + warp * 32 + c * 8) * 2;
         const uint32_t mine_at = tc::smem_u32(smem) + g * ROW_BYTES + warp * 64 + c * 16;
-        // A lane's activations of a piece: sent for a piece ahead (from L2), or from shared memory (DIRECT).
-        auto there = [&](int k0, int i) { return g < M && k0 + i * (CW * 32) + warp * 32 < K && i * (CW * 32) + warp * 32 < PIECE; };
-        auto fetch = [&](uint4* x, int k0) {
-#pragma unroll
-            for (int i = 0; i < STEPS; ++i) {
-                if (!there(k0, i)) x[i] = make_uint4(0, 0, 0, 0);
-                else if constexpr (DIRECT) x[i] = lds16(act + (k0 + i * (CW * 32)) * 2);
-                else x[i] = ld_l2_16(mine + k0 + i * (CW * 32));
-            }
-        };
 #pragma unroll 1
         for (int u0 = 0; u0 < units; u0 += per) {
             const int n = min(per, units - u0);
@@ -421,18 +373,13 @@ struct Block {
             for (int u = 0; u < UNITS / 2; ++u)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[u][0][i] = acc[u][1][i] = 0.f;
-            uint4 x[STEPS], next[STEPS];
-            if (!DIRECT) fetch(next, 0);
 #pragma unroll 1
             for (int k0 = 0; k0 < K; k0 += PIECE) {
-                if constexpr (DIRECT) {
-                    fetch(x, k0);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < STEPS; ++i) x[i] = next[i];
-                    if (k0 + PIECE < K) fetch(next, k0 + PIECE);
-                }
                 const int steps = min(PIECE, K - k0) / 32;
+                uint4 x[STEPS];                                 // this lane's activations of the piece
+#pragma unroll
+                for (int i = 0; i < STEPS; ++i)
+                    x[i] = g < M && i * CW + warp < steps ? lds16(act + (k0 + i * (CW * 32)) * 2) : make_uint4(0, 0, 0, 0);
 #pragma unroll
                 for (int u = 0; u < UNITS / 2; ++u) {
                     if (2 * u < n) {
@@ -473,7 +420,7 @@ struct Block {
             for (int u = 0; u < UNITS / 2; ++u)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    red[((warp * UNITS + 2 * u + i / 2) * TOKENS + 2 * c + i % 2) * 8 + g] = acc[u][0][i] + acc[u][1][i];
+                    red[((warp * UNITS + 2 * u + i / 2) * 8 + 2 * c + i % 2) * 8 + g] = acc[u][0][i] + acc[u][1][i];
             consumers_sync();
             each(u0 * 8, min(rows - u0 * 8, n * 8));
             consumers_sync();                                   // (the sums' place is free again)
@@ -481,36 +428,32 @@ struct Block {
     }
     // the sum of all warps for row `row` of the group and token t
     __device__ __forceinline__ float total(int row, int t) const {
-        const float* at = red + ((row >> 3) * TOKENS + t) * 8 + (row & 7);
+        const float* at = red + ((row >> 3) * 8 + t) * 8 + (row & 7);
         float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < CW; ++w) v += at[w * UNITS * TOKENS * 8];
+        for (int w = 0; w < CW; ++w) v += at[w * UNITS * 64];
         return v;
     }
 
     // 1 / rms of every token from the blocks' sums of squares [parts][tokens]: a warp per token
-    __device__ __forceinline__ void load_rms(const float* sums, int parts, float eps, uint32_t tag) {
+    __device__ __forceinline__ void load_rms(const uint2* sums, int parts, float eps, uint32_t tag) {
         for (int t = warp; t < s().n_tok; t += CW) {
             float v = 0.f;
-            if (DIRECT) {
-                uint2 w[8];                                     // (parts is at most 256)
-                until([&] {
-                    bool all = true;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (k * 32 + lane < parts) w[k] = look8(reinterpret_cast<const uint2*>(sums) + (k * 32 + lane) * DIRECT_TOKENS + t);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (k * 32 + lane < parts) all &= w[k].y == tag;
-                    return all;
-                });
-                __syncwarp();
+            uint2 w[8];                                         // (parts is at most 256)
+            until([&] {
+                bool all = true;
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    if (k * 32 + lane < parts) v += __uint_as_float(w[k].x);
-            } else {
-                for (int i = lane; i < parts; i += 32) v += ld_l2(sums + i * TOKENS + t);
-            }
+                    if (k * 32 + lane < parts) w[k] = look8(sums + (k * 32 + lane) * TOKENS + t);
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k * 32 + lane < parts) all &= w[k].y == tag;
+                return all;
+            });
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k * 32 + lane < parts) v += __uint_as_float(w[k].x);
             v = warp_sum(v);
             if (lane == 0) rms[t] = 1.0f / sqrtf(v * s().inv_hidden + eps);
         }
@@ -541,7 +484,7 @@ struct Block {
         }
         // q of the group's heads, and the token's own key and value where they are this block's: rotated, in bf16
         const bool own = g.s1 == keys.slices(t);
-        const float* row = s().qkv + (size_t)t * nqkv;
+        const uint2* row = s().qkv + (size_t)t * nqkv;
         const int n_q = group * (D / 2), n_all = n_q + (own ? D : 0);
         const int page = own ? L.table[(size_t)entries[t] * s().max_blocks + at_pos / s().page_size] : -1;
         const size_t cache_row = (((size_t)max(page, 0) * s().n_kv + g.kvh) * s().page_size + at_pos % s().page_size) * D;
@@ -551,19 +494,13 @@ struct Block {
             // the pair: (i, i + half) where it rotates, else neighbouring columns (behind the rotated ones)
             const bool turns = !is_v && i < half;
             const int c0 = turns ? i : is_v ? 2 * i : rot + 2 * (i - half), c1 = turns ? i + half : c0 + 1;
-            const float* src = row + (size_t)(is_q ? h0 + r : is_v ? s().n_heads + s().n_kv + g.kvh : s().n_heads + g.kvh) * D;
-            float a, b;
-            if (DIRECT) {
-                const uint2* words = reinterpret_cast<const uint2*>(s().qkv) + (src - s().qkv);
-                uint2 wa, wb;
-                until([&] {
-                    wa = look8(words + c0), wb = look8(words + c1);
-                    return wa.y == tag && wb.y == tag;
-                });
-                a = __uint_as_float(wa.x), b = __uint_as_float(wb.x);
-            } else {
-                a = ld_l2(src + c0), b = ld_l2(src + c1);
-            }
+            const uint2* src = row + (size_t)(is_q ? h0 + r : is_v ? s().n_heads + s().n_kv + g.kvh : s().n_heads + g.kvh) * D;
+            uint2 wa, wb;
+            until([&] {
+                wa = look8(src + c0), wb = look8(src + c1);
+                return wa.y == tag && wb.y == tag;
+            });
+            float a = __uint_as_float(wa.x), b = __uint_as_float(wb.x);
             if (turns) {
                 const float2 w = at[i];
                 const float ra = a * w.y - b * w.x, rb = a * w.x + b * w.y;
@@ -646,12 +583,8 @@ struct Block {
                 if (alone) {
                     const float inv = 1.0f / sum;
                     const size_t to = ((size_t)t * s().n_heads + h0 + r) * D + col;
-                    if (DIRECT) {
-                        tell(reinterpret_cast<uint32_t*>(s().attn) + to, tagged(v0 * inv, tag));
-                        tell(reinterpret_cast<uint32_t*>(s().attn) + to + 1, tagged(v1 * inv, tag));
-                    } else {
-                        *reinterpret_cast<uint32_t*>(s().attn + to) = pack_bf16(v0 * inv, v1 * inv);
-                    }
+                    tell(s().attn + to, tagged(v0 * inv, tag));
+                    tell(s().attn + to + 1, tagged(v1 * inv, tag));
                 } else {
                     *reinterpret_cast<float2*>(po + r * D + col) = make_float2(v0, v1);
                     if (col == 0) pml[r] = make_float2(M, sum);
@@ -669,44 +602,39 @@ struct Block {
             if (*s_last) s().counters[g.pair] = 0;
         }
         consumers_sync();
-        if (*s_last) merge<D, DIRECT>(s(), g, tag);
+        if (*s_last) merge<D>(s(), g, tag);
         consumers_sync();
     }
 
     // ---- the consumers' step ---------------------------------------------------------------------------------------------------
-    // A layer's meetings: 5 l before its q/k/v product (the step's first needs none), then one before each of the other phases.
-    __device__ __forceinline__ bool attention(int l) {
+    __device__ __forceinline__ void attention(int l) {
         const Keys keys{pos, s().n_tok, p.layer[l].window};
         const Line line = keys.line(s().n_kv, gridDim.x);
         int turned = -1;                                        // the token whose angles are there
         for_segments(keys, line, s().n_kv, blockIdx.x, [&](const Segment g) {
             if (turned < 0) angles(g.token, p.layer[l].inv_freq), turned = g.token;
         });
-        if (DIRECT) consumers_sync();
-        else if (!meet(5 * l + 1)) return false;
+        consumers_sync();
         for_segments(keys, line, s().n_kv, blockIdx.x, [&](const Segment g) {
             segment(l, g, turned == g.token);
             turned = g.token;
         });
-        if (!DIRECT) arrive();
-        return true;
     }
     // One of the four products of a layer: q/k/v, output, gate/up, down.
-    __device__ __forceinline__ bool multiply(int l, int which) {
+    __device__ __forceinline__ void multiply(int l, int which) {
         const int G = gridDim.x, b = blockIdx.x, H = s().hidden, M = s().n_tok, da = s().n_heads * D, nqkv = (s().n_heads + 2 * s().n_kv) * D;
         const ResidentLayer& L = p.layer[l];
-        if (!DIRECT && l + which > 0 && !meet(5 * l + which + (which > 0))) return false;
         const uint32_t tag = l + 1, next_tag = which == 3 ? l + 2 : l + 1;      // of what this product reads and of h behind it
         const bool last = which == 3 && l + 1 == s().n_layers, residual = which == 1 || which == 3;
         const int n = which == 0 ? nqkv : which == 2 ? s().ff : H, pairs = which == 2 ? 2 : 1;
         const int r0 = share(b, n, G) * pairs, rows = share(b + 1, n, G) * pairs - r0;
-        const bf16* in = which == 0 ? s().h[0] : which == 1 ? s().attn : which == 2 ? s().h[1] : s().act;
-        if (DIRECT) gather(in, M * (which == 1 ? da : which == 3 ? s().ff : H), tag);
+        const uint32_t* in = which == 0 ? s().h[0] : which == 1 ? s().attn : which == 2 ? s().h[1] : s().act;
+        gather(in, M * (which == 1 ? da : which == 3 ? s().ff : H), tag);
         if (!residual) load_rms(s().sums[which / 2], l + which == 0 ? 1 : G, which == 0 ? L.eps_mixer : L.eps_ffn, tag);
         const void* bias = which == 0 ? L.b_qkv : which == 1 ? L.b_o : nullptr;
         const void* norm_w = which == 1 ? L.norm_ffn : which == 3 && !last ? p.layer[l + 1].norm_mixer : nullptr;
         const int next = which == 1;                            // whose h and sums a residual product hands on
-        product(in, which == 1 ? da : which == 3 ? s().ff : H, rows, [&](int first, int here) {
+        product(which == 1 ? da : which == 3 ? s().ff : H, rows, [&](int first, int here) {
             const int mine = here / pairs;                      // results of this block (a gate and its up row make one)
 #pragma unroll 1
             for (int e = threadIdx.x; e < mine * M; e += CT) {
@@ -714,8 +642,7 @@ struct Block {
                 if (which == 2) {
                     const float v = glu_act(total(2 * i, t) * rms[t], total(2 * i + 1, t) * rms[t], GLU_SILU, 0.f, 0.f);
                     const size_t to = (size_t)t * s().ff + col;
-                    if (DIRECT) tell(reinterpret_cast<uint32_t*>(s().act) + to, tagged(v, tag));
-                    else s().act[to] = __float2bfloat16_rn(v);
+                    tell(s().act + to, tagged(v, tag));
                     continue;
                 }
                 float v = total(i, t);
@@ -723,8 +650,7 @@ struct Block {
                 if (bias) v += load_any(bias, which == 0 ? s().qkv_bias_dtype : s().o_bias_dtype, col);
                 if (which == 0) {
                     const size_t to = (size_t)t * nqkv + col;
-                    if (DIRECT) tell(reinterpret_cast<uint2*>(s().qkv) + to, v, tag);
-                    else s().qkv[to] = v;
+                    tell(s().qkv + to, v, tag);
                     continue;
                 }
                 float* x = x_s + t * MAX_ROWS + first + i;
@@ -735,67 +661,33 @@ struct Block {
                     continue;
                 }
                 v *= load_any(norm_w, s().norm_dtype, col);
-                if (DIRECT) tell(reinterpret_cast<uint32_t*>(s().h[next]) + to, tagged(v, next_tag));
-                else s().h[next][to] = __float2bfloat16_rn(v);
+                tell(s().h[next] + to, tagged(v, next_tag));
             }
         });
-        if (last) return true;
-        if (residual)
+        if (residual && !last)
             for (int t = warp; t < M; t += CW) {
                 float v = 0.f;
                 for (int i = lane; i < rows; i += 32) v += x_s[t * MAX_ROWS + i] * x_s[t * MAX_ROWS + i];
                 v = warp_sum(v);
-                if (lane == 0) {
-                    if (DIRECT) tell(reinterpret_cast<uint2*>(s().sums[next]) + b * DIRECT_TOKENS + t, v, next_tag);
-                    else s().sums[next][b * TOKENS + t] = v;
-                }
+                if (lane == 0) tell(s().sums[next] + b * TOKENS + t, v, next_tag);
             }
-        if (!DIRECT) arrive();
-        return true;
+    }
+    __device__ __forceinline__ void consume() {
+        const int G = gridDim.x, H = s().hidden, x0 = share(blockIdx.x, H, G), x_rows = share(blockIdx.x + 1, H, G) - x0;
+        for (int e = threadIdx.x; e < x_rows * s().n_tok; e += CT) x_s[e / x_rows * MAX_ROWS + e % x_rows] = s().x[(size_t)(e / x_rows) * H + x0 + e % x_rows];
+        consumers_sync();
+#pragma unroll 1
+        for (int step = 0; step < 4 * s().n_layers; ++step) {   // (one body for the four products)
+            if (step % 4 == 1) attention(step / 4);
+            multiply(step / 4, step % 4);
+        }
     }
 };
 
-// The loader and the two kinds of phase as calls: in one body with one another hundreds of bytes of registers spilled.  The phases
-// return how far the ring has been passed, or GIVE_UP.
-constexpr uint32_t GIVE_UP = 0xffffffffu;
-template <int D, bool DIRECT>
-__device__ __forceinline__ uint32_t attend(const Params& p, uint8_t* smem, int layer, uint32_t seq) {
-    Block<D, DIRECT> block(p, smem, seq);
-    return block.attention(layer) ? block.seq : GIVE_UP;
-}
-template <int D, bool DIRECT>
-__device__ __forceinline__ uint32_t multiply(const Params& p, uint8_t* smem, int layer, int which, uint32_t seq) {
-    Block<D, DIRECT> block(p, smem, seq);
-    return block.multiply(layer, which) ? block.seq : GIVE_UP;
-}
 template <int D>
-__device__ __noinline__ void load(const Params& p, uint8_t* smem) {
-    Block<D, false> block(p, smem);
-    block.loader();
-}
-
-template <int D, bool DIRECT>
-__device__ __forceinline__ void consume(const Params& p, uint8_t* smem) {
-    const int G = gridDim.x, H = p.s.hidden, x0 = share(blockIdx.x, H, G), x_rows = share(blockIdx.x + 1, H, G) - x0;
-    float* x_s = reinterpret_cast<float*>(smem + Smem::X);
-    for (int e = threadIdx.x; e < x_rows * p.s.n_tok; e += CT) x_s[e / x_rows * MAX_ROWS + e % x_rows] = p.s.x[(size_t)(e / x_rows) * H + x0 + e % x_rows];
-    consumers_sync();
-    uint32_t seq = 0;
-#pragma unroll 1
-    for (int step = 0; step < 4 * p.s.n_layers; ++step) {
-        if (step % 4 == 1) {
-            seq = attend<D, DIRECT>(p, smem, step / 4, seq);
-            if (seq == GIVE_UP) return;
-        }
-        seq = multiply<D, DIRECT>(p, smem, step / 4, step % 4, seq);
-        if (seq == GIVE_UP) return;
-    }
-}
-
-template <int D, bool DIRECT>
 __global__ void __launch_bounds__(THREADS, 1) decode_resident_kernel(const __grid_constant__ Params p) {
     extern __shared__ uint8_t smem_raw[];
-    Block<D, DIRECT> block(p, smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
+    Block<D> block(p, smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
     if (threadIdx.x < p.s.n_tok) {
         block.pos[threadIdx.x] = p.s.positions[threadIdx.x];
         block.entries[threadIdx.x] = p.s.tok_entry[threadIdx.x];
@@ -807,31 +699,30 @@ __global__ void __launch_bounds__(THREADS, 1) decode_resident_kernel(const __gri
         tc::fence_proxy_async();
     }
     __syncthreads();
-    if (block.warp == CW) load<D>(p, block.smem);
-    else consume<D, DIRECT>(p, block.smem);
+    if (block.warp == CW) block.loader();
+    else block.consume();
 }
 
-// The step's first kernel: a token's embedding, bf16(x * w) for the first product and the sum of squares behind its norm; the
-// meeting counter and the pairs' arrival counters start at zero, and no word has a tag (direct).
+// The step's first kernel: a token's embedding, bf16(x * w) for the first product and the sum of squares behind its norm; no other
+// word has a tag, and the pairs' arrival counters start at zero.
+constexpr int BEGIN_BLOCKS = 64;
 template <typename TE>
 __global__ void __launch_bounds__(256) resident_begin_kernel(const TE* __restrict__ table, const int* __restrict__ ids,
                                                               const int* __restrict__ device_tokens, int vocab, float scale,
-                                                              const void* __restrict__ w, const ResidentStep s, int head_dim, int blocks, int direct) {
+                                                              const void* __restrict__ w, const ResidentStep s, int head_dim, int blocks) {
     __shared__ float red[32];
     const int at = blockIdx.x * 256 + threadIdx.x, all = gridDim.x * 256;
-    if (direct) {
-        auto clear = [&](void* p, long long words) {
-            for (long long i = at; i < words; i += all) reinterpret_cast<uint32_t*>(p)[i] = 0;
-        };
-        clear(s.h[1], (long long)s.n_tok * s.hidden);
-        clear(s.attn, (long long)s.n_tok * s.n_heads * head_dim);
-        clear(s.act, (long long)s.n_tok * s.ff);
-        clear(s.qkv, 2ll * s.n_tok * (s.n_heads + 2 * s.n_kv) * head_dim);
-        clear(s.sums[1], 2ll * blocks * DIRECT_TOKENS);
-        clear(reinterpret_cast<uint2*>(s.sums[0]) + DIRECT_TOKENS, 2ll * (blocks - 1) * DIRECT_TOKENS);
-    }
-    if (at < 2) s.sync[at] = 0;
-    for (int i = at; i < TOKENS * s.n_kv; i += all) s.counters[i] = 0;
+    auto clear = [&](void* p, long long words) {
+        for (long long i = at; i < words; i += all) reinterpret_cast<uint32_t*>(p)[i] = 0;
+    };
+    clear(s.h[1], (long long)s.n_tok * s.hidden);
+    clear(s.attn, (long long)s.n_tok * s.n_heads * head_dim);
+    clear(s.act, (long long)s.n_tok * s.ff);
+    clear(s.qkv, 2ll * s.n_tok * (s.n_heads + 2 * s.n_kv) * head_dim);
+    clear(s.sums[1], 2ll * blocks * TOKENS);
+    clear(s.sums[0] + TOKENS, 2ll * (blocks - 1) * TOKENS);
+    clear(s.stop, 1);
+    clear(s.counters, TOKENS * s.n_kv);
     const int t = blockIdx.x;
     if (t >= s.n_tok) return;
     int id = ids[t];
@@ -839,37 +730,32 @@ __global__ void __launch_bounds__(256) resident_begin_kernel(const TE* __restric
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
     float ss = 0.f;
     for (int i = threadIdx.x; i < s.hidden; i += 256) {
-        const float v = to_f32(table[(size_t)id * s.hidden + i]) * scale, h = v * load_any(w, s.norm_dtype, i);
+        const float v = to_f32(table[(size_t)id * s.hidden + i]) * scale;
         const size_t to = (size_t)t * s.hidden + i;
         s.x[to] = v;
-        if (direct) reinterpret_cast<uint32_t*>(s.h[0])[to] = tagged(h, 1);
-        else s.h[0][to] = __float2bfloat16_rn(h);
+        s.h[0][to] = tagged(v * load_any(w, s.norm_dtype, i), 1);
         ss += v * v;
     }
     ss = block_sum(ss, red);
-    if (threadIdx.x == 0) {
-        if (direct) reinterpret_cast<uint2*>(s.sums[0])[t] = make_uint2(__float_as_uint(ss), 1);
-        else s.sums[0][t] = ss;
-    }
+    if (threadIdx.x == 0) s.sums[0][t] = make_uint2(__float_as_uint(ss), 1);
 }
 
 long long up(long long v) { return (v + 255) / 256 * 256; }
 
 }  // namespace
 
-// Scratch of a step of up to TOKENS tokens; sets the step's pointers into `at`.  (The tagged words of DIRECT_TOKENS tokens take no
-// more than the plain values of TOKENS.)
+// Scratch of a step of up to TOKENS tokens; sets the step's pointers into `at`.
 long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, int blocks) {
     long long off = 0;
     auto take = [&](long long bytes) { const long long here = off; off += up(bytes); return at ? at + here : nullptr; };
     const long long da = (long long)s->n_heads * head_dim, nqkv = (long long)(s->n_heads + 2 * s->n_kv) * head_dim, pieces = blocks + TOKENS * s->n_kv;
-    for (int i = 0; i < 2; ++i) s->h[i] = (bf16*)take(TOKENS * (long long)s->hidden * 2), s->sums[i] = (float*)take((long long)blocks * TOKENS * 4);
-    s->qkv = (float*)take(TOKENS * nqkv * 4);
-    s->attn = (bf16*)take(TOKENS * da * 2);
-    s->act = (bf16*)take(TOKENS * (long long)s->ff * 2);
+    for (int i = 0; i < 2; ++i) s->h[i] = (uint32_t*)take(TOKENS * (long long)s->hidden * 4), s->sums[i] = (uint2*)take((long long)blocks * TOKENS * 8);
+    s->qkv = (uint2*)take(TOKENS * nqkv * 8);
+    s->attn = (uint32_t*)take(TOKENS * da * 4);
+    s->act = (uint32_t*)take(TOKENS * (long long)s->ff * 4);
     s->part_o = (float*)take(pieces * GROUP * head_dim * 4);
     s->part_ml = (float*)take(pieces * GROUP * 8);
-    s->sync = (unsigned int*)take(8);
+    s->stop = (unsigned int*)take(4);
     s->counters = (int*)take((long long)TOKENS * s->n_kv * 4);
     return off;
 }
@@ -880,7 +766,8 @@ int infero_resident_supported(const ResidentStep* s, int head_dim, int blocks) {
     return s->n_tok >= 1 && s->n_tok <= TOKENS && s->n_layers >= 1 && s->n_layers <= RESIDENT_LAYERS && (head_dim == 64 || head_dim == 128) &&
            s->page_size % 16 == 0 && s->n_kv > 0 && s->n_heads % s->n_kv == 0 && s->n_heads / s->n_kv <= GROUP && s->hidden % 64 == 0 &&
            s->ff % 64 == 0 && (s->n_heads * head_dim) % 64 == 0 && s->hidden / blocks + 1 <= MAX_ROWS && s->rotary_dim % 2 == 0 &&
-           s->rotary_dim <= head_dim && blocks <= 256 && s->ff >= blocks && s->hidden >= 4 * blocks;
+           s->rotary_dim <= head_dim && blocks <= 256 && s->ff >= blocks && s->hidden >= 4 * blocks &&
+           s->n_tok * std::max({s->ff, s->hidden, s->n_heads * head_dim}) * 2 <= ACT_BYTES;
 }
 
 // Returns 0, 1 with the error recorded, or 2 when the device cannot hold the blocks all at once (nothing was launched).
@@ -888,14 +775,11 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
                            int embed_dtype, const int* ids, const int* device_tokens, int vocab, float embed_scale, int blocks,
                            cudaStream_t stream) {
     static std::mutex mutex;
-    static int fits[4] = {-1, -1, -1, -1};                      // blocks a multiprocessor holds, by kernel
-    const int widest = std::max({s->ff, s->hidden, s->n_heads * head_dim});
-    const bool direct = s->n_tok <= DIRECT_TOKENS && s->n_tok * widest * 2 <= ACT_BYTES;
-    void* kernel = head_dim == 64 ? (direct ? (void*)decode_resident_kernel<64, true> : (void*)decode_resident_kernel<64, false>)
-                                  : (direct ? (void*)decode_resident_kernel<128, true> : (void*)decode_resident_kernel<128, false>);
+    static int fits[2] = {-1, -1};                              // blocks a multiprocessor holds, by head size
+    void* kernel = head_dim == 64 ? (void*)decode_resident_kernel<64> : (void*)decode_resident_kernel<128>;
     {
         std::lock_guard<std::mutex> lock(mutex);
-        int& n = fits[2 * (head_dim == 128) + direct];
+        int& n = fits[head_dim == 128];
         if (n < 0) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, THREADS, Smem::TOTAL);
@@ -913,8 +797,7 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
             return 1;
     }
     auto begin = [&](auto* table) {
-        resident_begin_kernel<<<direct ? 64 : s->n_tok, 256, 0, stream>>>(table, ids, device_tokens, vocab, embed_scale, layers[0].norm_mixer, *s,
-                                                                          head_dim, blocks, direct ? 1 : 0);
+        resident_begin_kernel<<<BEGIN_BLOCKS, 256, 0, stream>>>(table, ids, device_tokens, vocab, embed_scale, layers[0].norm_mixer, *s, head_dim, blocks);
     };
     if (embed_dtype == INFERO_F32) begin((const float*)embed);
     else begin((const bf16*)embed);

@@ -23,13 +23,13 @@ struct ResidentStep {
     float inv_hidden;
     const int *positions, *tok_entry;
     float* x;                            // residual stream [n_tok, hidden]
-    // scratch (infero_resident_scratch): h, sums [0] of the first norm, [1] of the second
-    __nv_bfloat16* h[2];
-    float* sums[2];
-    float* qkv;
-    __nv_bfloat16 *attn, *act;
+    // scratch (infero_resident_scratch), values beside tags: h, sums [0] of the first norm, [1] of the second
+    uint32_t* h[2];
+    uint2* sums[2];
+    uint2* qkv;
+    uint32_t *attn, *act;
     float *part_o, *part_ml;
-    unsigned int* sync;                  // the blocks' meeting counter, and a flag that one has given up
+    unsigned int* stop;                  // a block has given up
     int* counters;                       // arrivals per (token, kv head)
 };
 
