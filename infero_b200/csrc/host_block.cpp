@@ -279,13 +279,13 @@ void infero_block_set_fusion(int fused_decode_on, int fused_norm_on) {
     g_fused_norm = fused_norm_on ? 1 : 0;
 }
 
-// A step of a few single tokens through blocks of equal sizes, each with a cache of its own, can run as one resident kernel
-// (decode_resident.cu), where INFERO_RESIDENT=1 asks for it and neither of the two switches above is off.
+// A step of one or two single tokens through blocks of equal sizes, each with a cache of its own, runs as one resident kernel
+// (decode_resident.cu; INFERO_RESIDENT=0 keeps the launches layer by layer, as do the two switches above).
 static int g_resident = -1;
 void infero_block_set_resident(int on) { g_resident = on ? 1 : 0; }
 static bool resident_step(const InferoBlock* b, int n, const InferoStep& s, const int* const* tables, const int* entry_group, int max_blocks,
                           ResidentStep* r, ResidentLayer* layers, int* num_pages) {
-    if (g_resident < 0) { const char* e = getenv("INFERO_RESIDENT"); g_resident = e && e[0] == '1' ? 1 : 0; }
+    if (g_resident < 0) g_resident = env_on("INFERO_RESIDENT") ? 1 : 0;
     if (g_fused_decode < 0) g_fused_decode = env_on("INFERO_FUSED_DECODE") ? 1 : 0;
     if (!g_resident || !g_fused_decode || !fused_norm_wanted() || n < 1 || n > RESIDENT_LAYERS) return false;
     if (s.n_decode != s.n_entries || s.n_decode != s.n_tokens) return false;
