@@ -323,7 +323,7 @@ int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
     const int least = a.head_dim > 64 || a.value_dim > 64 ? WARPS : WARPS / 2;
     const int warps = few ? (group < least ? least : group < WARPS ? group : WARPS) : WARPS;
     // Where blocks of 32 rows are fewer than two a multiprocessor, half as many rows a warp: what a chunk costs a warp is latency, and
-    // twice the warps cover it.
+    // twice the warps cover it (14 heads of 64 over 2, 32-bit, 301 tokens: 152 blocks 63 us, 302 blocks 42).
     const long long wide = few ? 0 : (a.singles + (long long)(a.n_tokens - a.singles + tokens - 1) / tokens) * ((group + WIDE_ROWS - 1) / WIDE_ROWS) *
                                          a.n_kv * (a.cross ? a.n_kv : 1);
     const bool half = !few && wide < 2 * infero_sm_count();
