@@ -416,7 +416,7 @@ int infero_add_rmsnorm_scaled(float* x, const void* delta, int delta_dtype, int 
 #define LAUNCH_RING(TD, TO)                                                                      \
             do {                                                                                 \
                 auto k = add_rmsnorm_ring_kernel<TD, TO>;                                        \
-                if (ring_bytes > 48 * 1024)                                                      \
+                if (ring_bytes > 47 * 1024)      /* (the barriers are shared memory too) */      \
                     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes); \
                 launch_pdl(k, dim3(blocks), dim3(threads), ring_bytes, stream, x, (const TD*)delta, dbias, dbias_dtype, \
                            w, w_dtype, eps, (TO*)out, n_rows, d, ring, err, ds);                      \
