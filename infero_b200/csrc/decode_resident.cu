@@ -779,13 +779,18 @@ long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, in
 }
 
 // Can a step of these sizes run here?  All of K must come in whole 32 columns and rows start on 16 bytes; a block's part of the
-// residual stream and a kv head's query heads have to fit their places; every block needs a part of every product worth a unit.
+// residual stream, a product's activations and a kv head's query heads have to fit their places; every block needs a part of every
+// product worth a unit.  And it is only worth it where a layer is small: at 200 KB of a layer's weights a block (Qwen2.5-0.5B sizes)
+// what counts are the waits between phases (one token at 300 keys 757 us a step in launches, 675 here; at 20 keys 732 and 644; two
+// tokens at 300 782 and 730), at 3.2 MB (7B sizes) the stream, which the launches keep up as well.
+constexpr long long LAYER_BYTES = 256 * 1024;
 int infero_resident_supported(const ResidentStep* s, int head_dim, int blocks) {
+    const long long H = s->hidden, da = (long long)s->n_heads * head_dim, nqkv = (long long)(s->n_heads + 2 * s->n_kv) * head_dim;
     return s->n_tok >= 1 && s->n_tok <= TOKENS && s->n_layers >= 1 && s->n_layers <= RESIDENT_LAYERS && (head_dim == 64 || head_dim == 128) &&
-           s->page_size % 16 == 0 && s->n_kv > 0 && s->n_heads % s->n_kv == 0 && s->n_heads / s->n_kv <= GROUP && s->hidden % 64 == 0 &&
-           s->ff % 64 == 0 && (s->n_heads * head_dim) % 64 == 0 && s->hidden / blocks + 1 <= MAX_ROWS && s->rotary_dim % 2 == 0 &&
-           s->rotary_dim <= head_dim && blocks <= 256 && s->ff >= blocks && s->hidden >= 4 * blocks &&
-           s->n_tok * std::max({s->ff, s->hidden, s->n_heads * head_dim}) * 2 <= ACT_BYTES;
+           s->page_size % 16 == 0 && s->n_kv > 0 && s->n_heads % s->n_kv == 0 && s->n_heads / s->n_kv <= GROUP && H % 64 == 0 &&
+           s->ff % 64 == 0 && da % 64 == 0 && H / blocks + 1 <= MAX_ROWS && s->rotary_dim % 2 == 0 && s->rotary_dim <= head_dim &&
+           blocks <= 256 && s->ff >= blocks && H >= 4 * blocks && s->n_tok * std::max({(long long)s->ff, H, da}) * 2 <= ACT_BYTES &&
+           2 * H * (nqkv + da + 3ll * s->ff) <= LAYER_BYTES * blocks;
 }
 
 // Returns 0, 1 with the error recorded, or 2 when the device cannot hold the blocks all at once (nothing was launched).
