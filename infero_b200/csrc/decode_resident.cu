@@ -9,8 +9,8 @@
 // a barrier; meanwhile the ring fills with the weights of the phases behind it.
 //
 //   products   Every block has an equal share of a matrix's rows, and all of K: no partial sums leave a block.  Rows come eight
-//              at a time (a unit), K in pieces of 896 columns; a unit's piece is one slot of the ring and one
-//              TMA box (a copy a row took the loader 1,000 cycles a slot, half the memory's rate at 7B sizes).  The seven consumer
+//              at a time (a unit), K in pieces of 896 columns; a unit's piece is one slot of the ring, a bulk
+//              copy a row.  The seven consumer
 //              warps share a slot's columns, 32 at a time in turns, on mma.sync m16n8k16 (rows of A: two units, columns of B: the
 //              tokens); their sums meet in shared memory, in warp order.  A lane reads 16 bytes of a weight row and 16 of
 //              an activation row and takes them for two k-steps (k is permuted alike on both sides, so no ldmatrix is needed).
@@ -64,7 +64,7 @@ static_assert(Smem::TOTAL <= 232448, "");
 static_assert(Smem::BARS % 8 == 0 && Smem::X % 16 == 0 && Smem::Q % 16 == 0 && Smem::KV % 16 == 0, "");
 
 struct alignas(64) Params {
-    CUtensorMap k_map[RESIDENT_LAYERS], v_map[RESIDENT_LAYERS], w_map[RESIDENT_LAYERS][4];    // (w: q/k/v, output, gate/up, down)
+    CUtensorMap k_map[RESIDENT_LAYERS], v_map[RESIDENT_LAYERS];
     ResidentLayer layer[RESIDENT_LAYERS];
     ResidentStep s;
     int* err_flag;
@@ -86,10 +86,6 @@ __device__ __forceinline__ uint4 lds16(uint32_t at) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
     return v;
-}
-__device__ __forceinline__ void tile_load(uint32_t dst, const CUtensorMap* map, int row, int k64, uint64_t* bar, uint64_t policy) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
-                 ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(k64), "r"(tc::smem_u32(bar)), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void arrive_n(uint64_t* bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
@@ -267,7 +263,7 @@ struct Block {
     __device__ __forceinline__ bool acquire() {                 // the slot `seq` is free
         return seq < SLOTS || wait(&empty[seq % SLOTS], (seq / SLOTS - 1) & 1u);
     }
-    __device__ __forceinline__ bool load_matrix(const bf16* w, const CUtensorMap* map, int r0, int r1, int K, uint64_t policy) {
+    __device__ __forceinline__ bool load_matrix(const bf16* w, int r0, int r1, int K, uint64_t policy) {
         const int units = (r1 - r0 + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
         for (int u0 = 0; u0 < units; u0 += per)
             for (int k0 = 0; k0 < K; k0 += PIECE) {
@@ -276,13 +272,6 @@ struct Block {
                     if (!acquire()) return false;
                     const int rows = min(8, r1 - r0 - u * 8);
                     uint64_t* bar = &full[seq % SLOTS];
-                    if (rows == 8) {                            // a whole unit: one box (what lies beyond K arrives as zeros)
-                        if (lane == 0) {
-                            tc::mbar_expect_tx(bar, 8 * PIECE * 2);
-                            tile_load(tc::smem_u32(smem) + (seq % SLOTS) * SLOT, map, r0 + u * 8, k0 / 64, bar, policy);
-                        }
-                        continue;
-                    }
                     if (lane == 0) tc::mbar_expect_tx(bar, rows * bytes);
                     __syncwarp();
                     if (lane < rows)
@@ -328,11 +317,11 @@ struct Block {
         bool ok = true;
         for (int l = 0; ok && l < s().n_layers; ++l) {
             const ResidentLayer& L = p.layer[l];
-            ok = load_matrix(L.w_qkv, &p.w_map[l][0], share(b, nqkv, G), share(b + 1, nqkv, G), H, policy) &&
+            ok = load_matrix(L.w_qkv, share(b, nqkv, G), share(b + 1, nqkv, G), H, policy) &&
                  load_keys(l, Keys{pos, s().n_tok, L.window}, policy) &&
-                 load_matrix(L.w_o, &p.w_map[l][1], share(b, H, G), share(b + 1, H, G), da, policy) &&
-                 load_matrix(L.w_gate_up, &p.w_map[l][2], 2 * share(b, s().ff, G), 2 * share(b + 1, s().ff, G), H, policy) &&
-                 load_matrix(L.w_down, &p.w_map[l][3], share(b, H, G), share(b + 1, H, G), s().ff, policy);
+                 load_matrix(L.w_o, share(b, H, G), share(b + 1, H, G), da, policy) &&
+                 load_matrix(L.w_gate_up, 2 * share(b, s().ff, G), 2 * share(b + 1, s().ff, G), H, policy) &&
+                 load_matrix(L.w_down, share(b, H, G), share(b + 1, H, G), s().ff, policy);
         }
         if (!ok && lane == 0) *abort_flag = 1;
         // whatever is still on its way lands before the block (and its shared memory) goes away
@@ -371,18 +360,7 @@ struct Block {
         const int units = (rows + 7) / 8, groups = (units + UNITS - 1) / UNITS, per = groups ? (units + groups - 1) / groups : 0;
         const int g = lane >> 2, c = lane & 3, M = s().n_tok;
         const uint32_t act = tc::smem_u32(smem) + Smem::ACT + (g * K + warp * 32 + c * 8) * 2;
-        // Where a lane's 16 bytes of step i lie in a slot: rows ROW_BYTES apart (units of fewer than eight rows), or as the box leaves
-        // them, eight rows of 128 bytes for every 64 columns with their 16-byte pieces in turned places.
-        const uint32_t ring = tc::smem_u32(smem);
-        uint32_t in_box[STEPS];
-#pragma unroll
-        for (int i = 0; i < STEPS; ++i) {
-            const int q = (i * CW + warp) * 4 + c;
-            in_box[i] = (q >> 3) * 1024 + g * 128 + ((q & 7) ^ g) * 16;
-        }
-        auto piece_at = [&](uint32_t q, bool box, int i) {
-            return ring + (q % SLOTS) * SLOT + (box ? in_box[i] : g * ROW_BYTES + (i * CW + warp) * 64 + c * 16);
-        };
+        const uint32_t mine_at = tc::smem_u32(smem) + g * ROW_BYTES + warp * 64 + c * 16;
 #pragma unroll 1
         for (int u0 = 0; u0 < units; u0 += per) {
             const int n = min(per, units - u0);
@@ -402,17 +380,17 @@ struct Block {
                 for (int u = 0; u < UNITS / 2; ++u) {
                     if (2 * u < n) {
                         const bool two = 2 * u + 1 < n;
-                        const bool box0 = rows - (u0 + 2 * u) * 8 >= 8, box1 = rows - (u0 + 2 * u + 1) * 8 >= 8;
+                        const uint32_t w0 = mine_at + (seq % SLOTS) * SLOT, w1 = mine_at + ((seq + 1) % SLOTS) * SLOT;
                         uint4 a0[STEPS], a1[STEPS];
                         arrived(seq);
 #pragma unroll
                         for (int i = 0; i < STEPS; ++i)
-                            if (i * CW + warp < steps) a0[i] = lds16(piece_at(seq, box0, i));
+                            if (i * CW + warp < steps) a0[i] = lds16(w0 + i * (CW * 64));
                         if (two) {
                             arrived(seq + 1);
 #pragma unroll
                             for (int i = 0; i < STEPS; ++i)
-                                if (i * CW + warp < steps) a1[i] = lds16(piece_at(seq + 1, box1, i));
+                                if (i * CW + warp < steps) a1[i] = lds16(w1 + i * (CW * 64));
                         } else {
 #pragma unroll
                             for (int i = 0; i < STEPS; ++i) a1[i] = make_uint4(0, 0, 0, 0);
@@ -782,7 +760,8 @@ long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, in
 // residual stream, a product's activations and a kv head's query heads have to fit their places; every block needs a part of every
 // product worth a unit.  And it is only worth it where a layer is small: at 200 KB of a layer's weights a block (Qwen2.5-0.5B sizes)
 // what counts are the waits between phases (one token at 300 keys 757 us a step in launches, 675 here; at 20 keys 732 and 644; two
-// tokens at 300 782 and 730), at 3.2 MB (7B sizes) the stream, which the launches keep up as well.
+// tokens at 300 782 and 730), from 0.6 MB on (1.5B
+// sizes) the stream, which the launches keep up better: 1,160 and 1,316, at 7B sizes 2,689 and 3,381.
 constexpr long long LAYER_BYTES = 256 * 1024;
 int infero_resident_supported(const ResidentStep* s, int head_dim, int blocks) {
     const long long H = s->hidden, da = (long long)s->n_heads * head_dim, nqkv = (long long)(s->n_heads + 2 * s->n_kv) * head_dim;
@@ -817,12 +796,6 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
         p.layer[l] = layers[l];
         if (infero_tensor_map_bf16(layers[l].k_cache, num_pages[l] * s->n_kv * s->page_size, head_dim, head_dim, 16, &p.k_map[l]) ||
             infero_tensor_map_bf16(layers[l].v_cache, num_pages[l] * s->n_kv * s->page_size, head_dim, head_dim, 16, &p.v_map[l]))
-            return 1;
-        const int da = s->n_heads * head_dim, nqkv = (s->n_heads + 2 * s->n_kv) * head_dim;
-        if (infero_tensor_map_bf16_k64(layers[l].w_qkv, nqkv, s->hidden, 8, PIECE / 64, &p.w_map[l][0]) ||
-            infero_tensor_map_bf16_k64(layers[l].w_o, s->hidden, da, 8, PIECE / 64, &p.w_map[l][1]) ||
-            infero_tensor_map_bf16_k64(layers[l].w_gate_up, 2 * s->ff, s->hidden, 8, PIECE / 64, &p.w_map[l][2]) ||
-            infero_tensor_map_bf16_k64(layers[l].w_down, s->hidden, s->ff, 8, PIECE / 64, &p.w_map[l][3]))
             return 1;
     }
     auto begin = [&](auto* table) {

@@ -4,7 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
-constexpr int RESIDENT_LAYERS = 36;      // layers a launch takes (their descriptors are kernel parameters)
+constexpr int RESIDENT_LAYERS = 48;      // layers a launch takes (their descriptors are kernel parameters)
 
 struct ResidentLayer {
     const __nv_bfloat16 *w_qkv, *w_o, *w_gate_up, *w_down;      // w_gate_up: rows alternate gate_j, up_j

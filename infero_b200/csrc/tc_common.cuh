@@ -294,6 +294,4 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32_b_mn(int m, int n) { return
 // Host side (tc_host.cu): a cached TMA descriptor for a [rows, cols] bf16 matrix with row
 // stride ld elements and boxes of box_rows x 64 elements, 128-byte swizzle.
 int infero_tensor_map_bf16(const void* ptr, int rows, int cols, int ld, int box_rows, CUtensorMap* out);
-// The same matrix (rows of whole 64 columns, one after the other) as [cols / 64, rows, 64], boxes of box_blocks x box_rows x 64.
-int infero_tensor_map_bf16_k64(const void* ptr, int rows, int cols, int box_rows, int box_blocks, CUtensorMap* out);
 int infero_tc_err_flag(int** out);

@@ -47,47 +47,34 @@ int load_encoder() {
 
 }  // namespace
 
-namespace {
-
-// ptr's map of the given rank, made once per key.
-int cached_map(const MapKey& key, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, CUtensorMap* out) {
+// A [rows, cols] bf16 matrix with row stride ld (elements), tiles of box_rows x 64 elements,
+// 128-byte swizzle, zero fill outside the matrix.  Returns 0, or 1 with the error recorded.
+int infero_tensor_map_bf16(const void* ptr, int rows, int cols, int ld, int box_rows, CUtensorMap* out) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (load_encoder()) return 1;
+    MapKey key{ptr, rows, cols, ld, box_rows};
     auto it = g_maps.find(key);
     if (it != g_maps.end()) {
         *out = it->second;
         return 0;
     }
-    cuuint32_t estr[3] = {1, 1, 1};
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {(cuuint32_t)TILE_K, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
-    CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(key.ptr), dims, strides, box, estr,
+    CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         infero_set_error("tensor map: cuTensorMapEncodeTiled failed (%d) for a [%d, %d] matrix, row stride %d, box %d",
-                         (int)r, key.rows, key.cols, key.ld, key.box_rows);
+                         (int)r, rows, cols, ld, box_rows);
         return 1;
     }
     if (g_maps.size() > 8192) g_maps.clear();
     g_maps.emplace(key, m);
     *out = m;
     return 0;
-}
-
-}  // namespace
-
-// A [rows, cols] bf16 matrix with row stride ld (elements), tiles of box_rows x 64 elements,
-// 128-byte swizzle, zero fill outside the matrix.  Returns 0, or 1 with the error recorded.
-int infero_tensor_map_bf16(const void* ptr, int rows, int cols, int ld, int box_rows, CUtensorMap* out) {
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, (cuuint32_t)box_rows};
-    return cached_map(MapKey{ptr, rows, cols, ld, box_rows}, 2, dims, strides, box, out);
-}
-
-int infero_tensor_map_bf16_k64(const void* ptr, int rows, int cols, int box_rows, int box_blocks, CUtensorMap* out) {
-    const cuuint64_t dims[3] = {(cuuint64_t)TILE_K, (cuuint64_t)rows, (cuuint64_t)(cols / TILE_K)}, strides[2] = {(cuuint64_t)cols * 2, TILE_K * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)TILE_K, (cuuint32_t)box_rows, (cuuint32_t)box_blocks};
-    return cached_map(MapKey{ptr, rows, cols, -box_blocks, box_rows}, 3, dims, strides, box, out);      // (no row stride is negative)
 }
 
 namespace {

@@ -35,6 +35,7 @@ def main(argv=None) -> int:
     args = ap.parse_args(argv)
 
     os.environ["INFERO_TIMELINE"] = "1"            # before the library is built and loaded
+    os.environ["INFERO_RESIDENT"] = "0"            # the launches of a layer, also where one resident kernel would run the step
     import ctypes
     import random
 
