@@ -591,13 +591,13 @@ struct Block {
             consumers_sync();
         }
         if (alone) return;
-        // ---- the block that arrives last merges the blocks' results
+        // ---- the block that arrives last merges the blocks' results (a counter of the layer's own: one that was set back for the
+        // next layer would have nothing that orders the reset before that layer's arrivals)
         int* s_last = reinterpret_cast<int*>(smem + Smem::MISC) + 28;
         if (threadIdx.x == 0) {
             int old;
-            asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(s().counters + g.pair) : "memory");
+            asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(s().counters + (size_t)layer * TOKENS * s().n_kv + g.pair) : "memory");
             *s_last = old == g.last - g.first;
-            if (*s_last) s().counters[g.pair] = 0;
         }
         consumers_sync();
         if (*s_last) merge<D>(s(), g, tag);
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(256) resident_begin_kernel(const TE* __restric
     clear(s.sums[1], 2ll * blocks * TOKENS);
     clear(s.sums[0] + TOKENS, 2ll * (blocks - 1) * TOKENS);
     clear(s.stop, 1);
-    clear(s.counters, TOKENS * s.n_kv);
+    clear(s.counters, (long long)s.n_layers * TOKENS * s.n_kv);
     const int t = blockIdx.x;
     if (t >= s.n_tok) return;
     int id = ids[t];
@@ -754,7 +754,7 @@ long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, in
     s->part_o = (float*)take(pieces * GROUP * head_dim * 4);
     s->part_ml = (float*)take(pieces * GROUP * 8);
     s->stop = (unsigned int*)take(4);
-    s->counters = (int*)take((long long)TOKENS * s->n_kv * 4);
+    s->counters = (int*)take((long long)RESIDENT_LAYERS * TOKENS * s->n_kv * 4);
     return off;
 }
 
