@@ -104,17 +104,18 @@ __device__ __forceinline__ uint4 look16(const uint32_t* p) {
     asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
+// (a 32-bit value and its tag are one access of 64 bits: a vector of two would be two accesses in no order)
 __device__ __forceinline__ uint2 look8(const uint2* p) {
-    uint2 v;
-    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-    return v;
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return make_uint2((unsigned)v, (unsigned)(v >> 32));
 }
 __device__ __forceinline__ uint32_t tagged(float v, uint32_t tag) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v)) | tag << 16;
 }
 __device__ __forceinline__ void tell(uint32_t* p, uint32_t word) { asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(p), "r"(word) : "memory"); }
 __device__ __forceinline__ void tell(uint2* p, float v, uint32_t tag) {
-    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory");
 }
 
 // ---- who takes which keys ------------------------------------------------------------------------------------------------
