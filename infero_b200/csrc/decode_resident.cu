@@ -89,9 +89,6 @@ __device__ __forceinline__ uint4 lds16(uint32_t at) {
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
     return v;
 }
-__device__ __forceinline__ void arrive_n(uint64_t* bar, uint32_t n) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
-}
 
 // ---- values that carry a tag --------------------------------------------------------------------------------------------------
 // What one block hands to the others needs no meeting.  Every value lies in a word of its own beside a tag (bf16 with 16 bits of
@@ -524,7 +521,16 @@ struct Block {
         int turn = 0;
         for (int b0 = g.s0; b0 < g.s1; b0 += 32)
             for (int i = b0; i < min(g.s1, b0 + 32); i += per, ++seq, turn = turn + 1 == CW ? 0 : turn + 1) {
-                if (turn != warp) continue;
+                if (turn != warp) {
+                    // Another warp's slot, watched all the same: a parity wait tells a phase from the next only, so a warp has to have
+                    // seen the barrier's phase before the one it waits for, and the slot is not filled again before all have.
+                    if (lane == 0) {
+                        arrived(seq);
+                        tc::mbar_arrive(&empty[seq % SLOTS]);
+                    }
+                    continue;
+                }
+                __syncwarp();                                   // (lane 0 has seen the slots in between)
                 arrived(seq);
                 const int n = min(per, min(g.s1, b0 + 32) - i);
                 for (int j = 0; j < n; ++j) {
@@ -544,7 +550,7 @@ struct Block {
                     slice16<D, Swizzled128<D, 16>>(qf, kt, vt, 0, kb, lo, at_pos, lo, at_pos, L.scale_log2, m, l, o, lane);
                 }
                 __syncwarp();
-                if (lane == 0) arrive_n(&empty[seq % SLOTS], CW);
+                if (lane == 0) tc::mbar_arrive(&empty[seq % SLOTS]);
             }
         // ---- the warps' results, 64 columns at a time
         const int gr = lane >> 2, c = lane & 3;
