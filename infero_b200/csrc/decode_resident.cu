@@ -767,18 +767,37 @@ long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, in
 
 // Can a step of these sizes run here?  All of K must come in whole 32 columns and rows start on 16 bytes; a block's part of the
 // residual stream, a product's activations and a kv head's query heads have to fit their places; every block needs a part of every
-// product worth a unit.  And it is only worth it where a layer is small: at 200 KB of a layer's weights a block (Qwen2.5-0.5B sizes)
-// what counts are the waits between phases (one token at 300 keys 757 us a step in launches, 675 here; at 20 keys 732 and 644; two
-// tokens at 300 782 and 730), from 0.6 MB on (1.5B
-// sizes) the stream, which the launches keep up better: 1,160 and 1,316, at 7B sizes 2,689 and 3,381.
-constexpr long long LAYER_BYTES = 256 * 1024;
+// product worth a unit.
 int infero_resident_supported(const ResidentStep* s, int head_dim, int blocks) {
-    const long long H = s->hidden, da = (long long)s->n_heads * head_dim, nqkv = (long long)(s->n_heads + 2 * s->n_kv) * head_dim;
+    const long long H = s->hidden, da = (long long)s->n_heads * head_dim;
     return s->n_tok >= 1 && s->n_tok <= TOKENS && s->n_layers >= 1 && s->n_layers <= RESIDENT_LAYERS && (head_dim == 64 || head_dim == 128) &&
            s->page_size % 16 == 0 && s->n_kv > 0 && s->n_heads % s->n_kv == 0 && s->n_heads / s->n_kv <= GROUP && H % 64 == 0 &&
            s->ff % 64 == 0 && da % 64 == 0 && H / blocks + 1 <= MAX_ROWS && s->rotary_dim % 2 == 0 && s->rotary_dim <= head_dim &&
-           blocks <= 256 && s->ff >= blocks && H >= 4 * blocks && s->n_tok * std::max({(long long)s->ff, H, da}) * 2 <= ACT_BYTES &&
-           2 * H * (nqkv + da + 3ll * s->ff) <= LAYER_BYTES * blocks;
+           blocks <= 256 && s->ff >= blocks && H >= 4 * blocks && s->n_tok * std::max({(long long)s->ff, H, da}) * 2 <= ACT_BYTES;
+}
+
+// Is it the faster way?  What it saves are the waits between launches; what it pays are a copy per slot and block (about 7 us a slot
+// of a layer, over 24 layers) and keys that few warps go through (22 us a thousand, where the launches hardly notice them).  `visible`:
+// keys of the longest request that some layer sees.  Launches and this, replayed, us a step of 24 layers:
+//   width 896, 14 heads of 64 over 2, ff 4,864 (197 KiB of a layer's weights a block, 17 slots): one token at 20 keys 643 and 520, 300 687
+//   and 585, 1,000 695 and 609, 2,000 699 and 627, 3,000 684 and 649, 4,095 684 and 660, 8,191 750 and 766, 16,383 805 and 858; two at 300 706 and
+//   610, at 2,000 692 and 659, at 4,095 each 700 and 695, at 8,191 769 and 817.
+//   up to 256 KiB: width 640, ff 8,192 (26 slots) one token at 2,040 684 and 662, at 4,090 668 and 704; 1,024, ff 5,120 (30 slots) 677 and
+//   664, 685 and 707; 2,048, ff 1,536 767 and 766, 775 and 853; 640, ff 6,144 (20 slots) at 4,090 652 and 653; 896, ff 6,272 (20 slots) 695
+//   and 654.  So 2,048 keys in all, 4,096 where a layer takes up to 20 slots.
+//   beyond: width 1,024, ff 5,504 (258 KiB) one token at 300 683 and 644, two 671 and 675; ff 6,912 (315) 698 and 699, two 713 and 739; 1,536, ff
+//   8,960 (616) 886 and 920; at 7B sizes 2,689 and 3,381.
+//   where the pairs' rounds of 112 keys are more than the blocks, a block has pieces of several pairs: 1,024, ff 4,096, 8 heads of 128 over 8,
+//   one token at 2,040 688 and 752; 16 heads of 64 over 16, ff 4,608 696 and 747.  Layers of up to 128 KiB bear it: 640, ff 2,560, 10 of 64
+//   over 10 at 4,090 (2.5 times the blocks) 686 and 615; 640, ff 1,024, 16 of 128 over 16 at 2,040 (2.05) 731 and 705, at 4,090 (4) 706 and 811.
+int infero_resident_worth(const ResidentStep* s, int head_dim, int blocks, int visible) {
+    const long long H = s->hidden, da = (long long)s->n_heads * head_dim, nqkv = (long long)(s->n_heads + 2 * s->n_kv) * head_dim;
+    const long long bytes = 2 * H * (nqkv + da + 3ll * s->ff) / blocks, keys = (long long)s->n_tok * visible;
+    auto slots = [&](long long n, long long K, int pairs) { return (((n + blocks - 1) / blocks) * pairs + 7) / 8 * ((K + PIECE - 1) / PIECE); };
+    const long long a_layer = slots(nqkv, H, 1) + slots(H, da, 1) + slots(s->ff, H, 2) + slots(H, s->ff, 1);
+    const long long rounds = (long long)s->n_tok * s->n_kv * ((visible / KEYS16 + CW) / CW);
+    return bytes <= 256 * 1024 && keys <= (a_layer <= 20 || bytes <= 128 * 1024 ? 4096 : 2048) &&
+           2 * rounds <= (bytes <= 128 * 1024 ? 5 : 2) * blocks;
 }
 
 // Returns 0, 1 with the error recorded, or 2 when the device cannot hold the blocks all at once (nothing was launched).

@@ -36,6 +36,7 @@ struct ResidentStep {
 extern "C" {
 long long infero_resident_scratch(ResidentStep* s, uint8_t* at, int head_dim, int blocks);
 int infero_resident_supported(const ResidentStep* s, int head_dim, int blocks);
+int infero_resident_worth(const ResidentStep* s, int head_dim, int blocks, int visible);
 int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, int head_dim, const int* num_pages, const void* embed,
                            int embed_dtype, const int* ids, const int* device_tokens, int vocab, float embed_scale, int blocks,
                            cudaStream_t stream);

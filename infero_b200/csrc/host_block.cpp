@@ -281,11 +281,12 @@ void infero_block_set_fusion(int fused_decode_on, int fused_norm_on) {
 
 // A step of one or two single tokens through blocks of equal sizes, each with a cache of its own, runs as one resident kernel
 // (decode_resident.cu; INFERO_RESIDENT=0 keeps the launches layer by layer, as do the two switches above).
+// (0 no, 1 wherever it can run, 2 where it is the faster way: what a run has unless a test says otherwise)
 static int g_resident = -1;
-void infero_block_set_resident(int on) { g_resident = on ? 1 : 0; }
+void infero_block_set_resident(int on) { g_resident = on; }
 static bool resident_step(const InferoBlock* b, int n, const InferoStep& s, const int* const* tables, const int* entry_group, int max_blocks,
                           ResidentStep* r, ResidentLayer* layers, int* num_pages) {
-    if (g_resident < 0) g_resident = env_on("INFERO_RESIDENT") ? 1 : 0;
+    if (g_resident < 0) g_resident = env_on("INFERO_RESIDENT") ? 2 : 0;
     if (g_fused_decode < 0) g_fused_decode = env_on("INFERO_FUSED_DECODE") ? 1 : 0;
     if (!g_resident || !g_fused_decode || !fused_norm_wanted() || n < 1 || n > RESIDENT_LAYERS) return false;
     if (s.n_decode != s.n_entries || s.n_decode != s.n_tokens) return false;
@@ -295,6 +296,7 @@ static bool resident_step(const InferoBlock* b, int n, const InferoStep& s, cons
     r->norm_dtype = b->norm_dtype, r->qkv_bias_dtype = b->qkv_bias_dtype, r->o_bias_dtype = b->o_bias_dtype;
     r->inv_hidden = 1.0f / (float)b->hidden, r->positions = s.positions, r->tok_entry = s.tok_entry, r->x = s.x;
     if (!infero_resident_supported(r, b->head_dim, s.sm_count)) return false;
+    int visible = 0;                                    // keys of the longest request that some layer sees, at most
     for (int i = 0; i < n; ++i) {
         const InferoBlock& o = b[i];
         if (o.hidden != b->hidden || o.n_heads != b->n_heads || o.n_kv != b->n_kv || o.head_dim != b->head_dim || o.intermediate != b->intermediate ||
@@ -309,7 +311,9 @@ static bool resident_step(const InferoBlock* b, int n, const InferoStep& s, cons
                                   o.b_qkv, o.b_o, o.w_norm_mixer, o.w_norm_ffn, o.inv_freq, (__nv_bfloat16*)o.k_cache, (__nv_bfloat16*)o.v_cache,
                                   tables[entry_group[i]], o.eps_mixer, o.eps_ffn, o.scale * 1.4426950408889634f, o.window};
         num_pages[i] = o.num_pages;
+        visible = std::max(visible, o.window > 0 ? std::min(s.decode_visible, o.window) : s.decode_visible);
     }
+    if (g_resident == 2 && !infero_resident_worth(r, b->head_dim, s.sm_count, visible)) return false;
     return infero_resident_scratch(r, s.arena, b->head_dim, s.sm_count) <= s.arena_bytes;
 }
 
