@@ -32,7 +32,7 @@ struct Tile {
     static constexpr int TX = BN / TN, TY = BM / TM, WORK = TX * TY, THREADS = WORK < 32 ? 32 : WORK;
     static constexpr int LY = TY < 4 ? TY : 4, LX = WORK < 32 ? TX : 32 / LY;              // a warp has LX x LY threads
     static constexpr int LD = BK + 4, A_FLOATS = BM * LD, STAGE = (BM + BN) * LD;
-    static constexpr int Q = BK / 4, ROWS = THREADS / Q;                                   // rows that one round of copies covers
+    static constexpr int Q = BK / 4;                                                       // copies a row
     static constexpr int FLOATS = STAGES * STAGE > BM * BN ? STAGES * STAGE : BM * BN;     // (a part's results take the ring's place)
     static constexpr size_t SMEM = (size_t)FLOATS * sizeof(float);
     static_assert(SMEM <= 48 * 1024, "more shared memory than a launch gets without asking");
@@ -63,12 +63,17 @@ __device__ __forceinline__ void copy_rows(unsigned int dst, const float* src, co
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * STEP * LD * 4), "l"(ok ? src : any), "r"(ok ? 16 : 0) : "memory");
     }
 }
-template <int ROWS, int BK, int LD, int THREADS, typename T>
-__device__ __forceinline__ void widen_rows(float* dst, const T* src, int row0, int n_rows, int k0, int k_end, long long ld, int tid) {
-    for (int e = tid; e < ROWS * BK; e += THREADS) {
-        const int r = e / BK, k = k0 + e % BK;
-        dst[r * LD + e % BK] = row0 + r < n_rows && k < k_end ? to_f32(src[(long long)(row0 + r) * ld + k]) : 0.f;
-    }
+// The same element by element, widened on the way: this thread takes a column of every STEP-th row; its loads are on their way
+// together before the first is stored.
+template <int ROWS, int LD, int STEP, typename T>
+__device__ __forceinline__ void widen_rows(float* dst, const T* src, long long ld, int row, int n_rows, bool in) {
+    constexpr int N = (ROWS + STEP - 1) / STEP;
+    float v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i, src += ld * STEP) v[i] = in && row + i * STEP < n_rows && (ROWS % STEP == 0 || row + i * STEP < ROWS) ? to_f32(*src) : 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if (ROWS % STEP == 0 || row + i * STEP < ROWS) dst[i * STEP * LD] = v[i];
 }
 __device__ __forceinline__ void cluster_meet() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -86,7 +91,7 @@ gemm_tiled_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const void
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const bool works = TL::WORK == TL::THREADS || tid < TL::WORK;
     const int k_first = SPLIT ? blockIdx.z * part_len : 0, k_last = SPLIT ? min(K, k_first + part_len) : K;
-    const int row = tid / TL::Q, col = tid % TL::Q * 4;
+    const int row = tid / (VEC ? TL::Q : BK), col = VEC ? tid % TL::Q * 4 : tid % BK;
     const TA* a_src = A + (long long)(m0 + row) * lda + col;
     const TW* w_src = W + (long long)(n0 + row) * K + col;
     const unsigned int ring_at = (unsigned int)__cvta_generic_to_shared(ring);
@@ -96,12 +101,13 @@ gemm_tiled_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const void
             if constexpr (VEC) {
                 const unsigned int dst = ring_at + (slot * TL::STAGE + row * LD + col) * 4;
                 const bool in = next_k + col < next_end;        // (K is a multiple of 4 here)
-                copy_rows<BM, LD, TL::ROWS>(dst, a_src + next_k, A, lda, row, M - m0, in);
-                copy_rows<BN, LD, TL::ROWS>(dst + TL::A_FLOATS * 4, w_src + next_k, W, K, row, N - n0, in);
+                copy_rows<BM, LD, TL::THREADS / TL::Q>(dst, a_src + next_k, A, lda, row, M - m0, in);
+                copy_rows<BN, LD, TL::THREADS / TL::Q>(dst + TL::A_FLOATS * 4, w_src + next_k, W, K, row, N - n0, in);
             } else {
-                float* at = ring + slot * TL::STAGE;
-                widen_rows<BM, BK, LD, TL::THREADS>(at, A, m0, M, next_k, next_end, lda, tid);
-                widen_rows<BN, BK, LD, TL::THREADS>(at + TL::A_FLOATS, W, n0, N, next_k, next_end, K, tid);
+                float* dst = ring + slot * TL::STAGE + row * LD + col;
+                const bool in = next_k + col < next_end;
+                widen_rows<BM, LD, TL::THREADS / BK>(dst, a_src + next_k, lda, row, M - m0, in);
+                widen_rows<BN, LD, TL::THREADS / BK>(dst + TL::A_FLOATS, w_src + next_k, K, row, N - n0, in);
             }
             next_k += BK;
             if (next_k >= next_end) next_k = next_end, next_end = min(K, next_end + part_len);
@@ -299,24 +305,40 @@ int launch_tiled(const void* A, const void* W, const void* bias, int bias_dtype,
     bool split = VEC && parts >= 2 && parts <= MAX_SPLIT;
     const int by = split ? parts : 1;
     auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
-    if (M <= 16) {
-        const bool narrow = blocks(16, 32) < 2 * sms;
-        split = split && blocks(16, 32) < 4 * sms;
-        if (M == 1 && narrow && split) TILE(1, 16, 1, 1, 128, 4);
-        if (M == 1 && narrow) TILE(1, 8, 1, 1, 128, 6);
-        if (M == 1) TILE(1, 32, 1, 1, 64, 4);
-        if (M <= 4 && narrow) TILE(4, 8, 1, 1, 128, 4);
-        if (M <= 4) TILE(4, 32, 4, 1, 64, 4);
-        if (M <= 8 && narrow) TILE(4, 16, 2, 1, 64, 5);
-        if (M <= 8) TILE(8, 32, 4, 1, 64, 3);
-        if (narrow) TILE(16, 16, 2, 1, 64, 4);
-        TILE(16, 32, 4, 1, 64, 3);
+    // Operands that are widened on the way have no copies in flight while a block works, so what counts is that many threads load.
+    // (us before K came in parts, with tiles for 16-byte copies, now; bf16 on both sides but for the rows of 897 and 4,865 32-bit columns:
+    // 8 x 896, K = 896 24, 37, 11; 8 x 896, K = 4,865 121, 191, 41; 4 x 32,000, K = 896 126, 126, 47; 16 x 6,144, K = 2,048 93, 91, 48;
+    // 64 x 2,048, K = 2,048 116, 137, 52; 150 x 896, K = 4,864 215, 324, 126; 301 x 9,728, K = 897 210, 242, 198; 2,048 x 9,728, K = 896 1,221,
+    // 1,311, 1,064.  Wider tiles at 64 x 9,728: 65 against 59; 16 x 32 for 301 x 896, K = 4,864: above 197 against 186.)
+    if constexpr (!VEC) {
+        if (M <= 16) {
+            if (blocks(16, 64) >= 2 * sms) TILE(16, 64, 4, 2, 64, 2);
+            if (M <= 8 || blocks(8, 16) < 2 * sms) TILE(8, 16, 1, 1, 64, 4);
+            TILE(16, 16, 2, 1, 64, 4);
+        }
+        if (blocks(64, 64) >= sms && (M + 63) / 64 * 64 <= (M + 31) / 32 * 35) TILE(64, 64, 4, 4, 32, 2);
+        if (5 * blocks(32, 32) >= 8 * sms) TILE(32, 32, 4, 2, 32, 3);
+        TILE(32, 16, 2, 1, 64, 3);
+    } else {
+        if (M <= 16) {
+            const bool narrow = blocks(16, 32) < 2 * sms;
+            split = split && blocks(16, 32) < 4 * sms;
+            if (M == 1 && narrow && split) TILE(1, 16, 1, 1, 128, 4);
+            if (M == 1 && narrow) TILE(1, 8, 1, 1, 128, 6);
+            if (M == 1) TILE(1, 32, 1, 1, 64, 4);
+            if (M <= 4 && narrow) TILE(4, 8, 1, 1, 128, 4);
+            if (M <= 4) TILE(4, 32, 4, 1, 64, 4);
+            if (M <= 8 && narrow) TILE(4, 16, 2, 1, 64, 5);
+            if (M <= 8) TILE(8, 32, 4, 1, 64, 3);
+            if (narrow) TILE(16, 16, 2, 1, 64, 4);
+            TILE(16, 32, 4, 1, 64, 3);
+        }
+        if (blocks(64, 64) * by >= 3 * sms && (M + 63) / 64 * 64 <= (M + 31) / 32 * 35) TILE(64, 64, 8, 4, 32, 2);
+        if (blocks(32, 64) * by >= 3 * sms) TILE(32, 64, 4, 4, 32, 3);
+        if (blocks(32, 32) * by >= sms) TILE(32, 32, 4, 2, 32, 3);
+        if (3 * blocks(32, 32) * by >= 2 * sms) TILE(32, 32, 2, 2, 32, 3);
+        TILE(32, 16, 2, 1, 32, 4);
     }
-    if (blocks(64, 64) * by >= 3 * sms && (M + 63) / 64 * 64 <= (M + 31) / 32 * 35) TILE(64, 64, 8, 4, 32, 2);
-    if (blocks(32, 64) * by >= 3 * sms) TILE(32, 64, 4, 4, 32, 3);
-    if (blocks(32, 32) * by >= sms) TILE(32, 32, 4, 2, 32, 3);
-    if (3 * blocks(32, 32) * by >= 2 * sms) TILE(32, 32, 2, 2, 32, 3);
-    TILE(32, 16, 2, 1, 32, 4);
 #undef TILE
 }
 

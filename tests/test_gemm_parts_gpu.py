@@ -29,3 +29,23 @@ def test_products_over_parts_of_k(N, K, lda):
     Kn.gemm_tiled(a[:3].bfloat16(), w, bias, wide)
     ref = (a[:3].bfloat16().double() @ w.double().T + bias.double())
     assert float((wide.double() - ref).norm() / ref.norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("N,K", [(70, 641), (1152, 896), (9000, 300), (200, 1925), (19000, 72)])
+@pytest.mark.parametrize("ta,tw", [("bfloat16", "bfloat16"), ("float32", "bfloat16"), ("bfloat16", "float32")])
+def test_widened_operands_over_the_tiles(N, K, ta, tw):
+    from infero_b200 import kernels as Kn
+    g = torch.Generator(device=DEV).manual_seed(N)
+    big = 301
+    a = torch.randn((big, K), generator=g, device=DEV).to(getattr(torch, ta))
+    w = torch.randn((N, K), generator=g, device=DEV).to(getattr(torch, tw))
+    bias = torch.randn((N,), generator=g, device=DEV)
+    full = torch.empty((big, N), device=DEV)
+    Kn.gemm_tiled(a, w, bias, full)
+    ref = a.double() @ w.double().T + bias.double()
+    bound = (340 + K / 640 + 3) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T + bias.double().abs())     # (as above)
+    assert bool(((full.double() - ref).abs() <= bound).all())
+    for M in (1, 8, 9, 16, 17, 33, 63, 64, 65, 100, 128, 200):
+        out = torch.full((M, N), 7.0, device=DEV)
+        Kn.gemm_tiled(a[:M], w, bias, out)
+        assert torch.equal(out, full[:M]), M
