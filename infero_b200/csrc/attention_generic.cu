@@ -315,6 +315,21 @@ int block_tokens(int n_tokens, int singles, int portions, int group) {
     return rest <= FEW_TOKENS || 2 * rest < (long long)portions * tokens ? 0 : tokens;
 }
 
+// Blocks of 16 rows that a multiprocessor holds.
+template <typename T, typename TO, bool VEC>
+int resident_half(int head_dim, int value_dim) {
+    const size_t smem = generic_smem<typename Stored<T, VEC>::type>(head_dim, value_dim, WIDE_ROWS / 2);
+    auto ask = [&](auto* kernel) {
+        int n = 0;
+        if ((smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, WARPS * 32, smem) != cudaSuccess)
+            n = 0, cudaGetLastError();
+        return n;
+    };
+    return head_dim > 128 || value_dim > 128 ? ask(attention_generic_kernel<T, TO, 2, 8, VEC>) : value_dim > 64 ? ask(attention_generic_kernel<T, TO, 2, 4, VEC>)
+                                                                                              : ask(attention_generic_kernel<T, TO, 2, 2, VEC>);
+}
+
 template <typename T, typename TO, bool VEC>
 int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
     const int group = a.n_heads / a.n_kv, tokens = block_tokens(a.n_tokens, a.singles, portions, group);
@@ -323,11 +338,19 @@ int launch_rows(GenericArgs& a, int portions, cudaStream_t stream) {
     const int least = a.head_dim > 64 || a.value_dim > 64 ? WARPS : WARPS / 2;
     const int warps = few ? (group < least ? least : group < WARPS ? group : WARPS) : WARPS;
     // Where blocks of 32 rows are fewer than two a multiprocessor, half as many rows a warp: what a chunk costs a warp is latency, and
-    // twice the warps cover it (14 heads of 64 over 2, 32-bit, 301 tokens: 152 blocks 63 us, 302 blocks 42).
-    const long long wide = few ? 0 : (a.singles + (long long)(a.n_tokens - a.singles + tokens - 1) / tokens) * ((group + WIDE_ROWS - 1) / WIDE_ROWS) *
-                                         a.n_kv * (a.cross ? a.n_kv : 1);
-    const bool half = !few && wide < 2 * infero_sm_count();
-    const int rows = few ? warps : half ? WIDE_ROWS / 2 : WIDE_ROWS;
+    // twice the warps cover it, as long as all the blocks run at once: they fetch a key up to three times as often, and a second wave takes
+    // as long as the first.  (us in blocks of 32 rows and of 16, 32-bit, 301 tokens: 14 heads of 64 over 2, 302 blocks of 16, 62 and 43,
+    // behind 1,500 cached ones 385 and 244; 16 of 64 over 1, 301 blocks of the 444 that fit, 289 and 252; 18 of 64 over 2, 602 blocks, 400 and 446,
+    // without cached ones 69 and 61; 9 of 128 over 1, 301 of 296, 455 and 546, without 82 and 60, 270 tokens behind 2,000 570 and 396.)
+    const long long sides = (long long)a.n_kv * (a.cross ? a.n_kv : 1), rest = a.n_tokens - a.singles;
+    auto blocks = [&](int rows) {
+        const int each = group > rows ? 1 : rows / group;
+        return (a.singles + (rest + each - 1) / each) * ((group + rows - 1) / rows) * sides;
+    };
+    const int sms = infero_sm_count(), half_rows = WIDE_ROWS / 2;
+    bool half = !few && blocks(WIDE_ROWS) < 2 * sms;
+    if (half) half = blocks(half_rows) <= (long long)sms * resident_half<T, TO, VEC>(a.head_dim, a.value_dim);
+    const int rows = few ? warps : half ? half_rows : WIDE_ROWS;
     a.tokens_per_block = few ? 1 : half ? (group > rows ? 1 : rows / group) : tokens;
     a.head_chunks = (group + rows - 1) / rows;
 #define COLUMNS(R)                                                                                      \
