@@ -290,7 +290,10 @@ int launch_tile(const void* A, const void* W, const void* bias, int bias_dtype, 
 // multiprocessor, 64 rows only where they are not much more than 32 would be (301 x 896, K = 4,864: 148 before, 73 with 64 x 64,
 // 104 with 32 x 64; 301 x 9,728, K = 896: 156 before, 138 and 141; 150 x 9,728 121 before, 93 with 32 x 64; 301 x 1,152 35 before,
 // 29 with 32 x 32, 31 with 32 x 64; 64 x 896 14.5 before, 12.4 with four results a thread, 14.4 with eight).  In large products
-// (2,048 x 9,728, K = 896: 857 before, 795 now) the bound is the rate of the paired multiply-adds, two thirds of it reached.
+// (2,048 x 9,728, K = 896: 857 before, 795 now) the bound is the rate of the paired multiply-adds, 0.6 of it reached.
+// Where blocks are few (few rows of W, and of K one part, two, or more than a cluster has blocks), a tile with fewer results a
+// thread (us before parts, with the larger tile, now: 16 x 512, K = 512 4.6, 5.5, 3.9; 16 x 1,152, K = 896 7.1, 7.3, 6.2; 16 x 200, K = 5,124
+// 33, 41, 27; 64 x 200 60, 65, 41; 17 x 2,048, K = 6,144 73, 77, 68; 16 x 2,048, K = 6,144 with 8 x 16 51, with 16 x 16 50).
 template <bool VEC, typename TA, typename TW, typename TC>
 int launch_tiled(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N,
                  int K, int lda, int ldc, cudaStream_t stream) {
@@ -330,6 +333,7 @@ int launch_tiled(const void* A, const void* W, const void* bias, int bias_dtype,
             if (M <= 4) TILE(4, 32, 4, 1, 64, 4);
             if (M <= 8 && narrow) TILE(4, 16, 2, 1, 64, 5);
             if (M <= 8) TILE(8, 32, 4, 1, 64, 3);
+            if (narrow && blocks(8, 16) * by < (split ? 2 : 1) * sms) TILE(8, 16, 1, 1, 64, 4);
             if (narrow) TILE(16, 16, 2, 1, 64, 4);
             TILE(16, 32, 4, 1, 64, 3);
         }
@@ -337,6 +341,7 @@ int launch_tiled(const void* A, const void* W, const void* bias, int bias_dtype,
         if (blocks(32, 64) * by >= 3 * sms) TILE(32, 64, 4, 4, 32, 3);
         if (blocks(32, 32) * by >= sms) TILE(32, 32, 4, 2, 32, 3);
         if (3 * blocks(32, 32) * by >= 2 * sms) TILE(32, 32, 2, 2, 32, 3);
+        if (!split) TILE(16, 16, 2, 1, 64, 4);
         TILE(32, 16, 2, 1, 32, 4);
     }
 #undef TILE
