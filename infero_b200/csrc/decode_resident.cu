@@ -33,6 +33,8 @@
 #include <algorithm>
 #include <mutex>
 
+extern "C" int infero_sm_count();
+
 namespace {
 
 using namespace attn;
@@ -800,7 +802,9 @@ int infero_resident_worth(const ResidentStep* s, int head_dim, int blocks, int v
            2 * rounds <= (bytes <= 128 * 1024 ? 5 : 2) * blocks;
 }
 
-// Returns 0, 1 with the error recorded, or 2 when the device cannot hold the blocks all at once (nothing was launched).
+// Returns 0, 1 with the error recorded, or 2 when the device cannot hold the blocks all at once: a multiprocessor has no room for one, there are
+// fewer multiprocessors than blocks, or the launch is refused because part of them is set aside (all that has run then is the step's first
+// kernel, whose results nobody else reads).
 int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, int head_dim, const int* num_pages, const void* embed,
                            int embed_dtype, const int* ids, const int* device_tokens, int vocab, float embed_scale, int blocks,
                            cudaStream_t stream) {
@@ -815,7 +819,7 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, THREADS, Smem::TOTAL);
             if (e != cudaSuccess) n = 0, cudaGetLastError();
         }
-        if (n < 1) return 2;
+        if (n < 1 || blocks > (long long)n * infero_sm_count()) return 2;
     }
     Params p;
     p.s = *s;
@@ -843,6 +847,9 @@ int infero_decode_resident(const ResidentStep* s, const ResidentLayer* layers, i
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void* args[] = {&p};
-    cudaLaunchKernelExC(&cfg, kernel, args);
+    if (cudaLaunchKernelExC(&cfg, kernel, args) == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return 2;
+    }
     return infero_check_launch("decode_resident");
 }
