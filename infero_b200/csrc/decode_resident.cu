@@ -242,7 +242,7 @@ struct Block {
     __device__ __forceinline__ void give_up() {
         *abort_flag = 1;
         *(volatile unsigned int*)s().stop = 1;
-        atomicExch(p.err_flag, 6);
+        atomicExch(p.err_flag, 10);
     }
     // The bytes of the ring's q-th slot are here.
     __device__ __forceinline__ void arrived(uint32_t q) {

@@ -39,3 +39,29 @@ def test_more_blocks_than_multiprocessors_keep_the_launches(monkeypatch):
     plain, many = _step(_runner(), 0)
     other, launches = _step(_runner(), 1)
     assert launches == many and torch.equal(plain, other)
+
+
+def test_a_wait_that_runs_out_names_the_kernel(monkeypatch):
+    """A token at position -1 sees no keys: nobody writes its attention, the wait for it ends at its limit and the step returns."""
+    from infero_b200.kernels import tc_gemm
+    runner = _runner()
+    good, launches = _step(runner, 1)
+    assert launches < 6, "the resident kernel was meant to run this step (the launches layer by layer must not see such a position)"
+    build = runner._build_context
+
+    def nowhere(entries, rcs):
+        ctx, rows = build(entries, rcs)
+        if len(entries[0].tokens) == 1:
+            ctx.positions.fill_(-1)
+        return ctx, rows
+
+    with monkeypatch.context() as m:
+        m.setattr(runner, "_build_context", nowhere)
+        runner.drop_graphs()
+        _step(runner, 1)
+        torch.cuda.synchronize()
+    assert tc_gemm.error_flag() == 10
+    assert tc_gemm.error_flag() == 0
+    runner.drop_graphs()
+    again, _ = _step(runner, 1)
+    assert torch.equal(good, again) and tc_gemm.error_flag() == 0
