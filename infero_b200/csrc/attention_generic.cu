@@ -22,7 +22,7 @@
 // block take turns, so single tokens and short portions get a block per token, with warps that only fetch where a kv head has
 // fewer query heads than a block wants warps.
 // What bounds it: long prompts the multiply-adds and what feeds them from shared memory, single tokens the chain over the
-// chunks.  A warp per row reading keys where they lie, and now, in us.  32-bit, 14 heads of 64 over 2: 301 tokens 265 and 64, one token
+// chunks.  A warp per row reading keys where they lie, and now, in us.  32-bit, 14 heads of 64 over 2: 301 tokens 265 and 43, one token
 // at 300 keys 127 and 24, 64 at 1,000 518 and 68; 16 heads of 64 over 16: 250 single tokens at 1,000 keys 1,248 and 426, 10 of them at
 // 2,000 beside 250 prompt tokens 1,412 and 208; 16 of 128 over 16: 1,500 tokens 9,560 and 742.  bf16, 16 of 36 over 16: 250 single
 // tokens 523 and 308.  (A chunk ahead is enough: two or three ahead made blocks too large, 707 instead of 428 for the 250 of 64.)
@@ -36,7 +36,7 @@ namespace {
 constexpr int WARPS = 8;
 constexpr int MAX_D = 256;
 constexpr int CHUNK = 32, STAGES = 2;
-constexpr int FEW_TOKENS = 256;         // portions of up to so many tokens: a block per token, one row a warp; beyond, 32 rows a block
+constexpr int FEW_TOKENS = 256;         // portions of up to so many tokens: a block per token, one row a warp; beyond, 32 or 16 rows a block
 constexpr int WIDE_ROWS = WARPS * 4;
 
 struct GenericArgs {
@@ -307,7 +307,7 @@ int launch(GenericArgs& a, int warps, cudaStream_t stream) {
     return infero_check_launch("attention_generic");
 }
 
-// Tokens a block of 32 rows takes at a time, 0 for a block per token.  A block's tokens of different requests take turns and all but
+// Tokens a block of 32 rows takes at a time (launch_rows may halve them), 0 for a block per token.  A block's tokens of different requests take turns and all but
 // one request's rows idle meanwhile, so what counts is the portions' tokens (the single ones in front have blocks of their own
 // either way) and that a portion has about a block's tokens and more.
 int block_tokens(int n_tokens, int singles, int portions, int group) {

@@ -22,8 +22,9 @@
 //   norms      The block that owns a column of the residual stream keeps it in shared memory in 32 bits; it hands on
 //              bf16(x * w) and its columns' sum of squares, and the product behind applies 1 / rms to its 32-bit results.
 //
-// A step of one token at 300 keys, 24 layers of Qwen2.5-0.5B sizes: 696 us as 196 launches, 576 so (0.15 ms of bytes); what bounds it
-// are five phases a layer that each wait for the one before, a store and a load through L2 and a few rows of work a block.
+// A step of one token at 300 keys, 24 layers of Qwen2.5-0.5B sizes, as one pass of a runner: 694 us as 195 launches, 584 so (0.15 ms of
+// bytes; infero_resident_worth has more lengths and sizes, as replays of the captured step alone).  What bounds it are five phases a
+// layer that each wait for the one before, a store and a load through L2 and a few rows of work a block.
 // Every wait has a time limit: a wait that runs out raises the error flag and every block runs to its end without waiting.
 // The reference's counterpart of the step: crates/model/src/lib.rs:3423-4243.
 #include "attn_common.cuh"

@@ -1,7 +1,8 @@
 // One layer of the built-in kind (pre-norm block: RMSNorm, grouped-query attention with rotary
 // positions over the paged cache, RMSNorm, SwiGLU) launched from native code.  In steps with a prompt
-// portion: the same kernels with the same arguments, in the same order, as the Python parts launch
-// them one by one, so the results are the same bit for bit and only the host's time per layer
+// portion: the same kernels with the same arguments as the Python parts launch them one by one (but for
+// attention of the single tokens, which comes behind that of the portions, to run beside it), so the
+// results are the same bit for bit and only the host's time per layer
 // differs (one call instead of a dozen Python wrappers).  In steps of single tokens, where a launch
 // costs more than its work, the layer is five launches instead of eight: decode attention finishes
 // the q/k/v product itself, and the two norms are folded into the products around them (see
@@ -460,7 +461,8 @@ int infero_block_forward(const InferoBlock* b, const InferoStep* s, const int* b
 // The whole model in one call: embedding, the schedule of built-in blocks, the final norm on the rows whose
 // logits are wanted, the output product.  What ``DecoderModel.forward`` does when every entry of its
 // schedule is a built-in block that goes the native way, launch for launch (the same functions with the
-// same arguments), so the logits are the same bit for bit; the host's share of a step that is not replayed
+// same arguments), so the logits are the same bit for bit (but for steps that the resident kernel takes, see
+// resident_step: one launch for all blocks, the same roundings, sums in another order); the host's share of a step that is not replayed
 // from a CUDA graph drops from a Python call per layer to this one call.  The reference runs its layer
 // loop natively too (crates/model/src/lib.rs:3423-4243).
 struct InferoDecoder {

@@ -5,7 +5,9 @@ When every execution of a model's schedule is a built-in block that goes the nat
 tensor-core kernel, ``DecoderModel.forward`` hands the step to ``infero_decoder_forward``
 (``csrc/host_block.cpp``): embedding, the blocks, the final norm on the wanted rows and the output product,
 launch for launch what the Python loop does (the same native functions with the same arguments, so the
-logits are the same bit for bit).  The host's share of a step that is not replayed from a CUDA graph drops
+logits are the same bit for bit), except that a step of one or two single tokens through small layers
+and short contexts runs all blocks in one resident kernel, whose sums come in another order
+(``csrc/decode_resident.cu``).  The host's share of a step that is not replayed from a CUDA graph drops
 from a Python call per layer to one call; ``INFERO_NATIVE_STEP=0`` keeps the loop.
 
 The reference runs its whole pass natively (crates/model/src/lib.rs:3423-4243).

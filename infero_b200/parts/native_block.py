@@ -3,7 +3,8 @@
 ``PreNormBlock`` made of exactly the package's own parts (RMSNorm, grouped-query attention with
 NeoX rotary positions or none, SwiGLU) in a bf16 step can hand its whole layer to
 ``infero_block_forward`` (``csrc/host_block.cpp``).  In steps with a prompt portion that call launches
-the same kernels with the same arguments in the same order as the parts launch one by one, so the
+the same kernels with the same arguments as the parts launch one by one (attention of the single tokens
+behind that of the portions, to run beside it), so the
 results are the same bit for bit; what changes is the host's time per layer (one call instead of a
 dozen wrappers), which is what bounds steps that are not replayed from a CUDA graph.  In steps of
 single tokens the native layer is made of fewer launches than the parts' (decode attention finishes
