@@ -841,7 +841,7 @@ int infero_attn_decode_tma(const void* q, int q_stride, void* out, int out_strid
                       scratch, counters, n_counters, 0, stream);
 }
 
-// The same right behind infero_attn_prefill_tc of the same step's prompt portions (see FusedQkv::beside).
+// The same right behind infero_attn_prefill_tc_beside of the same step's prompt portions (see FusedQkv::beside).
 int infero_attn_decode_tma_beside(const void* q, int q_stride, void* out, int out_stride, const void* k_cache,
                                   const void* v_cache, int num_pages, const int* block_table, int max_blocks,
                                   const int* tok_entry, const int* positions, int tok_first, int n_tok, int n_heads,

@@ -68,7 +68,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const int* __restrict__ entry_q_len, const int* __restrict__ entry_pos0, int n_entries,
                        int first_entry, int n_tiles, int n_heads, int n_kv, int heads_per_cta, int page_size, int slice,
                        int window, float scale_log2, int sink, int* __restrict__ err_flag,
-                       const attn::Extras ex) {
+                       const attn::Extras ex, int beside) {
     using Plan = PfPlan<D>;
     constexpr int DB = Plan::DB, ST = Plan::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -88,6 +88,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     volatile int* never_flag = abort_flag + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (!beside) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_q);
         prefetch_tensormap(&map_k);
@@ -119,8 +120,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                                        // q, the tables and this step's keys come from earlier kernels
-    // (behind the wait: decode attention of the same step may follow and take what is here for granted, see attention_decode.cu)
-    pdl_launch_dependents();
+    // (behind the wait where decode attention of the same step follows, which takes what is here for granted, see attention_decode.cu;
+    // in steps of portions alone the product behind is let in at the start: a prompt of 37 tokens, 24 layers, 1,050 us and 1,060)
+    if (beside) pdl_launch_dependents();
 
     // ---- which kv head and pair of heads, which request and which block of 128 query rows? ------
     const int group = n_heads / n_kv;
@@ -455,7 +457,7 @@ template <int D>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, int out_stride,
            const int* block_table, int max_blocks, const int* entry_q_start, const int* entry_q_len,
            const int* entry_pos0, int n_entries, int first_entry, int n_tiles, int n_heads, int n_kv, int page_size,
-           int slice, int window, float scale_log2, int sink, int* err, const attn::Extras& ex, cudaStream_t stream) {
+           int slice, int window, float scale_log2, int sink, int* err, const attn::Extras& ex, int beside, cudaStream_t stream) {
     using Plan = PfPlan<D>;
     // Two heads per CTA halve the key and value traffic, but a grid that does not fill the SMs that way
     // runs faster with one head per CTA: measured at 7B sizes 25 against 35 us at 1,024 tokens (128
@@ -481,7 +483,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
     }
     launch_pdl(kern, dim3(n_kv * sides * ((group + hpc - 1) / hpc), n_tiles), dim3(PFT_THREADS), Plan::TOTAL, stream, mq, mk, mv, (bf16*)out, out_stride,
                block_table, max_blocks, entry_q_start, entry_q_len, entry_pos0, n_entries, first_entry, n_tiles, n_heads,
-               n_kv, hpc, page_size, slice, window, scale_log2, sink, err, ex);
+               n_kv, hpc, page_size, slice, window, scale_log2, sink, err, ex, beside);
     return infero_check_launch("attn_prefill_tc");
 }
 
@@ -493,19 +495,12 @@ int infero_attn_prefill_tc_supported(int head_dim, int page_size, int q_stride, 
     return (head_dim == 64 || head_dim == 128) && page_size % 16 == 0 && q_stride % 8 == 0 && out_stride % 8 == 0;
 }
 
-// The same contract as infero_attn_prefill (attention_mma.cu) with 128 query rows per block:
-// n_tiles = sum over the requests first_entry .. n_entries - 1 of ceil(q_len / 128).  q is
-// [n_tokens, >= n_heads * head_dim] bf16 with row stride q_stride; the caches are
-// [num_pages, n_kv, page_size, head_dim] bf16, contiguous; all 16-byte aligned.
-// ``sink``: the softmax's sum has one more term exp(0) that carries no value.  ``slopes`` (float32 [n_heads] or null):
-// head h's score loses slopes[h] times the distance between the query and the key.  rel, rel_len, cross, sinks: see attn::Extras;
-// softcap > 0 soft-caps the scaled score (in the score's own units).
-int infero_attn_prefill_tc_ex(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
+static int prefill_tc(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
                                 const void* v_cache, int num_pages, const int* block_table, int max_blocks,
                                 const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int n_entries,
                                 int first_entry, int n_tiles, int n_heads, int n_kv, int head_dim, int page_size,
                                 int window, float scale, int sink, const float* slopes, const float* rel, int rel_len,
-                              int cross, const float* sinks, float softcap, cudaStream_t stream) {
+                              int cross, const float* sinks, float softcap, int beside, cudaStream_t stream) {
     if (n_tiles == 0) return 0;
     INFERO_REQUIRE((!slopes && !rel && softcap <= 0.f) || scale > 0.f, "attn_prefill_tc: a distance bias or a soft cap needs a positive scale");
     INFERO_REQUIRE(!rel || rel_len >= 1, "attn_prefill_tc: an empty table of distances");
@@ -530,9 +525,27 @@ int infero_attn_prefill_tc_ex(const void* q, int q_stride, int n_tokens, void* o
     const float sl2 = scale * 1.4426950408889634f;
     if (head_dim == 128)
         return launch<128>(mq, mk, mv, out, out_stride, block_table, max_blocks, entry_q_start, entry_q_len, entry_pos0,
-                           n_entries, first_entry, n_tiles, n_heads, n_kv, page_size, slice, window, sl2, sink, err, ex, stream);
+                           n_entries, first_entry, n_tiles, n_heads, n_kv, page_size, slice, window, sl2, sink, err, ex, beside, stream);
     return launch<64>(mq, mk, mv, out, out_stride, block_table, max_blocks, entry_q_start, entry_q_len, entry_pos0,
-                      n_entries, first_entry, n_tiles, n_heads, n_kv, page_size, slice, window, sl2, sink, err, ex, stream);
+                      n_entries, first_entry, n_tiles, n_heads, n_kv, page_size, slice, window, sl2, sink, err, ex, beside, stream);
+}
+
+// The same contract as infero_attn_prefill (attention_mma.cu) with 128 query rows per block:
+// n_tiles = sum over the requests first_entry .. n_entries - 1 of ceil(q_len / 128).  q is
+// [n_tokens, >= n_heads * head_dim] bf16 with row stride q_stride; the caches are
+// [num_pages, n_kv, page_size, head_dim] bf16, contiguous; all 16-byte aligned.
+// ``sink``: the softmax's sum has one more term exp(0) that carries no value.  ``slopes`` (float32 [n_heads] or null):
+// head h's score loses slopes[h] times the distance between the query and the key.  rel, rel_len, cross, sinks: see attn::Extras;
+// softcap > 0 soft-caps the scaled score (in the score's own units).
+int infero_attn_prefill_tc_ex(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
+                                const void* v_cache, int num_pages, const int* block_table, int max_blocks,
+                                const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int n_entries,
+                                int first_entry, int n_tiles, int n_heads, int n_kv, int head_dim, int page_size,
+                                int window, float scale, int sink, const float* slopes, const float* rel, int rel_len,
+                              int cross, const float* sinks, float softcap, cudaStream_t stream) {
+    return prefill_tc(q, q_stride, n_tokens, out, out_stride, k_cache, v_cache, num_pages, block_table, max_blocks, entry_q_start,
+                      entry_q_len, entry_pos0, n_entries, first_entry, n_tiles, n_heads, n_kv, head_dim, page_size, window, scale, sink,
+                      slopes, rel, rel_len, cross, sinks, softcap, 0, stream);
 }
 
 int infero_attn_prefill_tc_bias(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
@@ -563,6 +576,17 @@ int infero_attn_prefill_tc(const void* q, int q_stride, int n_tokens, void* out,
     return infero_attn_prefill_tc_sink(q, q_stride, n_tokens, out, out_stride, k_cache, v_cache, num_pages, block_table,
                                        max_blocks, entry_q_start, entry_q_len, entry_pos0, n_entries, first_entry, n_tiles,
                                        n_heads, n_kv, head_dim, page_size, window, scale, 0, stream);
+}
+
+// The same in front of infero_attn_decode_tma_beside of the same step's single tokens.
+int infero_attn_prefill_tc_beside(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
+                                  const void* v_cache, int num_pages, const int* block_table, int max_blocks,
+                                  const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int n_entries,
+                                  int first_entry, int n_tiles, int n_heads, int n_kv, int head_dim, int page_size,
+                                  int window, float scale, cudaStream_t stream) {
+    return prefill_tc(q, q_stride, n_tokens, out, out_stride, k_cache, v_cache, num_pages, block_table, max_blocks, entry_q_start,
+                      entry_q_len, entry_pos0, n_entries, first_entry, n_tiles, n_heads, n_kv, head_dim, page_size, window, scale, 0,
+                      nullptr, nullptr, 0, 0, nullptr, 0.f, 1, stream);
 }
 
 }  // extern "C"

@@ -85,6 +85,11 @@ int infero_attn_prefill_tc(const void* q, int q_stride, int n_tokens, void* out,
                            const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int n_entries,
                            int first_entry, int n_tiles, int n_heads, int n_kv, int head_dim, int page_size,
                            int window, float scale, cudaStream_t stream);
+int infero_attn_prefill_tc_beside(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,
+                           const void* v_cache, int num_pages, const int* block_table, int max_blocks,
+                           const int* entry_q_start, const int* entry_q_len, const int* entry_pos0, int n_entries,
+                           int first_entry, int n_tiles, int n_heads, int n_kv, int head_dim, int page_size,
+                           int window, float scale, cudaStream_t stream);
 }
 void infero_set_error(const char* fmt, ...);
 
@@ -380,10 +385,9 @@ int infero_block_forward(const InferoBlock* b, const InferoStep* s, const int* b
     // the portions first: single tokens then run on the multiprocessors and in the shared memory that these leave
     const bool beside = s->n_decode > 0 && s->n_decode < s->n_entries && s->prefill_tiles > 0;
     if (s->n_decode < s->n_entries) {
-        if (int rc = infero_attn_prefill_tc(q, q_stride, T, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table,
-                                            max_blocks, s->entry_q_start, s->entry_q_len, s->entry_pos0, s->n_entries,
-                                            s->n_decode, s->prefill_tiles, H, Hkv, D, b->page_size, b->window, b->scale,
-                                            s->stream))
+        if (int rc = (beside ? infero_attn_prefill_tc_beside : infero_attn_prefill_tc)(
+                q, q_stride, T, attn, da, b->k_cache, b->v_cache, b->num_pages, block_table, max_blocks, s->entry_q_start, s->entry_q_len,
+                s->entry_pos0, s->n_entries, s->n_decode, s->prefill_tiles, H, Hkv, D, b->page_size, b->window, b->scale, s->stream))
             return rc;
     }
     if (s->n_decode > 0) {
