@@ -91,6 +91,7 @@ gemm_tiled_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const void
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const bool works = TL::WORK == TL::THREADS || tid < TL::WORK;
     const int k_first = SPLIT ? blockIdx.z * part_len : 0, k_last = SPLIT ? min(K, k_first + part_len) : K;
+    static_assert(VEC || TL::THREADS % BK == 0, "a round of loads is whole rows");
     const int row = tid / (VEC ? TL::Q : BK), col = VEC ? tid % TL::Q * 4 : tid % BK;
     const TA* a_src = A + (long long)(m0 + row) * lda + col;
     const TW* w_src = W + (long long)(n0 + row) * K + col;
